@@ -377,6 +377,7 @@ int plan_batch(int64_t n_tiles, const fpgb_volume *vols, const fpgb_fibers *fibe
       T.Z = (int32_t)P.Z;
       T.max_layer = P.max_layer;
       T.layer_base = (int32_t)B->layers.size();
+      T.n_bundles = (int32_t)std::max<int64_t>(P.n_bundles, 1);
       B->tile_dev.push_back(T);
       seg_base[t + 1] = seg_base[t] + P.segs.size();
       for (int64_t b = 0; b < P.n_bundles; b++)
@@ -451,7 +452,7 @@ int plan_batch(int64_t n_tiles, const fpgb_volume *vols, const fpgb_fibers *fibe
 
    // workspace
    size_t w = 0;
-   B->ws_bricks = take(w, brick_workspace_bytes(B->n_bricks, B->brick_pairs));
+   B->ws_bricks = take(w, brick_workspace_bytes(B->n_bricks, B->brick_pairs, B->n_segs));
    B->ws_segs = take(w, sizeof(SegDev) * B->n_segs);
    B->ws_segtile = take(w, sizeof(int32_t) * B->seg_tile.size());
    B->ws_layers = take(w, sizeof(LayerDev) * B->layers.size());

@@ -9,15 +9,12 @@
 //
 //   binning       every segment's clipped bounding box is binned to the
 //                 8 x 8 x 32 voxel bricks it overlaps;
-//   voxel_bricks  one CTA per brick keeps the brick's 64-bit keys
-//                 (float bits of dist_squ) << 32 | (0xFFFFFFFF - seg), i.e.
-//                 smallest distance, then largest segment index, in shared
-//                 memory: a first sweep stores FP32 upper bounds of the
-//                 candidates certainly inside, a second the exact
-//                 double->float distance of the reference for every
-//                 candidate that can still win; then it decodes each
-//                 voxel's winner and writes its label and orientation
-//                 (voxel_bricks.cu).
+//   voxel_bricks  one CTA per brick sweeps the brick's candidates once with
+//                 FP32 bounds of dist_squ that almost always name a voxel's
+//                 winner; the voxels where two candidates are too close are
+//                 marked and decided with the exact double->float distance
+//                 of the reference; then every voxel's label and orientation
+//                 are written (voxel_bricks.cu).
 //
 // This translation unit is compiled with -fmad=false: the label and vector
 // decisions depend on separately rounded double products and sums
@@ -109,18 +106,45 @@ void split2(double d, float &hi, float &lo) {
    lo = (float)(d - (double)hi);
 }
 
+// Bound on |estimate - reference float| of the sweep's FP32 dist^2
+// (sweep_dist2) over the voxels of the segment's box that lie within or next
+// to the segment's thickest end: |w| <= |v| + r' for the voxel's offset w
+// from p.  With u = 2^-24, the rounding of the inputs (w: u (|w0| + |w| + 1)
+// for the offset w0 of the sub-box's first cell, v, c2: u each), of the six
+// operations and of the sum of the margin itself stays below u (15 |w|^2 +
+// 2 |w| |w0| + 12 c2 + 4) (the error of t enters squared: the value is the
+// squared distance to some point of the segment); the reference's own double
+// arithmetic adds 2^-50 pscale |w| and its final rounding u |w|^2.  18 u and
+// 12 u are 1.08e-6 and 7.2e-7.  For a voxel farther away, d >= |w| - |v|, so
+// that error is below 3.3e-6 d^2 + 4e-6 c2 and the estimate stays past the
+// thickest end as the distance does: r' has more than that on top.
+float seg_margin(const SegDev &S, double thr) {
+   double w2 = 0.0;
+   for (int i = 0; i < 3; i++) {
+      const double a = (double)S.lo[i] + 0.5 - S.p[i];
+      const double b = a + (double)(S.ext[i] > 0 ? S.ext[i] - 1 : 0);
+      w2 += std::max(a * a, b * b);
+   }
+   const double box = std::sqrt(w2), v = std::sqrt(S.c2), ps = 1e-14 * (double)S.pscale;
+   const double near = v + std::sqrt(thr * (1.0 + 1e-4) + 0.01 + 1e-4 * S.c2 +
+                                     10.0 * ps * (v + std::sqrt(thr) + 1.0));
+   const double w = std::min(box, near);
+   return (float)(1.001 * (1.08e-6 * w * w + 1.5e-7 * w * box + 7.2e-7 * S.c2 + 2e-6 +
+                           ps * (w + 1.0)));
+}
+
 // Host-side constants of the two-float path, all derived in double exactly
 // as the reference derives the corresponding values.
 void fill_fast_fields(SegDev &S, const fpgb_volume *vol) {
    double ps = 0;
    for (int i = 0; i < 3; i++) {
-      split2(S.p[i] - (double)S.base[i], S.pl_hi[i], S.pl_lo[i]);
-      split2(S.v[i], S.v_hi[i], S.v_lo[i]);
+      split2(S.p[i] - (double)S.base[i], S.pf[i], S.pl_lo[i]);
+      split2(S.v[i], S.vf[i], S.v_lo[i]);
       ps = std::max(ps, std::max(std::fabs(S.p[i]), std::fabs(S.q[i])));
       ps = std::max(ps, (double)vol->dim[i]);
    }
    S.pscale = (float)(ps + 2.0);
-   split2(S.c2, S.c2_hi, S.c2_lo);
+   split2(S.c2, S.c2f, S.c2_lo);
    S.c2_rcp = S.c2 > 0 ? (float)(1.0 / S.c2) : 0.f;
    split2(S.r0, S.r0_hi, S.r0_lo);
    split2(S.r1 - S.r0, S.dr_hi, S.dr_lo);
@@ -138,6 +162,7 @@ void fill_fast_fields(SegDev &S, const fpgb_volume *vol) {
       if (a == b)
          S.rsq_const = a;
    }
+   S.dec_rsq = S.rsq_const == S.rsq0 && S.rsq_const == S.rsq1 ? S.rsq_const : NAN;
    // 'p' layer vector: vm::unit(q - p) (generator.cpp:372-373, vemath.hpp:390-402)
    double n2 = 0.0;
    n2 = n2 + S.v[0] * S.v[0];
@@ -217,6 +242,7 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
          }
          L.scale_sq[i] = fb->layer_scale[l] * fb->layer_scale[l];
          L.model[i] = m;
+         L.models |= (uint32_t)(m == 'p' ? 1 : m == 'r' ? 2 : 0) << (2 * i);
          L.dn[i] = fb->layer_dn[l];
          L.mu[i] = fb->layer_mu[l];
       }
@@ -398,8 +424,6 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
             S.v[i] = Q[i] - P[i];
             const double base = std::floor(P[i]);
             S.base[i] = (int32_t)std::max(-2147483647.0, std::min(2147483647.0, base));
-            S.pf[i] = (float)(P[i] - (double)S.base[i]);
-            S.vf[i] = (float)S.v[i];
          }
          {
             double c = 0.0;
@@ -408,12 +432,12 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
             c = c + S.v[2] * S.v[2];
             S.c2 = c;
          }
-         S.c2f = (float)S.c2;
          S.r0 = r0;
          S.r1 = r1;
          fill_fast_fields(S, vol);
          const double rm = r0 < r1 ? r1 : r0;
-         S.thr_f = (float)((double)L.f_ly_squ * rm * rm * (1.0 + 1e-3) + 1e-3);
+         S.thr_f = (float)((double)L.f_ly_squ * rm * rm * (1.0 + 1e-5)) * (1.f + 0x1p-22f);
+         S.mg = seg_margin(S, S.thr_f);
          {
             const double rn = r0 < r1 ? r0 : r1;
             const double a = (double)L.f_ly_squ * rn * rn * (1.0 - 1e-5);
@@ -460,7 +484,7 @@ size_t tissue_workspace_bytes(const TissuePlan &p) {
    b += align_up(sizeof(SegDev) * std::max<size_t>(p.segs.size(), 1), 256);
    b += align_up(sizeof(LayerDev) * p.layers.size(), 256);
    b += align_up(sizeof(unsigned long long) * kCounterWords, 256);
-   b += brick_workspace_bytes(n_bricks, p.brick_pairs);
+   b += brick_workspace_bytes(n_bricks, p.brick_pairs, (int64_t)p.segs.size());
    return b;
 }
 
@@ -503,6 +527,7 @@ int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
    h.t.Z = (int32_t)p.Z;
    h.t.max_layer = p.max_layer;
    h.t.layer_base = 0;
+   h.t.n_bundles = (int32_t)p.layers.size();
    for (int i = 0; i < 3; i++)
       h.t.nb[i] = nb[i];
    h.label = d_label;

@@ -14,15 +14,17 @@ constexpr int kMaxLayers = 16;
 
 // One fiber segment after translate + resize (voxel units), in the
 // reference's processing order; its table index is the tie-break index.
+// 256 bytes: two whole 128-byte lines per segment.
 struct __align__(16) SegDev {
    double p[3];   // segment start s0
    double q[3];   // segment end s1
    double v[3];   // s1 - s0 (generator.cpp:479)
    double r0, r1; // radii at s0, s1
    double c2;     // dot(v, v) (generator.cpp:486)
-   // inputs of the voxelizer's sweeps: five 16-byte words at offset 96,
-   // read with vector loads (SegSweep)
-   float pf[3];   // p - base, for the FP32 prefilter
+   // inputs of the voxelizer's sweep: five 16-byte words at offset 96, read
+   // with vector loads (SegSweep), then the word {mg, dec_rsq, rsq0, rsq1}.
+   // pf, vf and c2f are also the high parts of the two-float inputs below.
+   float pf[3];   // float(p - base)
    float vf[3];   // float(v)
    float c2f;     // float(c2)
    float c2_rcp;  // float(1 / c2)
@@ -33,25 +35,33 @@ struct __align__(16) SegDev {
    int32_t lo[3];   // clipped box start (generator.cpp:304)
    int32_t ext[3];  // clipped box extent
    int32_t bundle;
-   // two-float copies (hi, lo) of the double inputs, for the fast path
-   float pl_hi[3], pl_lo[3]; // p - base
-   float v_hi[3], v_lo[3];   // v
-   float c2_hi, c2_lo;       // c2
-   float r0_hi, r0_lo;       // r0
-   float dr_hi, dr_lo;       // r1 - r0
-   float rsq0, rsq1;         // float(r^2) at t = 0 and t = 1 (exact)
-   float rsq_const;          // float(r^2) for every interior t when r0 == r1
-                             // and that rounding is certain; NaN otherwise
-   float pscale;             // max |coordinate| met by this segment's arithmetic
-   float vp[3];              // float(unit(q - p)): the 'p' layer vector (exact)
+   float mg;         // bound on |sweep estimate - dist^2| over the box (seg_margin)
+   float dec_rsq;    // float(r^2) at every t of the segment when that is one
+                     // certain value (constant radius); NaN otherwise
+   float rsq0, rsq1; // float(r^2) at t = 0 and t = 1 (exact)
+   // low parts of the two-float inputs of the fast path (and whole pairs
+   // where the high part is not above)
+   float pl_lo[3];   // p - base
+   float v_lo[3];    // v
+   float c2_lo;      // c2
+   float r0_hi, r0_lo; // r0
+   float dr_hi, dr_lo; // r1 - r0
+   float rsq_const;  // float(r^2) for every interior t when r0 == r1
+                     // and that rounding is certain; NaN otherwise
+   float pscale;     // max |coordinate| met by this segment's arithmetic
+   float vp[3];      // float(unit(q - p)): the 'p' layer vector (exact)
 };
-static_assert(offsetof(SegDev, pf) == 96 && offsetof(SegDev, bundle) == 172,
-              "the sweep inputs of SegDev are five aligned 16-byte words");
+static_assert(offsetof(SegDev, pf) == 96 && offsetof(SegDev, bundle) == 172 &&
+                  offsetof(SegDev, mg) == 176 && sizeof(SegDev) == 256,
+              "the sweep inputs of SegDev are aligned 16-byte words");
 
 // Layers of one bundle, sorted by scale (fiber_bundle.cpp:83-86).
 struct LayerDev {
    int32_t n = 0;
    float f_ly_squ = 0.f; // float(scale^2 of the outermost layer)
+   // the layers' models, two bits each: 0 'b' (and past the last layer), 1
+   // 'p', 2 'r'
+   uint32_t models = 0;
    double sqrt_last = 0.0;
    double scale_sq[kMaxLayers] = {};
    // largest float <= scale_sq[l]: for a float q, (double)q > scale_sq[l]

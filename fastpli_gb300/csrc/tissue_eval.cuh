@@ -77,6 +77,21 @@ FPGB_HD float approx_dist2(float wx, float wy, float wz, float vx, float vy, flo
                          margin);
 }
 
+// The same estimate as the sweep takes it, with the segment's own bound
+// S.mg (seg_margin) already in the sum: c1n2 = -2 (w.v)'s y and z parts and
+// b = wy^2 + wz^2 + mg come once per cell, vn2 = -2 vx, rch = -1/2 float(1 / c2).
+// The value is an upper bound hi of the reference's float, hi - 2 mg a lower
+// bound (mg covers the rounding of the two differences as well).
+FPGB_HD float sweep_dist2(float wx, float a2, float b, float vn2, float c2f, float rch) {
+   const float c1n = fmaf(wx, vn2, a2); // -2 w.v
+#ifdef __CUDA_ARCH__
+   const float t = __saturatef(c1n * rch);
+#else
+   const float t = fminf(fmaxf(c1n * rch, 0.f), 1.f);
+#endif
+   return fmaf(t, fmaf(t, c2f, c1n), fmaf(wx, wx, b));
+}
+
 // float(|cl - pt|^2) and float(r(t)^2) exactly as generator.cpp:327-328.
 FPGB_HD void exact_dist(const SegDev &S, const double pt[3],
                                            double cl[3], float &dist_squ,
@@ -104,109 +119,113 @@ FPGB_HD void exact_dist(const SegDev &S, const double pt[3],
 // else returns false and the caller replays the reference in FP64, so the
 // outcome is always the reference's, bit for bit.
 // ----------------------------------------------------------------------
+//
+// The pairs are kept unnormalised where the next operation does not need
+// them normalised: products contribute their rounding error (one fused
+// multiply-add) to a single low word, whose own rounding is a few units of
+// 2^-48 of the terms' magnitudes — the form every bound here is stated in
+// (2^-41 and 2^-42 of them, at least 2^3 units of slack).
 struct FastCand {
    float dist_squ, r_sqr;
    ff d[3];  // closest - point
-   float dn; // |d|
-   float m;  // magnitude scale of the terms that make up d
+   ff D;     // |d|^2
+   float y0; // ~ 1 / |d| (0 for d = 0)
+   float dn; // ~ |d|
+   float m;  // magnitude scale of the terms that make up d (>= their 2-norm)
 };
 
-// Per-(y, z) row terms of the candidate evaluation (hoisted out of the x loop).
-struct FastRow {
-   ff wy, wz, c1yz; // point - p along y and z, and their part of dot(w, v)
-   float wyz2;      // float estimate of wy^2 + wz^2
-};
-
-FPGB_HD void fast_row(const SegDev &S, float ly, float lz, FastRow &r) {
-   r.wy = ff_add_f(ff{-S.pl_hi[1], -S.pl_lo[1]}, ly);
-   r.wz = ff_add_f(ff{-S.pl_hi[2], -S.pl_lo[2]}, lz);
-   r.c1yz = ff_add_sloppy(ff_mul(r.wy, ff{S.v_hi[1], S.v_lo[1]}),
-                          ff_mul(r.wz, ff{S.v_hi[2], S.v_lo[2]}));
-   r.wyz2 = r.wy.hi * r.wy.hi + r.wz.hi * r.wz.hi;
+// 1 / sqrt(x) within a few units of 2^-23
+FPGB_HD float rsqrt_est(float x) {
+#ifdef __CUDA_ARCH__
+   return rsqrtf(x);
+#else
+   return 1.0f / sqrtf(x);
+#endif
 }
 
-FPGB_HD bool fast_candidate_row(const SegDev &S, float lx, const FastRow &row, FastCand &c) {
+// closest - point of the candidate (generator.cpp:475-494) with its squared
+// length, and r^2 where it needs no rounding decision (rsq0, rsq1, rsq_const;
+// NaN: interior of a segment whose radius changes, b holds the parameter).
+// False when the clamp of the closest-point parameter is undecided.
+FPGB_HD bool fast_offset(const SegDev &S, const float pt[3], FastCand &c, ff &b) {
    ff w[3], v[3];
-   w[0] = ff_add_f(ff{-S.pl_hi[0], -S.pl_lo[0]}, lx); // point - p
-   w[1] = row.wy;
-   w[2] = row.wz;
+   float wm = 0.f, vm = 0.f; // 1-norms: bounds of the 2-norms
 #pragma unroll
-   for (int i = 0; i < 3; i++)
-      v[i] = ff{S.v_hi[i], S.v_lo[i]};
-   const ff c1 = ff_add_sloppy(ff_mul(w[0], v[0]), row.c1yz);
-   const float wn = sqrtf(w[0].hi * w[0].hi + row.wyz2);
-   const ff c2{S.c2_hi, S.c2_lo};
-   const float vn = sqrtf(S.c2_hi);
-   const float ec = 0x1p-42f * (wn * vn + 1.f);
-   int branch;
-   if (c1.hi < -ec) {
-      branch = 0; // c1 < 0: closest = s0, t = 0 (generator.cpp:483-484)
-   } else {
-      const ff dq = ff_sub_sloppy(c1, c2);
-      if (dq.hi > ec)
-         branch = 1; // c2 <= c1: closest = s1, t = 1 (:487-488)
-      else if (c1.hi > ec && dq.hi < -ec)
-         branch = 2; // interior: b = c1 / c2 (:490-493)
-      else
-         return false;
+   for (int i = 0; i < 3; i++) { // point - p; pt is exact
+      const ff s = two_sum(pt[i], -S.pf[i]);
+      w[i] = ff{s.hi, s.lo - S.pl_lo[i]};
+      v[i] = ff{S.vf[i], S.v_lo[i]};
+      wm += fabsf(s.hi);
+      vm += fabsf(S.vf[i]);
    }
-   float bmag;
-   if (branch == 0) {
-      bmag = 0.f;
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-         c.d[i] = ff_neg(w[i]);
+   const ff c1 = ff_dot3(w, v);
+   const float ec = 0x1p-42f * (wm * vm + 1.f);
+   const float dq = (c1.hi - S.c2f) + (c1.lo - S.c2_lo);
+   b = ff{0.f, 0.f};
+   if (c1.hi < -ec) { // c1 < 0: closest = s0, t = 0 (generator.cpp:483-484)
       c.r_sqr = S.rsq0;
-   } else if (branch == 1) {
-      bmag = 1.f;
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-         c.d[i] = ff_sub_sloppy(v[i], w[i]);
+   } else if (dq > ec) { // c2 <= c1: closest = s1, t = 1 (:487-488)
+      b.hi = 1.f;
       c.r_sqr = S.rsq1;
+   } else if (c1.hi > ec && dq < -ec) { // interior: b = c1 / c2 (:490-493)
+      // one residual correction of the FP32 quotient: c1.hi - q c2 is exact
+      const float q = c1.hi * S.c2_rcp;
+      const ff p = two_prod(S.c2f, q);
+      const float e = ((c1.hi - p.hi) - p.lo) + fmaf(-S.c2_lo, q, c1.lo);
+      b = quick_two_sum(q, e * S.c2_rcp);
+      c.r_sqr = S.rsq_const;
    } else {
-      const ff b = ff_div_rcp(c1, c2, S.c2_rcp);
-      bmag = b.hi;
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-         c.d[i] = ff_sub_sloppy(ff_mul(v[i], b), w[i]);
-      if (!std::isnan(S.rsq_const)) {
-         c.r_sqr = S.rsq_const;
-      } else { // r = r0 (1 - t) + r1 t  (fiber.cpp:115-120)
-         const ff R = ff_add(ff{S.r0_hi, S.r0_lo}, ff_mul(ff{S.dr_hi, S.dr_lo}, b));
-         const ff R2 = ff_sqr(R);
-         const float er =
-             0x1p-40f * (R2.hi + fabsf(R.hi) * fabsf(S.dr_hi) * (bmag + wn / vn + 1.f));
-         if (!ff_round_unique(R2, er, c.r_sqr))
-            return false;
-      }
+      return false;
    }
-   const ff D = ff_norm2_sloppy(c.d);
-   c.dn = sqrtf(fmaxf(D.hi, 0.f));
-   c.m = wn + vn * bmag + 1.f;
-   const float ed = 0x1p-41f * c.m * (c.dn + 0x1p-20f * c.m) +
-                    0x1p-47f * S.pscale * (2.f * c.dn + 1.f);
-   return ff_round_unique(D, ed, c.dist_squ);
+#pragma unroll
+   for (int i = 0; i < 3; i++) { // v b - w
+      const ff p = two_prod(v[i].hi, b.hi);
+      const ff s = two_sum(p.hi, -w[i].hi);
+      const float lo = fmaf(v[i].hi, b.lo, fmaf(v[i].lo, b.hi, p.lo));
+      c.d[i] = quick_two_sum(s.hi, (lo - w[i].lo) + s.lo);
+   }
+   c.D = ff_dot3(c.d, c.d);
+   c.y0 = c.D.hi > 0.f ? rsqrt_est(c.D.hi) : 0.f;
+   c.dn = c.D.hi * c.y0;
+   c.m = wm + vm * b.hi + 1.f;
+   return true;
 }
 
 FPGB_HD bool fast_candidate(const SegDev &S, const float pt[3], FastCand &c) {
-   FastRow row;
-   fast_row(S, pt[1], pt[2], row);
-   return fast_candidate_row(S, pt[0], row, c);
+   ff b;
+   if (!fast_offset(S, pt, c, b))
+      return false;
+   if (!(c.r_sqr == c.r_sqr)) { // r = r0 (1 - t) + r1 t  (fiber.cpp:115-120)
+      const ff R = ff_add(ff{S.r0_hi, S.r0_lo}, ff_mul(ff{S.dr_hi, S.dr_lo}, b));
+      const ff R2 = ff_sqr(R);
+      // b's error is that of c1: 2^-42 (|w| |v| + 1) / c2
+      const float eb = c.m * c.m * S.c2_rcp + b.hi + 1.f;
+      const float er = 0x1p-40f * (R2.hi + fabsf(R.hi) * fabsf(S.dr_hi) * eb);
+      if (!ff_round_unique(R2, er, c.r_sqr))
+         return false;
+   }
+   const float ed = 0x1p-43f * c.m * (c.dn + 0x1p-20f * c.m) +
+                    0x1p-49f * S.pscale * (2.f * c.dn + 1.f);
+   return ff_round_unique(c.D, ed, c.dist_squ);
 }
 
 // float(unit(point - closest)) of the 'r' layer (generator.cpp:370-371)
 FPGB_HD bool fast_radial(const SegDev &S, const FastCand &c, float out[3]) {
    if (!(c.dn > 0x1p-10f))
       return false;
-   const ff n2 = ff_norm2(c.d);
-   const ff inv = ff_div(ff_from(-1.f), ff_sqrt(n2)); // nv = -d
-   const float ex = (0x1p-41f * c.m + 0x1p-47f * S.pscale) / c.dn + 0x1p-43f;
+   // 1 / |d| = y0 (1 + e/2 + 3 e^2/8 + ...), e = 1 - D y0^2 (|e| < 2^-20)
+   const ff t = two_prod(c.y0, c.y0);
+   const float e = fmaf(-c.D.lo, t.hi, fmaf(-c.D.hi, t.lo, fmaf(-c.D.hi, t.hi, 1.f)));
+   const ff inv = quick_two_sum(c.y0, c.y0 * fmaf(0.375f * e, e, 0.5f * e));
+   const float ex = (0x1p-43f * c.m + 0x1p-49f * S.pscale) * (1.001f * c.y0) + 0x1p-44f;
 #pragma unroll
-   for (int i = 0; i < 3; i++)
-      if (!ff_round_unique(ff_mul(c.d[i], inv), ex, out[i]))
+   for (int i = 0; i < 3; i++) { // nv = -d
+      const ff p = two_prod(-c.d[i].hi, inv.hi);
+      const float lo = fmaf(-c.d[i].hi, inv.lo, fmaf(-c.d[i].lo, inv.hi, p.lo));
+      if (!ff_round_unique(quick_two_sum(p.hi, lo), ex, out[i]))
          return false;
+   }
    return true;
 }
-
 
 } // namespace fpgb

@@ -4,33 +4,37 @@
 // (tissue_eval.cuh) must round every product and sum separately, and the
 // FP32 estimate of the key passes must be the same in both passes.
 //
-// Winner keys.  A voxel's key is float_bits(dist^2) << 32 |
-// (0xFFFFFFFF - segment): the minimum over every accepted (segment, voxel)
-// candidate is the smallest distance, ties going to the LAST segment, which
-// is the reference's `>=` overwrite rule (generator.cpp:329-340).  Keys live
-// in shared memory for the lifetime of the brick's CTA and are minimised
-// with shared-memory atomics.
+// The winner of a voxel is the segment with the smallest dist^2 (float, in
+// the reference's arithmetic) among those it is inside of, ties going to the
+// LAST segment: the reference's `>=` overwrite rule (generator.cpp:329-340).
+// Most voxels need no exact distance to find it.  One sweep over the brick's
+// segments gives every candidate an FP32 upper bound hi of its dist^2
+// (sweep_dist2; hi - 2 mg is a lower bound).  A candidate whose lower bound is
+// not past the thickest end of its segment lowers the voxel's 32-bit key (hi
+// in quanta of 1 / scale, slot in the brick's list) with a shared-memory
+// atomicMin that returns the old key.  When old and new lie within W = 2
+// max(mg) of each other the order of the two may be the other way round: the
+// voxel's key is marked (its lowest bit; a key that replaces it from farther
+// below drops the mark, which only spoke of candidates that have lost).
 //
-// Two key passes over the brick's segments:
+// Every pair that could be out of order at the end marks the final key.  Let
+// o hold it and c be another candidate with hi_c <= hi_o + W.  If c came
+// after o, it met o's key.  If c came before o, o met some key between its
+// own and c's.  So an unmarked key whose segment o the voxel is inside of
+// names the winner: every other one is farther (ties are within W).
 //
-//   BOUND  every candidate that is certainly accepted (FP32 estimate plus its
-//          bound at or below f_ly_squ * min(r0, r1)^2) stores an upper bound
-//          ub of its exact dist^2 as the key ub << 32 | 0xFFFFFFFF, and its
-//          bundle in the bundle minimum;
-//   EXACT  a candidate whose lower bound exceeds the voxel's current key
-//          cannot be the minimum and is skipped; the rest are evaluated with
-//          the reference's arithmetic (two-float fast path, FP64 replay) and
-//          stored as exact keys.
+// Whether the voxel is inside of o, and in which of its layers, follows from
+// the interval [hi - 2 mg, hi] unless that straddles a layer's boundary (the
+// voxel is marked as well) or the radius changes along the segment; then o is
+// evaluated with the reference's arithmetic (two-float fast path, FP64
+// replay), and the voxel marked if it lies outside.
 //
-// The true winner w (smallest exact dist^2 among accepted candidates, last
-// segment on ties) is never skipped: every stored value is >= its distance
-// (an upper bound belongs to an accepted candidate, whose exact distance is
-// >= w's), and w's lower bound is <= its own distance.  Candidates tied with
-// w are not skipped either, so the tie rule holds.  An upper-bound key is
-// >= w's exact key (equal only when w is segment 0: the same value), so the
-// final key is w's, bit for bit.  A candidate that the bound filter skips
-// but that was not certainly accepted is still decided exactly when the
-// bundle minimum is kept (multi-bundle volumes), so that stays exact too.
+// voxel_bricks leaves kMarkedLabel in the marked voxels (0.3% on the uneven
+// tiles) and lists them; voxel_marks resolves them with the reference's
+// arithmetic: every candidate whose lower bound is at or below the smallest
+// upper bound of the certain ones is evaluated, and the smallest
+// float_bits(dist^2) << 32 | (0xFFFFFFFF - segment) wins.  A kernel of its own
+// has no barriers, and its code and registers stay out of the sweep's.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -65,11 +69,22 @@ int64_t segment_brick_pairs(const SegDev &S) {
           brick_range(S.lo[2], S.ext[2], kBrickZ, b0);
 }
 
-size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs) {
+// The marked voxels' records, a share of the space per launch: entry 0 counts
+// {entries taken, records}; a record is {brick, number} and the brick's marked
+// voxels, four 16-bit places to an entry.  The launch's part of the bricks'
+// count array becomes the records' directory.  32 bytes per segment hold
+// several times the marks of the synthetic volumes; a brick whose record does
+// not fit is found again by the labels of its voxels.
+static int64_t mark_entries(int64_t n_segs) {
+   return std::max<int64_t>(0, 4 * n_segs - 32);
+}
+
+size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs, int64_t n_segs) {
    size_t w = 0;
    w += align_up(sizeof(unsigned) * (n_bricks + 1), 256); // offsets
    w += align_up(sizeof(unsigned) * std::max<int64_t>(n_bricks, 1), 256); // counts, then cursors
    w += align_up(sizeof(unsigned) * std::max<int64_t>(n_pairs, 1), 256);  // segment lists
+   w += align_up(sizeof(uint2) * mark_entries(n_segs), 256);              // marked voxels
    return w;
 }
 
@@ -116,7 +131,10 @@ constexpr int kScanPer = 8;
 
 __global__ void __launch_bounds__(1024)
 brick_scan(const unsigned *__restrict__ counts, int64_t n, unsigned *__restrict__ offsets,
+           uint2 *__restrict__ marks, int64_t mark_share, int n_shares,
            unsigned long long *__restrict__ counters) {
+   if (mark_share > 0 && (int)threadIdx.x < n_shares) // the marked voxels' lists start empty
+      marks[threadIdx.x * mark_share] = make_uint2(0u, 0u);
    __shared__ unsigned long long wsum[32];
    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
    // the callers' workspaces are 256-byte aligned; checked anyway before any
@@ -187,31 +205,33 @@ brick_scan(const unsigned *__restrict__ counts, int64_t n, unsigned *__restrict_
    }
 }
 
-// ------------------------------------------------------------ key passes ---
-// The inputs of the sweeps of one segment (SegDev offsets 96..175: pf, vf,
-// c2f, c2_rcp, thr_f, acc_f, base, lo, ext, bundle) in five 16-byte loads.
+// ----------------------------------------------------------------- sweep ---
+// The inputs of the sweep of one segment (SegDev offsets 96..191: pf, vf,
+// c2f, c2_rcp, thr_f, acc_f, base, lo, ext, bundle, mg) in 16-byte loads.
 struct SegSweep {
    float4 a; // pf[0..2], vf[0]
    float4 b; // vf[1..2], c2f, c2_rcp
    float4 c; // thr_f, acc_f, base[0..1] (int bits)
    int4 d;   // base[2], lo[0..2]
    int4 e;   // ext[0..2], bundle
+   float mg;
 };
 
 __device__ __forceinline__ SegSweep load_sweep(const SegDev &S) {
    const float4 *f = reinterpret_cast<const float4 *>(&S.pf[0]);
    const int4 *i = reinterpret_cast<const int4 *>(&S.pf[0]);
-   return SegSweep{__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(i + 3), __ldg(i + 4)};
+   return SegSweep{__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(i + 3), __ldg(i + 4),
+                   __ldg(&S.mg)};
 }
 
 // The part of segment S's clipped box inside the brick (origin o, extent n),
 // swept as columns along x: its ey x ez (y, z) cells are numbered z fastest,
 // lane l of chunk c owns cell 32 c + l and visits the ex voxels of that
 // cell's x column.  The y and z parts of the estimate are computed once per
-// cell; each voxel then costs six fused operations (approx_dist2_x).
+// cell; each voxel then costs six fused operations (sweep_dist2).
 struct SubBox {
    int x0, y0, z0, ex, ey, ez, ncell;
-   float inv_ez; // 1/ez for the division-free cell split
+   float ezf, inv_ez; // 1/ez for the division-free cell split
 };
 
 __device__ __forceinline__ bool sub_box(const SegSweep &w, int ox, int oy, int oz, int nx,
@@ -225,7 +245,8 @@ __device__ __forceinline__ bool sub_box(const SegSweep &w, int ox, int oy, int o
    if (b.ex <= 0 || b.ey <= 0 || b.ez <= 0)
       return false;
    b.ncell = b.ey * b.ez;
-   b.inv_ez = __frcp_rn((float)b.ez);
+   b.ezf = (float)b.ez;
+   b.inv_ez = __fdividef(1.f, b.ezf);
    return true;
 }
 
@@ -233,68 +254,135 @@ __device__ __forceinline__ int brick_index(int x, int y, int z, int ox, int oy, 
    return ((x - ox) * kBrickY + (y - oy)) * kBrickZ + (z - oz);
 }
 
+// The brick's quantisation of the keys: hi * scale rounds to an integer below
+// 2^min(23, 32 - slot_bits) (added to 2^23 it sits in the float's mantissa),
+// the slot takes the low slot_bits >= 8 bits but the last, the mark.  win: W
+// in key units.
+struct BrickScale {
+   float scale, quantum; // quantum >= 1 / scale
+   float mg2;            // 2 max(mg)
+   int bits;             // slot_bits
+   unsigned mul;         // 1 << slot_bits
+   unsigned win, win2;   // W, 2 W (all ones: every two keys are close)
+};
+
+constexpr unsigned kNoKey = 0xFFFFFFFFu;
+
+__device__ __forceinline__ bool key_marked(unsigned key) { return (key & 1u) && key != kNoKey; }
+
+__device__ BrickScale brick_scale(unsigned n_seg, float max_thr2, float max_mg) {
+   BrickScale k;
+   const int bits = n_seg <= 128u ? 8 : min(31, 33 - __clz((int)(n_seg - 1u)));
+   const int qbits = min(23, 32 - bits);
+   k.bits = bits;
+   k.mul = 1u << bits;
+   const float top = qbits > 3 ? (float)((1u << qbits) - 4u) : 0.f;
+   k.scale = 0.999999f * __fdividef(top, max_thr2);
+   if (!(k.scale > 0.f && k.scale < 1e30f))
+      k.scale = 0.f;
+   k.quantum = k.scale > 0.f ? __fdividef(1.000001f, k.scale) : INFINITY;
+   k.mg2 = 2.f * max_mg;
+   const float w = fmaf(k.mg2, k.scale, 4.f) * (float)k.mul;
+   if (w < 1e9f) {
+      k.win = (unsigned)w;
+      k.win2 = 2u * k.win;
+   } else { // NaN too
+      k.win = 0x7FFFFFFFu;
+      k.win2 = 0xFFFFFFFFu;
+   }
+   return k;
+}
+
+// Upper bound of the hi that a voxel's key stands for.
+__device__ __forceinline__ float key_bound(const BrickScale &k, unsigned key) {
+   return ((float)(key >> k.bits) + 1.f) * k.quantum;
+}
+
 // Per-segment inputs of the FP32 estimate, held in registers over a sweep.
 struct SegFP32 {
-   float pfx, pfy, pfz, vx, vy, vz, c2f, rc2, thr, acc;
+   float pfx, pfy, pfz, vn2x, vn2y, vn2z, c2f, rch, mg;
    int bx, by, bz;
 };
 
 __device__ __forceinline__ SegFP32 seg_fp32(const SegSweep &w) {
-   return SegFP32{w.a.x, w.a.y, w.a.z, w.a.w, w.b.x, w.b.y, w.b.z, w.b.w, w.c.x, w.c.y,
-                  __float_as_int(w.c.z), __float_as_int(w.c.w), w.d.x};
+   return SegFP32{w.a.x, w.a.y, w.a.z, -2.f * w.a.w, -2.f * w.b.x, -2.f * w.b.y, w.b.z,
+                  -0.5f * w.b.w, w.mg, __float_as_int(w.c.z), __float_as_int(w.c.w), w.d.x};
 }
 
-// A lane's (y, z) cell of a chunk: its brick index at x = x0, and the y / z
-// parts of the estimate.  (c + 1/2) / ez lies at least 1/(2 ez) >= 2^-6 from
-// an integer for c < 256 and ez <= 32, far beyond the float error of the
-// product, so the truncation is the exact quotient.
+// A lane's (y, z) cell of a chunk of 32, numbered z fastest, in float
+// arithmetic (all integers below 2^24).  (c + 1/2) / ez lies at least
+// 1/(2 ez) >= 2^-6 from an integer for c < 256 and ez <= 32, far beyond the
+// error of the product with the approximate reciprocal, so the truncation is
+// the exact quotient.
 struct Cell {
-   int li;
-   float a, b;
+   int yz;      // y * 32 + z from the sub-box's first cell
+   float a2, b; // the y / z parts of the estimate
 };
 
-__device__ __forceinline__ Cell cell_of(const SubBox &b, const SegFP32 &g, int c, int ox, int oy,
-                                        int oz) {
-   const int iy = (int)(((float)c + 0.5f) * b.inv_ez);
-   const int y = b.y0 + iy, z = b.z0 + (c - iy * b.ez);
-   // voxel centre - float(p - base): (y - base) + 1/2 is exact in float
-   const float wy = ((float)(y - g.by) + 0.5f) - g.pfy;
-   const float wz = ((float)(z - g.bz) + 0.5f) - g.pfz;
-   return Cell{brick_index(b.x0, y, z, ox, oy, oz), dist2_yz_dot(wy, wz, g.vy, g.vz),
-               dist2_yz_len(wy, wz)};
+// wy0, wz0: voxel centre - float(p - base) of the first cell ((y - base) + 1/2
+// is exact in float)
+__device__ __forceinline__ Cell cell_of(const SubBox &b, const SegFP32 &g, float wy0, float wz0,
+                                        float c) {
+   const float iy = truncf((c + 0.5f) * b.inv_ez);
+   const float iz = fmaf(-iy, b.ezf, c);
+   const float wy = wy0 + iy, wz = wz0 + iz;
+   return Cell{(int)fmaf(iy, (float)kBrickZ, iz), fmaf(wz, g.vn2z, wy * g.vn2y),
+               fmaf(wz, wz, fmaf(wy, wy, g.mg))};
 }
 
-// FP32 estimate of the candidate at x offset gx = (x - base) + 1/2 of a
-// cell: its dist^2 lies in [lo, hi] (directed rounding of estimate -/+
-// bound).
-__device__ __forceinline__ void candidate_bounds(const SegFP32 &g, const Cell &c, float gx,
-                                                 float &lo, float &hi) {
-   float mg;
-   const float d2f = approx_dist2_x(gx - g.pfx, c.a, c.b, g.vx, g.c2f, g.rc2, mg);
-   lo = __fsub_rd(d2f, mg);
-   hi = __fadd_ru(d2f, mg);
-}
+constexpr int kPlane = kBrickY * kBrickZ; // distance of x neighbours in the shared arrays
+constexpr int kSweepStep = 2;
 
-// BOUND pass of one segment over its sub-box: the upper bound of every
-// certainly accepted candidate goes to the voxel's 32-bit bound (a float
-// >= 0, so its bits order like the value).  Lanes take cells independently.
+// The sweep of one segment over its sub-box, kSweepStep voxels of a column at
+// a time (their atomics are in flight together).  A candidate outside sends
+// kNoKey, which changes nothing and needs no branch; the last step may reach
+// past the column (and into skey's padding).  multi: the smallest bundle whose
+// fiber a voxel is certainly inside of is kept as well; voxels that are only
+// possibly inside get a mark of their own, which stays.
 template <bool MULTI>
-__device__ __forceinline__ void brick_bound(const SegSweep &sw, const SubBox &b, int ox, int oy,
-                                            int oz, unsigned *sub, unsigned *sminb, int lane) {
+__device__ __forceinline__ void brick_sweep(const SegSweep &sw, unsigned slot, const SubBox &b,
+                                            int ox, int oy, int oz, const BrickScale &k,
+                                            bool multi, unsigned *skey, unsigned *smark,
+                                            unsigned *sminb, int lane) {
    const SegFP32 g = seg_fp32(sw);
-   const unsigned bundle = (unsigned)sw.e.w;
-   const float gx0 = (float)(b.x0 - g.bx) + 0.5f;
+   // bound of hi (finite: an infinite hi is outside)
+   const float thr = fminf(fmaf(2.00001f, g.mg, sw.c.x), 3e38f);
+   const float wy0 = ((float)(b.y0 - g.by) + 0.5f) - g.pfy;
+   const float wz0 = ((float)(b.z0 - g.bz) + 0.5f) - g.pfz;
+   const float wx0 = ((float)(b.x0 - g.bx) + 0.5f) - g.pfx;
+   const int first = ((b.x0 - ox) * kBrickY + (b.y0 - oy)) * kBrickZ + (b.z0 - oz);
    for (int c0 = lane; c0 < b.ncell; c0 += 32) {
-      const Cell c = cell_of(b, g, c0, ox, oy, oz);
-      float gx = gx0;
-      int li = c.li;
-      for (int i = 0; i < b.ex; i++, gx += 1.f, li += kBrickY * kBrickZ) {
-         float lo, hi;
-         candidate_bounds(g, c, gx, lo, hi);
-         if (hi <= g.acc) {
-            atomicMin(&sub[li], __float_as_uint(hi));
-            if (MULTI)
-               atomicMin(&sminb[li], bundle);
+      const Cell c = cell_of(b, g, wy0, wz0, (float)c0);
+      unsigned *key = skey + first + c.yz;
+      float wx = wx0;
+      for (int i = 0; i < b.ex;
+           i += kSweepStep, wx += (float)kSweepStep, key += kSweepStep * kPlane) {
+         float hi[kSweepStep];
+         unsigned mine[kSweepStep], old[kSweepStep];
+#pragma unroll
+         for (int u = 0; u < kSweepStep; u++) {
+            hi[u] = sweep_dist2(u ? wx + (float)u : wx, c.a2, c.b, g.vn2x, g.c2f, g.rch);
+            mine[u] = __float_as_uint(fmaf(hi[u], k.scale, 8388608.f)) * k.mul + 2u * slot;
+            if (u && i + u >= b.ex)
+               hi[u] = INFINITY;
+         }
+         // (NaN, from an infinite bound, counts as inside)
+#pragma unroll
+         for (int u = 0; u < kSweepStep; u++)
+            old[u] = atomicMin(key + u * kPlane, !(hi[u] > thr) ? mine[u] : kNoKey);
+#pragma unroll
+         for (int u = 0; u < kSweepStep; u++)
+            if (!(hi[u] > thr) && old[u] - mine[u] + k.win <= k.win2)
+               atomicOr(key + u * kPlane, 1u);
+         if (MULTI && multi) {
+#pragma unroll
+            for (int u = 0; u < kSweepStep; u++)
+               if (hi[u] <= fminf(sw.c.y, 3e38f))
+                  atomicMin(sminb + (key - skey) + u * kPlane, (unsigned)sw.e.w);
+               else if (!(hi[u] > thr)) {
+                  const int yz = (int)(key - skey) & (kPlane - 1), x = b.x0 - ox + i + u;
+                  atomicOr(&smark[yz >> 2], 1u << (8 * (yz & 3) + x));
+               }
          }
       }
    }
@@ -353,149 +441,36 @@ __device__ __noinline__ bool cand_radial(const SegDev &S, int x, int y, int z, f
    return true;
 }
 
-// Queue entry flags (bits 0-10: voxel of the brick)
-constexpr unsigned short kQueueCertain = 1u << 14;    // certainly accepted
-constexpr unsigned short kQueueBundleOnly = 1u << 15; // cannot win; bundle minimum only
-constexpr int kQueueCap = 64;
+// Segments of a brick's list whose index, r^2 and bundle are kept in shared
+// memory (the lists of the uneven tiles hold 30 on average, of a dense volume
+// 180).
+constexpr unsigned kSegCache = 512;
+constexpr int32_t kMarkedLabel = INT32_MIN; // until voxel_marks has resolved it
 
-struct WarpQueue {
-   unsigned slot[kQueueCap];       // position in the brick's segment list
-   unsigned short entry[kQueueCap];
+// The layers of the tile's first bundles, in shared memory.
+struct LayerLut {
+   int n;
+   unsigned models; // two bits per layer: 0 'b', 1 'p', 2 'r'
+   float sq[kMaxLayers]; // sq_fdown
 };
+constexpr int kLayerCache = 4;
 
-// Exact evaluation of one queued candidate (reference arithmetic: two-float
-// fast path, FP64 replay) and its atomics.
-template <bool MULTI>
-__device__ __forceinline__ void brick_eval(const SegDev *__restrict__ segs,
-                                           const unsigned *__restrict__ list,
-                                           const LayerDev *__restrict__ layers, int layer_base,
-                                           unsigned slot, unsigned short e, int ox, int oy, int oz,
-                                           unsigned long long *skey, unsigned *sminb,
-                                           unsigned long long &n_slow) {
-   const unsigned s = list[slot];
-   const SegDev &S = segs[s];
-   const int li = e & (kBrickVoxels - 1);
-   const int x = ox + (li >> 8), y = oy + ((li >> 5) & 7), z = oz + (li & 31);
-   float dist_squ, r_sqr;
-   if (cand_dist(S, x, y, z, dist_squ, r_sqr))
-      n_slow++;
-   if (dist_squ > layers[layer_base + S.bundle].f_ly_squ * r_sqr) // generator.cpp:329-331
-      return;
-   if (!(e & kQueueBundleOnly))
-      atomicMin(&skey[li], ((unsigned long long)__float_as_uint(dist_squ) << 32) |
-                               (unsigned long long)(0xFFFFFFFFu - s));
-   if (MULTI && !(e & kQueueCertain))
-      atomicMin(&sminb[li], (unsigned)S.bundle);
-}
-
-// EXACT pass, filter side: one segment over its sub-box; candidates that can
-// still win (or, for the bundle minimum, might be accepted) go to the warp's
-// queue, which is drained 32 entries at a time by all lanes together.
-template <bool MULTI>
-__device__ __forceinline__ void brick_filter(const SegSweep &sw, unsigned slot, const SubBox &b,
-                                             int ox, int oy, int oz, unsigned long long *skey,
-                                             WarpQueue &q, int &qn, int lane,
-                                             const SegDev *__restrict__ segs,
-                                             const unsigned *__restrict__ list,
-                                             const LayerDev *__restrict__ layers, int layer_base,
-                                             unsigned *sminb, unsigned long long &n_slow) {
-   const SegFP32 g = seg_fp32(sw);
-   const float gx0 = (float)(b.x0 - g.bx) + 0.5f;
-   for (int c0 = 0; c0 < b.ncell; c0 += 32) { // whole warps: the queue is filled by ballot
-      const bool in = c0 + lane < b.ncell;
-      const Cell c = cell_of(b, g, in ? c0 + lane : 0, ox, oy, oz);
-      float gx = gx0;
-      int li = c.li;
-      for (int i = 0; i < b.ex; i++, gx += 1.f, li += kBrickY * kBrickZ) {
-         bool need = false;
-         unsigned short e = 0;
-         if (in) {
-            float lo, hi;
-            candidate_bounds(g, c, gx, lo, hi);
-            if (!(lo > g.thr)) { // inside the outermost layer at the thickest end
-               const bool certain = hi <= g.acc;
-               // keys only decrease, so any value read bounds the final one
-               // from above; the initial ~0 reads as NaN and skips nothing
-               const unsigned long long cur =
-                   *reinterpret_cast<volatile unsigned long long *>(&skey[li]);
-               const bool loser = lo > __uint_as_float((unsigned)(cur >> 32));
-               need = !(loser && (certain || !MULTI));
-               e = (unsigned short)(li | (certain ? kQueueCertain : 0) |
-                                    (loser ? kQueueBundleOnly : 0));
-            }
-         }
-         const unsigned m = __ballot_sync(0xFFFFFFFFu, need);
-         if (need) {
-            const int at = qn + __popc(m & ((1u << lane) - 1u));
-            q.slot[at] = slot;
-            q.entry[at] = e;
-         }
-         qn += __popc(m);
-         if (qn >= 32) { // drain 32 entries with every lane
-            __syncwarp();
-            const int at = qn - 32 + lane;
-            brick_eval<MULTI>(segs, list, layers, layer_base, q.slot[at], q.entry[at], ox, oy,
-                              oz, skey, sminb, n_slow);
-            qn -= 32;
-            __syncwarp();
-         }
-      }
+// Layer of a winner whose dist^2 lies in [lo, hi] with r^2 = r_sqr: the
+// reference's lower_bound over scale^2 of the float dist^2 / r^2
+// (generator.cpp:345-349).  2^-20 covers the rounding of the quotient and of
+// the products here.  -1 when the interval straddles a boundary, the
+// outermost one included.
+__device__ __forceinline__ int certain_layer(const float *sq, int n, float lo, float hi,
+                                             float r_sqr) {
+   int w = 0;
+   bool sure = true;
+   for (int l = 0; l < n; l++) {
+      const float b = sq[l] * r_sqr;
+      const bool past = hi > b * (1.f - 0x1p-20f);
+      w += past ? 1 : 0;
+      sure = sure && (!past || lo > b * (1.f + 0x1p-20f));
    }
-}
-
-// --------------------------------------------------------- winner decode ---
-// Label and orientation of voxel (x, y, z) of a tile from its winner key
-// (generator.cpp:343-372): the layer by lower_bound on the squared layer
-// scales, the vector by the layer's model ('p' segment direction, 'r'
-// radial, 'b' none).
-__device__ __forceinline__ void decode_voxel(unsigned long long key, int x, int y, int z,
-                                             const SegDev *__restrict__ segs,
-                                             const LayerDev *__restrict__ layers,
-                                             int layer_base, int max_layer, unsigned minb,
-                                             int32_t &label_out, float o[3], bool &defer,
-                                             unsigned long long &n_overlap,
-                                             unsigned long long &n_overflow,
-                                             unsigned long long &n_slow) {
-   o[0] = o[1] = o[2] = 0.f;
-   defer = false;
-   if (key == ~0ull) {
-      label_out = 0;
-      return;
-   }
-   const unsigned seg = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
-   const float dist_squ = __uint_as_float((unsigned)(key >> 32));
-   const SegDev &S = segs[seg];
-   const LayerDev &L = layers[layer_base + S.bundle];
-   // With a constant radius whose square rounds the same at every t
-   // (rsq_const) and at both ends, r^2 at the winner is known without
-   // evaluating the candidate again.
-   const bool r_known = S.rsq_const == S.rsq0 && S.rsq_const == S.rsq1; // false for NaN
-   float r_sqr = S.rsq_const;
-   if (!r_known) {
-      float d_chk;
-      if (cand_dist(S, x, y, z, d_chk, r_sqr))
-         n_slow++;
-   }
-   // std::lower_bound(scale^2, double(dist_squ / r_sqr)) (generator.cpp:345-349)
-   const float qv = dist_squ / r_sqr;
-   int ly = 0;
-   while (ly < L.n && qv > L.sq_fdown[ly])
-      ly++;
-   label_out = ly + 1 + S.bundle * max_layer;
-   if (minb < (unsigned)S.bundle)
-      n_overlap++;
-   char m = 'b';
-   if (ly < L.n)
-      m = L.model[ly];
-   else
-      n_overflow++;
-   if (m == 'p') {
-      o[0] = S.vp[0];
-      o[1] = S.vp[1];
-      o[2] = S.vp[2];
-   } else if (m == 'r') { // the caller evaluates it with radial_vector, 32 at a time
-      defer = true;
-   }
+   return sure && w < n ? w : -1;
 }
 
 // The 'r' orientation of voxel (x, y, z) for winner S: unit(point - closest)
@@ -506,156 +481,554 @@ __device__ __forceinline__ void radial_vector(const SegDev &S, int x, int y, int
       n_slow++;
 }
 
+// A brick: its tile and place.
+struct BrickPlace {
+   const TileDev *T;
+   int64_t tile;
+   int ox, oy, oz, nx, ny, nz;
+};
+
+__device__ __forceinline__ BrickPlace brick_place(const TileDev *__restrict__ tiles,
+                                                  int64_t n_tiles, int64_t brick) {
+   // last tile whose brick_base <= brick
+   int64_t lo = 0, hi = n_tiles - 1;
+   while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) >> 1;
+      if (tiles[mid].brick_base <= brick)
+         lo = mid;
+      else
+         hi = mid - 1;
+   }
+   BrickPlace p;
+   p.tile = lo;
+   p.T = tiles + lo;
+   const unsigned lb = (unsigned)(brick - p.T->brick_base); // below 2^32: the lists are 32-bit
+   const unsigned rxy = lb / (unsigned)p.T->nb[2], bx = rxy / (unsigned)p.T->nb[1];
+   p.ox = (int)bx * kBrickX;
+   p.oy = (int)(rxy - bx * (unsigned)p.T->nb[1]) * kBrickY;
+   p.oz = (int)(lb - rxy * (unsigned)p.T->nb[2]) * kBrickZ;
+   p.nx = min(kBrickX, p.T->X - p.ox);
+   p.ny = min(kBrickY, p.T->Y - p.oy);
+   p.nz = min(kBrickZ, p.T->Z - p.oz);
+   return p;
+}
+
+// --------------------------------------------------------- marked voxels ---
+constexpr int kMarkThreads = 128, kMarkQueue = 192;
+constexpr unsigned kScanBrick = 0x80000000u; // directory entry without a record: a brick
+
+// What one warp of voxel_marks works on: up to 32 marked voxels of its brick,
+// and the candidates found for them.
+struct MarkWarp {
+   unsigned long long exact[32]; // winner keys
+   unsigned bound[32];           // float bits of the smallest certain upper bound
+   unsigned minb[32];            // smallest bundle a voxel is inside of
+   unsigned short voxel[32];     // place in the brick
+   unsigned q_seg[kMarkQueue];
+   float q_lo[kMarkQueue];
+   unsigned char q_mark[kMarkQueue]; // voxel; bit 7: certainly inside
+};
+
+struct MarkCtx {
+   BrickPlace p;
+   unsigned n_seg;
+   const unsigned *list;
+   const SegDev *segs;
+   const LayerDev *layers;
+   int32_t *label;
+   float *vec;
+   bool multi; // the overlap warning is still open
+};
+
+// Label and orientation of a marked voxel from its winner's key
+// (generator.cpp:343-372).
+__device__ __forceinline__ void finish_voxel(const MarkCtx &C, unsigned long long key, int x,
+                                             int y, int z, unsigned minb,
+                                             unsigned long long &n_slow,
+                                             unsigned long long &n_overlap,
+                                             unsigned long long &n_overflow) {
+   const int64_t i = ((int64_t)x * C.p.T->Y + y) * C.p.T->Z + z;
+   int32_t lab = 0;
+   float o[3] = {0.f, 0.f, 0.f};
+   if (key != ~0ull) {
+      const SegDev &S = C.segs[0xFFFFFFFFu - (unsigned)key];
+      const LayerDev &L = C.layers[S.bundle];
+      float dist_squ = __uint_as_float((unsigned)(key >> 32)), r_sqr = S.dec_rsq;
+      if (!(r_sqr == r_sqr) && cand_dist(S, x, y, z, dist_squ, r_sqr))
+         n_slow++;
+      // std::lower_bound(scale^2, double(dist_squ / r_sqr)) (generator.cpp:345-349)
+      const float qv = dist_squ / r_sqr;
+      int w = 0;
+      while (w < L.n && qv > L.sq_fdown[w])
+         w++;
+      if (w == L.n)
+         n_overflow++;
+      if (C.multi && minb < (unsigned)S.bundle)
+         n_overlap++;
+      lab = w + 1 + S.bundle * C.p.T->max_layer;
+      const unsigned m = w < L.n ? L.models >> (2 * w) & 3u : 0u;
+      if (m == 1u) {
+         o[0] = S.vp[0];
+         o[1] = S.vp[1];
+         o[2] = S.vp[2];
+      } else if (m == 2u && C.vec) {
+         radial_vector(S, x, y, z, o, n_slow);
+      }
+   }
+   C.label[i] = lab;
+   if (C.vec) {
+      C.vec[3 * i + 0] = o[0];
+      C.vec[3 * i + 1] = o[1];
+      C.vec[3 * i + 2] = o[2];
+   }
+}
+
+// Evaluates the queued candidates that can still win, 32 at a time.
+__device__ __forceinline__ void drain_marks(const MarkCtx &C, MarkWarp &W, int qn, int lane,
+                                            unsigned long long &n_slow) {
+   __syncwarp();
+   int n = 0; // the ones kept, at the front of the queue
+   for (int i = 0; i < qn; i += 32) {
+      unsigned s = 0, m = 0;
+      bool need = false;
+      if (i + lane < qn) {
+         s = W.q_seg[i + lane];
+         m = W.q_mark[i + lane];
+         need = !(W.q_lo[i + lane] > __uint_as_float(W.bound[m & 31u])) ||
+                (C.multi && !(m & 128u) && (unsigned)C.segs[s].bundle < W.minb[m & 31u]);
+      }
+      const unsigned b = __ballot_sync(0xFFFFFFFFu, need);
+      if (need) {
+         const int at = n + __popc(b & ((1u << lane) - 1u));
+         W.q_seg[at] = s;
+         W.q_mark[at] = (unsigned char)m;
+      }
+      n += __popc(b);
+      __syncwarp();
+   }
+   for (int i = lane; i < n; i += 32) {
+      const unsigned s = W.q_seg[i], m = W.q_mark[i] & 31u;
+      const SegDev &S = C.segs[s];
+      const int v = W.voxel[m];
+      float dist_squ, r_sqr;
+      if (cand_dist(S, C.p.ox + (v >> 8), C.p.oy + (v >> 5 & 7), C.p.oz + (v & 31), dist_squ,
+                    r_sqr))
+         n_slow++;
+      if (dist_squ > C.layers[S.bundle].f_ly_squ * r_sqr) // generator.cpp:329-331
+         continue;
+      atomicMin(&W.exact[m], ((unsigned long long)__float_as_uint(dist_squ) << 32) |
+                                 (unsigned long long)(0xFFFFFFFFu - s));
+      atomicMin(&W.bound[m], __float_as_uint(dist_squ));
+      if (C.multi)
+         atomicMin(&W.minb[m], (unsigned)S.bundle);
+   }
+   __syncwarp();
+}
+
+// The nm <= 32 marked voxels W.voxel: a segment of the list per lane, its
+// inputs in registers while the voxels pass by.
+__device__ __forceinline__ void resolve_marks(const MarkCtx &C, MarkWarp &W, int nm, int lane,
+                                              unsigned long long &n_slow,
+                                              unsigned long long &n_overlap,
+                                              unsigned long long &n_overflow) {
+   W.exact[lane] = ~0ull;
+   W.bound[lane] = __float_as_uint(INFINITY);
+   W.minb[lane] = ~0u;
+   __syncwarp();
+   int qn = 0;
+   for (unsigned j = 0; j < C.n_seg; j += 32) {
+      const bool have = j + lane < C.n_seg;
+      const unsigned s = C.list[have ? j + lane : C.n_seg - 1];
+      const SegSweep w = load_sweep(C.segs[s]);
+      for (int m = 0; m < nm; m++) {
+         const int v = W.voxel[m];
+         const int x = C.p.ox + (v >> 8), y = C.p.oy + (v >> 5 & 7), z = C.p.oz + (v & 31);
+         float lo = 0.f;
+         bool in = have && x >= w.d.y && x < w.d.y + w.e.x && y >= w.d.z && y < w.d.z + w.e.y &&
+                   z >= w.d.w && z < w.d.w + w.e.z;
+         bool certain = false;
+         if (in) {
+            float mg;
+            const float d2 = approx_dist2(((float)(x - __float_as_int(w.c.z)) + 0.5f) - w.a.x,
+                                          ((float)(y - __float_as_int(w.c.w)) + 0.5f) - w.a.y,
+                                          ((float)(z - w.d.x) + 0.5f) - w.a.z, w.a.w, w.b.x,
+                                          w.b.y, w.b.z, w.b.w, mg);
+            lo = __fsub_rd(d2, mg);
+            const float hi = __fadd_ru(d2, mg);
+            certain = hi <= w.c.y;
+            in = !(lo > w.c.x);
+            if (certain) {
+               atomicMin(&W.bound[m], __float_as_uint(hi));
+               if (C.multi)
+                  atomicMin(&W.minb[m], (unsigned)w.e.w);
+            }
+         }
+         const unsigned b = __ballot_sync(0xFFFFFFFFu, in);
+         if (!b)
+            continue;
+         if (in) {
+            const int at = qn + __popc(b & ((1u << lane) - 1u));
+            W.q_seg[at] = s;
+            W.q_lo[at] = lo;
+            W.q_mark[at] = (unsigned char)(m | (certain ? 128 : 0));
+         }
+         qn += __popc(b);
+         if (qn > kMarkQueue - 32) {
+            drain_marks(C, W, qn, lane, n_slow);
+            qn = 0;
+         }
+      }
+   }
+   drain_marks(C, W, qn, lane, n_slow);
+   if (lane < nm) {
+      const int v = W.voxel[lane];
+      finish_voxel(C, W.exact[lane], C.p.ox + (v >> 8), C.p.oy + (v >> 5 & 7), C.p.oz + (v & 31),
+                   W.minb[lane], n_slow, n_overlap, n_overflow);
+   }
+   __syncwarp();
+}
+
+// Resolves the marked voxels of the bricks [brick_begin, brick_end), a brick
+// per warp (bound by latency: 16 warps per SM, each a chain of list, segment
+// and evaluation; a voxel per lane walking the list by itself took 260 us on
+// the crossing volume instead of 153, 6 CTAs per SM at 80 registers 166): from its record, or from the labels of a brick without one (every
+// brick when the launch has no space for records).
+__global__ void __launch_bounds__(kMarkThreads)
+voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
+            int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
+            const unsigned *__restrict__ list, unsigned n_pairs,
+            const unsigned *__restrict__ directory, const uint2 *__restrict__ marks,
+            int64_t mark_share, const LayerDev *__restrict__ layers,
+            int32_t *const *__restrict__ labels, float *const *__restrict__ vecs,
+            unsigned long long *__restrict__ counters) {
+   __shared__ MarkWarp s_warps[kMarkThreads / 32];
+   MarkWarp &W = s_warps[threadIdx.x >> 5];
+   const int lane = threadIdx.x & 31;
+   const int64_t warp = (blockIdx.x * (int64_t)kMarkThreads + threadIdx.x) >> 5;
+   const int64_t n_warps = (int64_t)gridDim.x * (kMarkThreads / 32);
+   unsigned long long n_slow = 0, n_overlap = 0, n_overflow = 0;
+   const bool open = *reinterpret_cast<volatile unsigned long long *>(&counters[0]) == 0;
+   const int64_t n = mark_share > 0 ? (int64_t)marks[0].y : brick_end - brick_begin;
+   for (int64_t r = warp; r < n; r += n_warps) {
+      const unsigned at = mark_share > 0 ? directory[r] : kScanBrick;
+      int64_t brick = brick_begin + r;
+      if (mark_share > 0)
+         brick = brick_begin + ((at & kScanBrick) ? at & ~kScanBrick : marks[at].x);
+      const unsigned j1 = min(offsets[brick + 1], n_pairs), j0 = min(offsets[brick], j1);
+      if (j0 == j1)
+         continue;
+      MarkCtx C;
+      C.p = brick_place(tiles, n_tiles, brick);
+      C.n_seg = j1 - j0;
+      C.list = list + j0;
+      C.segs = segs;
+      C.layers = layers + C.p.T->layer_base;
+      C.label = labels[C.p.tile];
+      C.vec = vecs[C.p.tile];
+      C.multi = open && C.p.T->n_bundles > 1;
+      if (!(at & kScanBrick)) {
+         const int total = (int)marks[at].y;
+         const unsigned short *voxel = reinterpret_cast<const unsigned short *>(marks + at + 1);
+         for (int m = 0; m < total; m += 32) {
+            if (m + lane < total)
+               W.voxel[lane] = voxel[m + lane];
+            __syncwarp();
+            resolve_marks(C, W, min(32, total - m), lane, n_slow, n_overlap, n_overflow);
+         }
+         continue;
+      }
+      for (int row = 0; row < C.p.nx * C.p.ny; row++) {
+         const int lx = row / C.p.ny, ly = row - lx * C.p.ny;
+         const int64_t i =
+             ((int64_t)(C.p.ox + lx) * C.p.T->Y + (C.p.oy + ly)) * C.p.T->Z + C.p.oz + lane;
+         const bool on = lane < C.p.nz && C.label[i] == kMarkedLabel;
+         const unsigned b = __ballot_sync(0xFFFFFFFFu, on);
+         if (!b)
+            continue;
+         if (on)
+            W.voxel[__popc(b & ((1u << lane) - 1u))] =
+                (unsigned short)(lx * kPlane + ly * kBrickZ + lane);
+         __syncwarp();
+         resolve_marks(C, W, __popc(b), lane, n_slow, n_overlap, n_overflow);
+      }
+   }
+   if (n_overlap)
+      atomicAdd(&counters[0], n_overlap);
+   if (n_overflow)
+      atomicAdd(&counters[5], n_overflow);
+   if (n_slow)
+      atomicAdd(&counters[9], n_slow);
+}
+
 // ------------------------------------------------------------- the brick ---
-// 4 resident bricks per SM (64 registers, ~130 bytes of spill): 6% faster
-// than 3 on config 2 — the passes are latency-bound and the extra warps hide
-// more of it than the spills cost.
+static_assert(kBrickWarps == kBrickY && kBrickX <= 8, "the decode gives each y a warp");
+
+// Marked voxels of one brick that get a record; with more of them the labels
+// are as good.
+constexpr unsigned kMarkList = 128;
+
+// Radial orientations a warp has still to compute.
+struct RadialQueue {
+   unsigned seg[64];
+   unsigned short entry[64]; // voxel of the brick
+};
+
+// One CTA per brick, 256 threads: 8 warps share the brick's segments in the
+// sweep, then each owns the voxels of one y.  4 CTAs per SM (64 registers).
+// Bound by instruction issue (66-75% of the slots): per (segment, brick) pair
+// about 110 warp instructions of setup and 19 per 32 x-steps of the sweep,
+// then the decode of every voxel and a two-float unit vector per 'r' voxel.
+// With the marked voxels in a kernel of their own (voxel_marks) against two
+// sweeps with an exact evaluation of 0.9 candidates per voxel in this one:
+// 397 x 283 x 77 with 15,013 segments 523 -> 219 + 45 us, crossing
+// 512 x 512 x 120 2,216 -> 929 + 153 us, Watson 1024 x 1024 x 240 44.3 -> 24 ms
+// in all; the marked voxels resolved here instead (a list, a queue and two
+// barriers per brick): 330 and 1,290 us.
 template <bool MULTI>
 __global__ void __launch_bounds__(kBrickThreads, 4)
 voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
              int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
-             const unsigned *__restrict__ list, unsigned n_pairs,
-             const LayerDev *__restrict__ layers,
+             const unsigned *__restrict__ list, unsigned n_pairs, unsigned *__restrict__ directory,
+             uint2 *__restrict__ marks, int64_t mark_share, const LayerDev *__restrict__ layers,
              int32_t *const *__restrict__ labels, float *const *__restrict__ vecs,
              unsigned long long *__restrict__ counters) {
-   __shared__ unsigned long long skey[kBrickVoxels];
-   __shared__ unsigned sub[kBrickVoxels]; // BOUND pass: upper bound of the winner's dist^2
+   __shared__ unsigned skey[kBrickVoxels + kSweepStep * kPlane];
+   __shared__ unsigned smark[MULTI ? kPlane / 4 : 1]; // a byte per (y, z), a bit per x
+   // the first segments of the list: index, dec_rsq, bundle
+   __shared__ unsigned s_seg[kSegCache];
+   __shared__ float s_rsq[kSegCache];
+   __shared__ int s_bundle[MULTI ? kSegCache : 1];
    __shared__ unsigned sminb[MULTI ? kBrickVoxels : 1];
-   __shared__ WarpQueue queues[kBrickWarps];
-   __shared__ unsigned s_next[2]; // next segment of the brick's list, per pass
+   __shared__ LayerLut s_layers[MULTI ? kLayerCache : 1];
+   __shared__ RadialQueue queues[kBrickWarps];
+   __shared__ unsigned short s_list[kMarkList];
+   __shared__ unsigned s_next, s_thr, s_mg, s_marked;
+   __shared__ bool s_multi;
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   unsigned long long n_slow = 0, n_overlap = 0, n_overflow = 0;
+   unsigned long long n_slow = 0, n_overlap = 0;
 
    for (int64_t brick = brick_begin + blockIdx.x; brick < brick_end; brick += gridDim.x) {
-      // tile of the brick: last tile whose brick_base <= brick
-      int64_t lo = 0, hi = n_tiles - 1;
-      while (lo < hi) {
-         const int64_t mid = (lo + hi + 1) >> 1;
-         if (tiles[mid].brick_base <= brick)
-            lo = mid;
-         else
-            hi = mid - 1;
+      const BrickPlace p = brick_place(tiles, n_tiles, brick);
+      const int ox = p.ox, oy = p.oy, oz = p.oz, nx = p.nx, ny = p.ny, nz = p.nz;
+      const int Y = p.T->Y, Z = p.T->Z, layer_base = p.T->layer_base;
+      const int max_layer = p.T->max_layer, n_bundles = p.T->n_bundles;
+      int32_t *label = labels[p.tile];
+      float *vec = vecs[p.tile];
+      // (clamped to the planned list size: every slot below it is written)
+      const unsigned j1 = min(offsets[brick + 1], n_pairs), j0 = min(offsets[brick], j1);
+
+      if (j0 == j1) { // no segment: background
+         if (warp < ny)
+            for (int lx = 0; lx < nx; lx++) {
+               const int64_t i0 = ((int64_t)(ox + lx) * Y + (oy + warp)) * Z + oz;
+               if (lane < nz)
+                  label[i0 + lane] = 0;
+               if (vec)
+                  for (int e = lane; e < 3 * nz; e += 32)
+                     vec[3 * i0 + e] = 0.f;
+            }
+         continue;
       }
-      const TileDev &T = tiles[lo];
-      const int X = T.X, Y = T.Y, Z = T.Z;
-      const int64_t lb = brick - T.brick_base;
-      const int bz = (int)(lb % T.nb[2]);
-      const int64_t rxy = lb / T.nb[2];
-      const int by = (int)(rxy % T.nb[1]), bx = (int)(rxy / T.nb[1]);
-      const int ox = bx * kBrickX, oy = by * kBrickY, oz = bz * kBrickZ;
-      const int nx = min(kBrickX, X - ox), ny = min(kBrickY, Y - oy), nz = min(kBrickZ, Z - oz);
-      const int layer_base = T.layer_base, max_layer = T.max_layer;
 
       for (int i = threadIdx.x; i < kBrickVoxels; i += kBrickThreads) {
-         sub[i] = ~0u;
+         skey[i] = kNoKey;
          if (MULTI)
             sminb[i] = ~0u;
       }
-      // (clamped to the planned list size: every slot below it is written)
-      const unsigned j1 = min(offsets[brick + 1], n_pairs), j0 = min(offsets[brick], j1);
-      if (threadIdx.x < 2)
-         s_next[threadIdx.x] = 0;
+      if (MULTI && threadIdx.x < kPlane / 4)
+         smark[threadIdx.x] = 0;
+      {
+         const int b = threadIdx.x / kMaxLayers, l = threadIdx.x % kMaxLayers;
+         if (b < (MULTI ? min(kLayerCache, n_bundles) : 1)) {
+            const LayerDev &L = layers[layer_base + b];
+            s_layers[b].sq[l] = L.sq_fdown[l];
+            if (l == 0) {
+               s_layers[b].n = L.n;
+               s_layers[b].models = L.models;
+            }
+         }
+      }
+      if (threadIdx.x == 0) {
+         s_next = s_thr = s_mg = s_marked = 0;
+         // the overlap warning is one bit for the whole volume: once some
+         // brick has raised it, the bundle minima are of no more use
+         s_multi = MULTI && n_bundles > 1 &&
+                   *reinterpret_cast<volatile unsigned long long *>(&counters[0]) == 0;
+      }
       __syncthreads();
-      // BOUND pass: warps take segments from a shared counter
+      { // the largest bounds of the list's segments (floats >= 0: bits order like values)
+         unsigned th = 0, mg = 0;
+         for (unsigned j = threadIdx.x; j < j1 - j0; j += kBrickThreads) {
+            const unsigned s = list[j0 + j];
+            const SegDev &S = segs[s];
+            const float m = __ldg(&S.mg);
+            if (j < kSegCache) {
+               s_seg[j] = s;
+               s_rsq[j] = __ldg(&S.dec_rsq);
+               if (MULTI)
+                  s_bundle[j] = __ldg(&S.bundle);
+            }
+            th = max(th, __float_as_uint(fmaf(2.0001f, m, __ldg(&S.thr_f))));
+            mg = max(mg, __float_as_uint(m));
+         }
+#pragma unroll
+         for (int o = 16; o > 0; o >>= 1) {
+            th = max(th, __shfl_xor_sync(0xFFFFFFFFu, th, o));
+            mg = max(mg, __shfl_xor_sync(0xFFFFFFFFu, mg, o));
+         }
+         if (lane == 0 && th) {
+            atomicMax(&s_thr, th);
+            atomicMax(&s_mg, mg);
+         }
+      }
+      __syncthreads();
+      const BrickScale k = brick_scale(j1 - j0, __uint_as_float(s_thr), __uint_as_float(s_mg));
+      const bool multi = MULTI && s_multi;
+      // sweep: warps take segments from a shared counter
       for (;;) {
          unsigned j = 0;
          if (lane == 0)
-            j = atomicAdd(&s_next[0], 1u);
-         j = __shfl_sync(0xFFFFFFFFu, j, 0) + j0;
-         if (j >= j1)
+            j = atomicAdd(&s_next, 1u);
+         j = __shfl_sync(0xFFFFFFFFu, j, 0);
+         if (j >= j1 - j0)
             break;
-         const SegSweep sw = load_sweep(segs[list[j]]);
+         const SegSweep sw = load_sweep(segs[j < kSegCache ? s_seg[j] : list[j0 + j]]);
          SubBox b;
          if (sub_box(sw, ox, oy, oz, nx, ny, nz, b))
-            brick_bound<MULTI>(sw, b, ox, oy, oz, sub, sminb, lane);
+            brick_sweep<MULTI>(sw, j, b, ox, oy, oz, k, multi, skey, smark, sminb, lane);
       }
       __syncthreads();
-      // the bounds become the keys ub << 32 | 0xFFFFFFFF the EXACT pass
-      // filters against and lowers (no bound: ~0, which reads as NaN)
-      for (int i = threadIdx.x; i < kBrickVoxels; i += kBrickThreads)
-         skey[i] = sub[i] == ~0u ? ~0ull : ((unsigned long long)sub[i] << 32) | 0xFFFFFFFFull;
-      __syncthreads();
-      // EXACT pass: warps take segments from a shared counter again
-      {
-         WarpQueue &q = queues[warp];
-         int qn = 0;
-         for (;;) {
-            unsigned j = 0;
-            if (lane == 0)
-               j = atomicAdd(&s_next[1], 1u);
-            j = __shfl_sync(0xFFFFFFFFu, j, 0) + j0;
-            if (j >= j1)
-               break;
-            const SegSweep sw = load_sweep(segs[list[j]]);
-            SubBox b;
-            if (sub_box(sw, ox, oy, oz, nx, ny, nz, b))
-               brick_filter<MULTI>(sw, j, b, ox, oy, oz, skey, q, qn, lane, segs, list, layers,
-                                   layer_base, sminb, n_slow);
-         }
-         __syncwarp();
-         if (lane < qn)
-            brick_eval<MULTI>(segs, list, layers, layer_base, q.slot[lane], q.entry[lane], ox, oy,
-                              oz, skey, sminb, n_slow);
-      }
-      __syncthreads();
-      // one warp per (x, y) row of the brick, lane = z: coalesced stores.
-      // Radial ('r') orientations of winners whose candidate the decode did
-      // not evaluate go to the warp's queue and are computed 32 at a time
-      // (a warp's row mixes 'b' and 'r' voxels: in place, half the lanes
+      // decode: a warp per y, lane = z, along x: coalesced stores.  Radial
+      // ('r') orientations go to the warp's queue and are computed 32 at a
+      // time (a warp's row mixes 'b' and 'r' voxels: in place, half the lanes
       // would idle through the two-float unit vector).
-      int32_t *label = labels[lo];
-      float *vec = vecs[lo];
-      WarpQueue &rq = queues[warp];
+      RadialQueue &rq = queues[warp];
+      const LayerDev *tile_layers = layers + layer_base;
       int qn = 0;
-      auto radial = [&](unsigned short li) {
+      auto radial = [&](int at) {
+         const int li = rq.entry[at];
          const int rx = ox + (li >> 8), ry = oy + ((li >> 5) & 7), rz = oz + (li & 31);
-         const unsigned seg = 0xFFFFFFFFu - (unsigned)(skey[li] & 0xFFFFFFFFull);
          float o[3];
-         radial_vector(segs[seg], rx, ry, rz, o, n_slow);
+         radial_vector(segs[rq.seg[at]], rx, ry, rz, o, n_slow);
          const int64_t i = ((int64_t)rx * Y + ry) * Z + rz;
          vec[3 * i + 0] = o[0];
          vec[3 * i + 1] = o[1];
          vec[3 * i + 2] = o[2];
       };
-      for (int r = warp; r < nx * ny; r += kBrickWarps) {
-         const int lx = r / ny, ly = r - (r / ny) * ny;
-         const int li = (lx * kBrickY + ly) * kBrickZ + lane;
+      const int yz = threadIdx.x; // warp * 32 + lane
+      const unsigned sticky = MULTI ? reinterpret_cast<const uint8_t *>(smark)[yz] : 0u;
+      const int y = oy + warp, z = oz + lane;
+      int64_t i = ((int64_t)ox * Y + y) * Z + z;
+      for (int lx = 0; lx < (warp < ny ? nx : 0); lx++, i += (int64_t)Y * Z) {
+         const int li = lx * kPlane + yz;
          bool defer = false;
+         unsigned seg = 0;
+         int32_t lab = 0;
          if (lane < nz) {
-            const int x = ox + lx, y = oy + ly, z = oz + lane;
-            int32_t lab;
-            float o[3];
-            decode_voxel(skey[li], x, y, z, segs, layers, layer_base, max_layer,
-                         MULTI ? sminb[li] : ~0u, lab, o, defer, n_overlap, n_overflow, n_slow);
-            const int64_t i = ((int64_t)x * Y + y) * Z + z;
+            const unsigned key = skey[li];
+            float o0 = 0.f, o1 = 0.f, o2 = 0.f;
+            if (key != kNoKey || (MULTI && (sticky >> lx & 1u))) {
+               const unsigned slot = (key & (k.mul - 1u)) >> 1;
+               int w = -1, bundle = 0;
+               if (!(key & 1u) && !(MULTI && (sticky >> lx & 1u))) { // not marked
+                  float rsq;
+                  if (slot < kSegCache) {
+                     seg = s_seg[slot];
+                     rsq = s_rsq[slot];
+                     bundle = MULTI ? s_bundle[slot] : 0;
+                  } else {
+                     seg = list[j0 + slot];
+                     rsq = segs[seg].dec_rsq;
+                     bundle = MULTI ? segs[seg].bundle : 0;
+                  }
+                  // 4e-6: the rounding of the quantum and of the product
+                  const float up = key_bound(k, key);
+                  float lo = up * (1.f - 4e-6f) - 2.f * k.quantum - k.mg2, hi = up;
+                  if (!(rsq == rsq)) { // the radius changes: evaluate
+                     float dist_squ;
+                     if (cand_dist(segs[seg], ox + lx, y, z, dist_squ, rsq))
+                        n_slow++;
+                     lo = hi = dist_squ;
+                     if (dist_squ > tile_layers[bundle].f_ly_squ * rsq)
+                        hi = INFINITY; // outside (generator.cpp:329-331): no layer is certain
+                  }
+                  if (!MULTI || bundle < kLayerCache)
+                     w = certain_layer(s_layers[MULTI ? bundle : 0].sq,
+                                       s_layers[MULTI ? bundle : 0].n, lo, hi, rsq);
+                  else
+                     w = certain_layer(tile_layers[bundle].sq_fdown, tile_layers[bundle].n, lo,
+                                       hi, rsq);
+               }
+               if (w >= 0) {
+                  lab = w + 1 + bundle * max_layer;
+                  if (MULTI && multi && sminb[li] < (unsigned)bundle)
+                     n_overlap++;
+                  const unsigned models = !MULTI || bundle < kLayerCache
+                                              ? s_layers[MULTI ? bundle : 0].models
+                                              : tile_layers[bundle].models;
+                  const unsigned m = models >> (2 * w) & 3u;
+                  if (m == 1u) {
+                     o0 = segs[seg].vp[0];
+                     o1 = segs[seg].vp[1];
+                     o2 = segs[seg].vp[2];
+                  }
+                  defer = m == 2u && vec;
+               } else {
+                  lab = kMarkedLabel;
+               }
+            }
             label[i] = lab;
-            defer = defer && vec;
             if (vec && !defer) {
-               vec[3 * i + 0] = o[0];
-               vec[3 * i + 1] = o[1];
-               vec[3 * i + 2] = o[2];
+               vec[3 * i + 0] = o0;
+               vec[3 * i + 1] = o1;
+               vec[3 * i + 2] = o2;
             }
          }
+         if (lab == kMarkedLabel) {
+            const unsigned at = atomicAdd(&s_marked, 1u);
+            if (at < kMarkList)
+               s_list[at] = (unsigned short)li;
+         }
          const unsigned m = __ballot_sync(0xFFFFFFFFu, defer);
-         if (defer)
-            rq.entry[qn + __popc(m & ((1u << lane) - 1u))] = (unsigned short)li;
+         if (defer) {
+            const int at = qn + __popc(m & ((1u << lane) - 1u));
+            rq.entry[at] = (unsigned short)li;
+            rq.seg[at] = seg;
+         }
          qn += __popc(m);
          if (qn >= 32) {
             __syncwarp();
-            radial(rq.entry[qn - 32 + lane]);
+            radial(qn - 32 + lane);
             qn -= 32;
             __syncwarp();
          }
       }
       __syncwarp();
       if (lane < qn)
-         radial(rq.entry[lane]);
-      __syncthreads(); // shared keys are re-initialised for the next brick
+         radial(lane);
+      __syncthreads();
+      if (warp == 0 && s_marked && mark_share > 0) { // the brick's record
+         const unsigned n = s_marked, place = (unsigned)(brick - brick_begin);
+         unsigned long long got = 0; // {entries taken, records}
+         if (lane == 0) // (a record that does not fit takes no entries)
+            got = atomicAdd(reinterpret_cast<unsigned long long *>(marks),
+                            (1ull << 32) | (n <= kMarkList ? 1u + (n + 3u) / 4u : 0u));
+         got = __shfl_sync(0xFFFFFFFFu, got, 0);
+         const uint64_t at = 1u + (unsigned)got;
+         const bool fits = n <= kMarkList && at + 1 + (n + 3) / 4 <= (uint64_t)mark_share;
+         if (lane == 0) {
+            directory[got >> 32] = fits ? (unsigned)at : kScanBrick | place;
+            if (fits)
+               marks[at] = make_uint2(place, n);
+         }
+         if (fits)
+            for (unsigned e = lane; e < n; e += 32)
+               reinterpret_cast<unsigned short *>(marks + at + 1)[e] = s_list[e];
+      }
+      __syncthreads();
    }
    if (n_overlap)
       atomicAdd(&counters[0], n_overlap);
-   if (n_overflow)
-      atomicAdd(&counters[5], n_overflow);
    if (n_slow)
       atomicAdd(&counters[9], n_slow);
 }
@@ -682,6 +1055,11 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
    auto *counts = reinterpret_cast<unsigned *>(w);
    w += align_up(sizeof(unsigned) * std::max<int64_t>(n_bricks, 1), 256);
    auto *list = reinterpret_cast<unsigned *>(w);
+   w += align_up(sizeof(unsigned) * std::max<int64_t>(n_pairs, 1), 256);
+   auto *marks = reinterpret_cast<uint2 *>(w);
+   const int n_launch = chunks ? chunks->n : 1;
+   // entries of one launch (entry 0 counts)
+   const int64_t mark_share = n_launch <= 1024 ? mark_entries(n_segs) / n_launch : 0;
 
    FPGB_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(unsigned) * n_bricks, st));
    if (n_segs > 0) {
@@ -690,7 +1068,8 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
                                           nullptr, n_pairs, counters);
       FPGB_CUDA_TRY(cudaGetLastError());
    }
-   brick_scan<<<1, 1024, 0, st>>>(counts, n_bricks, offsets, counters);
+   brick_scan<<<1, 1024, 0, st>>>(counts, n_bricks, offsets, marks, mark_share, n_launch,
+                                  counters);
    FPGB_CUDA_TRY(cudaGetLastError());
    if (n_segs > 0) {
       FPGB_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(unsigned) * n_bricks, st));
@@ -699,7 +1078,6 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
                                          n_pairs, counters);
       FPGB_CUDA_TRY(cudaGetLastError());
    }
-   const int n_launch = chunks ? chunks->n : 1;
    cudaStream_t alt = chunks && chunks->n > 1 ? chunks->alt : nullptr;
    cudaEvent_t joined[2] = {};
    auto launch_all = [&]() -> int {
@@ -714,14 +1092,19 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
          cudaStream_t s = (alt && (c & 1)) ? alt : st;
          if (b1 > b0) {
             const unsigned grid = (unsigned)std::min<int64_t>(b1 - b0, 0x7FFFFFFF);
-            if (multi_bundle)
-               voxel_bricks<true><<<grid, kBrickThreads, 0, s>>>(segs, tiles, n_tiles, b0, b1,
-                                                                offsets, list, (unsigned)n_pairs,
-                                                                layers, labels, vecs, counters);
-            else
-               voxel_bricks<false><<<grid, kBrickThreads, 0, s>>>(segs, tiles, n_tiles, b0, b1,
-                                                                 offsets, list, (unsigned)n_pairs,
-                                                                 layers, labels, vecs, counters);
+            // a warp per brick, up to about two waves
+            const unsigned mark_grid = (unsigned)std::min<int64_t>(
+                (b1 - b0 + kMarkThreads / 32 - 1) / (kMarkThreads / 32), 152 * 8);
+            uint2 *share = marks + c * mark_share;
+            auto kernel = multi_bundle ? voxel_bricks<true> : voxel_bricks<false>;
+            kernel<<<grid, kBrickThreads, 0, s>>>(segs, tiles, n_tiles, b0, b1, offsets, list,
+                                                  (unsigned)n_pairs, counts + b0, share,
+                                                  mark_share, layers, labels, vecs, counters);
+            FPGB_CUDA_TRY(cudaGetLastError());
+            // (the fill's cursors have become the directory of the records)
+            voxel_marks<<<mark_grid, kMarkThreads, 0, s>>>(
+                segs, tiles, n_tiles, b0, b1, offsets, list, (unsigned)n_pairs, counts + b0,
+                share, mark_share, layers, labels, vecs, counters);
             FPGB_CUDA_TRY(cudaGetLastError());
          }
          if (chunks && chunks->after)

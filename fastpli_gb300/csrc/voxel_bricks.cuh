@@ -4,11 +4,10 @@
 // The volume (or every tile of a batch) is cut into bricks of
 // kBrickX x kBrickY x kBrickZ voxels.  Each segment is binned to the bricks
 // its clipped box overlaps (count, scan, fill on the device); one CTA then
-// owns one brick: it keeps the brick's 64-bit winner keys
-// (float_bits(dist^2) << 32 | (0xFFFFFFFF - segment), see below) and, for
-// multi-bundle volumes, the per-voxel bundle minimum in shared memory, runs
-// both key passes over the brick's segments, and finally decodes every
-// voxel's winner into label and orientation, written once to HBM.
+// owns one brick: it keeps the voxels' winner keys and, for multi-bundle
+// volumes, the per-voxel bundle minimum in shared memory, sweeps the brick's
+// segments over them, and finally decodes every voxel's winner into label
+// and orientation, written once to HBM.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,7 +30,9 @@ struct TileDev {
    int32_t X, Y, Z;
    int32_t max_layer;
    int32_t layer_base; // first LayerDev of the tile
+   int32_t n_bundles;  // LayerDevs of the tile (at least 1)
    int32_t nb[3];      // bricks along x, y, z
+   int32_t pad_;
 };
 
 // Bricks of an X x Y x Z volume along each axis and in total.
@@ -40,8 +41,9 @@ void tile_bricks(int64_t X, int64_t Y, int64_t Z, int32_t nb[3], int64_t *n_bric
 // Number of (segment, brick) pairs of one segment (its clipped box).
 int64_t segment_brick_pairs(const SegDev &S);
 
-// Device scratch of the voxelizer for n_bricks bricks and n_pairs pairs.
-size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs);
+// Device scratch of the voxelizer for n_bricks bricks, n_pairs pairs and
+// n_segs segments.
+size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs, int64_t n_segs);
 
 // Brick ranges to voxelize as separate launches, in order: launch c covers
 // bricks [bound[c], bound[c + 1]), and after(ctx, c, s) runs on the host once
@@ -62,7 +64,7 @@ struct BrickChunks {
 // Bins the segments to bricks and voxelizes every tile.  labels[t] / vecs[t]
 // are the tile's output arrays (vecs[t] may be null: labels only).
 // seg_tile may be null when there is one tile.  `ws` holds
-// brick_workspace_bytes(n_bricks, n_pairs) bytes, 256-byte aligned.
+// brick_workspace_bytes(n_bricks, n_pairs, n_segs) bytes, 256-byte aligned.
 // `chunks` may be null: one launch over every brick.
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
