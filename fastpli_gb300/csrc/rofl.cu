@@ -50,13 +50,45 @@ struct RoflParams {
    double incl[6], trel[6];    // start grid
 };
 
-// numpy.remainder for b > 0: result in [0, b)
+// numpy.remainder for b > 0: result in [0, b).  Within two periods of 0 the
+// truncated remainder is the argument or one exact subtraction away (Sterbenz),
+// which is what fmod's digit loop gives.
 __device__ __forceinline__ double pymod(double a, double b) {
-   double m = fmod(a, b);
+   const double x = fabs(a);
+   double m;
+   if (x < b)
+      m = a;
+   else if (x < 2.0 * b)
+      m = a < 0.0 ? a + b : a - b;
+   else
+      m = fmod(a, b); // (NaN too)
    if (m != 0.0 && m < 0.0)
       m += b;
    return m == 0.0 ? 0.0 : m;
 }
+
+// Many quotients by one divisor, each rounded once: with y = 1 / b rounded,
+// q = a y is within 2 ulps of a / b, one residual correction makes it faithful
+// and a second one correct (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  Outside of
+// the range where every step is free of under- and overflow, and for zeros,
+// the division itself.
+struct Divisor {
+   double b, y;
+   bool safe;
+   __device__ __forceinline__ explicit Divisor(double d) : b(d), y(1.0 / d) {
+      const double m = fabs(d);
+      safe = m > 0x1p-300 && m < 0x1p300;
+   }
+   __device__ __forceinline__ double quotient(double a) const {
+      const double m = fabs(a);
+      if (!(safe && m > 0x1p-300 && m < 0x1p300))
+         return a / b;
+      double q = a * y;
+      q = fma(fma(-b, q, a), y, q);
+      return fma(fma(-b, q, a), y, q);
+   }
+};
 
 // CUDA's FP64 sin, cos, sincos, atan and asin called out of line: one copy
 // of each in the kernel's code instead of one per call site (the fit is
@@ -70,7 +102,15 @@ __device__ __noinline__ double ol_asin(double x) { return asin(x); }
 
 // _symmetrize_angles (_ROFL_with_jacobi.py:64-74)
 __device__ __forceinline__ void symmetrize(double &dir, double &incl) {
-   const double s = -pymod(floor(dir / M_PI), 2.0) + 0.5; // +-0.5
+   // floor(dir / pi) is 0 or -1 without the division, away from its steps
+   double turns;
+   if (dir >= 0.0 && dir < 3.14159265)
+      turns = 0.0;
+   else if (dir < -1e-300 && dir > -3.14159265)
+      turns = -1.0;
+   else
+      turns = floor(dir / M_PI);
+   const double s = -pymod(turns, 2.0) + 0.5; // +-0.5
    incl = (pymod(incl + M_PI / 2.0, M_PI) - M_PI / 2.0) * (s > 0.0 ? 1.0 : -1.0);
    dir = pymod(dir, M_PI);
 }
@@ -116,25 +156,47 @@ __device__ __forceinline__ void tilted(const RoflParams &P, double phi, double a
    }
 }
 
-// weighted residuals r[i] = w[i] (model_i - c[i]) (_residuum, :407-410) of
-// the 5 R measurements, i = tilt * R + rotation (the order of the
-// reference's flattened intensity curves, :186-212).  Out of line, like the
-// Jacobian and the trust-region step below: one copy of each large body
-// keeps the kernel's code in the instruction cache while the threads of a
+// The model's factors at one point of the fit: wave[i] = sin 2 (rho - phi) of
+// every measurement, i = tilt * R + rotation (the order of the reference's
+// flattened intensity curves, :186-212), and cos^2 of each tilt's inclination.
+// t_rel enters neither, so the 6 start points of one inclination and the
+// forward difference in t_rel share them.  base (or null): the waves of a
+// point with the same phi, whose untilted ones are the same.  Out of line,
+// like the Jacobian and the trust-region step below: one copy of each large
+// body keeps the kernel's code in the instruction cache while the threads of a
 // warp are in different phases of their fits.
-__device__ __noinline__ void px_residuals(const RoflParams &P, const double *c,
-                                             const double *w, double phi, double alpha,
-                                             double trel, double *r) {
+__device__ __noinline__ void px_waves(const RoflParams &P, double phi, double alpha,
+                                      const double *base, double *wave, double cos2[5]) {
    Tilted T;
-   tilted(P, phi, alpha, trel, T);
+   tilted(P, phi, alpha, 0.0, T);
    const int R = P.n_rot;
-#pragma unroll
+#pragma unroll 1
    for (int j = 0; j < 5; j++) {
       const double ca = ol_cos(T.alpha[j]);
-      const double amp = ol_sin(M_PI / 2.0 * T.trel[j] * (ca * ca));
+      cos2[j] = ca * ca;
+      const int i0 = j * R;
+      if (j == 0 && base) {
+         for (int k = 0; k < R; k++)
+            wave[k] = base[k];
+         continue;
+      }
+      for (int k = 0; k < R; k++)
+         wave[i0 + k] = ol_sin(2.0 * (P.rho[k] - T.phi[j]));
+   }
+}
+
+// weighted residuals r[i] = w[i] (model_i - c[i]) (_residuum, :407-410)
+__device__ __noinline__ void px_residuals(const RoflParams &P, const double *c, const double *w,
+                                          const double *wave, const double cos2[5], double trel,
+                                          double *r) {
+   const int R = P.n_rot;
+   const double t0 = fabs(trel), t1 = fabs(trel / P.cos_tau); // |t_rel| seen in the tilts
+#pragma unroll 1
+   for (int j = 0; j < 5; j++) {
+      const double amp = ol_sin(M_PI / 2.0 * (j == 0 ? t0 : t1) * cos2[j]);
       const int i0 = j * R;
       for (int k = 0; k < R; k++)
-         r[i0 + k] = w[i0 + k] * (amp * ol_sin(2.0 * (P.rho[k] - T.phi[j])) - c[i0 + k]);
+         r[i0 + k] = w[i0 + k] * (amp * wave[i0 + k] - c[i0 + k]);
    }
 }
 
@@ -420,16 +482,19 @@ __device__ __noinline__ void mp_lmpar(double r[3][3], const int ipvt[3], const d
 
 // The fit for one pixel (one thread): x in: the start point, out: the last
 // accepted point; F (2 x MAXM) holds the residuals, *cur the half that
-// holds them at x on return; J (3 x MAXM) is the Jacobian's workspace.
+// holds them at x on return, S (2 x MAXM) the model's waves likewise; J
+// (3 x MAXM) is the Jacobian's workspace.
 // Returns MINPACK's info (5: evaluation budget spent); nfev counts as
 // MINPACK counts (lmdif: 1 + 3 per Jacobian + 1 per trial step; lmder:
 // 1 + 1 per trial step).
 template <int MAXM>
 __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int M, double x[3],
-                      double *F, int &cur, double *J, int &nfev) {
+                      double *F, int &cur, double *J, double *S, int &nfev) {
    const double epsfd = sqrt(kMpEps); // sqrt(max(epsfcn, epsmch)), epsfcn = eps
+   double cos2[10], cos2p[5]; // of both points, as F and S
    cur = 0;
-   px_residuals(P, c, w, x[0], x[1], x[2], F);
+   px_waves(P, x[0], x[1], nullptr, S, cos2);
+   px_residuals(P, c, w, S, cos2, x[2], F);
    nfev = 1;
    double fnorm = sqrt(seq_sumsq(F, M));
    double par = 0.0, delta = 0.0, xnorm = 0.0;
@@ -448,12 +513,19 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
             double h = epsfd * fabs(temp);
             if (h == 0.0)
                h = epsfd;
-            double xp[3] = {x[0], x[1], x[2]};
-            xp[j] = temp + h;
             double *Jj = J + col[j];
-            px_residuals(P, c, w, xp[0], xp[1], xp[2], Jj);
+            const double *Sc = S + cur * MAXM, *wave = Sc, *cc = cos2 + 5 * cur;
+            if (j < 2) { // (the waves take column 2's place, not yet filled)
+               double *Sp = J + col[2];
+               px_waves(P, j == 0 ? temp + h : x[0], j == 1 ? temp + h : x[1],
+                        j == 1 ? Sc : nullptr, Sp, cos2p);
+               wave = Sp;
+               cc = cos2p;
+            }
+            px_residuals(P, c, w, wave, cc, j == 2 ? temp + h : x[2], Jj);
+            const Divisor by_h(h);
             for (int i = 0; i < M; i++)
-               Jj[i] = (Jj[i] - fv[i]) / h;
+               Jj[i] = by_h.quotient(Jj[i] - fv[i]);
          }
          nfev += 3;
       }
@@ -489,8 +561,9 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
          if (ajnorm != 0.0) {
             if (aj[j] < 0.0)
                ajnorm = -ajnorm;
+            const Divisor by_norm(ajnorm);
             for (int i = j; i < M; i++)
-               aj[i] = aj[i] / ajnorm;
+               aj[i] = by_norm.quotient(aj[i]);
             aj[j] = aj[j] + 1.0;
 #pragma unroll
             for (int k = j + 1; k < 3; k++) {
@@ -584,7 +657,11 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
          const double pnorm = mp_norm3(w3);
          if (iter == 1)
             delta = fmin(delta, pnorm);
-         px_residuals(P, c, w, w2[0], w2[1], w2[2], wa4);
+         {
+            double *Sn = S + (1 - cur) * MAXM, *cn = cos2 + 5 * (1 - cur);
+            px_waves(P, w2[0], w2[1], nullptr, Sn, cn);
+            px_residuals(P, c, w, Sn, cn, w2[2], wa4);
+         }
          nfev++;
          const double fnorm1 = sqrt(seq_sumsq(wa4, M));
          double actred = -1.0;
@@ -653,17 +730,20 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
 
 // One thread per pixel.  MAXR bounds n_rot: the measurement arrays of the
 // pixel (7 x 5 MAXR doubles) live in the thread's local memory, which is
-// interleaved across the threads of a warp and cached in L1.  Held to 80
-// registers (6 CTAs per SM, some values spilled to L1): on 512 x 512 pixels
-// of 5 x 9 measurements 319 ms, against 334 ms at 96 registers (5 CTAs),
-// 361 ms at 128 (4 CTAs) and 462 ms at 168 (3 CTAs).
+// interleaved across the threads of a warp and cached in L1.  One warp per
+// CTA: an SM issues one FP64 warp instruction per 19 cycles, whatever its warps,
+// and a lone warp one per 64, so a map of a few warps per SM ends with its
+// fullest SM (160 x 150 pixels: 188 CTAs of 4 warps gave 36 SMs twice the
+// work).  80 registers (24 warps per SM).
+constexpr int kRoflThreads = 32;
+
 template <int MAXR>
-__global__ void __launch_bounds__(128, 6)
+__global__ void __launch_bounds__(kRoflThreads, 24)
 rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__restrict__ mask,
          const RoflParams P, double *__restrict__ out, unsigned long long *__restrict__ status) {
    constexpr int MAXM = 5 * MAXR;
    const int R = P.n_rot, M = 5 * R;
-   double c[MAXM], w[MAXM], F[2 * MAXM], J[3 * MAXM];
+   double c[MAXM], w[MAXM], F[2 * MAXM], J[3 * MAXM], S[2 * MAXM];
    // pixels are taken one at a time from a counter (status[1]): a thread
    // whose fit ended early starts the next pixel instead of idling until
    // the slowest pixel of a fixed share is done
@@ -697,11 +777,12 @@ rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__
 #pragma unroll
       for (int t = 0; t < 5; t++) {
          const double *d = data + (t * n_pix + p) * R;
-         const double tr = trans[t], tr2 = tr * tr, tr3r = cube_rn(tr) * R;
+         const double tr = trans[t];
+         const Divisor by_tr(tr), by_tr2(tr * tr), by_tr3r(cube_rn(tr) * R);
          for (int k = 0; k < R; k++) {
             const double v = d[k];
-            c[t * R + k] = v / tr - 1.0;
-            w[t * R + k] = 1.0 / sqrt(P.gain * (v / tr2 + v * v / tr3r));
+            c[t * R + k] = by_tr.quotient(v) - 1.0;
+            w[t * R + k] = 1.0 / sqrt(P.gain * (by_tr2.quotient(v) + by_tr3r.quotient(v * v)));
          }
       }
       // start grid (:261-328): inclination outer, t_rel inner, the first
@@ -709,9 +790,11 @@ rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__
       double x[3] = {phi0, P.incl[0], P.trel[0]};
       {
          double best = INFINITY;
-         for (int a = 0; a < 6; a++)
+         for (int a = 0; a < 6; a++) {
+            double cos2[5];
+            px_waves(P, phi0, P.incl[a], a ? S : nullptr, S, cos2);
             for (int t = 0; t < 6; t++) {
-               px_residuals(P, c, w, phi0, P.incl[a], P.trel[t], F);
+               px_residuals(P, c, w, S, cos2, P.trel[t], F);
                const double cost = np_sum([&](int i) { return F[i] * F[i]; }, M);
                if (cost < best || (isnan(cost) && !isnan(best))) {
                   best = cost;
@@ -719,10 +802,11 @@ rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__
                   x[2] = P.trel[t];
                }
             }
+         }
       }
       // MINPACK's fit, as scipy.optimize.leastsq runs it for the reference
       int n_fev = 0, cur = 0;
-      const int info = mp_fit<MAXM>(P, c, w, M, x, F, cur, J, n_fev);
+      const int info = mp_fit<MAXM>(P, c, w, M, x, F, cur, J, S, n_fev);
       if (info == 5)
          atomicAdd(&status[0], 1ull); // evaluation budget reached
       const double *fv = F + cur * MAXM;
@@ -829,15 +913,15 @@ int fpgb_rofl_device(const double *d_data, int64_t n_pix, int64_t n_rot, double 
       FPGB_CUDA_TRY(cudaGetDevice(&dev));
       FPGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       FPGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, small ? rofl_fit<kRoflSmallRot> : rofl_fit<kRoflMaxRot>, 128, 0));
+          &per_sm, small ? rofl_fit<kRoflSmallRot> : rofl_fit<kRoflMaxRot>, kRoflThreads, 0));
       const int64_t blocks =
-          std::max<int64_t>(1, std::min<int64_t>((n_pix + 127) / 128,
+          std::max<int64_t>(1, std::min<int64_t>((n_pix + kRoflThreads - 1) / kRoflThreads,
                                                  (int64_t)sms * std::max(per_sm, 1)));
       if (small)
-         rofl_fit<kRoflSmallRot><<<(unsigned)blocks, 128, 0, st>>>(d_data, n_pix, d_mask, P,
+         rofl_fit<kRoflSmallRot><<<(unsigned)blocks, kRoflThreads, 0, st>>>(d_data, n_pix, d_mask, P,
                                                                    d_out, status);
       else
-         rofl_fit<kRoflMaxRot><<<(unsigned)blocks, 128, 0, st>>>(d_data, n_pix, d_mask, P,
+         rofl_fit<kRoflMaxRot><<<(unsigned)blocks, kRoflThreads, 0, st>>>(d_data, n_pix, d_mask, P,
                                                                  d_out, status);
       FPGB_CUDA_TRY(cudaGetLastError());
    }
