@@ -103,7 +103,7 @@ constexpr int kBatchThreads = 128; // one work item = one CTA-width block of ray
 // MODE, TILT, COOP and WIDE are then unused.  (A min-blocks bound of 0 leaves
 // the other instantiations as compiled without one.)
 template <int MODE, bool TILT, bool COOP, bool WIDE, bool COLUMNS = false>
-__global__ void __launch_bounds__(128, COLUMNS ? 6 : 0)
+__global__ void __launch_bounds__(128, COLUMNS || COOP ? 6 : 0)
 batch_march(const MarchParams *__restrict__ prm, const BatchItem *__restrict__ items,
             int64_t n_items, int chunk, unsigned long long *__restrict__ next,
             unsigned long long *__restrict__ counters, int shape) {
@@ -112,6 +112,7 @@ batch_march(const MarchParams *__restrict__ prm, const BatchItem *__restrict__ i
    // plain kernel reads its by-value parameters)
    __shared__ __align__(16) MarchParams sP;
    __shared__ CoopScratch scratch[(COOP && !COLUMNS) ? kBatchThreads / 32 : 1];
+   __shared__ CoopLut lut; // the pair's
    int cur = -1;
    for (;;) {
       if (threadIdx.x == 0)
@@ -131,6 +132,8 @@ batch_march(const MarchParams *__restrict__ prm, const BatchItem *__restrict__ i
             for (int i = threadIdx.x; i < (int)(sizeof(MarchParams) / 16); i += blockDim.x)
                dst[i] = src[i];
             cur = w.pair;
+            if (COOP && !COLUMNS)
+               fill_lut(prm[w.pair], lut, threadIdx.x, blockDim.x);
             __syncthreads();
          }
          int64_t ray;
@@ -159,7 +162,8 @@ batch_march(const MarchParams *__restrict__ prm, const BatchItem *__restrict__ i
                                          sP.epa_d, sP.epa_r, counters);
          } else {
             march_ray_coop<MODE, TILT, WIDE>(sP, ray, valid, sP.label, sP.vec, sP.image, sP.epa_t,
-                                       sP.epa_d, sP.epa_r, counters, scratch[threadIdx.x >> 5]);
+                                       sP.epa_d, sP.epa_r, counters, scratch[threadIdx.x >> 5],
+                                       lut);
          }
       }
       __syncthreads(); // s_item is rewritten for the next chunk

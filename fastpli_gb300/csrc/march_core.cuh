@@ -22,7 +22,9 @@ namespace fpgb {
 struct F3 {
    float x, y, z;
 };
-__device__ __forceinline__ bool is_zero(F3 v) { return v.x == 0.f && v.y == 0.f && v.z == 0.f; }
+__device__ __forceinline__ bool is_zero(F3 v) { // +-0 in every component
+   return ((__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z)) << 1) == 0u;
+}
 __device__ __forceinline__ float dot3(F3 a, F3 b) {
    return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x));
 }
@@ -57,6 +59,14 @@ __device__ __forceinline__ float sinc_sq(float y) {
    return fmaf(p, y, 1.f);
 }
 
+// __fdividef(1, x) for x around 1: without its scaling of large divisors, which
+// changes nothing there (the same bits for every float in [0.5, 2]).
+__device__ __forceinline__ float rcp_near_one(float x) {
+   float r;
+   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+   return r;
+}
+
 // acos(1 - x)^2 for x = 1 - cos(th) in [0, 1 - cos 0.6]: 2x g(x) with g a
 // cubic least-squares fit (on Chebyshev nodes of that interval) of
 // g(x) = (2 asin(sqrt(x / 2)))^2 / (2x), relative error < 2e-7.  The
@@ -78,30 +88,40 @@ __device__ __forceinline__ float acos_sq(float x) {
 // from cos(th) directly (acos_sq): no inverse cosine and no sine calls, and
 // accurate as th -> 0.  Larger angles use acosf and the hardware sine.  The
 // reference's flip of u (when v.u < 0) is carried as the sign of u's weight.
+//
+// Out of line, as are the rare wide angles within, and the zero cases are
+// weights, not branches of their own: seven copies of this body in a marching
+// kernel, which the warps run through out of step, do not fit the instruction
+// cache.
+static __device__ __noinline__ float2 slerp_weights_wide(float c, float t) {
+   // th in [0.6, pi/2]: the hardware sine is accurate to ~5e-7 here
+   const float th = acosf(c);
+   const float inv = __fdividef(1.f, __sinf(th));
+   return make_float2(__sinf((1.f - t) * th) * inv, __sinf(t * th) * inv);
+}
+
 __device__ __forceinline__ F3 slerp_axis(F3 v, F3 u, float t) {
-   if (is_zero(v))
-      return u;
-   if (is_zero(u))
-      return v;
-   const float d0 = dot3(v, u);
-   const float sg = d0 < 0.f ? -1.f : 1.f;
-   const F3 df{fmaf(-sg, u.x, v.x), fmaf(-sg, u.y, v.y), fmaf(-sg, u.z, v.z)};
-   if (dot3(df, df) < 1e-12f)
-      return v;
-   const float c = fminf(fabsf(d0) * rsqrtf(dot3(v, v) * dot3(u, u)), 1.f);
-   float w0, w1;
-   if (c > 0.825335615f) { // th < 0.6
-      const float y = acos_sq(1.f - c), s = 1.f - t;
-      const float inv = __fdividef(1.f, sinc_sq(y));
-      w0 = s * sinc_sq(s * s * y) * inv;
-      w1 = t * sinc_sq(t * t * y) * inv;
-   } else { // th in [0.6, pi/2]: the hardware sine is accurate to ~5e-7 here
-      const float th = acosf(c);
-      const float inv = __fdividef(1.f, __sinf(th));
-      w0 = __sinf((1.f - t) * th) * inv;
-      w1 = __sinf(t * th) * inv;
+   const bool vz = is_zero(v), uz = is_zero(u);
+   float w0 = vz ? 0.f : 1.f, w1 = vz ? 1.f : 0.f; // v, or u where v is zero
+   if (!(vz || uz)) {
+      const float d0 = dot3(v, u);
+      const float sg = d0 < 0.f ? -1.f : 1.f;
+      const F3 df{fmaf(-sg, u.x, v.x), fmaf(-sg, u.y, v.y), fmaf(-sg, u.z, v.z)};
+      if (!(dot3(df, df) < 1e-12f)) {
+         const float c = fminf(fabsf(d0) * rsqrtf(dot3(v, v) * dot3(u, u)), 1.f);
+         if (c > 0.825335615f) { // th < 0.6
+            const float y = acos_sq(1.f - c), s = 1.f - t;
+            const float inv = rcp_near_one(sinc_sq(y)); // sinc_sq in [0.94, 1]
+            w0 = s * sinc_sq(s * s * y) * inv;
+            w1 = t * sinc_sq(t * t * y) * inv;
+         } else {
+            const float2 w = slerp_weights_wide(c, t);
+            w0 = w.x;
+            w1 = w.y;
+         }
+         w1 *= sg;
+      }
    }
-   w1 *= sg;
    return F3{fmaf(v.x, w0, u.x * w1), fmaf(v.y, w0, u.y * w1), fmaf(v.z, w0, u.z * w1)};
 }
 
@@ -673,103 +693,103 @@ __device__ __forceinline__ void march_one_ray_column(const MarchParams &P, int64
 // need it at different steps, so a one-ray-per-thread loop pays it on almost
 // every step.  Here each warp takes its 32 rays through kCoopSteps steps at a
 // time in three phases:
-//   1. every lane classifies its steps (label, optics) and writes one job
-//      descriptor per birefringent step into shared memory;
-//   2. the warp's jobs are compacted and shared out to all 32 lanes, each job
-//      producing that step's rotation (cos 2phi, sin 2phi, cos/sin ret) from
-//      the interpolated axis — the interpolated axis of a step depends only on
-//      its position, not on the state;
-//   3. every lane applies its steps' rotations and attenuations in order.
-// The arithmetic per step is the same as march_one_ray's.  Windows of 4 steps
-// keep the scratch at 17 KB per 128-thread block: the march lives on L1 hits
-// of its 8-corner gathers, and shared memory comes out of the same 256 KB
-// (8-step windows: 2.30 ms for config 2's five tilts, 4 steps: 2.12 ms,
-// 2 steps: 2.43 ms, the compaction then having too few jobs to fill warps).
+//   1. every lane loads its steps' labels (all in flight together), adds up
+//      their attenuation and lists its birefringent steps, packed by ballot;
+//   2. the warp's jobs are shared out to all 32 lanes, each job producing that
+//      step's rotation (cos 2phi, sin 2phi, cos/sin ret) from the interpolated
+//      axis, which depends only on the step's position, not on the state;
+//   3. every lane applies its own jobs' rotations in order.
+// The arithmetic per step is the same as march_one_ray's.  The attenuation is
+// taken ahead of phase 2, which may find that an interpolated axis is zero and
+// the step has no effect at all (simulator.cpp:292-297): such a ray's window
+// is added up again without it.
+// Bound by instruction issue (56% of the slots) and the latency of the 8-corner
+// gathers: about 250 issue slots per ray and step on the crossing volume, 670
+// per job.  Against windows of 4 steps with the corners worked out in phase 1
+// (a warp pays for it when one lane has a job), a shuffle scan and every step
+// applied in turn: crossing, one tilt 478 -> 430 us, Lerp tile 146 -> 106 us;
+// with windows of 4 steps 5% slower, of 16 (half the L1 gone to scratch) 30%.
+// The loops below stay rolled: unrolled, the kernel outgrows the instruction
+// cache (119 KB: 660 us).
 // ----------------------------------------------------------------------------
-constexpr int kCoopSteps = 4;
+constexpr int kCoopSteps = 8;
 constexpr int kCoopSlots = kCoopSteps * 32; // per warp
-constexpr int kCoopFields = 8;
+constexpr float kNoRotation = 2.f;          // in the place of cos 2phi
 
 struct CoopScratch {
-   float f[kCoopFields][kCoopSlots]; // slot = step * 32 + lane
-   unsigned short list[kCoopSlots];
+   float f[4][kCoopSlots]; // cos 2phi, sin 2phi, cos ret, sin ret; slot = step * 32 + lane
+   int64_t px[32], py[32]; // the rays' positions at the window's first step
+   int lab[kCoopSlots];    // of a job
+   unsigned flags[32];     // per ray: bit j: the axis of step j is zero; bit 31: not normalised
+   unsigned char list[kCoopSlots]; // slots of the jobs
+};
+static_assert(kCoopSlots <= 256 && kCoopSteps < 31, "slots are bytes, steps flag bits");
+
+// Label optics in shared memory (labels below kLutCache).
+constexpr int kLutCache = 64;
+struct CoopLut {
+   float2 step[kLutCache]; // alog, kind (int bits)
+   float kret[kLutCache];
 };
 
-// job status codes written to field 4
-constexpr int kJobRotate = 0, kJobIdentity = 1, kJobZero = 2, kJobNorm = 4;
+__device__ __forceinline__ void fill_lut(const MarchParams &P, CoopLut &lut, int tid, int n) {
+   for (int l = tid; l < min(P.n_props, kLutCache); l += n) {
+      const LabelOptics o = P.lut[l];
+      lut.step[l] = make_float2(o.alog, __int_as_float(o.kind));
+      lut.kret[l] = o.kret;
+   }
+}
+
+// Label of a ray's step at (px, py) in the z layer of step k (0 outside).
+template <bool WIDE>
+__device__ __forceinline__ int step_label(const MarchParams &P, const int32_t *__restrict__ label,
+                                          int64_t px, int64_t py, int k) {
+   using C = typename MarchIdx<WIDE>::C;
+   const C ix = fx_floor<WIDE>(px, P.frac_bits), iy = fx_floor<WIDE>(py, P.frac_bits);
+   if (ix < 0 || ix >= (C)P.X || iy < 0 || iy >= (C)P.Y)
+      return 0;
+   return __ldg(label + voxel_index<WIDE>(P, ix, iy, (C)P.ztab[k].iz));
+}
+
+__device__ __forceinline__ float2 step_optics(const MarchParams &P, const CoopLut &lut, int lab) {
+   if (lab < kLutCache)
+      return lut.step[lab];
+   const LabelOptics o = P.lut[lab];
+   return make_float2(o.alog, __int_as_float(o.kind));
+}
 
 template <int MODE, bool TILT, bool WIDE>
-__device__ __forceinline__ void coop_job(const MarchParams &P, const int32_t *__restrict__ label,
-                                         const float *__restrict__ vec, CoopScratch &S,
-                                         int slot) {
-   const int x0 = __float_as_int(S.f[0][slot]);
-   const int y0 = __float_as_int(S.f[1][slot]);
-   const int z0 = __float_as_int(S.f[2][slot]);
-   const int fl = __float_as_int(S.f[3][slot]);
-   const float xd = S.f[4][slot], yd = S.f[5][slot], zd = S.f[6][slot];
-   const int lab = __float_as_int(S.f[7][slot]);
-   const bool ax = fl & 1, ay = fl & 2, az = fl & 4;
-   using C = typename MarchIdx<WIDE>::C;
-   using U = typename MarchIdx<WIDE>::U;
-   const int dz = ((fl >> 3) & 3) - 1; // z1 - z0
-   const U base = voxel_index<WIDE>(P, (C)x0, (C)y0, (C)z0);
-   F3 v;
-   if (!ax && !ay && !az) {
-      v = load_vec(vec, base);
-   } else {
-      const U ox = (U)P.Y * (U)P.Z, oy = (U)P.Z, oz = (U)(C)dz;
-      F3 c[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-         if (((k & 1) && !ax) || ((k & 2) && !ay) || ((k & 4) && !az))
-            continue;
-         const U idx =
-             base + ((k & 1) ? ox : U(0)) + ((k & 2) ? oy : U(0)) + ((k & 4) ? oz : U(0));
-         // GetVec(...) * (GetLabel(...) == label) (simulator.cpp:533-540);
-         // label and axis loads are issued together
-         const float m = (__ldg(label + idx) == lab) ? 1.f : 0.f;
-         const F3 u = load_vec(vec, idx);
-         c[k] = F3{u.x * m, u.y * m, u.z * m};
-      }
-      F3 c00 = c[0], c10 = c[2], c01 = c[4], c11 = c[6];
-      if (ax) {
-         c00 = interp_axis<MODE>(c[0], c[1], xd);
-         if (az)
-            c01 = interp_axis<MODE>(c[4], c[5], xd);
-         if (ay) {
-            c10 = interp_axis<MODE>(c[2], c[3], xd);
-            if (az)
-               c11 = interp_axis<MODE>(c[6], c[7], xd);
-         }
-      }
-      F3 c0 = c00, c1 = c01;
-      if (ay) {
-         c0 = interp_axis<MODE>(c00, c10, yd);
-         if (az)
-            c1 = interp_axis<MODE>(c01, c11, yd);
-      }
-      v = az ? interp_axis<MODE>(c0, c1, zd) : c0;
+__device__ __forceinline__ void coop_job(const MarchParams &P, const CoopLut &lut,
+                                         const int32_t *__restrict__ label,
+                                         const float *__restrict__ vec, CoopScratch &S, int k0,
+                                         int t) {
+   const int slot = S.list[t], lab = S.lab[t], ray = slot & 31, j = slot >> 5;
+   int64_t px = S.px[ray], py = S.py[ray];
+   if (TILT) {
+      px += j * P.dx_fx;
+      py += j * P.dy_fx;
    }
-   int status;
-   float c = 1.f, s = 0.f, cr = 1.f, sr = 0.f;
+   F3 v = axis_interp<MODE, WIDE>(P, label, vec, px, py, P.ztab[k0 + j], lab);
+   float c = kNoRotation, s = 0.f, cr = 1.f, sr = 0.f;
    if (is_zero(v)) {
-      status = kJobZero;
+      atomicOr(&S.flags[ray], 1u << j);
    } else {
       const float n2 = dot3(v, v);
-      status = (n2 - 1.f > 1e-5f) ? kJobNorm : 0;
+      if (n2 - 1.f > 1e-5f)
+         atomicOr(&S.flags[ray], 1u << 31);
       if (TILT && P.rotate) {
          v = F3{dot3(F3{P.rot[0], P.rot[1], P.rot[2]}, v),
                 dot3(F3{P.rot[3], P.rot[4], P.rot[5]}, v),
                 dot3(F3{P.rot[6], P.rot[7], P.rot[8]}, v)};
       }
-      if (!retard_params(v, n2, P.lut[lab].kret, c, s, cr, sr))
-         status |= kJobIdentity;
+      const float kret = lab < kLutCache ? lut.kret[lab] : P.lut[lab].kret;
+      if (!retard_params(v, n2, kret, c, s, cr, sr))
+         c = kNoRotation;
    }
    S.f[0][slot] = c;
    S.f[1][slot] = s;
    S.f[2][slot] = cr;
    S.f[3][slot] = sr;
-   S.f[4][slot] = __int_as_float(status);
 }
 
 template <int MODE, bool TILT, bool WIDE>
@@ -781,115 +801,88 @@ __device__ __forceinline__ void march_ray_coop(const MarchParams &P, int64_t ray
                                                double *__restrict__ epa_d,
                                                double *__restrict__ epa_r,
                                                unsigned long long *__restrict__ counters,
-                                               CoopScratch &S) {
-   using C = typename MarchIdx<WIDE>::C;
+                                               CoopScratch &S, const CoopLut &lut) {
    const int lane = threadIdx.x & 31;
-   const int F = P.frac_bits;
    int64_t px = 0, py = 0;
    if (active)
       ray_setup(P, ray, px, py);
-   const int64_t half = int64_t(1) << (F - 1);
-   const C xm = (C)P.X - 1, ym = (C)P.Y - 1, zm = (C)P.Z - 1;
+   else
+      px = py = INT64_MIN; // outside at every step
    float u1 = 0.f, u2 = 0.f, u3 = -1.f, L = 0.f;
    bool w_zero = false, w_norm = false, bad_label = false;
+   S.flags[lane] = 0;
    for (int k0 = 0; k0 < P.n_z; k0 += kCoopSteps) {
-      // phase 1: classify this lane's steps, write job descriptors
-      unsigned kinds = 0; // 2 bits per step
-      float alog[kCoopSteps];
+      // phase 1: labels, attenuation, jobs
+      const float L0 = L;
+      int lab[kCoopSteps];
+      S.px[lane] = px;
+      S.py[lane] = py;
 #pragma unroll
       for (int j = 0; j < kCoopSteps; j++) {
-         const int k = k0 + j;
-         alog[j] = 0.f;
-         if (!active || k >= P.n_z)
-            continue;
-         if (TILT && k > 0) {
+         lab[j] = k0 + j < P.n_z ? step_label<WIDE>(P, label, px, py, k0 + j) : 0;
+         if (TILT && active) {
             px += P.dx_fx;
             py += P.dy_fx;
          }
-         const C ix = fx_floor<WIDE>(px, F), iy = fx_floor<WIDE>(py, F);
-         const ZStep zs = P.ztab[k];
-         int lab = 0;
-         if (ix >= 0 && ix <= xm && iy >= 0 && iy <= ym) {
-            lab = __ldg(label + voxel_index<WIDE>(P, ix, iy, (C)zs.iz));
-            if (lab < 0 || lab >= P.n_props) {
-               bad_label = true;
-               lab = 0;
-            }
-         }
-         const LabelOptics o = P.lut[lab];
-         alog[j] = o.alog;
-         kinds |= (unsigned)o.kind << (2 * j);
-         if (o.kind != 2)
-            continue;
-         // trilinear corners as in axis_interp (simulator.cpp:510-530)
-         const int64_t hx = px - half, hy = py - half;
-         const C fx0 = fx_floor<WIDE>(hx, F), fy0 = fx_floor<WIDE>(hy, F);
-         const C x0 = clampc<C>(fx0, xm), x1 = clampc<C>(fx0 + (C)fx_has_frac(hx, F), xm);
-         const C y0 = clampc<C>(fy0, ym), y1 = clampc<C>(fy0 + (C)fx_has_frac(hy, F), ym);
-         C z0 = clampc<C>((C)zs.z0, zm), z1 = clampc<C>((C)zs.z0 + (C)(zs.zf != 0.f), zm);
-         const int ax = x0 != x1, ay = y0 != y1, az = z0 != z1;
-         const float xf = ax ? fx_frac(hx, F) : 0.f;
-         const float yf = ay ? fx_frac(hy, F) : 0.f;
-         const float zd = az ? zs.zf : 0.f;
-         if (P.flip_z) {
-            z0 = zm - z0;
-            z1 = zm - z1;
-         }
-         const int slot = j * 32 + lane;
-         S.f[0][slot] = __int_as_float((int)x0);
-         S.f[1][slot] = __int_as_float((int)y0);
-         S.f[2][slot] = __int_as_float((int)z0);
-         S.f[3][slot] = __int_as_float(ax | (ay << 1) | (az << 2) | ((int)(z1 - z0 + 1) << 3));
-         S.f[4][slot] = xf;
-         S.f[5][slot] = yf;
-         S.f[6][slot] = zd;
-         S.f[7][slot] = __int_as_float(lab);
       }
-      // phase 2: compact the warp's jobs and share them out
       unsigned jobs = 0;
-#pragma unroll
-      for (int j = 0; j < kCoopSteps; j++)
-         jobs |= (((kinds >> (2 * j)) & 3u) == 2u) ? (1u << j) : 0u;
-      const int cnt = __popc(jobs);
-      int pre = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-         const int v = __shfl_up_sync(0xffffffffu, pre, o);
-         if (lane >= o)
-            pre += v;
-      }
-      const int total = __shfl_sync(0xffffffffu, pre, 31);
-      pre -= cnt;
-      for (unsigned m = jobs; m; m &= m - 1) {
-         const int j = __ffs(m) - 1;
-         S.list[pre++] = (unsigned short)(j * 32 + lane);
-      }
-      __syncwarp();
-      for (int t = lane; t < total; t += 32)
-         coop_job<MODE, TILT, WIDE>(P, label, vec, S, S.list[t]);
-      __syncwarp();
-      // phase 3: apply this lane's steps in order
+      int total = 0;
 #pragma unroll
       for (int j = 0; j < kCoopSteps; j++) {
-         const unsigned kind = (kinds >> (2 * j)) & 3u;
-         if (kind == 1u) {
-            L += alog[j];
-         } else if (kind == 2u) {
-            const int slot = j * 32 + lane;
-            const int st = __float_as_int(S.f[4][slot]);
-            if (st & kJobZero) { // simulator.cpp:292-297: no attenuation either
-               w_zero = true;
-               continue;
-            }
-            if (st & kJobNorm)
-               w_norm = true;
-            if (!(st & kJobIdentity))
-               apply_retard(u1, u2, u3, S.f[0][slot], S.f[1][slot], S.f[2][slot],
-                            S.f[3][slot]);
-            L += alog[j];
+         if ((unsigned)lab[j] >= (unsigned)P.n_props) {
+            bad_label = true;
+            lab[j] = 0;
          }
+         const float2 o = step_optics(P, lut, lab[j]);
+         L += k0 + j < P.n_z ? o.x : 0.f; // (0 for labels without effect)
+         const bool job = active && __float_as_int(o.y) == 2;
+         const unsigned m = __ballot_sync(0xffffffffu, job);
+         if (job) {
+            const int at = total + __popc(m & ((1u << lane) - 1u));
+            S.list[at] = (unsigned char)(j * 32 + lane);
+            S.lab[at] = lab[j];
+            jobs |= 1u << j;
+         }
+         total += __popc(m);
       }
-      __syncwarp(); // the scratch is rewritten by the next block of steps
+      __syncwarp();
+      // phase 2: the jobs
+#pragma unroll 1
+      for (int t = lane; t < total; t += 32)
+         coop_job<MODE, TILT, WIDE>(P, lut, label, vec, S, k0, t);
+      __syncwarp();
+      // phase 3: this lane's rotations, in order
+#pragma unroll 1
+      for (unsigned m = jobs; m; m &= m - 1) {
+         const int slot = (__ffs((int)m) - 1) * 32 + lane;
+         const float c = S.f[0][slot];
+         if (c != kNoRotation)
+            apply_retard(u1, u2, u3, c, S.f[1][slot], S.f[2][slot], S.f[3][slot]);
+      }
+      const unsigned flags = jobs ? S.flags[lane] : 0u;
+      if (flags) {
+         w_norm = w_norm || (flags >> 31);
+         const unsigned zero = flags & 0x7fffffffu;
+         if (zero) { // simulator.cpp:292-297: no attenuation either
+            w_zero = true;
+            L = L0;
+            int64_t qx = S.px[lane], qy = S.py[lane];
+#pragma unroll 1
+            for (int j = 0; j < kCoopSteps && k0 + j < P.n_z; j++) {
+               int l = step_label<WIDE>(P, label, qx, qy, k0 + j);
+               if ((unsigned)l >= (unsigned)P.n_props)
+                  l = 0;
+               if (!(zero >> j & 1u))
+                  L += step_optics(P, lut, l).x;
+               if (TILT) {
+                  qx += P.dx_fx;
+                  qy += P.dy_fx;
+               }
+            }
+         }
+         S.flags[lane] = 0;
+      }
+      __syncwarp(); // the scratch is rewritten by the next window
    }
    if (active)
       ray_epilogue(P, ray, u1, u2, L, image, epa_t, epa_d, epa_r, w_zero, w_norm, bad_label,

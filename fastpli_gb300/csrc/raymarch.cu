@@ -317,10 +317,11 @@ int plan_march(const fpgb_setup *s, const int64_t *dim, const double *props, int
 // ======================================================================
 // 7 resident blocks per SM for the per-thread and column kernels (72
 // registers: 3% faster than the 80-register default on config 2; 8 blocks
-// spill too much); the cooperative kernel keeps the 5 its registers give it
-// (6 measured the same).
+// spill too much); the cooperative kernels 5 for Slerp (96 registers, and less
+// of L1 gone to scratch: five tilts of the crossing volume 1,657 us against
+// 1,726 with 6) and 6 for Lerp (a tile 181 us against 233 with 5).
 template <int MODE, bool TILT, bool COOP, bool WIDE>
-__global__ void __launch_bounds__(128, COOP ? 6 : 7)
+__global__ void __launch_bounds__(128, COOP ? (MODE == 2 ? 5 : 6) : 7)
 march_rays(const MarchParams P, int64_t unit0, const int32_t *__restrict__ label,
            const float *__restrict__ vec, double *__restrict__ image,
            double *__restrict__ epa_t, double *__restrict__ epa_d, double *__restrict__ epa_r,
@@ -342,8 +343,11 @@ march_rays(const MarchParams P, int64_t unit0, const int32_t *__restrict__ label
                                          counters);
    } else { // whole warps take part in the cooperative march
       __shared__ CoopScratch scratch[4];
+      __shared__ CoopLut lut;
+      fill_lut(P, lut, threadIdx.x, blockDim.x);
+      __syncthreads();
       march_ray_coop<MODE, TILT, WIDE>(P, valid ? ray : 0, valid, label, vec, image, epa_t, epa_d,
-                                 epa_r, counters, scratch[threadIdx.x >> 5]);
+                                       epa_r, counters, scratch[threadIdx.x >> 5], lut);
    }
 }
 
@@ -444,7 +448,9 @@ static int launch_march_units(const MarchParams &P, const int32_t *d_label, cons
                                                       d_d, d_r, d_counters)
    const bool coop = P.coop != 0;
    const bool narrow = march_narrow(P);
-   switch (P.mode * 4 + (tilt ? 2 : 0) + (coop ? 1 : 0)) {
+   // (vertical columns need no interpolation: the kernel with the fewest
+   // registers and no scratch; 1024 x 1024 x 240 1,120 -> 940 us)
+   switch (!tilt && P.column ? 0 : P.mode * 4 + (tilt ? 2 : 0) + (coop ? 1 : 0)) {
    case 0: case 1: FPGB_LAUNCH(0, false, false); break;
    case 2: case 3: FPGB_LAUNCH(0, true, false); break;
    case 4: FPGB_LAUNCH(1, false, false); break;
