@@ -100,8 +100,9 @@ constexpr int kBatchThreads = 128; // one work item = one CTA-width block of ray
 // the untilted pairs of a batch with step 1): the kernel carries only the
 // column path and its few registers (more resident warps for its streaming
 // loads; held to 6 CTAs per SM, 80 registers: 0.3% faster than 5 at 92);
-// MODE, TILT, COOP and WIDE are then unused.  (A min-blocks bound of 0 leaves
-// the other instantiations as compiled without one.)
+// MODE, TILT, COOP and WIDE are then unused.  The cooperative kernels are held
+// to 6 CTAs per SM as well (8 tiles x 5 tilts 2,787 us against 2,875 with 5);
+// a min-blocks bound of 0 leaves the others as compiled without one.
 template <int MODE, bool TILT, bool COOP, bool WIDE, bool COLUMNS = false>
 __global__ void __launch_bounds__(128, COLUMNS || COOP ? 6 : 0)
 batch_march(const MarchParams *__restrict__ prm, const BatchItem *__restrict__ items,

@@ -392,26 +392,32 @@ int sm_count() {
 }
 } // namespace
 
-// The launch form of the plan: tables copied into caller-provided device
-// memory (lut then ztab, 256-byte aligned) and pointed to from P.
-static int prepare_march(const MarchPlan &mp, const int32_t *d_label, const float *d_vec,
-                         void *d_tables, cudaStream_t st, MarchParams &P) {
-   P = mp.prm;
-   char *w = static_cast<char *>(d_tables);
-   LabelOptics *lut = reinterpret_cast<LabelOptics *>(w);
-   w += align_up(sizeof(LabelOptics) * mp.lut.size(), 256);
-   ZStep *zt = reinterpret_cast<ZStep *>(w);
-   FPGB_CUDA_TRY(cudaMemcpyAsync(lut, mp.lut.data(), sizeof(LabelOptics) * mp.lut.size(),
-                                 cudaMemcpyHostToDevice, st));
-   FPGB_CUDA_TRY(cudaMemcpyAsync(zt, mp.ztab.data(), sizeof(ZStep) * mp.ztab.size(),
-                                 cudaMemcpyHostToDevice, st));
-   P.lut = lut;
-   P.ztab = zt;
+// A plan's tables (lut then ztab, 256-byte aligned) in h, for one upload.
+static void stage_march(const MarchPlan &mp, char *h) {
+   std::memcpy(h, mp.lut.data(), sizeof(LabelOptics) * mp.lut.size());
+   std::memcpy(h + align_up(sizeof(LabelOptics) * mp.lut.size(), 256), mp.ztab.data(),
+               sizeof(ZStep) * mp.ztab.size());
+}
+
+// A counter block as a march starts with it.
+static void stage_counters(char *h) {
+   unsigned long long c[kCounterWords] = {0};
+   c[7] = ~0ull; // smallest label
+   std::memcpy(h, c, sizeof c);
+}
+
+// The launch form of the plan, its tables at d_tables.
+static MarchParams bind_march(const MarchPlan &mp, const int32_t *d_label, const float *d_vec,
+                              char *d_tables) {
+   MarchParams P = mp.prm;
+   P.lut = reinterpret_cast<LabelOptics *>(d_tables);
+   P.ztab = reinterpret_cast<ZStep *>(d_tables +
+                                      align_up(sizeof(LabelOptics) * mp.lut.size(), 256));
    // 16-byte column loads (Z % 4 == 0) need 16-byte aligned fields
    if (P.Z % 4 == 0 &&
        (reinterpret_cast<uintptr_t>(d_label) % 16 || reinterpret_cast<uintptr_t>(d_vec) % 16))
       P.column = 0;
-   return FPGB_OK;
+   return P;
 }
 
 static bool march_tilted(const MarchParams &P) {
@@ -467,11 +473,9 @@ static int launch_march_units(const MarchParams &P, const int32_t *d_label, cons
    return FPGB_OK;
 }
 
-int launch_march(const MarchPlan &mp, const int32_t *d_label, const float *d_vec,
-                 double *d_image, double *d_t, double *d_d, double *d_r,
-                 void *d_tables, unsigned long long *d_counters, cudaStream_t st) {
-   MarchParams P;
-   FPGB_TRY(prepare_march(mp, d_label, d_vec, d_tables, st, P));
+static int launch_march(MarchParams P, const int32_t *d_label, const float *d_vec,
+                        double *d_image, double *d_t, double *d_d, double *d_r,
+                        unsigned long long *d_counters, cudaStream_t st) {
    // start at the end of the volume the previous device-resident pass
    // (voxelizer or march) finished at: that part is still in L2
    std::atomic<int> &end = l2_end_state();
@@ -530,22 +534,10 @@ int launch_label_check(const int32_t *d_label, int64_t n, unsigned long long *d_
    return FPGB_OK;
 }
 
-// counters: [0..5] warnings, [6] status, [7] min label + 2^31, [8] max + 2^31
-int init_counters(unsigned long long *d_counters, cudaStream_t st) {
-   unsigned long long h[kCounterWords] = {0};
-   h[7] = ~0ull;
-   h[8] = 0;
-   FPGB_CUDA_TRY(cudaMemcpyAsync(d_counters, h, sizeof h, cudaMemcpyHostToDevice, st));
-   return FPGB_OK;
-}
-
-// Reads the counters back (synchronising) and turns status bits and label
-// range violations into errors.
-int finish_counters(const unsigned long long *d_counters, int64_t n_props, bool checked_all,
-                    fpgb_warnings *w, cudaStream_t st) {
-   unsigned long long h[kCounterWords];
-   FPGB_CUDA_TRY(cudaMemcpyAsync(h, d_counters, sizeof h, cudaMemcpyDeviceToHost, st));
-   FPGB_CUDA_TRY(cudaStreamSynchronize(st));
+// counters: [0..5] warnings, [6] status, [7] min label + 2^31, [8] max + 2^31.
+// Turns status bits and label range violations of a block into errors.
+static int check_counters(const unsigned long long *h, int64_t n_props, bool checked_all,
+                          fpgb_warnings *w) {
    if (checked_all) {
       const long long mn = (long long)h[7] - 2147483648LL;
       const long long mx = (long long)h[8] - 2147483648LL;
@@ -567,6 +559,46 @@ int finish_counters(const unsigned long long *d_counters, int64_t n_props, bool 
    return FPGB_OK;
 }
 
+// Reads n counter blocks back (synchronising) and checks them in order.
+static int finish_counters(const char *d_counters, int64_t n, int64_t n_props, bool checked_all,
+                           fpgb_warnings *w, cudaStream_t st) {
+   std::vector<unsigned long long> h((size_t)(kCounterWords * n));
+   FPGB_CUDA_TRY(cudaMemcpyAsync(h.data(), d_counters, sizeof(unsigned long long) * h.size(),
+                                 cudaMemcpyDeviceToHost, st));
+   FPGB_CUDA_TRY(cudaStreamSynchronize(st));
+   for (int64_t k = 0; k < n; k++)
+      FPGB_TRY(check_counters(h.data() + kCounterWords * k, n_props, checked_all,
+                              w ? w + k : nullptr));
+   return FPGB_OK;
+}
+
+constexpr size_t kCounterBytes = sizeof(unsigned long long) * kCounterWords;
+
+// The counter blocks and tables of the plans of one call, in one pool buffer
+// of st and by one upload: *d_counters, and *d_tables[k] per plan.
+static int upload_march(const MarchPlan *plans, int64_t n, char **d_counters,
+                        std::vector<char *> &d_tables, cudaStream_t st) {
+   size_t bytes = align_up(kCounterBytes * (size_t)n, 256);
+   std::vector<size_t> off((size_t)n);
+   for (int64_t k = 0; k < n; k++) {
+      off[k] = bytes;
+      bytes += march_table_bytes(plans[k]);
+   }
+   std::vector<char> h(bytes);
+   for (int64_t k = 0; k < n; k++) {
+      stage_counters(h.data() + kCounterBytes * (size_t)k);
+      stage_march(plans[k], h.data() + off[k]);
+   }
+   void *d = nullptr;
+   FPGB_TRY(pool_get(kSlotProps, bytes, &d, st));
+   FPGB_CUDA_TRY(cudaMemcpyAsync(d, h.data(), bytes, cudaMemcpyHostToDevice, st));
+   *d_counters = static_cast<char *>(d);
+   d_tables.resize((size_t)n);
+   for (int64_t k = 0; k < n; k++)
+      d_tables[k] = *d_counters + off[k];
+   return FPGB_OK;
+}
+
 static int run_sim_planned(const MarchPlan &mp, const int32_t *d_label, const float *d_vector,
                            int64_t n_props, double *d_image, double *d_t, double *d_d,
                            double *d_r, fpgb_warnings *warnings, bool check_all,
@@ -575,160 +607,23 @@ static int run_sim_planned(const MarchPlan &mp, const int32_t *d_label, const fl
       set_error("run_simulation: null label/vector buffer");
       return FPGB_EINVAL;
    }
-   void *tables = nullptr, *counters = nullptr;
-   FPGB_TRY(pool_get(kSlotProps, march_table_bytes(mp), &tables, st));
-   FPGB_TRY(pool_get(kSlotCounters, sizeof(unsigned long long) * kCounterWords, &counters, st));
-   auto *cnt = static_cast<unsigned long long *>(counters);
-   FPGB_TRY(init_counters(cnt, st));
+   char *counters = nullptr;
+   std::vector<char *> tables;
+   FPGB_TRY(upload_march(&mp, 1, &counters, tables, st));
+   auto *cnt = reinterpret_cast<unsigned long long *>(counters);
    if (check_all)
       FPGB_TRY(launch_label_check(d_label, mp.prm.X * mp.prm.Y * mp.prm.Z, cnt, st));
-   FPGB_TRY(launch_march(mp, d_label, d_vector, d_image, d_t, d_d, d_r, tables, cnt, st));
+   FPGB_TRY(launch_march(bind_march(mp, d_label, d_vector, tables[0]), d_label, d_vector, d_image,
+                         d_t, d_d, d_r, cnt, st));
    if (warnings || check_all)
-      return finish_counters(cnt, n_props, check_all, warnings, st);
+      return finish_counters(counters, 1, n_props, check_all, warnings, st);
    return FPGB_OK;
 }
 
-// Host-buffer march over page-locked label / vector fields: the volume goes
-// up in x-slabs on a second stream, and the rays are launched in chunks,
-// each as soon as every slab its rays can read (march_units_x_range) is on
-// the device, so most of the march runs under the copy.  Same kernels and
-// bits as the one-launch march.
-// Consecutive chunks that wait for the same slab go out as one launch: a
-// chunk alone fills a third of the GPU, and the chunks that need the last
-// slab would otherwise run one after another after the copy (measured on
-// config 2: 4 slabs / 8 single-chunk launches left 0.47 ms of march after
-// the 2.41 ms copy).
-// With a page-locked host image, the image rows each launch completes go
-// down on a third stream while the later launches run, so only the last
-// launch's rows are copied after the march.
-constexpr int kUpSlabs = 8, kRayChunks = 32;
-
-// Image rows (pixel columns x) every ray of which lies in blocks [0, u).
-static int64_t march_units_rows_done(const MarchParams &P, int64_t u) {
-   if (!march_tilted(P) && P.column)
-      return std::min(P.X, u * 128 / P.Y);
-   return std::min(P.X, (u / ((P.Y + kRayTileY - 1) / kRayTileY)) * kRayTileX);
-}
-
-static int run_sim_pipelined(const MarchPlan &mp, const int32_t *label, const float *vector,
-                             int32_t *d_label, float *d_vec, int64_t n_props, double *d_img,
-                             double *h_image, fpgb_warnings *warnings, cudaStream_t st) {
-   const int64_t X = mp.prm.X, row = mp.prm.Y * mp.prm.Z;
-   const int64_t img_row = mp.prm.Y * mp.prm.n_rho; // doubles per image row
-   void *tables = nullptr, *counters = nullptr;
-   FPGB_TRY(pool_get(kSlotProps, march_table_bytes(mp), &tables, st));
-   FPGB_TRY(pool_get(kSlotCounters, sizeof(unsigned long long) * kCounterWords, &counters, st));
-   auto *cnt = static_cast<unsigned long long *>(counters);
-   FPGB_TRY(init_counters(cnt, st));
-   MarchParams P;
-   FPGB_TRY(prepare_march(mp, d_label, d_vec, tables, st, P));
-   cudaStream_t up = nullptr, down = nullptr;
-   cudaEvent_t ev[kUpSlabs] = {};
-   cudaEvent_t done[kRayChunks + 1] = {};
-   int n_done = 0;
-   int64_t rows_copied = 0;
-   int64_t slab_end[kUpSlabs];
-   int rc = FPGB_OK;
-   // after a launch: copy the image rows [rows_copied, r1) it completed
-   auto copy_rows = [&](int64_t r1) -> int {
-      if (!h_image || r1 <= rows_copied)
-         return FPGB_OK;
-      FPGB_CUDA_TRY(cudaEventCreateWithFlags(&done[n_done], cudaEventDisableTiming));
-      FPGB_CUDA_TRY(cudaEventRecord(done[n_done], st));
-      FPGB_CUDA_TRY(cudaStreamWaitEvent(down, done[n_done++], 0));
-      FPGB_CUDA_TRY(cudaMemcpyAsync(h_image + rows_copied * img_row, d_img + rows_copied * img_row,
-                                    sizeof(double) * (r1 - rows_copied) * img_row,
-                                    cudaMemcpyDeviceToHost, down));
-      rows_copied = r1;
-      return FPGB_OK;
-   };
-   auto run = [&]() -> int {
-      FPGB_CUDA_TRY(cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking));
-      if (h_image)
-         FPGB_CUDA_TRY(cudaStreamCreateWithFlags(&down, cudaStreamNonBlocking));
-      // the slab copies must not start before the stream's earlier work
-      // (the previous call's march may still read these buffers)
-      FPGB_CUDA_TRY(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
-      FPGB_CUDA_TRY(cudaEventRecord(ev[0], st));
-      FPGB_CUDA_TRY(cudaStreamWaitEvent(up, ev[0], 0));
-      for (int s = 0; s < kUpSlabs; s++) {
-         const int64_t x0 = X * s / kUpSlabs, x1 = X * (s + 1) / kUpSlabs;
-         slab_end[s] = x1;
-         if (x1 > x0) {
-            FPGB_CUDA_TRY(cudaMemcpyAsync(d_label + x0 * row, label + x0 * row,
-                                          sizeof(int32_t) * (x1 - x0) * row,
-                                          cudaMemcpyHostToDevice, up));
-            FPGB_CUDA_TRY(cudaMemcpyAsync(d_vec + 3 * x0 * row, vector + 3 * x0 * row,
-                                          sizeof(float) * 3 * (x1 - x0) * row,
-                                          cudaMemcpyHostToDevice, up));
-         }
-         if (s > 0)
-            FPGB_CUDA_TRY(cudaEventCreateWithFlags(&ev[s], cudaEventDisableTiming));
-         FPGB_CUDA_TRY(cudaEventRecord(ev[s], up));
-      }
-      const int64_t nu = march_units(P);
-      int waited = -1;
-      int64_t g0 = 0; // first unit of the pending launch
-      for (int c = 0; c < kRayChunks; c++) {
-         const int64_t u0 = nu * c / kRayChunks, u1 = nu * (c + 1) / kRayChunks;
-         if (u1 <= u0)
-            continue;
-         int64_t lo, hi;
-         march_units_x_range(P, u0, u1, lo, hi);
-         int s = 0;
-         while (s < kUpSlabs - 1 && slab_end[s] <= hi)
-            s++;
-         s = std::max(s, waited);
-         if (s > waited && u0 > g0) { // launch the chunks that the slabs so far cover
-            FPGB_TRY(launch_march_units(P, d_label, d_vec, d_img, nullptr, nullptr, nullptr,
-                                        cnt, g0, u0, st));
-            FPGB_TRY(copy_rows(march_units_rows_done(P, u0)));
-            g0 = u0;
-         }
-         if (s > waited) {
-            FPGB_CUDA_TRY(cudaStreamWaitEvent(st, ev[s], 0));
-            waited = s;
-         }
-      }
-      FPGB_TRY(launch_march_units(P, d_label, d_vec, d_img, nullptr, nullptr, nullptr, cnt, g0,
-                                  nu, st));
-      FPGB_TRY(copy_rows(X)); // every launch is done: all remaining rows
-      if (waited < kUpSlabs - 1)
-         FPGB_CUDA_TRY(cudaStreamWaitEvent(st, ev[kUpSlabs - 1], 0));
-      return launch_label_check(d_label, X * row, cnt, st);
-   };
-   rc = run();
-   for (cudaStream_t s : {up, down})
-      if (s) {
-         cudaStreamSynchronize(s);
-         cudaStreamDestroy(s);
-      }
-   for (cudaEvent_t e : ev)
-      if (e)
-         cudaEventDestroy(e);
-   for (cudaEvent_t e : done)
-      if (e)
-         cudaEventDestroy(e);
-   FPGB_TRY(rc);
-   return finish_counters(cnt, n_props, true, warnings, st);
-}
-
-static int run_sim_device(const fpgb_setup *setup, const int64_t *dim, const int32_t *d_label,
-                          const float *d_vector, const double *props, int64_t n_props,
-                          double theta, double phi, double *d_image, double *d_t, double *d_d,
-                          double *d_r, fpgb_warnings *warnings, bool check_all,
-                          cudaStream_t st) {
-   MarchPlan mp;
-   FPGB_TRY(plan_march(setup, dim, props, n_props, theta, phi, &mp));
-   return run_sim_planned(mp, d_label, d_vector, n_props, d_image, d_t, d_d, d_r, warnings,
-                          check_all, st);
-}
-
 // The streams a multi-tilt call spreads its tilts over (per device, created
-// on first use and kept for the process), and the lock that keeps two
-// calls' work on them in one order: a tilt's tables live in the stream's
-// pool slot, so one call's uploads must not land between another call's
-// upload and march on the same stream.
+// on first use and kept for the process; the host-buffer march uses them as
+// well), and the lock under which they are made and a multi-tilt call forks
+// and joins them.
 constexpr int kTiltStreams = 4;
 
 static std::mutex &tilt_issue_mutex() {
@@ -750,6 +645,171 @@ static int tilt_streams(cudaStream_t *out) { // caller holds tilt_issue_mutex
       out[i] = streams[dev][i];
    }
    return FPGB_OK;
+}
+
+// Host-buffer march over page-locked label / vector fields: the volume goes
+// up in x-slabs on a second stream, and the rays are launched in chunks,
+// each as soon as every slab its rays can read (march_units_x_range) is on
+// the device, so most of the march runs under the copy.  Same kernels and
+// bits as the one-launch march.
+// Consecutive chunks that wait for the same slab go out as one launch: a
+// chunk alone fills a third of the GPU, and the chunks that need the last
+// slab would otherwise run one after another after the copy (measured on
+// config 2: 4 slabs / 8 single-chunk launches left 0.47 ms of march after
+// the 2.41 ms copy).
+// The launches take turns on the library's streams: one alone fills a part of
+// the GPU for as long as its slowest ray takes (75 us on a 256 x 256 x 60
+// volume, whose copy takes 300), and on one stream each would wait for the one
+// before it.
+// With a page-locked host image, the image rows each launch completes go
+// down on a third stream while the later launches run, so only the last
+// launch's rows are copied after the march.
+// Slabs of at least 8 MiB: smaller ones cost more in launches than they hide.
+constexpr int kUpSlabs = 8, kRayChunks = 32;
+constexpr int64_t kMinSlabBytes = int64_t(8) << 20;
+
+// Image rows (pixel columns x) every ray of which lies in blocks [0, u).
+static int64_t march_units_rows_done(const MarchParams &P, int64_t u) {
+   if (!march_tilted(P) && P.column)
+      return std::min(P.X, u * 128 / P.Y);
+   return std::min(P.X, (u / ((P.Y + kRayTileY - 1) / kRayTileY)) * kRayTileX);
+}
+
+static int run_sim_pipelined(const MarchPlan &mp, const int32_t *label, const float *vector,
+                             int32_t *d_label, float *d_vec, int64_t n_props, double *d_img,
+                             double *h_image, fpgb_warnings *warnings, cudaStream_t st) {
+   const int64_t X = mp.prm.X, row = mp.prm.Y * mp.prm.Z;
+   const int64_t img_row = mp.prm.Y * mp.prm.n_rho; // doubles per image row
+   char *counters = nullptr;
+   std::vector<char *> tables;
+   FPGB_TRY(upload_march(&mp, 1, &counters, tables, st));
+   auto *cnt = reinterpret_cast<unsigned long long *>(counters);
+   const MarchParams P = bind_march(mp, d_label, d_vec, tables[0]);
+   const int n_slabs =
+       (int)std::max<int64_t>(1, std::min<int64_t>(kUpSlabs, 16 * X * row / kMinSlabBytes));
+   cudaStream_t march[kTiltStreams];
+   {
+      std::lock_guard<std::mutex> lk(tilt_issue_mutex());
+      FPGB_TRY(tilt_streams(march));
+   }
+   int n_launch = 0; // launch i ran on march[i % kTiltStreams]
+   cudaStream_t up = nullptr, down = nullptr;
+   cudaEvent_t ready = nullptr, ev[kUpSlabs] = {}, joined[kTiltStreams] = {};
+   cudaEvent_t done[kRayChunks + 1] = {};
+   int n_done = 0;
+   int64_t rows_copied = 0;
+   int64_t slab_end[kUpSlabs];
+   int rc = FPGB_OK;
+   // after a launch: copy the image rows [rows_copied, r1) it completed
+   auto copy_rows = [&](cudaStream_t from, int64_t r1) -> int {
+      if (!h_image)
+         return FPGB_OK;
+      FPGB_CUDA_TRY(cudaEventCreateWithFlags(&done[n_done], cudaEventDisableTiming));
+      FPGB_CUDA_TRY(cudaEventRecord(done[n_done], from));
+      FPGB_CUDA_TRY(cudaStreamWaitEvent(down, done[n_done++], 0));
+      if (r1 <= rows_copied)
+         return FPGB_OK;
+      FPGB_CUDA_TRY(cudaMemcpyAsync(h_image + rows_copied * img_row, d_img + rows_copied * img_row,
+                                    sizeof(double) * (r1 - rows_copied) * img_row,
+                                    cudaMemcpyDeviceToHost, down));
+      rows_copied = r1;
+      return FPGB_OK;
+   };
+   auto run = [&]() -> int {
+      FPGB_CUDA_TRY(cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking));
+      if (h_image)
+         FPGB_CUDA_TRY(cudaStreamCreateWithFlags(&down, cudaStreamNonBlocking));
+      // the slab copies must not start before the stream's earlier work
+      // (the previous call's march may still read these buffers)
+      FPGB_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+      FPGB_CUDA_TRY(cudaEventRecord(ready, st));
+      FPGB_CUDA_TRY(cudaStreamWaitEvent(up, ready, 0));
+      for (int i = 0; i < kTiltStreams; i++)
+         FPGB_CUDA_TRY(cudaStreamWaitEvent(march[i], ready, 0));
+      for (int s = 0; s < n_slabs; s++) {
+         const int64_t x0 = X * s / n_slabs, x1 = X * (s + 1) / n_slabs;
+         slab_end[s] = x1;
+         if (x1 > x0) {
+            FPGB_CUDA_TRY(cudaMemcpyAsync(d_label + x0 * row, label + x0 * row,
+                                          sizeof(int32_t) * (x1 - x0) * row,
+                                          cudaMemcpyHostToDevice, up));
+            FPGB_CUDA_TRY(cudaMemcpyAsync(d_vec + 3 * x0 * row, vector + 3 * x0 * row,
+                                          sizeof(float) * 3 * (x1 - x0) * row,
+                                          cudaMemcpyHostToDevice, up));
+         }
+         FPGB_CUDA_TRY(cudaEventCreateWithFlags(&ev[s], cudaEventDisableTiming));
+         FPGB_CUDA_TRY(cudaEventRecord(ev[s], up));
+      }
+      const int64_t nu = march_units(P);
+      auto launch = [&](int64_t u0, int64_t u1, int slab, int64_t rows) -> int {
+         cudaStream_t s = march[n_launch++ % kTiltStreams];
+         if (slab >= 0)
+            FPGB_CUDA_TRY(cudaStreamWaitEvent(s, ev[slab], 0));
+         FPGB_TRY(launch_march_units(P, d_label, d_vec, d_img, nullptr, nullptr, nullptr, cnt, u0,
+                                     u1, s));
+         return copy_rows(s, rows);
+      };
+      int waited = -1; // the slabs up to here cover the pending launch
+      int64_t g0 = 0; // first unit of the pending launch
+      for (int c = 0; c < kRayChunks; c++) {
+         const int64_t u0 = nu * c / kRayChunks, u1 = nu * (c + 1) / kRayChunks;
+         if (u1 <= u0)
+            continue;
+         int64_t lo, hi;
+         march_units_x_range(P, u0, u1, lo, hi);
+         int s = 0;
+         while (s < n_slabs - 1 && slab_end[s] <= hi)
+            s++;
+         s = std::max(s, waited);
+         if (s > waited && u0 > g0) { // launch the chunks that the slabs so far cover
+            FPGB_TRY(launch(g0, u0, waited, march_units_rows_done(P, u0)));
+            g0 = u0;
+         }
+         waited = s;
+      }
+      // the rest; its rows are the last (down has waited for every launch)
+      FPGB_TRY(launch(g0, nu, waited, X));
+      for (int i = 0; i < kTiltStreams; i++) {
+         FPGB_CUDA_TRY(cudaEventCreateWithFlags(&joined[i], cudaEventDisableTiming));
+         FPGB_CUDA_TRY(cudaEventRecord(joined[i], march[i]));
+         FPGB_CUDA_TRY(cudaStreamWaitEvent(st, joined[i], 0));
+      }
+      FPGB_CUDA_TRY(cudaStreamWaitEvent(st, ev[n_slabs - 1], 0));
+      return launch_label_check(d_label, X * row, cnt, st);
+   };
+   rc = run();
+   if (rc != FPGB_OK) // whatever was queued is done before the buffers are used again
+      for (cudaStream_t s : march)
+         cudaStreamSynchronize(s);
+   for (cudaStream_t s : {up, down})
+      if (s) {
+         cudaStreamSynchronize(s);
+         cudaStreamDestroy(s);
+      }
+   for (cudaEvent_t e : ev)
+      if (e)
+         cudaEventDestroy(e);
+   for (cudaEvent_t e : done)
+      if (e)
+         cudaEventDestroy(e);
+   for (cudaEvent_t e : joined)
+      if (e)
+         cudaEventDestroy(e);
+   if (ready)
+      cudaEventDestroy(ready);
+   FPGB_TRY(rc);
+   return finish_counters(counters, 1, n_props, true, warnings, st);
+}
+
+static int run_sim_device(const fpgb_setup *setup, const int64_t *dim, const int32_t *d_label,
+                          const float *d_vector, const double *props, int64_t n_props,
+                          double theta, double phi, double *d_image, double *d_t, double *d_d,
+                          double *d_r, fpgb_warnings *warnings, bool check_all,
+                          cudaStream_t st) {
+   MarchPlan mp;
+   FPGB_TRY(plan_march(setup, dim, props, n_props, theta, phi, &mp));
+   return run_sim_planned(mp, d_label, d_vector, n_props, d_image, d_t, d_d, d_r, warnings,
+                          check_all, st);
 }
 
 } // namespace fpgb
@@ -814,10 +874,12 @@ int fpgb_run_simulations_device(const fpgb_setup *setup, const int64_t *dim,
    if (n_tilts == 0)
       return FPGB_OK;
    cudaStream_t st = as_stream(stream);
-   void *counters = nullptr;
-   FPGB_TRY(pool_get(kSlotCounters, sizeof(unsigned long long) * kCounterWords * n_tilts,
-                     &counters, st));
-   auto *cnt = static_cast<unsigned long long *>(counters);
+   // (the buffer is st's: the next call's upload into it follows this call's
+   // marches, which st waits for)
+   char *counters = nullptr;
+   std::vector<char *> tables;
+   FPGB_TRY(upload_march(plans.data(), n_tilts, &counters, tables, st));
+   auto *cnt = reinterpret_cast<unsigned long long *>(counters);
    {
       std::lock_guard<std::mutex> lk(tilt_issue_mutex());
       cudaStream_t side[kTiltStreams];
@@ -837,14 +899,10 @@ int fpgb_run_simulations_device(const fpgb_setup *setup, const int64_t *dim,
          for (; joined < n_side; joined++)
             FPGB_TRY(event_on(st, side[joined]));
          for (int64_t k = 0; k < n_tilts; k++) {
-            cudaStream_t s = side[k % kTiltStreams];
-            void *tables = nullptr;
-            FPGB_TRY(pool_get(kSlotProps, march_table_bytes(plans[k]), &tables, s));
-            FPGB_TRY(init_counters(cnt + k * kCounterWords, s));
-            FPGB_TRY(launch_march(plans[k], d_label, d_vector, d_images[k],
-                                  d_trans ? d_trans[k] : nullptr, d_dir ? d_dir[k] : nullptr,
-                                  d_ret ? d_ret[k] : nullptr, tables, cnt + k * kCounterWords,
-                                  s));
+            FPGB_TRY(launch_march(bind_march(plans[k], d_label, d_vector, tables[k]), d_label,
+                                  d_vector, d_images[k], d_trans ? d_trans[k] : nullptr,
+                                  d_dir ? d_dir[k] : nullptr, d_ret ? d_ret[k] : nullptr,
+                                  cnt + k * kCounterWords, side[k % kTiltStreams]));
          }
          return FPGB_OK;
       };
@@ -859,8 +917,7 @@ int fpgb_run_simulations_device(const fpgb_setup *setup, const int64_t *dim,
       FPGB_TRY(rc);
    }
    if (warnings)
-      for (int64_t k = 0; k < n_tilts; k++)
-         FPGB_TRY(finish_counters(cnt + k * kCounterWords, n_props, false, &warnings[k], st));
+      return finish_counters(counters, n_tilts, n_props, false, warnings, st);
    return FPGB_OK;
 }
 

@@ -97,7 +97,4 @@ int plan_march(const fpgb_setup *setup, const int64_t *dim, const double *props,
 namespace fpgb {
 int check_setup(const fpgb_setup *s);
 size_t march_table_bytes(const MarchPlan &mp);
-int init_counters(unsigned long long *d_counters, cudaStream_t st);
-int finish_counters(const unsigned long long *d_counters, int64_t n_props, bool checked_all,
-                    fpgb_warnings *w, cudaStream_t st);
 } // namespace fpgb

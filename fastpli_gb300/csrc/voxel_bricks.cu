@@ -89,35 +89,130 @@ size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs, int64_t n_segs) 
 }
 
 // ---------------------------------------------------------------- binning ---
+// Pair p of segment S in tile T (x slowest): its brick.
+struct SegBricks {
+   int bx0, by0, bz0;
+   unsigned nx, ny, nz;
+};
+
+__device__ __forceinline__ SegBricks seg_bricks(const SegDev &S) {
+   SegBricks r;
+   r.nx = (unsigned)brick_range(S.lo[0], S.ext[0], kBrickX, r.bx0);
+   r.ny = (unsigned)brick_range(S.lo[1], S.ext[1], kBrickY, r.by0);
+   r.nz = (unsigned)brick_range(S.lo[2], S.ext[2], kBrickZ, r.bz0);
+   return r;
+}
+
+__device__ __forceinline__ int64_t pair_brick(const SegBricks &r, const TileDev &T, unsigned p) {
+   const unsigned i = p / (r.ny * r.nz), q = p - i * (r.ny * r.nz), j = q / r.nz, k = q - j * r.nz;
+   return T.brick_base + ((int64_t)(r.bx0 + i) * T.nb[1] + (r.by0 + j)) * T.nb[2] + (r.bz0 + k);
+}
+
+// kBinLanes lanes share a segment's pairs: a pair is an atomic's latency, and
+// a segment has about ten (15,013 segments: 21 us with one lane each).
+constexpr int kBinLanes = 8;
+
 template <bool FILL>
 __global__ void brick_bin(const SegDev *__restrict__ segs, const int32_t *__restrict__ seg_tile,
                           int64_t n_segs, const TileDev *__restrict__ tiles,
                           unsigned *__restrict__ counts, const unsigned *__restrict__ offsets,
                           unsigned *__restrict__ list, int64_t n_pairs,
                           unsigned long long *__restrict__ counters) {
-   for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_segs;
-        s += (int64_t)gridDim.x * blockDim.x) {
-      const SegDev &S = segs[s];
+   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_segs * kBinLanes;
+        t += (int64_t)gridDim.x * blockDim.x) {
+      const int64_t s = t / kBinLanes;
+      const SegBricks r = seg_bricks(segs[s]);
       const TileDev &T = tiles[seg_tile ? seg_tile[s] : 0];
-      int bx0, by0, bz0;
-      const int64_t nx = brick_range(S.lo[0], S.ext[0], kBrickX, bx0);
-      const int64_t ny = brick_range(S.lo[1], S.ext[1], kBrickY, by0);
-      const int64_t nz = brick_range(S.lo[2], S.ext[2], kBrickZ, bz0);
-      for (int64_t i = 0; i < nx; i++)
-         for (int64_t j = 0; j < ny; j++)
-            for (int64_t k = 0; k < nz; k++) {
-               const int64_t b =
-                   T.brick_base + ((bx0 + i) * T.nb[1] + (by0 + j)) * T.nb[2] + (bz0 + k);
-               const unsigned slot = atomicAdd(&counts[b], 1u);
-               if (FILL) {
-                  const int64_t at = (int64_t)offsets[b] + slot;
-                  if (at < offsets[b + 1] && at < n_pairs)
-                     list[at] = (unsigned)s;
-                  else
-                     atomicOr(&counters[6], (unsigned long long)kStatusOverflow);
-               }
-            }
+      const int64_t n = (int64_t)r.nx * r.ny * r.nz;
+      for (int64_t p = t % kBinLanes; p < n; p += kBinLanes) {
+         const int64_t b = pair_brick(r, T, (unsigned)p);
+         const unsigned slot = atomicAdd(&counts[b], 1u);
+         if (FILL) {
+            const int64_t at = (int64_t)offsets[b] + slot;
+            if (at < offsets[b + 1] && at < n_pairs)
+               list[at] = (unsigned)s;
+            else
+               atomicOr(&counters[6], (unsigned long long)kStatusOverflow);
+         }
+      }
    }
+}
+
+// Count, scan and fill of a small volume by one CTA, its counts in shared
+// memory: one launch for five (25 us on 280 segments and 30 bricks).
+constexpr int64_t kSmallBricks = 4096, kSmallPairs = 16384;
+
+__global__ void __launch_bounds__(1024)
+brick_bin_small(const SegDev *__restrict__ segs, const int32_t *__restrict__ seg_tile,
+                int n_segs, const TileDev *__restrict__ tiles, int n_bricks,
+                unsigned *__restrict__ offsets, unsigned *__restrict__ list, int64_t n_pairs,
+                uint2 *__restrict__ marks, int64_t mark_share, int n_shares,
+                unsigned long long *__restrict__ counters) {
+   __shared__ unsigned count[kSmallBricks], wsum[32];
+   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+   if (mark_share > 0 && t < n_shares) // the marked voxels' lists start empty
+      marks[t * mark_share] = make_uint2(0u, 0u);
+   for (int b = t; b < n_bricks; b += 1024)
+      count[b] = 0;
+   __syncthreads();
+   auto pairs = [&](auto &&f) {
+      for (int i = t; i < n_segs * kBinLanes; i += 1024) {
+         const int s = i / kBinLanes;
+         const SegBricks r = seg_bricks(segs[s]);
+         const TileDev &T = tiles[seg_tile ? seg_tile[s] : 0];
+         const unsigned n = r.nx * r.ny * r.nz; // at most n_bricks
+         for (unsigned p = i % kBinLanes; p < n; p += kBinLanes)
+            f(s, (int)pair_brick(r, T, p));
+      }
+   };
+   pairs([&](int, int b) { atomicAdd(&count[b], 1u); });
+   __syncthreads();
+   // exclusive scan, 4 consecutive bricks per thread
+   const int b0 = 4 * t;
+   unsigned v[4], sum = 0;
+#pragma unroll
+   for (int i = 0; i < 4; i++) {
+      v[i] = b0 + i < n_bricks ? count[b0 + i] : 0u;
+      sum += v[i];
+   }
+   unsigned x = sum;
+#pragma unroll
+   for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o)
+         x += y;
+   }
+   if (lane == 31)
+      wsum[wid] = x;
+   __syncthreads();
+   if (wid == 0) {
+      unsigned w = wsum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+         const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
+         if (lane >= o)
+            w += y;
+      }
+      wsum[lane] = w;
+   }
+   __syncthreads();
+   unsigned run = (wid ? wsum[wid - 1] : 0u) + (x - sum);
+#pragma unroll
+   for (int i = 0; i < 4; i++)
+      if (b0 + i < n_bricks) {
+         offsets[b0 + i] = count[b0 + i] = run; // the fill's cursor
+         run += v[i];
+      }
+   if (t == 0)
+      offsets[n_bricks] = wsum[31];
+   __syncthreads();
+   pairs([&](int s, int b) {
+      const unsigned at = atomicAdd(&count[b], 1u);
+      if ((int64_t)at < n_pairs)
+         list[at] = (unsigned)s;
+      else
+         atomicOr(&counters[6], (unsigned long long)kStatusOverflow);
+   });
 }
 
 // Exclusive scan of the per-brick counts, one CTA walking the counts in tiles
@@ -1061,22 +1156,29 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
    // entries of one launch (entry 0 counts)
    const int64_t mark_share = n_launch <= 1024 ? mark_entries(n_segs) / n_launch : 0;
 
-   FPGB_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(unsigned) * n_bricks, st));
-   if (n_segs > 0) {
-      const unsigned g = (unsigned)std::min<int64_t>((n_segs + 255) / 256, 1 << 20);
-      brick_bin<false><<<g, 256, 0, st>>>(segs, seg_tile, n_segs, tiles, counts, nullptr,
-                                          nullptr, n_pairs, counters);
+   if (n_bricks <= kSmallBricks && n_pairs <= kSmallPairs && n_segs <= kSmallPairs) {
+      brick_bin_small<<<1, 1024, 0, st>>>(segs, seg_tile, (int)n_segs, tiles, (int)n_bricks,
+                                          offsets, list, n_pairs, marks, mark_share, n_launch,
+                                          counters);
       FPGB_CUDA_TRY(cudaGetLastError());
-   }
-   brick_scan<<<1, 1024, 0, st>>>(counts, n_bricks, offsets, marks, mark_share, n_launch,
-                                  counters);
-   FPGB_CUDA_TRY(cudaGetLastError());
-   if (n_segs > 0) {
+   } else {
+      const unsigned g =
+          (unsigned)std::min<int64_t>((n_segs * kBinLanes + 255) / 256, 1 << 20);
       FPGB_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(unsigned) * n_bricks, st));
-      const unsigned g = (unsigned)std::min<int64_t>((n_segs + 255) / 256, 1 << 20);
-      brick_bin<true><<<g, 256, 0, st>>>(segs, seg_tile, n_segs, tiles, counts, offsets, list,
-                                         n_pairs, counters);
+      if (n_segs > 0) {
+         brick_bin<false><<<g, 256, 0, st>>>(segs, seg_tile, n_segs, tiles, counts, nullptr,
+                                             nullptr, n_pairs, counters);
+         FPGB_CUDA_TRY(cudaGetLastError());
+      }
+      brick_scan<<<1, 1024, 0, st>>>(counts, n_bricks, offsets, marks, mark_share, n_launch,
+                                     counters);
       FPGB_CUDA_TRY(cudaGetLastError());
+      if (n_segs > 0) {
+         FPGB_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(unsigned) * n_bricks, st));
+         brick_bin<true><<<g, 256, 0, st>>>(segs, seg_tile, n_segs, tiles, counts, offsets, list,
+                                            n_pairs, counters);
+         FPGB_CUDA_TRY(cudaGetLastError());
+      }
    }
    cudaStream_t alt = chunks && chunks->n > 1 ? chunks->alt : nullptr;
    cudaEvent_t joined[2] = {};
