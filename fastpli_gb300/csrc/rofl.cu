@@ -1,7 +1,7 @@
 // ROFL tilt analysis (src/fastpli/analysis/rofl.py:16-63,
 // _ROFL_with_jacobi.py:47-522; Schmitz et al., Front. Neuroanat. 2018,
 // doi:10.3389/fnana.2018.00075) of every pixel of a 5-tilt image series,
-// one thread per pixel, FP64.
+// a few lanes of a warp per pixel, FP64.
 //
 // Per pixel, as the reference: the untilted direction (epa.direction) starts
 // the fit; the measurements are centered (I / mean - 1) and weighted by
@@ -17,12 +17,15 @@
 // reference's own Jacobian; the same tolerances, scaling and budget of 150
 // evaluations), restated below; n_fev is MINPACK's evaluation count.
 //
-// One thread per pixel, not one warp: GB300 runs FP64 at a small fraction
-// of its FP32 rate, so the kernel is bound by FP64 instructions issued, and
-// a warp per pixel would repeat every per-pixel step (the tilt rotations,
-// the 3 x 3 trust-region algebra) in all 32 lanes.  A thread walks the
-// 5 R measurements of its pixel in the reference's order, so every sum is
-// taken in the order MINPACK (sequential) or numpy (pairwise) takes it.
+// FP64 is what bounds it, in two ways: an SM issues one FP64 warp instruction
+// per 19 cycles whatever its warps, and a lone warp one per 64.  A thread per
+// pixel keeps the instructions of a warp few but makes a map of some thousand
+// pixels wait for the chain of its slowest fit (37 iterations of 13,000
+// instructions: 17 ms); a warp per pixel repeats every per-pixel step (the
+// 3 x 3 trust-region algebra, sums in a fixed order) in 32 lanes.  Four lanes
+// share the measurements, the tilts and the Jacobian's columns of a pixel: the
+// chain is a quarter as long, and the sums of the three columns, each in the
+// order MINPACK (sequential) or numpy (pairwise) takes it, run side by side.
 // Compiled with -fmad=false: products and sums round separately, as in the
 // reference, except where a fused multiply-add is written out.
 #include <cuda_runtime.h>
@@ -42,6 +45,7 @@ constexpr int kRoflSmallRot = 10; // the usual 6 - 9 rotations: 50 measurements
 struct RoflParams {
    int n_rot;
    int grad_mode;
+   int inv_rot; // i / n_rot = i * inv_rot >> 16 for i < 5 n_rot
    double tau, gain, dir_offset, cos_tau;
    double rho[kRoflMaxRot];    // linspace(0, pi, R + 1)[:-1] + dir_offset
    double rho2s[kRoflMaxRot];  // sin / cos of 2 linspace(0, pi, R, False)
@@ -124,109 +128,125 @@ __device__ __forceinline__ double np_dot3(const double *a, double v0, double v1,
    return fma(a[2], v2, fma(a[0], v0, a[1] * v1));
 }
 
-// (direction, inclination, t_rel) seen in tilt j (:150-183), folded and
-// |t_rel| as the model uses them (:186-212)
-struct Tilted {
-   double phi[5], alpha[5], trel[5];
+// The G lanes of one pixel.
+template <int G> struct Lanes {
+   int g;         // this lane's place
+   unsigned mask; // the lanes' bits in the warp
+   __device__ __forceinline__ Lanes() {
+      const int lane = threadIdx.x & 31;
+      g = lane % G;
+      mask = (G == 32 ? ~0u : (1u << (G & 31)) - 1u) << (lane - g);
+   }
+   __device__ __forceinline__ void sync() const {
+      if (G > 1)
+         __syncwarp(mask);
+   }
+   __device__ __forceinline__ double from(double v, int lane) const {
+      return G > 1 ? __shfl_sync(mask, v, lane, G) : v;
+   }
 };
 
-__device__ __forceinline__ void tilted(const RoflParams &P, double phi, double alpha,
-                                       double trel, Tilted &T) {
-   double sp, cp, sa, ca;
-   ol_sincos(phi, &sp, &cp);
-   ol_sincos(alpha, &sa, &ca);
-   const double v0 = ca * cp, v1 = ca * sp, v2 = sa;
-   T.phi[0] = phi;
-   T.alpha[0] = alpha;
-   T.trel[0] = trel;
-#pragma unroll
-   for (int t = 0; t < 4; t++) {
-      const double *M = P.mat[t];
-      const double w0 = np_dot3(M, v0, v1, v2);
-      const double w1 = np_dot3(M + 3, v0, v1, v2);
-      const double w2 = np_dot3(M + 6, v0, v1, v2);
-      T.phi[t + 1] = ol_atan(w1 / w0);
-      T.alpha[t + 1] = ol_asin(w2);
-      T.trel[t + 1] = trel / P.cos_tau;
-   }
-#pragma unroll
-   for (int j = 0; j < 5; j++) {
-      symmetrize(T.phi[j], T.alpha[j]);
-      T.trel[j] = fabs(T.trel[j]);
-   }
-}
+// Per-tilt values of the model at one point, next to the pixel's arrays.
+struct TiltValues {
+   double phi[5], alpha[5], amp[5];
+};
 
 // The model's factors at one point of the fit: wave[i] = sin 2 (rho - phi) of
 // every measurement, i = tilt * R + rotation (the order of the reference's
 // flattened intensity curves, :186-212), and cos^2 of each tilt's inclination.
-// t_rel enters neither, so the 6 start points of one inclination and the
+// (direction, inclination) in the tilts: :150-183, folded as the model uses
+// them.  t_rel enters neither, so the 6 start points of one inclination and the
 // forward difference in t_rel share them.  base (or null): the waves of a
 // point with the same phi, whose untilted ones are the same.  Out of line,
 // like the Jacobian and the trust-region step below: one copy of each large
-// body keeps the kernel's code in the instruction cache while the threads of a
+// body keeps the kernel's code in the instruction cache while the pixels of a
 // warp are in different phases of their fits.
+template <int G>
 __device__ __noinline__ void px_waves(const RoflParams &P, double phi, double alpha,
-                                      const double *base, double *wave, double cos2[5]) {
-   Tilted T;
-   tilted(P, phi, alpha, 0.0, T);
-   const int R = P.n_rot;
-#pragma unroll 1
-   for (int j = 0; j < 5; j++) {
-      const double ca = ol_cos(T.alpha[j]);
-      cos2[j] = ca * ca;
-      const int i0 = j * R;
-      if (j == 0 && base) {
-         for (int k = 0; k < R; k++)
-            wave[k] = base[k];
-         continue;
+                                      const double *base, double *wave, TiltValues &T,
+                                      double cos2[5]) {
+   const Lanes<G> L;
+   double sp, cp, sa, ca;
+   ol_sincos(phi, &sp, &cp);
+   ol_sincos(alpha, &sa, &ca);
+   const double v0 = ca * cp, v1 = ca * sp, v2 = sa;
+   for (int t = L.g; t < 5; t += G) { // tilts 1 .. 4, then the untilted
+      const int j = t < 4 ? t + 1 : 0;
+      double ph = phi, al = alpha;
+      if (t < 4) {
+         const double *M = P.mat[t];
+         const double w0 = np_dot3(M, v0, v1, v2);
+         const double w1 = np_dot3(M + 3, v0, v1, v2);
+         const double w2 = np_dot3(M + 6, v0, v1, v2);
+         ph = ol_atan(w1 / w0);
+         al = ol_asin(w2);
       }
-      for (int k = 0; k < R; k++)
-         wave[i0 + k] = ol_sin(2.0 * (P.rho[k] - T.phi[j]));
+      symmetrize(ph, al);
+      const double c = ol_cos(al);
+      T.phi[j] = ph;
+      T.alpha[j] = al;
+      cos2[j] = c * c;
    }
+   L.sync();
+   const int R = P.n_rot, M = 5 * R;
+   for (int i = L.g + (base ? R : 0); i < M; i += G) {
+      const int j = i * P.inv_rot >> 16;
+      wave[i] = ol_sin(2.0 * (P.rho[i - j * R] - T.phi[j]));
+   }
+   if (base && base != wave)
+      for (int k = L.g; k < R; k += G)
+         wave[k] = base[k];
+   L.sync();
+}
+
+// |t_rel| as the model uses it in tilt j
+__device__ __forceinline__ double tilt_trel(const RoflParams &P, int j, double trel) {
+   return fabs(j == 0 ? trel : trel / P.cos_tau);
 }
 
 // weighted residuals r[i] = w[i] (model_i - c[i]) (_residuum, :407-410)
+template <int G>
 __device__ __noinline__ void px_residuals(const RoflParams &P, const double *c, const double *w,
-                                          const double *wave, const double cos2[5], double trel,
-                                          double *r) {
-   const int R = P.n_rot;
-   const double t0 = fabs(trel), t1 = fabs(trel / P.cos_tau); // |t_rel| seen in the tilts
-#pragma unroll 1
-   for (int j = 0; j < 5; j++) {
-      const double amp = ol_sin(M_PI / 2.0 * (j == 0 ? t0 : t1) * cos2[j]);
-      const int i0 = j * R;
-      for (int k = 0; k < R; k++)
-         r[i0 + k] = w[i0 + k] * (amp * wave[i0 + k] - c[i0 + k]);
-   }
+                                          const double *wave, const double cos2[5],
+                                          TiltValues &T, double trel, double *r) {
+   const Lanes<G> L;
+   for (int j = L.g; j < 5; j += G)
+      T.amp[j] = ol_sin(M_PI / 2.0 * tilt_trel(P, j, trel) * cos2[j]);
+   L.sync();
+   const int R = P.n_rot, M = 5 * R;
+   for (int i = L.g; i < M; i += G)
+      r[i] = w[i] * (T.amp[i * P.inv_rot >> 16] * wave[i] - c[i]);
+   L.sync();
 }
 
 // the reference's Jacobian of the model with respect to each tilt's own
-// angles (_calc_Jacobi, :215-258), weighted (_weighted_jacobi, :393-403):
-// columns J[0..2][i] at J + col[0..2]; used by grad_mode and by the
-// covariance
-__device__ __noinline__ void px_jacobi(const RoflParams &P, const double *w, double phi,
-                                          double alpha, double trel, double *J,
-                                          const int col[3]) {
-   Tilted T;
-   tilted(P, phi, alpha, trel, T);
+// angles (_calc_Jacobi, :215-258), weighted (_weighted_jacobi, :393-403), at
+// the point that wave and T.alpha are of: columns J[0..2][i] at J + col[0..2];
+// used by grad_mode and by the covariance
+template <int G>
+__device__ __noinline__ void px_jacobi(const RoflParams &P, const double *w, const double *wave,
+                                       const TiltValues &T, double trel, double *J,
+                                       const int col[3]) {
+   const Lanes<G> L;
    const int R = P.n_rot;
-#pragma unroll
+#pragma unroll 1
    for (int j = 0; j < 5; j++) {
+      const double tr = tilt_trel(P, j, trel);
       const double ca = ol_cos(T.alpha[j]), sa = ol_sin(T.alpha[j]);
-      const double arg = M_PI / 2.0 * T.trel[j] * (ca * ca);
+      const double arg = M_PI / 2.0 * tr * (ca * ca);
       const double sarg = ol_sin(arg), carg = ol_cos(arg);
-      const double dal = -M_PI * T.trel[j] * ca * sa * carg; // times s2
-      const double dtr = M_PI / 2.0 * (ca * ca);             // times s2, cos(arg)
-      const int i0 = j * R;
-      for (int k = 0; k < R; k++) {
-         const double d2 = 2.0 * (P.rho[k] - T.phi[j]);
-         const double s2 = ol_sin(d2), c2 = ol_cos(d2);
-         const double wi = w[i0 + k];
-         J[col[0] + i0 + k] = -2.0 * c2 * sarg * wi;
-         J[col[1] + i0 + k] = dal * s2 * wi;
-         J[col[2] + i0 + k] = dtr * s2 * carg * wi;
+      const double dal = -M_PI * tr * ca * sa * carg; // times s2
+      const double dtr = M_PI / 2.0 * (ca * ca);      // times s2, cos(arg)
+      for (int k = L.g; k < R; k += G) {
+         const int i = j * R + k;
+         const double s2 = wave[i], c2 = ol_cos(2.0 * (P.rho[k] - T.phi[j]));
+         const double wi = w[i];
+         J[col[0] + i] = -2.0 * c2 * sarg * wi;
+         J[col[1] + i] = dal * s2 * wi;
+         J[col[2] + i] = dtr * s2 * carg * wi;
       }
    }
+   L.sync();
 }
 
 // numpy's pairwise sum (np.sum of a contiguous float64 array, n <= 256):
@@ -262,16 +282,51 @@ template <class Get> __device__ __forceinline__ double np_sum(Get get, int n) {
    return np_sum_block(get, 0, n2) + np_sum_block(get, n2, n - n2);
 }
 
-// sum of squares in MINPACK's enorm order (sequential; every value of these
-// fits lies in enorm's unscaled range or is zero)
-__device__ __noinline__ double seq_sumsq(const double *r, int n) {
-   double s = 0.0;
-   for (int i = 0; i < n; i++)
-      s = s + r[i] * r[i];
+// np.sum(np.square(r)) of n values, 8 <= n <= 256, by the pixel's lanes: numpy's
+// 8 partial sums are spread over them.
+template <int G> __device__ __forceinline__ double np_sumsq_block(const Lanes<G> &L,
+                                                                  const double *r, int n) {
+   constexpr int kOwn = G >= 8 ? 1 : 8 / G; // partial sums of a lane: g, g + G, ...
+   double a[kOwn];
+#pragma unroll
+   for (int o = 0; o < kOwn; o++) {
+      const double v = r[(L.g + o * G) & 7];
+      a[o] = v * v;
+   }
+   int i = 8;
+   for (; i + 8 <= n; i += 8)
+#pragma unroll
+      for (int o = 0; o < kOwn; o++) {
+         const double v = r[i + ((L.g + o * G) & 7)];
+         a[o] += v * v;
+      }
+   // ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7)): sums of two commute
+#pragma unroll
+   for (int o = 0; o < kOwn; o++) {
+      a[o] = a[o] + __shfl_xor_sync(L.mask, a[o], 1);
+      a[o] = a[o] + __shfl_xor_sync(L.mask, a[o], 2);
+   }
+   double s = kOwn == 2 ? a[0] + a[kOwn - 1] : a[0] + __shfl_xor_sync(L.mask, a[0], 4);
+   for (; i < n; i++)
+      s += r[i] * r[i];
    return s;
 }
 
-// sum over i of a[i] b[i], sequential (qrfac's and qtf's column products)
+template <int G> __device__ __forceinline__ double np_sumsq(const Lanes<G> &L, const double *r,
+                                                            int n) {
+   static_assert(G == 1 || G == 4 || G >= 8, "the partial sums pair up within the lanes");
+   if constexpr (G == 1)
+      return np_sum([&](int i) { return r[i] * r[i]; }, n);
+   if (n <= 128)
+      return np_sumsq_block(L, r, n);
+   int n2 = n / 2;
+   n2 -= n2 % 8;
+   return np_sumsq_block(L, r, n2) + np_sumsq_block(L, r + n2, n - n2);
+}
+
+// sum over i of a[i] b[i], sequential: MINPACK's enorm (a = b; every value of
+// these fits lies in its unscaled range or is zero), qrfac's and qtf's column
+// products.  By one lane; lanes may run different ones side by side.
 __device__ __noinline__ double seq_dot(const double *a, const double *b, int n) {
    double s = 0.0;
    for (int i = 0; i < n; i++)
@@ -279,10 +334,20 @@ __device__ __noinline__ double seq_dot(const double *a, const double *b, int n) 
    return s;
 }
 
-// b[i] = b[i] - t a[i] (qrfac's Householder update)
-__device__ __noinline__ void seq_axmy(const double *a, double *b, double t, int n) {
+// The same of one pair of vectors by all lanes: the products first, into t.
+template <int G>
+__device__ __noinline__ double lanes_dot(const double *a, const double *b, int n, double *t) {
+   if (G == 1)
+      return seq_dot(a, b, n);
+   const Lanes<G> L;
+   for (int i = L.g; i < n; i += G)
+      t[i] = a[i] * b[i];
+   L.sync();
+   double s = 0.0;
    for (int i = 0; i < n; i++)
-      b[i] = b[i] - t * a[i];
+      s = s + t[i];
+   L.sync();
+   return s;
 }
 
 // x^3 rounded once, as numpy's x**3 (pow) gives it: the exact cube as a
@@ -480,32 +545,41 @@ __device__ __noinline__ void mp_lmpar(double r[3][3], const int ipvt[3], const d
    }
 }
 
-// The fit for one pixel (one thread): x in: the start point, out: the last
-// accepted point; F (2 x MAXM) holds the residuals, *cur the half that
-// holds them at x on return, S (2 x MAXM) the model's waves likewise; J
-// (3 x MAXM) is the Jacobian's workspace.
-// Returns MINPACK's info (5: evaluation budget spent); nfev counts as
-// MINPACK counts (lmdif: 1 + 3 per Jacobian + 1 per trial step; lmder:
-// 1 + 1 per trial step).
-template <int MAXM>
-__device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int M, double x[3],
-                      double *F, int &cur, double *J, double *S, int &nfev) {
+// A pixel's arrays in shared memory: measurements c, weights w, residuals F and
+// waves S of two points, the Jacobian J (also a third wave's place) and
+// products t.
+template <int MAXM> struct PixelArrays {
+   double c[MAXM], w[MAXM], F[2 * MAXM], S[2 * MAXM], J[3 * MAXM], t[MAXM];
+   double cos2[3][5]; // of the points of S[0], S[1] and of a difference
+   double trans[5];
+   TiltValues T;
+};
+
+// The fit for one pixel (G lanes, which all hold the same scalars): x in: the
+// start point, out: the last accepted point; A.F + cur * MAXM holds its
+// residuals on return.  Returns MINPACK's info (5: evaluation budget spent);
+// nfev counts as MINPACK counts (lmdif: 1 + 3 per Jacobian + 1 per trial step;
+// lmder: 1 + 1 per trial step).
+template <int MAXM, int G>
+__device__ int mp_fit(const RoflParams &P, PixelArrays<MAXM> &A, int M, double x[3], int &cur,
+                      int &nfev) {
+   const Lanes<G> L;
    const double epsfd = sqrt(kMpEps); // sqrt(max(epsfcn, epsmch)), epsfcn = eps
-   double cos2[10], cos2p[5]; // of both points, as F and S
+   double *J = A.J;
    cur = 0;
-   px_waves(P, x[0], x[1], nullptr, S, cos2);
-   px_residuals(P, c, w, S, cos2, x[2], F);
+   px_waves<G>(P, x[0], x[1], nullptr, A.S, A.T, A.cos2[0]);
+   px_residuals<G>(P, A.c, A.w, A.S, A.cos2[0], A.T, x[2], A.F);
    nfev = 1;
-   double fnorm = sqrt(seq_sumsq(F, M));
+   double fnorm = sqrt(lanes_dot<G>(A.F, A.F, M, A.t));
    double par = 0.0, delta = 0.0, xnorm = 0.0;
    double dg[3] = {1.0, 1.0, 1.0};
    int iter = 1;
    for (;;) {
-      double *fv = F + cur * MAXM, *wa4 = F + (1 - cur) * MAXM;
+      double *fv = A.F + cur * MAXM, *wa4 = A.F + (1 - cur) * MAXM;
       // the Jacobian's columns, J + col[j] after the pivoting swaps
       int col[3] = {0, MAXM, 2 * MAXM};
-      if (P.grad_mode) {
-         px_jacobi(P, w, x[0], x[1], x[2], J, col);
+      if (P.grad_mode) { // (T is the accepted point's: the trial's, just evaluated)
+         px_jacobi<G>(P, A.w, A.S + cur * MAXM, A.T, x[2], J, col);
       } else { // fdjac2
 #pragma unroll 1
          for (int j = 0; j < 3; j++) {
@@ -514,28 +588,35 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
             if (h == 0.0)
                h = epsfd;
             double *Jj = J + col[j];
-            const double *Sc = S + cur * MAXM, *wave = Sc, *cc = cos2 + 5 * cur;
+            const double *Sc = A.S + cur * MAXM, *wave = Sc, *cc = A.cos2[cur];
             if (j < 2) { // (the waves take column 2's place, not yet filled)
                double *Sp = J + col[2];
-               px_waves(P, j == 0 ? temp + h : x[0], j == 1 ? temp + h : x[1],
-                        j == 1 ? Sc : nullptr, Sp, cos2p);
+               px_waves<G>(P, j == 0 ? temp + h : x[0], j == 1 ? temp + h : x[1],
+                           j == 1 ? Sc : nullptr, Sp, A.T, A.cos2[2]);
                wave = Sp;
-               cc = cos2p;
+               cc = A.cos2[2];
             }
-            px_residuals(P, c, w, wave, cc, j == 2 ? temp + h : x[2], Jj);
+            px_residuals<G>(P, A.c, A.w, wave, cc, A.T, j == 2 ? temp + h : x[2], Jj);
             const Divisor by_h(h);
-            for (int i = 0; i < M; i++)
+            for (int i = L.g; i < M; i += G)
                Jj[i] = by_h.quotient(Jj[i] - fv[i]);
          }
+         L.sync();
          nfev += 3;
       }
-      // qrfac with column pivoting
+      // qrfac with column pivoting; the columns' norms side by side
       double acnorm[3], rdiag[3], wa[3];
       int ipvt[3] = {0, 1, 2};
+      {
+         const double *a = J + min(L.g, 2) * MAXM;
+         const double norm = sqrt(seq_dot(a, a, M));
 #pragma unroll
-      for (int j = 0; j < 3; j++) {
-         acnorm[j] = sqrt(seq_sumsq(J + col[j], M));
-         rdiag[j] = wa[j] = acnorm[j];
+         for (int j = 0; j < 3; j++) {
+            acnorm[j] = L.from(norm, j);
+            if (G == 1 && j)
+               acnorm[j] = sqrt(seq_dot(J + j * MAXM, J + j * MAXM, M));
+            rdiag[j] = wa[j] = acnorm[j];
+         }
       }
 #pragma unroll
       for (int j = 0; j < 3; j++) {
@@ -557,30 +638,48 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
                ipvt[k] = t;
             }
          double *aj = J + col[j];
-         double ajnorm = sqrt(seq_sumsq(aj + j, M - j));
+         // (the first column is as it was for acnorm)
+         double ajnorm =
+             j == 0 ? (ipvt[0] == 0 ? acnorm[0] : ipvt[0] == 1 ? acnorm[1] : acnorm[2])
+                    : sqrt(lanes_dot<G>(aj + j, aj + j, M - j, A.t));
          if (ajnorm != 0.0) {
             if (aj[j] < 0.0)
                ajnorm = -ajnorm;
+            L.sync(); // every lane has read aj[j]
             const Divisor by_norm(ajnorm);
-            for (int i = j; i < M; i++)
-               aj[i] = by_norm.quotient(aj[i]);
-            aj[j] = aj[j] + 1.0;
+            for (int i = j + L.g; i < M; i += G) {
+               const double q = by_norm.quotient(aj[i]);
+               aj[i] = i == j ? q + 1.0 : q;
+            }
+            L.sync();
+            double sums[2] = {0.0, 0.0}; // of columns j + 1, j + 2
+            if (j == 0) {
+               const double sum = seq_dot(aj, J + ((L.g & 1) ? col[2] : col[1]), M);
+               sums[0] = L.from(sum, 0);
+               sums[1] = G == 1 ? seq_dot(aj, J + col[2], M) : L.from(sum, 1);
+            } else if (j == 1) {
+               sums[0] = lanes_dot<G>(aj + 1, J + col[2] + 1, M - 1, A.t);
+            }
 #pragma unroll
             for (int k = j + 1; k < 3; k++) {
                double *ak = J + col[k];
-               const double sum = seq_dot(aj + j, ak + j, M - j);
-               const double temp = sum / aj[j];
-               seq_axmy(aj + j, ak + j, temp, M - j);
+               const double temp = sums[k - j - 1] / aj[j];
+               for (int i = j + L.g; i < M; i += G)
+                  ak[i] = ak[i] - temp * aj[i];
+            }
+            L.sync();
+#pragma unroll
+            for (int k = j + 1; k < 3; k++)
                if (rdiag[k] != 0.0) {
+                  const double *ak = J + col[k];
                   const double t2 = ak[j] / rdiag[k];
                   rdiag[k] = rdiag[k] * sqrt(fmax(0.0, 1.0 - t2 * t2));
                   const double q2 = rdiag[k] / wa[k];
                   if (0.05 * (q2 * q2) <= kMpEps) {
-                     rdiag[k] = sqrt(seq_sumsq(ak + j + 1, M - j - 1));
+                     rdiag[k] = sqrt(seq_dot(ak + j + 1, ak + j + 1, M - j - 1));
                      wa[k] = rdiag[k];
                   }
                }
-            }
          }
          rdiag[j] = -ajnorm;
       }
@@ -597,20 +696,25 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
       // (Q^T fvec) in its first 3 rows (wa4 is the residual buffer's free
       // half), and R's diagonal restored
       double qtf[3];
-      for (int i = 0; i < M; i++)
+      for (int i = L.g; i < M; i += G)
          wa4[i] = fv[i];
+      L.sync();
 #pragma unroll
       for (int j = 0; j < 3; j++) {
          double *aj = J + col[j];
-         if (aj[j] != 0.0) {
-            const double sum = seq_dot(aj + j, wa4 + j, M - j);
-            const double temp = -sum / aj[j];
-            for (int i = j; i < M; i++)
+         const double ajj = aj[j];
+         if (ajj != 0.0) {
+            const double sum = lanes_dot<G>(aj + j, wa4 + j, M - j, A.t);
+            const double temp = -sum / ajj;
+            for (int i = j + L.g; i < M; i += G)
                wa4[i] = wa4[i] + aj[i] * temp;
          }
-         aj[j] = rdiag[j];
+         L.sync();
+         if (L.g == 0)
+            aj[j] = rdiag[j];
          qtf[j] = wa4[j];
       }
+      L.sync();
       double R[3][3];
 #pragma unroll
       for (int j = 0; j < 3; j++)
@@ -657,13 +761,10 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
          const double pnorm = mp_norm3(w3);
          if (iter == 1)
             delta = fmin(delta, pnorm);
-         {
-            double *Sn = S + (1 - cur) * MAXM, *cn = cos2 + 5 * (1 - cur);
-            px_waves(P, w2[0], w2[1], nullptr, Sn, cn);
-            px_residuals(P, c, w, Sn, cn, w2[2], wa4);
-         }
+         px_waves<G>(P, w2[0], w2[1], nullptr, A.S + (1 - cur) * MAXM, A.T, A.cos2[1 - cur]);
+         px_residuals<G>(P, A.c, A.w, A.S + (1 - cur) * MAXM, A.cos2[1 - cur], A.T, w2[2], wa4);
          nfev++;
-         const double fnorm1 = sqrt(seq_sumsq(wa4, M));
+         const double fnorm1 = sqrt(lanes_dot<G>(wa4, wa4, M, A.t));
          double actred = -1.0;
          if (0.1 * fnorm1 < fnorm) {
             const double t = fnorm1 / fnorm;
@@ -728,124 +829,169 @@ __device__ int mp_fit(const RoflParams &P, const double *c, const double *w, int
    }
 }
 
-// One thread per pixel.  MAXR bounds n_rot: the measurement arrays of the
-// pixel (7 x 5 MAXR doubles) live in the thread's local memory, which is
-// interleaved across the threads of a warp and cached in L1.  One warp per
-// CTA: an SM issues one FP64 warp instruction per 19 cycles, whatever its warps,
-// and a lone warp one per 64, so a map of a few warps per SM ends with its
-// fullest SM (160 x 150 pixels: 188 CTAs of 4 warps gave 36 SMs twice the
-// work).  80 registers (24 warps per SM).
-constexpr int kRoflThreads = 32;
-
-template <int MAXR>
-__global__ void __launch_bounds__(kRoflThreads, 24)
+// One warp per CTA, 32 / G pixels at a time, taken from a counter by the warp
+// (its pixels start together, so that their phases coincide).  MAXR bounds
+// n_rot.  The arrays of the pixels (10 x 5 MAXR doubles each) live in shared
+// memory, 33 KB per warp with G = 4 and 10 rotations, 26 KB with 16 and 32; with
+// a lane per pixel in its local memory, interleaved across the warp and cached
+// in L1 (held to 80 registers: 24 warps per SM).
+template <int MAXR, int G>
+__global__ void __launch_bounds__(32, G == 1 ? 24 : 0)
 rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__restrict__ mask,
          const RoflParams P, double *__restrict__ out, unsigned long long *__restrict__ status) {
-   constexpr int MAXM = 5 * MAXR;
-   const int R = P.n_rot, M = 5 * R;
-   double c[MAXM], w[MAXM], F[2 * MAXM], J[3 * MAXM], S[2 * MAXM];
-   // pixels are taken one at a time from a counter (status[1]): a thread
-   // whose fit ended early starts the next pixel instead of idling until
-   // the slowest pixel of a fixed share is done
+   constexpr int MAXM = 5 * MAXR, kPixels = 32 / G;
+   extern __shared__ __align__(16) unsigned char s_arrays[];
+   PixelArrays<G == 1 ? MAXM : 1> own; // (local memory)
+   const int lane = threadIdx.x & 31, R = P.n_rot, M = 5 * R;
+   PixelArrays<MAXM> &A =
+       G == 1 ? reinterpret_cast<PixelArrays<MAXM> &>(own)
+              : reinterpret_cast<PixelArrays<MAXM> *>(s_arrays)[lane / G];
+   const Lanes<G> L;
    for (;;) {
-      const int64_t p = (int64_t)atomicAdd(&status[1], 1ull);
-      if (p >= n_pix)
+      unsigned long long first = 0;
+      if (lane == 0)
+         first = atomicAdd(&status[1], (unsigned long long)kPixels);
+      first = __shfl_sync(0xFFFFFFFFu, first, 0);
+      if (first >= (unsigned long long)n_pix)
          break;
-      double *o = out + 8 * p;
-      if (mask && !mask[p]) {
-#pragma unroll
-         for (int e = 0; e < 8; e++)
-            o[e] = nan("");
-         continue;
-      }
-      // tilt t, rotation k of pixel p: data[(t * n_pix + p) * R + k]
-      double trans[5];
-#pragma unroll
-      for (int t = 0; t < 5; t++) {
-         const double *d = data + (t * n_pix + p) * R;
-         trans[t] = np_sum([&](int k) { return d[k]; }, R) / R; // np.mean
-      }
-      // epa.direction of the untilted series (epa.py:48-77) + dir_offset
-      double phi0;
-      {
-         const double *d0 = data + p * R;
-         const double a1 = 2.0 * np_sum([&](int k) { return d0[k] * P.rho2s[k]; }, R) / R;
-         const double b1 = 2.0 * np_sum([&](int k) { return d0[k] * P.rho2c[k]; }, R) / R;
-         phi0 = pymod(0.5 * atan2(-b1, a1) + M_PI, M_PI) + P.dir_offset;
-      }
-      // _calc_centered_vals (:47-61)
-#pragma unroll
-      for (int t = 0; t < 5; t++) {
-         const double *d = data + (t * n_pix + p) * R;
-         const double tr = trans[t];
-         const Divisor by_tr(tr), by_tr2(tr * tr), by_tr3r(cube_rn(tr) * R);
-         for (int k = 0; k < R; k++) {
-            const double v = d[k];
-            c[t * R + k] = by_tr.quotient(v) - 1.0;
-            w[t * R + k] = 1.0 / sqrt(P.gain * (by_tr2.quotient(v) + by_tr3r.quotient(v * v)));
+      const int64_t p = (int64_t)first + lane / G;
+      if (p < n_pix && mask && !mask[p]) {
+         for (int e = L.g; e < 8; e += G)
+            out[8 * p + e] = nan("");
+      } else if (p < n_pix) {
+         // tilt t, rotation k of pixel p: data[(t * n_pix + p) * R + k]
+         for (int t = L.g; t < 5; t += G) {
+            const double *d = data + (t * n_pix + p) * R;
+            A.trans[t] = np_sum([&](int k) { return d[k]; }, R) / R; // np.mean
          }
-      }
-      // start grid (:261-328): inclination outer, t_rel inner, the first
-      // minimum of the pairwise row sums (np.argmin: a NaN wins)
-      double x[3] = {phi0, P.incl[0], P.trel[0]};
-      {
-         double best = INFINITY;
-         for (int a = 0; a < 6; a++) {
-            double cos2[5];
-            px_waves(P, phi0, P.incl[a], a ? S : nullptr, S, cos2);
-            for (int t = 0; t < 6; t++) {
-               px_residuals(P, c, w, S, cos2, P.trel[t], F);
-               const double cost = np_sum([&](int i) { return F[i] * F[i]; }, M);
-               if (cost < best || (isnan(cost) && !isnan(best))) {
-                  best = cost;
-                  x[1] = P.incl[a];
-                  x[2] = P.trel[t];
+         L.sync();
+         // epa.direction of the untilted series (epa.py:48-77) + dir_offset
+         double phi0;
+         {
+            const double *d0 = data + p * R, *wave = (L.g & 1) ? P.rho2c : P.rho2s;
+            const double sum = np_sum([&](int k) { return d0[k] * wave[k]; }, R);
+            const double cosine = G == 1 ? np_sum([&](int k) { return d0[k] * P.rho2c[k]; }, R)
+                                         : L.from(sum, 1);
+            const double a1 = 2.0 * L.from(sum, 0) / R, b1 = 2.0 * cosine / R;
+            phi0 = pymod(0.5 * atan2(-b1, a1) + M_PI, M_PI) + P.dir_offset;
+         }
+         // _calc_centered_vals (:47-61)
+#pragma unroll 1
+         for (int t = 0; t < 5; t++) {
+            const double *d = data + (t * n_pix + p) * R;
+            const double tr = A.trans[t], tr2 = tr * tr, tr3r = cube_rn(tr) * R;
+            for (int k = L.g; k < R; k += G) {
+               const double v = d[k];
+               A.c[t * R + k] = v / tr - 1.0;
+               A.w[t * R + k] = 1.0 / sqrt(P.gain * (v / tr2 + v * v / tr3r));
+            }
+         }
+         L.sync();
+         // start grid (:261-328): inclination outer, t_rel inner, the first
+         // minimum of the pairwise row sums (np.argmin: a NaN wins)
+         double x[3] = {phi0, P.incl[0], P.trel[0]};
+         {
+            double best = INFINITY;
+#pragma unroll 1
+            for (int a = 0; a < 6; a++) {
+               px_waves<G>(P, phi0, P.incl[a], a ? A.S : nullptr, A.S, A.T, A.cos2[0]);
+#pragma unroll 1
+               for (int t = 0; t < 6; t++) {
+                  px_residuals<G>(P, A.c, A.w, A.S, A.cos2[0], A.T, P.trel[t], A.F);
+                  const double cost = np_sumsq(L, A.F, M);
+                  L.sync();
+                  if (cost < best || (isnan(cost) && !isnan(best))) {
+                     best = cost;
+                     x[1] = P.incl[a];
+                     x[2] = P.trel[t];
+                  }
                }
             }
          }
+         // MINPACK's fit, as scipy.optimize.leastsq runs it for the reference
+         int n_fev = 0, cur = 0;
+         const int info = mp_fit<MAXM, G>(P, A, M, x, cur, n_fev);
+         if (info == 5 && L.g == 0)
+            atomicAdd(&status[0], 1ull); // evaluation budget reached
+         const double cost = np_sumsq(L, A.F + cur * MAXM, M); // np.sum(np.square)
+         L.sync();
+         // result (:488-520): fold, |t_rel|, covariance from the reference's
+         // Jacobian at the folded point and its own 3x3 inverse
+         double d = x[0], a = x[1];
+         symmetrize(d, a);
+         const double t = fabs(x[2]);
+         const double sigma_sq = cost / (double)(M - 3);
+         const int col[3] = {0, MAXM, 2 * MAXM};
+         px_waves<G>(P, d, a, nullptr, A.S, A.T, A.cos2[0]);
+         px_jacobi<G>(P, A.w, A.S, A.T, t, A.J, col);
+         // the six sums of products, a lane each
+         double s[6], own[(6 + G - 1) / G];
+#pragma unroll
+         for (int o = 0; o < (6 + G - 1) / G; o++) {
+            const int e = min(L.g + o * G, 5); // (0 0) (0 1) (0 2) (1 1) (1 2) (2 2)
+            const int i = e < 3 ? 0 : e < 5 ? 1 : 2, j = e < 3 ? e : e < 5 ? e - 2 : 2;
+            own[o] = seq_dot(A.J + i * MAXM, A.J + j * MAXM, M);
+         }
+#pragma unroll
+         for (int e = 0; e < 6; e++)
+            s[e] = L.from(own[e / G], e % G);
+         const double mm[9] = {s[0], s[1], s[2], s[1], s[3], s[4], s[2], s[4], s[5]};
+         // _invertmatrix (:14-44) with the reference's determinant expression
+         // (its fourth term is m20 * m12, without a third factor)
+         const double det = mm[0] * mm[4] * mm[8] + mm[3] * mm[7] * mm[2] + mm[6] * mm[5] -
+                            mm[0] * mm[7] * mm[5] - mm[6] * mm[4] * mm[2] - mm[3] * mm[1] * mm[8];
+         const double i00 = (mm[4] * mm[8] - mm[5] * mm[7]) / det;
+         const double i11 = (mm[0] * mm[8] - mm[2] * mm[6]) / det;
+         const double i22 = (mm[0] * mm[4] - mm[1] * mm[3]) / det;
+         if (L.g == 0) {
+            double *o = out + 8 * p;
+            o[0] = d;
+            o[1] = a;
+            o[2] = t;
+            o[3] = sqrt(fabs(i00 * sigma_sq));
+            o[4] = sqrt(fabs(i11 * sigma_sq));
+            o[5] = sqrt(fabs(i22 * sigma_sq));
+            o[6] = cost;
+            o[7] = (double)n_fev;
+         }
       }
-      // MINPACK's fit, as scipy.optimize.leastsq runs it for the reference
-      int n_fev = 0, cur = 0;
-      const int info = mp_fit<MAXM>(P, c, w, M, x, F, cur, J, S, n_fev);
-      if (info == 5)
-         atomicAdd(&status[0], 1ull); // evaluation budget reached
-      const double *fv = F + cur * MAXM;
-      const double cost = np_sum([&](int i) { return fv[i] * fv[i]; }, M); // np.sum(np.square)
-      // result (:488-520): fold, |t_rel|, covariance from the reference's
-      // Jacobian at the folded point and its own 3x3 inverse
-      double d = x[0], a = x[1];
-      symmetrize(d, a);
-      const double t = fabs(x[2]);
-      const double sigma_sq = cost / (double)(M - 3);
-      const int col[3] = {0, MAXM, 2 * MAXM};
-      px_jacobi(P, w, d, a, t, J, col);
-      double s[6] = {0, 0, 0, 0, 0, 0};
-      for (int i = 0; i < M; i++) {
-         const double j0 = J[i], j1 = J[MAXM + i], j2 = J[2 * MAXM + i];
-         s[0] += j0 * j0;
-         s[1] += j0 * j1;
-         s[2] += j0 * j2;
-         s[3] += j1 * j1;
-         s[4] += j1 * j2;
-         s[5] += j2 * j2;
-      }
-      const double mm[9] = {s[0], s[1], s[2], s[1], s[3], s[4], s[2], s[4], s[5]};
-      // _invertmatrix (:14-44) with the reference's determinant expression
-      // (its fourth term is m20 * m12, without a third factor)
-      const double det = mm[0] * mm[4] * mm[8] + mm[3] * mm[7] * mm[2] + mm[6] * mm[5] -
-                         mm[0] * mm[7] * mm[5] - mm[6] * mm[4] * mm[2] - mm[3] * mm[1] * mm[8];
-      const double i00 = (mm[4] * mm[8] - mm[5] * mm[7]) / det;
-      const double i11 = (mm[0] * mm[8] - mm[2] * mm[6]) / det;
-      const double i22 = (mm[0] * mm[4] - mm[1] * mm[3]) / det;
-      o[0] = d;
-      o[1] = a;
-      o[2] = t;
-      o[3] = sqrt(fabs(i00 * sigma_sq));
-      o[4] = sqrt(fabs(i11 * sigma_sq));
-      o[5] = sqrt(fabs(i22 * sigma_sq));
-      o[6] = cost;
-      o[7] = (double)n_fev;
+      __syncwarp();
    }
+}
+
+// Lanes per pixel.  Up to kRoflFewPixels 16: four warps per SM of two pixels
+// each, which an SM's FP64 unit runs nearly as fast as one, so only the length
+// of a pixel's chain counts.  From kRoflManyPixels on 1: the map keeps every SM
+// busy for many times the longest chain, so only the number of instructions
+// counts.  Between them 4 (GB300, forward differences, 9 rotations):
+//   30 x 20     16: 1.70 ms   4:   2.72 ms   1:  6.3 ms
+//   77 x 77     16: 4.94      4:   4.68      1:  9.8
+//   160 x 150   16: 18.2      4:  13.8       1: 18.0
+//   320 x 320                 4:  44.0       1: 35.7
+//   512 x 512                 4: 109         1: 84.0
+constexpr int64_t kRoflFewPixels = 1216, kRoflManyPixels = 80000;
+
+// As many warps as are resident (the pixels are taken from the counter), fewer
+// for small maps.
+template <int MAXR, int G>
+static int launch_rofl(const double *d_data, int64_t n_pix, const unsigned char *d_mask,
+                       const RoflParams &P, double *d_out, unsigned long long *status,
+                       cudaStream_t st) {
+   constexpr int kPixels = 32 / G;
+   constexpr int kBytes = G == 1 ? 0 : kPixels * (int)sizeof(PixelArrays<5 * MAXR>);
+   int dev = 0, sms = 0, per_sm = 0;
+   FPGB_CUDA_TRY(cudaGetDevice(&dev));
+   FPGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+   FPGB_CUDA_TRY(cudaFuncSetAttribute(rofl_fit<MAXR, G>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
+   FPGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rofl_fit<MAXR, G>, 32,
+                                                               kBytes));
+   const int64_t blocks = std::max<int64_t>(
+       1, std::min<int64_t>((n_pix + kPixels - 1) / kPixels, (int64_t)sms * std::max(per_sm, 1)));
+   rofl_fit<MAXR, G><<<(unsigned)blocks, 32, kBytes, st>>>(d_data, n_pix, d_mask, P, d_out,
+                                                           status);
+   FPGB_CUDA_TRY(cudaGetLastError());
+   return FPGB_OK;
 }
 
 } // namespace fpgb
@@ -868,6 +1014,7 @@ int fpgb_rofl_device(const double *d_data, int64_t n_pix, int64_t n_rot, double 
    RoflParams P;
    std::memset(&P, 0, sizeof P);
    P.n_rot = (int)n_rot;
+   P.inv_rot = (1 << 16) / P.n_rot + 1;
    P.grad_mode = grad_mode ? 1 : 0;
    P.tau = tilt_angle;
    P.gain = gain;
@@ -906,24 +1053,13 @@ int fpgb_rofl_device(const double *d_data, int64_t n_pix, int64_t n_rot, double 
    // status[0]: pixels at the evaluation limit, status[1]: next pixel
    FPGB_CUDA_TRY(cudaMemsetAsync(status, 0, 2 * sizeof(unsigned long long), st));
    if (n_pix > 0) {
-      // as many CTAs as are resident at once (the pixels are taken from the
-      // counter), fewer for small maps
       const bool small = P.n_rot <= kRoflSmallRot;
-      int dev = 0, sms = 0, per_sm = 0;
-      FPGB_CUDA_TRY(cudaGetDevice(&dev));
-      FPGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      FPGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, small ? rofl_fit<kRoflSmallRot> : rofl_fit<kRoflMaxRot>, kRoflThreads, 0));
-      const int64_t blocks =
-          std::max<int64_t>(1, std::min<int64_t>((n_pix + kRoflThreads - 1) / kRoflThreads,
-                                                 (int64_t)sms * std::max(per_sm, 1)));
-      if (small)
-         rofl_fit<kRoflSmallRot><<<(unsigned)blocks, kRoflThreads, 0, st>>>(d_data, n_pix, d_mask, P,
-                                                                   d_out, status);
-      else
-         rofl_fit<kRoflMaxRot><<<(unsigned)blocks, kRoflThreads, 0, st>>>(d_data, n_pix, d_mask, P,
-                                                                 d_out, status);
-      FPGB_CUDA_TRY(cudaGetLastError());
+      auto launch = n_pix >= kRoflManyPixels
+                        ? (small ? launch_rofl<kRoflSmallRot, 1> : launch_rofl<kRoflMaxRot, 1>)
+                    : small && n_pix > kRoflFewPixels ? launch_rofl<kRoflSmallRot, 4>
+                    : small                           ? launch_rofl<kRoflSmallRot, 16>
+                                                      : launch_rofl<kRoflMaxRot, 16>;
+      FPGB_TRY(launch(d_data, n_pix, d_mask, P, d_out, status, st));
    }
    if (n_unconverged) {
       unsigned long long h = 0;
