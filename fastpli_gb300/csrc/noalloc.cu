@@ -78,7 +78,7 @@ extern "C" int fpgb_generate_tissue_noalloc(const fpgb_volume *vol, const fpgb_f
                                             int64_t props_cap, int64_t *n_props,
                                             fpgb_warnings *warnings, void *stream) {
    TissuePlan p;
-   FPGB_TRY(plan_tissue(vol, fibers, &p));
+   FPGB_TRY(plan_tissue(vol, fibers, &p, false));
    if (!d_label || (!only_label && !d_vector)) {
       set_error("generate_tissue_noalloc: null output buffer");
       return FPGB_EINVAL;
@@ -88,7 +88,7 @@ extern "C" int fpgb_generate_tissue_noalloc(const fpgb_volume *vol, const fpgb_f
       set_error("generate_tissue_noalloc: this volume (%lld voxels) and its %zu fiber "
                 "segments need %zu bytes of scratch, more than the fixed %zu bytes; "
                 "use fpgb_generate_tissue_device with a workspace instead",
-                (long long)(p.X * p.Y * p.Z), p.segs.size(), need, kNoAllocScratchBytes);
+                (long long)(p.X * p.Y * p.Z), (size_t)p.n_segs, need, kNoAllocScratchBytes);
       return FPGB_EINVAL;
    }
    const int64_t rows = (int64_t)p.props.size() / 2;

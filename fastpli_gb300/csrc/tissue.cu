@@ -37,6 +37,154 @@
 namespace fpgb {
 
 // ======================================================================
+// the segment table (double precision, reference operation order)
+// ======================================================================
+// double -> (hi, lo) float pair; |d - hi - lo| <= 2^-48 |d|
+FPGB_HD void split2(double d, float &hi, float &lo) {
+   hi = (float)d;
+   lo = (float)(d - (double)hi);
+}
+
+// Bound on |estimate - reference float| of the sweep's FP32 dist^2
+// (sweep_dist2) over the voxels of the segment's box that lie within or next
+// to the segment's thickest end: |w| <= |v| + r' for the voxel's offset w
+// from p.  With u = 2^-24, the rounding of the inputs (w: u (|w0| + |w| + 1)
+// for the offset w0 of the sub-box's first cell, v, c2: u each), of the six
+// operations and of the sum of the margin itself stays below u (15 |w|^2 +
+// 2 |w| |w0| + 12 c2 + 4) (the error of t enters squared: the value is the
+// squared distance to some point of the segment); the reference's own double
+// arithmetic adds 2^-50 pscale |w| and its final rounding u |w|^2.  18 u and
+// 12 u are 1.08e-6 and 7.2e-7.  For a voxel farther away, d >= |w| - |v|, so
+// that error is below 3.3e-6 d^2 + 4e-6 c2 and the estimate stays past the
+// thickest end as the distance does: r' has more than that on top.
+// Evaluated in float, whose own rounding (below 1e-5) the factor 1.001 covers.
+FPGB_HD float seg_margin(const SegDev &S, float thr) {
+   float w2 = 0.f;
+   for (int i = 0; i < 3; i++) {
+      const float a = (float)((double)S.lo[i] + 0.5 - S.p[i]);
+      const float b = a + (float)(S.ext[i] > 0 ? S.ext[i] - 1 : 0);
+      w2 += fmaxf(a * a, b * b);
+   }
+   const float box = sqrtf(w2), v = sqrtf(S.c2f), ps = 1e-14f * S.pscale;
+   const float near = v + sqrtf(thr * 1.0001f + 0.01f + 1e-4f * S.c2f +
+                                10.f * ps * (v + sqrtf(thr) + 1.f));
+   const float w = fminf(box, near);
+   return 1.001f * (1.08e-6f * w * w + 1.5e-7f * w * box + 7.2e-7f * S.c2f + 2e-6f +
+                    ps * (w + 1.f));
+}
+
+// Host-side constants of the two-float path, all derived in double exactly
+// as the reference derives the corresponding values.
+FPGB_HD void fill_fast_fields(SegDev &S, const int64_t dim[3]) {
+   double ps = 0;
+   for (int i = 0; i < 3; i++) {
+      split2(S.p[i] - (double)S.base[i], S.pf[i], S.pl_lo[i]);
+      split2(S.v[i], S.vf[i], S.v_lo[i]);
+      ps = fmax(ps, fmax(fabs(S.p[i]), fabs(S.q[i])));
+      ps = fmax(ps, (double)dim[i]);
+   }
+   S.pscale = (float)(ps + 2.0);
+   split2(S.c2, S.c2f, S.c2_lo);
+   S.c2_rcp = S.c2 > 0 ? (float)(1.0 / S.c2) : 0.f;
+   split2(S.r0, S.r0_hi, S.r0_lo);
+   split2(S.r1 - S.r0, S.dr_hi, S.dr_lo);
+   // Fiber::CalcRadius at t = 0 and t = 1 is exactly r0 and r1
+   // (fiber.cpp:115-120): r0*(1-0) + r1*0 = r0, r0*0 + r1*1 = r1
+   S.rsq0 = (float)(S.r0 * S.r0);
+   S.rsq1 = (float)(S.r1 * S.r1);
+   // r0 == r1: every interior r(t) is r0 within a few ulp, so float(r^2) is
+   // fixed unless r0^2 sits next to a float rounding boundary
+   S.rsq_const = NAN;
+   if (S.r0 == S.r1) {
+      const double r2 = S.r0 * S.r0;
+      const double eps = 64.0 * 0x1p-53;
+      const float a = (float)(r2 * (1.0 - eps)), b = (float)(r2 * (1.0 + eps));
+      if (a == b)
+         S.rsq_const = a;
+   }
+   S.dec_rsq = S.rsq_const == S.rsq0 && S.rsq_const == S.rsq1 ? S.rsq_const : NAN;
+   // 'p' layer vector: vm::unit(q - p) (generator.cpp:372-373, vemath.hpp:390-402)
+   double n2 = 0.0;
+   n2 = n2 + S.v[0] * S.v[0];
+   n2 = n2 + S.v[1] * S.v[1];
+   n2 = n2 + S.v[2] * S.v[2];
+   double u[3] = {S.v[0], S.v[1], S.v[2]};
+   if (n2 > 0) {
+      const double inv = 1.0 / sqrt(n2);
+      for (int i = 0; i < 3; i++)
+         u[i] = u[i] * inv;
+   }
+   for (int i = 0; i < 3; i++)
+      S.vp[i] = (float)u[i];
+}
+
+// The segment's box clipped to the volume (generator.cpp:295-312): its voxel
+// count, 0 when it is empty.
+FPGB_HD int64_t segment_box(const double *P, const double *Q, double r0, double r1, double rsl,
+                            const int64_t dim[3], int32_t lo_out[3], int32_t ext_out[3]) {
+   const double rmax = (r0 < r1 ? r1 : r0) * rsl;
+   int64_t count = 1;
+   for (int i = 0; i < 3; i++) {
+      double mn = P[i] < Q[i] ? P[i] : Q[i], mx = P[i] < Q[i] ? Q[i] : P[i];
+      const double top = (double)dim[i];
+      mn -= rmax;
+      mx += rmax;
+      if (0.0 > mn)
+         mn = 0.0;
+      if (top < mx)
+         mx = top;
+      if (!(mn <= mx)) { // empty or non-finite box
+         lo_out[i] = 0;
+         ext_out[i] = 0;
+         count = 0;
+         continue;
+      }
+      // (int64) truncation as generator.cpp:304-305; the clamp only
+      // restates that the box already lies in [0, dim]
+      int64_t lo = (int64_t)mn, hi = (int64_t)(mx + 0.5);
+      lo = lo < 0 ? 0 : lo;
+      hi = hi > dim[i] ? dim[i] : hi;
+      lo_out[i] = (int32_t)lo;
+      ext_out[i] = (int32_t)(hi > lo ? hi - lo : 0);
+      count *= ext_out[i];
+   }
+   return count;
+}
+
+// One segment of the table from its ends and radii, in double exactly as the
+// reference derives the corresponding values: host and device give the same
+// bits (IEEE operations, no contraction).
+FPGB_HD void fill_segment(const double *P, const double *Q, double r0, double r1, int32_t bundle,
+                          float f_ly_squ, double sqrt_last, const int64_t dim[3], SegDev &S) {
+   segment_box(P, Q, r0, r1, sqrt_last, dim, S.lo, S.ext);
+   for (int i = 0; i < 3; i++) {
+      S.p[i] = P[i];
+      S.q[i] = Q[i];
+      S.v[i] = Q[i] - P[i];
+      const double base = floor(P[i]);
+      S.base[i] = (int32_t)fmax(-2147483647.0, fmin(2147483647.0, base));
+   }
+   double c = 0.0;
+   c = c + S.v[0] * S.v[0];
+   c = c + S.v[1] * S.v[1];
+   c = c + S.v[2] * S.v[2];
+   S.c2 = c;
+   S.r0 = r0;
+   S.r1 = r1;
+   fill_fast_fields(S, dim);
+   const double rm = r0 < r1 ? r1 : r0;
+   S.thr_f = (float)((double)f_ly_squ * rm * rm * (1.0 + 1e-5)) * (1.f + 0x1p-22f);
+   S.mg = seg_margin(S, S.thr_f);
+   const double rn = r0 < r1 ? r0 : r1;
+   const double a = (double)f_ly_squ * rn * rn * (1.0 - 1e-5);
+   float af = (float)a;
+   if ((double)af > a)
+      af = nextafterf(af, 0.f);
+   S.acc_f = af > 0.f ? af : -1.f;
+   S.bundle = bundle;
+}
+
+// ======================================================================
 // host planning (double precision, reference operation order)
 // ======================================================================
 namespace {
@@ -100,91 +248,20 @@ Box fiber_box(const double *xyz, const double *r, int64_t n) {
    return b;
 }
 
-// double -> (hi, lo) float pair; |d - hi - lo| <= 2^-48 |d|
-void split2(double d, float &hi, float &lo) {
-   hi = (float)d;
-   lo = (float)(d - (double)hi);
-}
-
-// Bound on |estimate - reference float| of the sweep's FP32 dist^2
-// (sweep_dist2) over the voxels of the segment's box that lie within or next
-// to the segment's thickest end: |w| <= |v| + r' for the voxel's offset w
-// from p.  With u = 2^-24, the rounding of the inputs (w: u (|w0| + |w| + 1)
-// for the offset w0 of the sub-box's first cell, v, c2: u each), of the six
-// operations and of the sum of the margin itself stays below u (15 |w|^2 +
-// 2 |w| |w0| + 12 c2 + 4) (the error of t enters squared: the value is the
-// squared distance to some point of the segment); the reference's own double
-// arithmetic adds 2^-50 pscale |w| and its final rounding u |w|^2.  18 u and
-// 12 u are 1.08e-6 and 7.2e-7.  For a voxel farther away, d >= |w| - |v|, so
-// that error is below 3.3e-6 d^2 + 4e-6 c2 and the estimate stays past the
-// thickest end as the distance does: r' has more than that on top.
-float seg_margin(const SegDev &S, double thr) {
-   double w2 = 0.0;
-   for (int i = 0; i < 3; i++) {
-      const double a = (double)S.lo[i] + 0.5 - S.p[i];
-      const double b = a + (double)(S.ext[i] > 0 ? S.ext[i] - 1 : 0);
-      w2 += std::max(a * a, b * b);
-   }
-   const double box = std::sqrt(w2), v = std::sqrt(S.c2), ps = 1e-14 * (double)S.pscale;
-   const double near = v + std::sqrt(thr * (1.0 + 1e-4) + 0.01 + 1e-4 * S.c2 +
-                                     10.0 * ps * (v + std::sqrt(thr) + 1.0));
-   const double w = std::min(box, near);
-   return (float)(1.001 * (1.08e-6 * w * w + 1.5e-7 * w * box + 7.2e-7 * S.c2 + 2e-6 +
-                           ps * (w + 1.0)));
-}
-
-// Host-side constants of the two-float path, all derived in double exactly
-// as the reference derives the corresponding values.
-void fill_fast_fields(SegDev &S, const fpgb_volume *vol) {
-   double ps = 0;
-   for (int i = 0; i < 3; i++) {
-      split2(S.p[i] - (double)S.base[i], S.pf[i], S.pl_lo[i]);
-      split2(S.v[i], S.vf[i], S.v_lo[i]);
-      ps = std::max(ps, std::max(std::fabs(S.p[i]), std::fabs(S.q[i])));
-      ps = std::max(ps, (double)vol->dim[i]);
-   }
-   S.pscale = (float)(ps + 2.0);
-   split2(S.c2, S.c2f, S.c2_lo);
-   S.c2_rcp = S.c2 > 0 ? (float)(1.0 / S.c2) : 0.f;
-   split2(S.r0, S.r0_hi, S.r0_lo);
-   split2(S.r1 - S.r0, S.dr_hi, S.dr_lo);
-   // Fiber::CalcRadius at t = 0 and t = 1 is exactly r0 and r1
-   // (fiber.cpp:115-120): r0*(1-0) + r1*0 = r0, r0*0 + r1*1 = r1
-   S.rsq0 = (float)(S.r0 * S.r0);
-   S.rsq1 = (float)(S.r1 * S.r1);
-   // r0 == r1: every interior r(t) is r0 within a few ulp, so float(r^2) is
-   // fixed unless r0^2 sits next to a float rounding boundary
-   S.rsq_const = NAN;
-   if (S.r0 == S.r1) {
-      const double r2 = S.r0 * S.r0;
-      const double eps = 64.0 * 0x1p-53;
-      const float a = (float)(r2 * (1.0 - eps)), b = (float)(r2 * (1.0 + eps));
-      if (a == b)
-         S.rsq_const = a;
-   }
-   S.dec_rsq = S.rsq_const == S.rsq0 && S.rsq_const == S.rsq1 ? S.rsq_const : NAN;
-   // 'p' layer vector: vm::unit(q - p) (generator.cpp:372-373, vemath.hpp:390-402)
-   double n2 = 0.0;
-   n2 = n2 + S.v[0] * S.v[0];
-   n2 = n2 + S.v[1] * S.v[1];
-   n2 = n2 + S.v[2] * S.v[2];
-   double u[3] = {S.v[0], S.v[1], S.v[2]};
-   if (n2 > 0) {
-      const double inv = 1.0 / std::sqrt(n2);
-      for (int i = 0; i < 3; i++)
-         u[i] = u[i] * inv;
-   }
-   for (int i = 0; i < 3; i++)
-      S.vp[i] = (float)u[i];
-}
-
 } // namespace
 
 // Up to this many points one thread plans faster than waking the others takes
 // (320 points: 21 us against 42).
 [[maybe_unused]] constexpr int64_t kSerialPoints = 1000;
+// Segment tables up to this size are filled on the host and go up with the
+// small tables: a copy from pageable memory costs the host about 8 us however
+// small.  Larger ones are filled on the device from the points, a sixth of the
+// bytes (94,451 segments: 325 us of 16 host threads and a copy of 165 us before;
+// the kernel takes 36 us, and the whole call went from 2122 to 1501 us; 980,000 segments:
+// 29.6 and 22.7 ms).
+constexpr size_t kTogetherBytes = size_t(256) << 10;
 
-int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan) {
+int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan, bool fill) {
    if (!vol || !fb) {
       set_error("generate_tissue: null volume or fibers");
       return FPGB_EINVAL;
@@ -216,6 +293,7 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
    plan->Z = vol->dim[2];
    plan->n_bundles = nb;
    plan->segs.clear();
+   plan->source.clear();
    plan->layers.assign(nb > 0 ? nb : 1, LayerDev{});
    plan->single_point = 0;
 
@@ -281,9 +359,10 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
       set_error("generate_tissue: points == NULL");
       return FPGB_EINVAL;
    }
-   RawArray<double> xyz, rad;
-   xyz.reset((size_t)(3 * np));
-   rad.reset((size_t)np);
+   // (a fiber of n points has fewer than n segments)
+   plan->n_points = np;
+   plan->source.reset((32 + sizeof(SegSrc)) * (size_t)np);
+   double *xyz = reinterpret_cast<double *>(plan->source.data()), *rad = xyz + 3 * np;
    const bool translate =
        vol->origin[0] != 0 || vol->origin[1] != 0 || vol->origin[2] != 0;
    const double f = 1.0 / vol->voxel_size;
@@ -321,7 +400,7 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
 #pragma omp parallel for schedule(dynamic, 32) if (np > kSerialPoints)
    for (int64_t fi = 0; fi < nf; fi++) {
       const int64_t p0 = fb->fiber_point_off[fi], p1 = fb->fiber_point_off[fi + 1];
-      fbox[fi] = fiber_box(xyz.data() + 3 * p0, rad.data() + p0, p1 - p0);
+      fbox[fi] = fiber_box(xyz + 3 * p0, rad + p0, p1 - p0);
    }
    Box volbox;
    for (int i = 0; i < 3; i++) {
@@ -346,46 +425,20 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
       }
       bundle_on[b] = overlap(volbox, bb) ? 1 : 0;
    }
-   // pass 1: segments each fiber keeps (its boxes only); pass 2 fills the
-   // table in place at the fibers' prefix offsets
+   // pass 1: segments each fiber keeps (its boxes only), their candidates and
+   // bricks; pass 2 fills the table, or notes the segments' sources, in place at
+   // the fibers' prefix offsets
+   RawArray<char> kept;
+   kept.reset((size_t)np);
    std::vector<int64_t> fiber_segs(nf + 1, 0);
    std::vector<char> single(nf, 0);
-   auto seg_box = [&](int64_t s, double rsl, SegDev &S) -> int64_t {
-      const double *P = &xyz[3 * s], *Q = &xyz[3 * (s + 1)];
-      const double r0 = rad[s], r1 = rad[s + 1];
-      const double rmax = (r0 < r1 ? r1 : r0) * rsl;
-      Box sb;
-      sb.from_pq(P, Q);
-      int64_t count = 1;
-      for (int i = 0; i < 3; i++) {
-         sb.mn[i] -= rmax;
-         sb.mx[i] += rmax;
-         if (volbox.mn[i] > sb.mn[i])
-            sb.mn[i] = volbox.mn[i];
-         if (volbox.mx[i] < sb.mx[i])
-            sb.mx[i] = volbox.mx[i];
-         if (!(sb.mn[i] <= sb.mx[i])) { // empty or non-finite box
-            S.lo[i] = 0;
-            S.ext[i] = 0;
-            count = 0;
-            continue;
-         }
-         // (int64) truncation as generator.cpp:304-305; the clamp only
-         // restates that the box already lies in [0, dim]
-         const int64_t lo = std::max<int64_t>(0, (int64_t)sb.mn[i]);
-         const int64_t hi = std::min<int64_t>(vol->dim[i], (int64_t)(sb.mx[i] + 0.5));
-         S.lo[i] = (int32_t)lo;
-         S.ext[i] = (int32_t)(hi > lo ? hi - lo : 0);
-         count *= S.ext[i];
-      }
-      return count;
-   };
    auto fiber_used = [&](int64_t fi) -> bool {
       const int64_t b = fiber_bundle[fi];
       const int64_t p0 = fb->fiber_point_off[fi], p1 = fb->fiber_point_off[fi + 1];
       return bundle_on[b] && p1 - p0 > 1 && overlap(volbox, fbox[fi]) && plan->layers[b].n > 0;
    };
-#pragma omp parallel for schedule(dynamic, 32) if (np > kSerialPoints)
+   int64_t cand = 0, pairs = 0;
+#pragma omp parallel for schedule(dynamic, 32) reduction(+ : cand, pairs) if (np > kSerialPoints)
    for (int64_t fi = 0; fi < nf; fi++) {
       const int64_t b = fiber_bundle[fi];
       const int64_t p0 = fb->fiber_point_off[fi], p1 = fb->fiber_point_off[fi + 1];
@@ -395,79 +448,80 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan)
          continue;
       int64_t n = 0;
       SegDev S;
-      for (int64_t s = p0; s + 1 < p1; s++)
-         n += seg_box(s, plan->layers[b].sqrt_last, S) > 0;
+      for (int64_t s = p0; s + 1 < p1; s++) {
+         const int64_t count =
+             segment_box(&xyz[3 * s], &xyz[3 * (s + 1)], rad[s], rad[s + 1],
+                         plan->layers[b].sqrt_last, vol->dim, S.lo, S.ext);
+         kept[s] = count > 0;
+         if (count == 0)
+            continue;
+         n++;
+         cand += count;
+         pairs += segment_brick_pairs(S);
+      }
       fiber_segs[fi + 1] = n;
    }
    for (int64_t fi = 0; fi < nf; fi++) {
       fiber_segs[fi + 1] += fiber_segs[fi];
       plan->single_point += single[fi];
    }
-   plan->segs.reset((size_t)fiber_segs[nf]);
+   plan->n_segs = fiber_segs[nf];
+   plan->candidates = cand;
+   plan->brick_pairs = pairs;
+   if (plan->n_segs > 0xFFFFFFF0ll) {
+      set_error("too many fiber segments: %lld", (long long)plan->n_segs);
+      return FPGB_EINVAL;
+   }
+   fill = fill || sizeof(SegDev) * (size_t)plan->n_segs <= kTogetherBytes ||
+          np > 0xFFFFFFFFll; // SegSrc::point
+   if (fill)
+      plan->segs.reset((size_t)plan->n_segs);
    SegDev *table = plan->segs.data();
-   int64_t cand = 0, pairs = 0;
-#pragma omp parallel for schedule(dynamic, 32) reduction(+ : cand, pairs) if (np > kSerialPoints)
+   SegSrc *src = reinterpret_cast<SegSrc *>(rad + np);
+#pragma omp parallel for schedule(dynamic, 32) if (np > kSerialPoints)
    for (int64_t fi = 0; fi < nf; fi++) {
-      if (!fiber_used(fi))
+      if (fiber_segs[fi + 1] == fiber_segs[fi])
          continue;
       const int64_t b = fiber_bundle[fi];
       const LayerDev &L = plan->layers[b];
       const int64_t p0 = fb->fiber_point_off[fi], p1 = fb->fiber_point_off[fi + 1];
       int64_t at = fiber_segs[fi];
       for (int64_t s = p0; s + 1 < p1; s++) {
-         SegDev S;
-         std::memset(&S, 0, sizeof S);
-         const int64_t count = seg_box(s, L.sqrt_last, S);
-         if (count == 0)
+         if (!kept[s])
             continue;
-         const double *P = &xyz[3 * s], *Q = &xyz[3 * (s + 1)];
-         const double r0 = rad[s], r1 = rad[s + 1];
-         for (int i = 0; i < 3; i++) {
-            S.p[i] = P[i];
-            S.q[i] = Q[i];
-            S.v[i] = Q[i] - P[i];
-            const double base = std::floor(P[i]);
-            S.base[i] = (int32_t)std::max(-2147483647.0, std::min(2147483647.0, base));
-         }
-         {
-            double c = 0.0;
-            c = c + S.v[0] * S.v[0];
-            c = c + S.v[1] * S.v[1];
-            c = c + S.v[2] * S.v[2];
-            S.c2 = c;
-         }
-         S.r0 = r0;
-         S.r1 = r1;
-         fill_fast_fields(S, vol);
-         const double rm = r0 < r1 ? r1 : r0;
-         S.thr_f = (float)((double)L.f_ly_squ * rm * rm * (1.0 + 1e-5)) * (1.f + 0x1p-22f);
-         S.mg = seg_margin(S, S.thr_f);
-         {
-            const double rn = r0 < r1 ? r0 : r1;
-            const double a = (double)L.f_ly_squ * rn * rn * (1.0 - 1e-5);
-            float af = (float)a;
-            if ((double)af > a)
-               af = std::nextafter(af, 0.f);
-            S.acc_f = af > 0.f ? af : -1.f;
-         }
-         S.bundle = (int32_t)b;
-         table[at++] = S;
-         cand += count;
-         pairs += segment_brick_pairs(S);
+         if (fill)
+            fill_segment(&xyz[3 * s], &xyz[3 * (s + 1)], rad[s], rad[s + 1], (int32_t)b,
+                         L.f_ly_squ, L.sqrt_last, vol->dim, table[at]);
+         else
+            src[at] = SegSrc{(uint32_t)s, (int32_t)b};
+         at++;
       }
    }
-   if (plan->segs.size() > 0xFFFFFFF0ull) {
-      set_error("too many fiber segments: %zu", plan->segs.size());
-      return FPGB_EINVAL;
-   }
-   plan->candidates = cand;
-   plan->brick_pairs = pairs;
+   if (fill)
+      plan->source.clear();
    return FPGB_OK;
 }
 
 // ======================================================================
 // device code
 // ======================================================================
+// The segment table from the points, a thread per segment.  Bound by its FP64
+// arithmetic (the pipe 83% busy): 94,451 segments 36 us, 980,000 318 us.
+__global__ void __launch_bounds__(128)
+fill_segments(const double *__restrict__ xyz, const double *__restrict__ rad,
+              const SegSrc *__restrict__ src, int64_t n, const LayerDev *__restrict__ layers,
+              int64_t X, int64_t Y, int64_t Z, SegDev *__restrict__ segs) {
+   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+   if (i >= n)
+      return;
+   const int64_t dim[3] = {X, Y, Z};
+   const int64_t s = src[i].point;
+   const LayerDev &L = layers[src[i].bundle];
+   SegDev S;
+   fill_segment(xyz + 3 * s, xyz + 3 * (s + 1), rad[s], rad[s + 1], src[i].bundle, L.f_ly_squ,
+                L.sqrt_last, dim, S);
+   segs[i] = S;
+}
 
 // ======================================================================
 // launch
@@ -485,18 +539,15 @@ size_t tissue_workspace_bytes(const TissuePlan &p) {
    int32_t nb[3];
    const int64_t n_bricks = plan_bricks(p, nb);
    size_t b = align_up(sizeof(TileDev) + 2 * sizeof(void *), 256);
-   b += align_up(sizeof(SegDev) * std::max<size_t>(p.segs.size(), 1), 256);
+   b += align_up(sizeof(SegDev) * std::max<size_t>((size_t)p.n_segs, 1), 256);
    b += align_up(sizeof(LayerDev) * p.layers.size(), 256);
    b += align_up(sizeof(unsigned long long) * kCounterWords, 256);
-   b += brick_workspace_bytes(n_bricks, p.brick_pairs, (int64_t)p.segs.size());
+   b += brick_workspace_bytes(n_bricks, p.brick_pairs, p.n_segs);
    return b;
 }
 
 // Bricks of a slabbed launch, at least: a wave of 4 per SM.
 constexpr int64_t kSlabBricks = 608;
-// Segment tables up to this size go up with the head: a copy from pageable
-// memory costs the host about 8 us however small.
-constexpr size_t kTogetherBytes = size_t(256) << 10;
 
 int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
                float *d_vector, void *d_ws, size_t ws_bytes,
@@ -519,13 +570,13 @@ int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
    const size_t counter_off = layer_off + align_up(sizeof(LayerDev) * p.layers.size(), 256);
    const size_t seg_off =
        counter_off + align_up(sizeof(unsigned long long) * kCounterWords, 256);
-   const size_t seg_bytes = sizeof(SegDev) * p.segs.size();
+   const size_t seg_bytes = sizeof(SegDev) * (size_t)p.n_segs;
    char *w = static_cast<char *>(d_ws);
    char *head = w;
    auto *layers = reinterpret_cast<LayerDev *>(w + layer_off);
    auto *counters = reinterpret_cast<unsigned long long *>(w + counter_off);
    auto *segs = reinterpret_cast<SegDev *>(w + seg_off);
-   w += seg_off + align_up(sizeof(SegDev) * std::max<size_t>(p.segs.size(), 1), 256);
+   w += seg_off + align_up(sizeof(SegDev) * std::max<size_t>((size_t)p.n_segs, 1), 256);
 
    // the single volume as tile 0 of the brick voxelizer
    struct {
@@ -549,15 +600,44 @@ int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
 
    // one upload of the small tables (counters 0), with the segments where they
    // are few
-   const bool together = seg_bytes <= kTogetherBytes;
+   const bool together = seg_bytes <= kTogetherBytes && !p.segs.empty();
    std::vector<char> stage(seg_off + (together ? seg_bytes : 0));
    std::memcpy(stage.data(), &h, sizeof h);
    std::memcpy(stage.data() + layer_off, p.layers.data(), sizeof(LayerDev) * p.layers.size());
    if (together && seg_bytes)
       std::memcpy(stage.data() + seg_off, p.segs.data(), seg_bytes);
    FPGB_CUDA_TRY(cudaMemcpyAsync(head, stage.data(), stage.size(), cudaMemcpyHostToDevice, st));
-   if (!together)
-      FPGB_CUDA_TRY(cudaMemcpyAsync(segs, p.segs.data(), seg_bytes, cudaMemcpyHostToDevice, st));
+   if (!together && seg_bytes) {
+      // the points go where the brick lists will be, when they fit
+      const size_t bytes = p.source_bytes();
+      if (p.segs.empty() && bytes <= ws_bytes - (size_t)(w - static_cast<char *>(d_ws))) {
+         FPGB_CUDA_TRY(cudaMemcpyAsync(w, p.source.data(), bytes, cudaMemcpyHostToDevice, st));
+         auto *xyz = reinterpret_cast<const double *>(w);
+         fill_segments<<<(unsigned)((p.n_segs + 127) / 128), 128, 0, st>>>(
+             xyz, xyz + 3 * p.n_points, reinterpret_cast<const SegSrc *>(xyz + 4 * p.n_points),
+             p.n_segs, layers, p.X, p.Y, p.Z, segs);
+         FPGB_CUDA_TRY(cudaGetLastError());
+      } else {
+         RawArray<SegDev> table; // (long fibers of which little is in the volume)
+         const SegDev *from = p.segs.data();
+         if (p.segs.empty()) {
+            table.reset((size_t)p.n_segs);
+            const int64_t dim[3] = {p.X, p.Y, p.Z};
+            const double *xyz = reinterpret_cast<const double *>(p.source.data());
+            const double *rad = xyz + 3 * p.n_points;
+            auto *src = reinterpret_cast<const SegSrc *>(rad + p.n_points);
+#pragma omp parallel for schedule(static)
+            for (int64_t i = 0; i < p.n_segs; i++) {
+               const LayerDev &L = p.layers[src[i].bundle];
+               const int64_t a = src[i].point;
+               fill_segment(xyz + 3 * a, xyz + 3 * (a + 1), rad[a], rad[a + 1], src[i].bundle,
+                            L.f_ly_squ, L.sqrt_last, dim, table[i]);
+            }
+            from = table.data();
+         }
+         FPGB_CUDA_TRY(cudaMemcpyAsync(segs, from, seg_bytes, cudaMemcpyHostToDevice, st));
+      }
+   }
    auto *tile = reinterpret_cast<const TileDev *>(head);
    auto *lp = reinterpret_cast<int32_t *const *>(head + sizeof(TileDev));
    auto *vp = reinterpret_cast<float *const *>(head + sizeof(TileDev) + sizeof(void *));
@@ -590,7 +670,7 @@ int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
       }
       chunks = BrickChunks{n, bound, &Slabs::thunk, &slabs, alt};
    }
-   FPGB_TRY(launch_voxel_bricks(segs, nullptr, (int64_t)p.segs.size(), tile, 1, n_bricks,
+   FPGB_TRY(launch_voxel_bricks(segs, nullptr, p.n_segs, tile, 1, n_bricks,
                                 p.brick_pairs, layers, p.n_bundles > 1, lp, vp, w, counters, st,
                                 n > 1 ? &chunks : nullptr));
    if (n == 1 && after_slab)
@@ -681,7 +761,7 @@ extern "C" {
 
 size_t fpgb_generate_workspace_size(const fpgb_volume *vol, const fpgb_fibers *fibers) {
    TissuePlan p;
-   if (plan_tissue(vol, fibers, &p) != FPGB_OK)
+   if (plan_tissue(vol, fibers, &p, false) != FPGB_OK)
       return 0;
    return tissue_workspace_bytes(p);
 }
@@ -692,7 +772,7 @@ int fpgb_generate_tissue_device(const fpgb_volume *vol, const fpgb_fibers *fiber
                                 void *d_workspace, size_t workspace_bytes,
                                 fpgb_warnings *warnings, void *stream) {
    TissuePlan p;
-   FPGB_TRY(plan_tissue(vol, fibers, &p));
+   FPGB_TRY(plan_tissue(vol, fibers, &p, false));
    if (!d_label || (!only_label && !d_vector)) {
       set_error("generate_tissue_device: null output buffer");
       return FPGB_EINVAL;
@@ -714,7 +794,7 @@ int fpgb_generate_tissue(const fpgb_volume *vol, const fpgb_fibers *fibers, int 
                          int32_t *label, float *vector, double *props, int64_t props_cap,
                          int64_t *n_props, fpgb_warnings *warnings) {
    TissuePlan p;
-   FPGB_TRY(plan_tissue(vol, fibers, &p));
+   FPGB_TRY(plan_tissue(vol, fibers, &p, false));
    if (!label || (!only_label && !vector)) {
       set_error("generate_tissue: null output buffer");
       return FPGB_EINVAL;

@@ -95,6 +95,13 @@ template <class T> class RawArray {
    size_t n_ = 0;
 };
 
+// Where a segment of the table comes from: its start among the plan's points
+// (its end is the next one) and its bundle.
+struct SegSrc {
+   uint32_t point;
+   int32_t bundle;
+};
+
 struct TissuePlan {
    int64_t X = 0, Y = 0, Z = 0;
    int64_t n_bundles = 0;
@@ -102,12 +109,20 @@ struct TissuePlan {
    int64_t single_point = 0; // fibers skipped with a warning
    int64_t candidates = 0;   // sum of clipped box volumes
    int64_t brick_pairs = 0;  // (segment, brick) pairs of the brick voxelizer
+   int64_t n_segs = 0;
+   // the segment table; or, unfilled, what the device fills it from: n_points x
+   // (x, y, z) in voxels, n_points radii, n_segs SegSrc
    RawArray<SegDev> segs;
+   RawArray<char> source;
+   int64_t n_points = 0;
+   size_t source_bytes() const { return 32 * (size_t)n_points + sizeof(SegSrc) * (size_t)n_segs; }
    std::vector<LayerDev> layers;
    std::vector<double> props; // (dn, mu) rows
 };
 
-int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan);
+// fill = false leaves a large segment table to the device (run_tissue).
+int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
+                bool fill = true);
 size_t tissue_workspace_bytes(const TissuePlan &p);
 // Voxelizes the planned volume into d_label / d_vector on stream st.  With
 // n_slabs > 1 the bricks are voxelized in that many x-slabs, one launch each
