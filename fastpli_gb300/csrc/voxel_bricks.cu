@@ -47,8 +47,12 @@
 
 namespace fpgb {
 
-constexpr int kBrickThreads = 256;
-constexpr int kBrickWarps = kBrickThreads / 32;
+// A brick's threads: small CTAs wait less at its barriers, but those of a
+// volume of several bundles (31 KB of shared memory at 128 threads) then leave
+// too little L1 (one bundle, 397 x 283 x 77: 202 us with 128 threads, 214 with
+// 256; two, 512 x 512 x 120: 961 and 880).  As many sweep records at a time.
+template <bool MULTI> constexpr int kBrickThreads = MULTI ? 256 : 128;
+template <bool MULTI> constexpr unsigned kRecs = kBrickThreads<MULTI>;
 static_assert(kBrickZ == 32, "the write phase maps one lane to one z of a brick row");
 
 void tile_bricks(int64_t X, int64_t Y, int64_t Z, int32_t nb[3], int64_t *n_bricks) {
@@ -301,6 +305,15 @@ brick_scan(const unsigned *__restrict__ counts, int64_t n, unsigned *__restrict_
 }
 
 // ----------------------------------------------------------------- sweep ---
+constexpr int kPlane = kBrickY * kBrickZ; // distance of x neighbours in the shared arrays
+
+// Place of (y, z) in a plane of the shared arrays.  A row y is rotated by 9 y:
+// the lanes of a chunk cover several rows of a sub-box some 8 to 13 voxels
+// high, which would else share that many of the 32 banks.
+__device__ __forceinline__ int plane_place(int y, int z) {
+   return y * kBrickZ + ((z + 9 * y) & (kBrickZ - 1));
+}
+
 // The inputs of the sweep of one segment (SegDev offsets 96..191: pf, vf,
 // c2f, c2_rcp, thr_f, acc_f, base, lo, ext, bundle, mg) in 16-byte loads.
 struct SegSweep {
@@ -326,7 +339,7 @@ __device__ __forceinline__ SegSweep load_sweep(const SegDev &S) {
 // cell; each voxel then costs six fused operations (sweep_dist2).
 struct SubBox {
    int x0, y0, z0, ex, ey, ez, ncell;
-   float ezf, inv_ez; // 1/ez for the division-free cell split
+   float inv_ez; // 1/ez for the division-free cell split
 };
 
 __device__ __forceinline__ bool sub_box(const SegSweep &w, int ox, int oy, int oz, int nx,
@@ -340,8 +353,7 @@ __device__ __forceinline__ bool sub_box(const SegSweep &w, int ox, int oy, int o
    if (b.ex <= 0 || b.ey <= 0 || b.ez <= 0)
       return false;
    b.ncell = b.ey * b.ez;
-   b.ezf = (float)b.ez;
-   b.inv_ez = __fdividef(1.f, b.ezf);
+   b.inv_ez = __fdividef(1.f, (float)b.ez);
    return true;
 }
 
@@ -393,15 +405,35 @@ __device__ __forceinline__ float key_bound(const BrickScale &k, unsigned key) {
    return ((float)(key >> k.bits) + 1.f) * k.quantum;
 }
 
-// Per-segment inputs of the FP32 estimate, held in registers over a sweep.
-struct SegFP32 {
-   float pfx, pfy, pfz, vn2x, vn2y, vn2z, c2f, rch, mg;
-   int bx, by, bz;
+// A segment's inputs to the sweep of one brick, in shared memory: a thread
+// prepares a segment (about 100 instructions), a warp then reads it with three
+// 16-byte loads.
+struct __align__(16) SweepRec {
+   float wx0, wy0, wz0, mg;    // voxel centre - float(p - base) of the sub-box's first voxel
+   float vn2x, vn2y, vn2z, c2f; // -2 v, v.v
+   float rch, thr, inv_ez;     // -1/2 float(1 / c2), bound of hi
+   unsigned box;               // ncell, ez << 9, ex << 15, first voxel's place << 19
 };
 
-__device__ __forceinline__ SegFP32 seg_fp32(const SegSweep &w) {
-   return SegFP32{w.a.x, w.a.y, w.a.z, -2.f * w.a.w, -2.f * w.b.x, -2.f * w.b.y, w.b.z,
-                  -0.5f * w.b.w, w.mg, __float_as_int(w.c.z), __float_as_int(w.c.w), w.d.x};
+__device__ __forceinline__ SweepRec sweep_rec(const SegSweep &w, const SubBox &b, bool any,
+                                              int ox, int oy, int oz) {
+   SweepRec r;
+   r.wx0 = ((float)(b.x0 - __float_as_int(w.c.z)) + 0.5f) - w.a.x;
+   r.wy0 = ((float)(b.y0 - __float_as_int(w.c.w)) + 0.5f) - w.a.y;
+   r.wz0 = ((float)(b.z0 - w.d.x) + 0.5f) - w.a.z;
+   r.mg = w.mg;
+   r.vn2x = -2.f * w.a.w;
+   r.vn2y = -2.f * w.b.x;
+   r.vn2z = -2.f * w.b.y;
+   r.c2f = w.b.z;
+   r.rch = -0.5f * w.b.w;
+   // (finite: an infinite hi is outside)
+   r.thr = fminf(fmaf(2.00001f, w.mg, w.c.x), 3e38f);
+   r.inv_ez = b.inv_ez;
+   r.box = any ? (unsigned)b.ncell | (unsigned)b.ez << 9 | (unsigned)b.ex << 15 |
+                     (unsigned)brick_index(b.x0, b.y0, b.z0, ox, oy, oz) << 19
+               : 0u;
+   return r;
 }
 
 // A lane's (y, z) cell of a chunk of 32, numbered z fastest, in float
@@ -410,76 +442,115 @@ __device__ __forceinline__ SegFP32 seg_fp32(const SegSweep &w) {
 // error of the product with the approximate reciprocal, so the truncation is
 // the exact quotient.
 struct Cell {
-   int yz;      // y * 32 + z from the sub-box's first cell
+   int yz;      // plane_place
    float a2, b; // the y / z parts of the estimate
 };
 
-// wy0, wz0: voxel centre - float(p - base) of the first cell ((y - base) + 1/2
-// is exact in float)
-__device__ __forceinline__ Cell cell_of(const SubBox &b, const SegFP32 &g, float wy0, float wz0,
-                                        float c) {
-   const float iy = truncf((c + 0.5f) * b.inv_ez);
-   const float iz = fmaf(-iy, b.ezf, c);
-   const float wy = wy0 + iy, wz = wz0 + iz;
-   return Cell{(int)fmaf(iy, (float)kBrickZ, iz), fmaf(wz, g.vn2z, wy * g.vn2y),
+__device__ __forceinline__ Cell cell_of(const SweepRec &g, float ezf, float c) {
+   const float iy = truncf((c + 0.5f) * g.inv_ez);
+   const float iz = fmaf(-iy, ezf, c);
+   const float wy = g.wy0 + iy, wz = g.wz0 + iz;
+   return Cell{plane_place((int)(g.box >> 24 & 7u) + (int)iy, (int)(g.box >> 19 & 31u) + (int)iz),
+               fmaf(wz, g.vn2z, wy * g.vn2y),
                fmaf(wz, wz, fmaf(wy, wy, g.mg))};
 }
 
-constexpr int kPlane = kBrickY * kBrickZ; // distance of x neighbours in the shared arrays
-constexpr int kSweepStep = 2;
+constexpr int kSweepStep = 4; // candidates of a column at a time (2: 889 us, 8: 924)
 
-// The sweep of one segment over its sub-box, kSweepStep voxels of a column at
-// a time (their atomics are in flight together).  A candidate outside sends
-// kNoKey, which changes nothing and needs no branch; the last step may reach
-// past the column (and into skey's padding).  multi: the smallest bundle whose
-// fiber a voxel is certainly inside of is kept as well; voxels that are only
-// possibly inside get a mark of their own, which stays.
-template <bool MULTI>
-__device__ __forceinline__ void brick_sweep(const SegSweep &sw, unsigned slot, const SubBox &b,
-                                            int ox, int oy, int oz, const BrickScale &k,
-                                            bool multi, unsigned *skey, unsigned *smark,
-                                            unsigned *sminb, int lane) {
-   const SegFP32 g = seg_fp32(sw);
-   // bound of hi (finite: an infinite hi is outside)
-   const float thr = fminf(fmaf(2.00001f, g.mg, sw.c.x), 3e38f);
-   const float wy0 = ((float)(b.y0 - g.by) + 0.5f) - g.pfy;
-   const float wz0 = ((float)(b.z0 - g.bz) + 0.5f) - g.pfz;
-   const float wx0 = ((float)(b.x0 - g.bx) + 0.5f) - g.pfx;
-   const int first = ((b.x0 - ox) * kBrickY + (b.y0 - oy)) * kBrickZ + (b.z0 - oz);
-   for (int c0 = lane; c0 < b.ncell; c0 += 32) {
-      const Cell c = cell_of(b, g, wy0, wz0, (float)c0);
-      unsigned *key = skey + first + c.yz;
-      float wx = wx0;
-      for (int i = 0; i < b.ex;
-           i += kSweepStep, wx += (float)kSweepStep, key += kSweepStep * kPlane) {
-         float hi[kSweepStep];
-         unsigned mine[kSweepStep], old[kSweepStep];
+// What a warp carries through the sweep of one segment.
+struct SweepState {
+   float thr;       // the lane's bound of hi (below every hi without a cell)
+   float acc;       // hi at or below which the voxel is certainly inside
+   unsigned bundle, slot2; // bundle, 2 slot
+   unsigned *skey, *smark, *sminb;
+};
+
+// N candidates of the lane's x column, at wx, wx + 1, ... (their atomics are
+// in flight together).  The atomic is predicated: it takes time per active
+// lane (880 us; with kNoKey from the candidates outside 905).  multi: the
+// smallest bundle whose fiber a voxel is certainly inside of is kept as well;
+// voxels that are only possibly inside get a mark of their own, which stays.
+template <bool MULTI, int N>
+__device__ __forceinline__ void sweep_step(const SweepRec &g, const SweepState &w, const Cell &c,
+                                           const BrickScale &k, bool multi, float wx,
+                                           unsigned *key) {
+   float hi[N];
+   unsigned mine[N], old[N];
+   bool close[N], any = false;
 #pragma unroll
-         for (int u = 0; u < kSweepStep; u++) {
-            hi[u] = sweep_dist2(u ? wx + (float)u : wx, c.a2, c.b, g.vn2x, g.c2f, g.rch);
-            mine[u] = __float_as_uint(fmaf(hi[u], k.scale, 8388608.f)) * k.mul + 2u * slot;
-            if (u && i + u >= b.ex)
-               hi[u] = INFINITY;
-         }
-         // (NaN, from an infinite bound, counts as inside)
+   for (int u = 0; u < N; u++) {
+      hi[u] = sweep_dist2(u ? wx + (float)u : wx, c.a2, c.b, g.vn2x, g.c2f, g.rch);
+      mine[u] = __float_as_uint(fmaf(hi[u], k.scale, 8388608.f)) * k.mul + w.slot2;
+   }
+   // (NaN, from an infinite bound, counts as inside)
+   const unsigned a = (unsigned)__cvta_generic_to_shared(key);
 #pragma unroll
-         for (int u = 0; u < kSweepStep; u++)
-            old[u] = atomicMin(key + u * kPlane, !(hi[u] > thr) ? mine[u] : kNoKey);
+   for (int u = 0; u < N; u++) {
+      old[u] = 0;
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %3, %4;\n\t"
+                   "@!p atom.shared.min.u32 %0, [%1], %2;\n\t}"
+                   : "+r"(old[u])
+                   : "r"(a + 4u * kPlane * u), "r"(mine[u]), "f"(hi[u]), "f"(w.thr)
+                   : "memory");
+   }
 #pragma unroll
-         for (int u = 0; u < kSweepStep; u++)
-            if (!(hi[u] > thr) && old[u] - mine[u] + k.win <= k.win2)
-               atomicOr(key + u * kPlane, 1u);
-         if (MULTI && multi) {
+   for (int u = 0; u < N; u++) {
+      close[u] = !(hi[u] > w.thr) && old[u] - mine[u] + k.win <= k.win2;
+      any = any || close[u];
+   }
+   if (__any_sync(0xFFFFFFFFu, any)) {
 #pragma unroll
-            for (int u = 0; u < kSweepStep; u++)
-               if (hi[u] <= fminf(sw.c.y, 3e38f))
-                  atomicMin(sminb + (key - skey) + u * kPlane, (unsigned)sw.e.w);
-               else if (!(hi[u] > thr)) {
-                  const int yz = (int)(key - skey) & (kPlane - 1), x = b.x0 - ox + i + u;
-                  atomicOr(&smark[yz >> 2], 1u << (8 * (yz & 3) + x));
-               }
+      for (int u = 0; u < N; u++)
+         if (close[u])
+            atomicOr(key + u * kPlane, 1u);
+   }
+   if (MULTI && multi) {
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+         const int at = (int)(key - w.skey) + u * kPlane;
+         if (hi[u] <= fminf(w.acc, w.thr)) {
+            atomicMin(w.sminb + at, w.bundle);
+         } else if (!(hi[u] > w.thr)) {
+            const int yz = at & (kPlane - 1);
+            atomicOr(&w.smark[yz >> 2], 1u << (8 * (yz & 3) + at / kPlane));
          }
       }
+   }
+}
+
+// The sweep of one segment over its sub-box.  Every lane runs every step (the
+// control flow of a warp stays uniform: diverging branches cost a quarter of
+// the sweep's instructions); one without a cell of its own repeats the last
+// with a bound that nothing meets (a NaN does, and marks a voxel too many).
+template <bool MULTI>
+__device__ __forceinline__ void brick_sweep(const SweepRec &rec, unsigned slot, float acc,
+                                            unsigned bundle, const BrickScale &k, bool multi,
+                                            unsigned *skey, unsigned *smark, unsigned *sminb,
+                                            int lane) {
+   const SweepRec g = rec;
+   const float ezf = (float)(g.box >> 9 & 63u);
+   const int ncell = (int)(g.box & 511u), ex = (int)(g.box >> 15 & 15u);
+   unsigned *first = skey + (g.box >> 27) * kPlane;
+   SweepState w{g.thr, acc, bundle, 2u * slot, skey, smark, sminb};
+   for (int c0 = 0; c0 < ncell; c0 += 32) {
+      const int at = c0 + lane;
+      w.thr = at < ncell ? g.thr : -INFINITY;
+      const Cell c = cell_of(g, ezf, (float)min(at, ncell - 1));
+      unsigned *key = first + c.yz;
+      float wx = g.wx0;
+      int i = ex;
+      for (; i >= kSweepStep; i -= kSweepStep, wx += (float)kSweepStep, key += kSweepStep * kPlane)
+         sweep_step<MULTI, kSweepStep>(g, w, c, k, multi, wx, key);
+#pragma unroll
+      for (int n = kSweepStep / 2; n >= 1; n /= 2)
+         if (i & n) {
+            if (n == 2)
+               sweep_step<MULTI, 2>(g, w, c, k, multi, wx, key);
+            else
+               sweep_step<MULTI, 1>(g, w, c, k, multi, wx, key);
+            wx += (float)n;
+            key += n * kPlane;
+         }
    }
 }
 
@@ -512,7 +583,8 @@ __device__ __noinline__ bool cand_radial(const SegDev &S, int x, int y, int z, f
    const float lpt[3] = {(float)(x - S.base[0]) + 0.5f, (float)(y - S.base[1]) + 0.5f,
                          (float)(z - S.base[2]) + 0.5f};
    FastCand fc;
-   if (S.pscale < 0x1p22f && fast_candidate(S, lpt, fc) && fast_radial(S, fc, o))
+   ff t;
+   if (S.pscale < 0x1p22f && fast_offset(S, lpt, fc, t) && fast_radial(S, fc, o))
       return false;
    const double pt[3] = {(double)x + 0.5, (double)y + 0.5, (double)z + 0.5};
    double cl[3];
@@ -786,8 +858,9 @@ __device__ __forceinline__ void resolve_marks(const MarkCtx &C, MarkWarp &W, int
 // Resolves the marked voxels of the bricks [brick_begin, brick_end), a brick
 // per warp (bound by latency: 16 warps per SM, each a chain of list, segment
 // and evaluation; a voxel per lane walking the list by itself took 260 us on
-// the crossing volume instead of 153, 6 CTAs per SM at 80 registers 166): from its record, or from the labels of a brick without one (every
-// brick when the launch has no space for records).
+// the crossing volume instead of 153, 6 CTAs per SM at 80 registers 166): from
+// its record, or from the labels of a brick without one (every brick when the
+// launch has no space for records).
 __global__ void __launch_bounds__(kMarkThreads)
 voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
             int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
@@ -856,8 +929,6 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
 }
 
 // ------------------------------------------------------------- the brick ---
-static_assert(kBrickWarps == kBrickY && kBrickX <= 8, "the decode gives each y a warp");
-
 // Marked voxels of one brick that get a record; with more of them the labels
 // are as good.
 constexpr unsigned kMarkList = 128;
@@ -868,36 +939,43 @@ struct RadialQueue {
    unsigned short entry[64]; // voxel of the brick
 };
 
-// One CTA per brick, 256 threads: 8 warps share the brick's segments in the
-// sweep, then each owns the voxels of one y.  4 CTAs per SM (64 registers).
-// Bound by instruction issue (66-75% of the slots): per (segment, brick) pair
-// about 110 warp instructions of setup and 19 per 32 x-steps of the sweep,
-// then the decode of every voxel and a two-float unit vector per 'r' voxel.
+// One CTA per brick: its warps share the brick's segments in the sweep, then
+// its rows in the decode.  32 warps per SM (64 registers).  Bound by
+// instruction issue (66-75% of the slots) and the shared-memory atomics: about
+// a third of the time goes to the sweep, less than a third to the setup of
+// bricks and segments, the rest to the decode, near half of it for the unit
+// vectors of 'r' voxels.
+// Segments prepared by a thread each and uniform control flow in the sweep
+// against a warp's setup per segment and a branch per candidate: 397 x 283 x 77
+// with 15,013 segments 218 -> 202 us, crossing 512 x 512 x 120 928 -> 880 us;
+// work shared out by chunks of 32 cells instead of segments: 223 and 968 us.
 // With the marked voxels in a kernel of their own (voxel_marks) against two
 // sweeps with an exact evaluation of 0.9 candidates per voxel in this one:
-// 397 x 283 x 77 with 15,013 segments 523 -> 219 + 45 us, crossing
-// 512 x 512 x 120 2,216 -> 929 + 153 us, Watson 1024 x 1024 x 240 44.3 -> 24 ms
-// in all; the marked voxels resolved here instead (a list, a queue and two
-// barriers per brick): 330 and 1,290 us.
+// 523 -> 219 + 45 us and 2,216 -> 929 + 153 us; the marked voxels resolved here
+// instead (a list, a queue and two barriers per brick): 330 and 1,290 us.
 template <bool MULTI>
-__global__ void __launch_bounds__(kBrickThreads, 4)
+__global__ void __launch_bounds__(kBrickThreads<MULTI>, 1024 / kBrickThreads<MULTI>)
 voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
              int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
              const unsigned *__restrict__ list, unsigned n_pairs, unsigned *__restrict__ directory,
              uint2 *__restrict__ marks, int64_t mark_share, const LayerDev *__restrict__ layers,
              int32_t *const *__restrict__ labels, float *const *__restrict__ vecs,
              unsigned long long *__restrict__ counters) {
-   __shared__ unsigned skey[kBrickVoxels + kSweepStep * kPlane];
+   constexpr int kThreads = kBrickThreads<MULTI>, kWarps = kThreads / 32;
+   __shared__ __align__(16) unsigned skey[kBrickVoxels];
+   __shared__ SweepRec s_rec[kRecs<MULTI>];
+   __shared__ uint2 s_acc[MULTI ? kRecs<MULTI> : 1]; // acc_f, bundle
+   __shared__ uint2 s_max[kWarps];
    __shared__ unsigned smark[MULTI ? kPlane / 4 : 1]; // a byte per (y, z), a bit per x
    // the first segments of the list: index, dec_rsq, bundle
    __shared__ unsigned s_seg[kSegCache];
    __shared__ float s_rsq[kSegCache];
    __shared__ int s_bundle[MULTI ? kSegCache : 1];
-   __shared__ unsigned sminb[MULTI ? kBrickVoxels : 1];
+   __shared__ __align__(16) unsigned sminb[MULTI ? kBrickVoxels : 4];
    __shared__ LayerLut s_layers[MULTI ? kLayerCache : 1];
-   __shared__ RadialQueue queues[kBrickWarps];
+   __shared__ RadialQueue queues[kWarps];
    __shared__ unsigned short s_list[kMarkList];
-   __shared__ unsigned s_next, s_thr, s_mg, s_marked;
+   __shared__ unsigned s_next, s_marked;
    __shared__ bool s_multi;
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    unsigned long long n_slow = 0, n_overlap = 0;
@@ -913,9 +991,9 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
       const unsigned j1 = min(offsets[brick + 1], n_pairs), j0 = min(offsets[brick], j1);
 
       if (j0 == j1) { // no segment: background
-         if (warp < ny)
+         for (int ly = warp; ly < ny; ly += kWarps)
             for (int lx = 0; lx < nx; lx++) {
-               const int64_t i0 = ((int64_t)(ox + lx) * Y + (oy + warp)) * Z + oz;
+               const int64_t i0 = ((int64_t)(ox + lx) * Y + (oy + ly)) * Z + oz;
                if (lane < nz)
                   label[i0 + lane] = 0;
                if (vec)
@@ -925,10 +1003,12 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          continue;
       }
 
-      for (int i = threadIdx.x; i < kBrickVoxels; i += kBrickThreads) {
-         skey[i] = kNoKey;
+      const unsigned n_seg = j1 - j0;
+      const uint4 none = make_uint4(kNoKey, kNoKey, kNoKey, kNoKey);
+      for (int i = threadIdx.x; i < kBrickVoxels / 4; i += kThreads) {
+         reinterpret_cast<uint4 *>(skey)[i] = none;
          if (MULTI)
-            sminb[i] = ~0u;
+            reinterpret_cast<uint4 *>(sminb)[i] = none;
       }
       if (MULTI && threadIdx.x < kPlane / 4)
          smark[threadIdx.x] = 0;
@@ -944,16 +1024,26 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          }
       }
       if (threadIdx.x == 0) {
-         s_next = s_thr = s_mg = s_marked = 0;
+         s_next = kWarps;
+         s_marked = 0;
          // the overlap warning is one bit for the whole volume: once some
          // brick has raised it, the bundle minima are of no more use
          s_multi = MULTI && n_bundles > 1 &&
                    *reinterpret_cast<volatile unsigned long long *>(&counters[0]) == 0;
       }
-      __syncthreads();
-      { // the largest bounds of the list's segments (floats >= 0: bits order like values)
+      auto prepare = [&](unsigned j, unsigned s) {
+         const SegSweep w = load_sweep(segs[s]);
+         SubBox b;
+         const bool any = sub_box(w, ox, oy, oz, nx, ny, nz, b);
+         s_rec[j % kRecs<MULTI>] = sweep_rec(w, b, any, ox, oy, oz);
+         if (MULTI)
+            s_acc[j % kRecs<MULTI>] =
+                make_uint2(__float_as_uint(fminf(w.c.y, 3e38f)), (unsigned)w.e.w);
+      };
+      { // the first records, and the largest bounds of the list's segments
+        // (floats >= 0: bits order like values)
          unsigned th = 0, mg = 0;
-         for (unsigned j = threadIdx.x; j < j1 - j0; j += kBrickThreads) {
+         for (unsigned j = threadIdx.x; j < n_seg; j += kThreads) {
             const unsigned s = list[j0 + j];
             const SegDev &S = segs[s];
             const float m = __ldg(&S.mg);
@@ -963,34 +1053,50 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
                if (MULTI)
                   s_bundle[j] = __ldg(&S.bundle);
             }
+            if (j < kRecs<MULTI>)
+               prepare(j, s);
             th = max(th, __float_as_uint(fmaf(2.0001f, m, __ldg(&S.thr_f))));
             mg = max(mg, __float_as_uint(m));
          }
+         if (warp * 32 < n_seg) {
 #pragma unroll
-         for (int o = 16; o > 0; o >>= 1) {
-            th = max(th, __shfl_xor_sync(0xFFFFFFFFu, th, o));
-            mg = max(mg, __shfl_xor_sync(0xFFFFFFFFu, mg, o));
+            for (int o = 16; o > 0; o >>= 1) {
+               th = max(th, __shfl_xor_sync(0xFFFFFFFFu, th, o));
+               mg = max(mg, __shfl_xor_sync(0xFFFFFFFFu, mg, o));
+            }
          }
-         if (lane == 0 && th) {
-            atomicMax(&s_thr, th);
-            atomicMax(&s_mg, mg);
-         }
+         if (lane == 0)
+            s_max[warp] = make_uint2(th, mg);
       }
       __syncthreads();
-      const BrickScale k = brick_scale(j1 - j0, __uint_as_float(s_thr), __uint_as_float(s_mg));
+      unsigned th = 0, mg = 0;
+#pragma unroll
+      for (int i = 0; i < kWarps; i++) {
+         th = max(th, s_max[i].x);
+         mg = max(mg, s_max[i].y);
+      }
+      const BrickScale k = brick_scale(n_seg, __uint_as_float(th), __uint_as_float(mg));
       const bool multi = MULTI && s_multi;
-      // sweep: warps take segments from a shared counter
-      for (;;) {
-         unsigned j = 0;
-         if (lane == 0)
-            j = atomicAdd(&s_next, 1u);
-         j = __shfl_sync(0xFFFFFFFFu, j, 0);
-         if (j >= j1 - j0)
+      for (unsigned base = 0;;) {
+         // sweep: warps take segments from a shared counter, the next one
+         // while they are busy with one
+         const unsigned n = min(n_seg - base, kRecs<MULTI>);
+         for (unsigned j = warp, next; j < n; j = __shfl_sync(0xFFFFFFFFu, next, 0)) {
+            if (lane == 0)
+               next = atomicAdd(&s_next, 1u);
+            const uint2 a = MULTI ? s_acc[j] : make_uint2(0u, 0u);
+            brick_sweep<MULTI>(s_rec[j], base + j, __uint_as_float(a.x), a.y, k, multi, skey,
+                               smark, sminb, lane);
+         }
+         base += kRecs<MULTI>;
+         if (base >= n_seg)
             break;
-         const SegSweep sw = load_sweep(segs[j < kSegCache ? s_seg[j] : list[j0 + j]]);
-         SubBox b;
-         if (sub_box(sw, ox, oy, oz, nx, ny, nz, b))
-            brick_sweep<MULTI>(sw, j, b, ox, oy, oz, k, multi, skey, smark, sminb, lane);
+         __syncthreads();
+         if (threadIdx.x == 0)
+            s_next = kWarps;
+         for (unsigned e = threadIdx.x; e < min(kRecs<MULTI>, n_seg - base); e += kThreads)
+            prepare(base + e, list[j0 + base + e]);
+         __syncthreads();
       }
       __syncthreads();
       // decode: a warp per y, lane = z, along x: coalesced stores.  Radial
@@ -1010,92 +1116,94 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          vec[3 * i + 1] = o[1];
          vec[3 * i + 2] = o[2];
       };
-      const int yz = threadIdx.x; // warp * 32 + lane
-      const unsigned sticky = MULTI ? reinterpret_cast<const uint8_t *>(smark)[yz] : 0u;
-      const int y = oy + warp, z = oz + lane;
-      int64_t i = ((int64_t)ox * Y + y) * Z + z;
-      for (int lx = 0; lx < (warp < ny ? nx : 0); lx++, i += (int64_t)Y * Z) {
-         const int li = lx * kPlane + yz;
-         bool defer = false;
-         unsigned seg = 0;
-         int32_t lab = 0;
-         if (lane < nz) {
-            const unsigned key = skey[li];
-            float o0 = 0.f, o1 = 0.f, o2 = 0.f;
-            if (key != kNoKey || (MULTI && (sticky >> lx & 1u))) {
-               const unsigned slot = (key & (k.mul - 1u)) >> 1;
-               int w = -1, bundle = 0;
-               if (!(key & 1u) && !(MULTI && (sticky >> lx & 1u))) { // not marked
-                  float rsq;
-                  if (slot < kSegCache) {
-                     seg = s_seg[slot];
-                     rsq = s_rsq[slot];
-                     bundle = MULTI ? s_bundle[slot] : 0;
+      for (int ly = warp; ly < ny; ly += kWarps) {
+         const int yz = plane_place(ly, lane);
+         const unsigned sticky = MULTI ? reinterpret_cast<const uint8_t *>(smark)[yz] : 0u;
+         const int y = oy + ly, z = oz + lane;
+         int64_t i = ((int64_t)ox * Y + y) * Z + z;
+         for (int lx = 0; lx < nx; lx++, i += (int64_t)Y * Z) {
+            const int li = lx * kPlane + yz;
+            bool defer = false;
+            unsigned seg = 0;
+            int32_t lab = 0;
+            if (lane < nz) {
+               const unsigned key = skey[li];
+               float o0 = 0.f, o1 = 0.f, o2 = 0.f;
+               if (key != kNoKey || (MULTI && (sticky >> lx & 1u))) {
+                  const unsigned slot = (key & (k.mul - 1u)) >> 1;
+                  int w = -1, bundle = 0;
+                  if (!(key & 1u) && !(MULTI && (sticky >> lx & 1u))) { // not marked
+                     float rsq;
+                     if (slot < kSegCache) {
+                        seg = s_seg[slot];
+                        rsq = s_rsq[slot];
+                        bundle = MULTI ? s_bundle[slot] : 0;
+                     } else {
+                        seg = list[j0 + slot];
+                        rsq = segs[seg].dec_rsq;
+                        bundle = MULTI ? segs[seg].bundle : 0;
+                     }
+                     // 4e-6: the rounding of the quantum and of the product
+                     const float up = key_bound(k, key);
+                     float lo = up * (1.f - 4e-6f) - 2.f * k.quantum - k.mg2, hi = up;
+                     if (!(rsq == rsq)) { // the radius changes: evaluate
+                        float dist_squ;
+                        if (cand_dist(segs[seg], ox + lx, y, z, dist_squ, rsq))
+                           n_slow++;
+                        lo = hi = dist_squ;
+                        if (dist_squ > tile_layers[bundle].f_ly_squ * rsq)
+                           hi = INFINITY; // outside (generator.cpp:329-331): no layer is certain
+                     }
+                     if (!MULTI || bundle < kLayerCache)
+                        w = certain_layer(s_layers[MULTI ? bundle : 0].sq,
+                                          s_layers[MULTI ? bundle : 0].n, lo, hi, rsq);
+                     else
+                        w = certain_layer(tile_layers[bundle].sq_fdown, tile_layers[bundle].n, lo,
+                                          hi, rsq);
+                  }
+                  if (w >= 0) {
+                     lab = w + 1 + bundle * max_layer;
+                     if (MULTI && multi && sminb[li] < (unsigned)bundle)
+                        n_overlap++;
+                     const unsigned models = !MULTI || bundle < kLayerCache
+                                                 ? s_layers[MULTI ? bundle : 0].models
+                                                 : tile_layers[bundle].models;
+                     const unsigned m = models >> (2 * w) & 3u;
+                     if (m == 1u) {
+                        o0 = segs[seg].vp[0];
+                        o1 = segs[seg].vp[1];
+                        o2 = segs[seg].vp[2];
+                     }
+                     defer = m == 2u && vec;
                   } else {
-                     seg = list[j0 + slot];
-                     rsq = segs[seg].dec_rsq;
-                     bundle = MULTI ? segs[seg].bundle : 0;
+                     lab = kMarkedLabel;
                   }
-                  // 4e-6: the rounding of the quantum and of the product
-                  const float up = key_bound(k, key);
-                  float lo = up * (1.f - 4e-6f) - 2.f * k.quantum - k.mg2, hi = up;
-                  if (!(rsq == rsq)) { // the radius changes: evaluate
-                     float dist_squ;
-                     if (cand_dist(segs[seg], ox + lx, y, z, dist_squ, rsq))
-                        n_slow++;
-                     lo = hi = dist_squ;
-                     if (dist_squ > tile_layers[bundle].f_ly_squ * rsq)
-                        hi = INFINITY; // outside (generator.cpp:329-331): no layer is certain
-                  }
-                  if (!MULTI || bundle < kLayerCache)
-                     w = certain_layer(s_layers[MULTI ? bundle : 0].sq,
-                                       s_layers[MULTI ? bundle : 0].n, lo, hi, rsq);
-                  else
-                     w = certain_layer(tile_layers[bundle].sq_fdown, tile_layers[bundle].n, lo,
-                                       hi, rsq);
                }
-               if (w >= 0) {
-                  lab = w + 1 + bundle * max_layer;
-                  if (MULTI && multi && sminb[li] < (unsigned)bundle)
-                     n_overlap++;
-                  const unsigned models = !MULTI || bundle < kLayerCache
-                                              ? s_layers[MULTI ? bundle : 0].models
-                                              : tile_layers[bundle].models;
-                  const unsigned m = models >> (2 * w) & 3u;
-                  if (m == 1u) {
-                     o0 = segs[seg].vp[0];
-                     o1 = segs[seg].vp[1];
-                     o2 = segs[seg].vp[2];
-                  }
-                  defer = m == 2u && vec;
-               } else {
-                  lab = kMarkedLabel;
+               label[i] = lab;
+               if (vec && !defer) {
+                  vec[3 * i + 0] = o0;
+                  vec[3 * i + 1] = o1;
+                  vec[3 * i + 2] = o2;
                }
             }
-            label[i] = lab;
-            if (vec && !defer) {
-               vec[3 * i + 0] = o0;
-               vec[3 * i + 1] = o1;
-               vec[3 * i + 2] = o2;
+            if (lab == kMarkedLabel) {
+               const unsigned at = atomicAdd(&s_marked, 1u);
+               if (at < kMarkList)
+                  s_list[at] = (unsigned short)(lx * kPlane + ly * kBrickZ + lane);
             }
-         }
-         if (lab == kMarkedLabel) {
-            const unsigned at = atomicAdd(&s_marked, 1u);
-            if (at < kMarkList)
-               s_list[at] = (unsigned short)li;
-         }
-         const unsigned m = __ballot_sync(0xFFFFFFFFu, defer);
-         if (defer) {
-            const int at = qn + __popc(m & ((1u << lane) - 1u));
-            rq.entry[at] = (unsigned short)li;
-            rq.seg[at] = seg;
-         }
-         qn += __popc(m);
-         if (qn >= 32) {
-            __syncwarp();
-            radial(qn - 32 + lane);
-            qn -= 32;
-            __syncwarp();
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, defer);
+            if (defer) {
+               const int at = qn + __popc(m & ((1u << lane) - 1u));
+               rq.entry[at] = (unsigned short)(lx * kPlane + ly * kBrickZ + lane);
+               rq.seg[at] = seg;
+            }
+            qn += __popc(m);
+            if (qn >= 32) {
+               __syncwarp();
+               radial(qn - 32 + lane);
+               qn -= 32;
+               __syncwarp();
+            }
          }
       }
       __syncwarp();
@@ -1199,7 +1307,8 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
                 (b1 - b0 + kMarkThreads / 32 - 1) / (kMarkThreads / 32), 152 * 8);
             uint2 *share = marks + c * mark_share;
             auto kernel = multi_bundle ? voxel_bricks<true> : voxel_bricks<false>;
-            kernel<<<grid, kBrickThreads, 0, s>>>(segs, tiles, n_tiles, b0, b1, offsets, list,
+            const int threads = multi_bundle ? kBrickThreads<true> : kBrickThreads<false>;
+            kernel<<<grid, threads, 0, s>>>(segs, tiles, n_tiles, b0, b1, offsets, list,
                                                   (unsigned)n_pairs, counts + b0, share,
                                                   mark_share, layers, labels, vecs, counters);
             FPGB_CUDA_TRY(cudaGetLastError());
