@@ -681,6 +681,9 @@ __device__ __forceinline__ BrickPlace brick_place(const TileDev *__restrict__ ti
 }
 
 // --------------------------------------------------------- marked voxels ---
+// Marked voxels of one brick that get a record; with more of them the labels
+// are as good.
+constexpr unsigned kMarkList = 128;
 constexpr int kMarkThreads = 128, kMarkQueue = 192;
 constexpr unsigned kScanBrick = 0x80000000u; // directory entry without a record: a brick
 
@@ -860,13 +863,14 @@ __device__ __forceinline__ void resolve_marks(const MarkCtx &C, MarkWarp &W, int
 // and evaluation; a voxel per lane walking the list by itself took 260 us on
 // the crossing volume instead of 153, 6 CTAs per SM at 80 registers 166): from
 // its record, or from the labels of a brick without one (every brick when the
-// launch has no space for records).
+// launch has no space for records).  Units: 2^split parts of a brick, `part`
+// marked voxels of one of them.
 __global__ void __launch_bounds__(kMarkThreads)
 voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
             int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
             const unsigned *__restrict__ list, unsigned n_pairs,
             const unsigned *__restrict__ directory, const uint2 *__restrict__ marks,
-            int64_t mark_share, const LayerDev *__restrict__ layers,
+            int64_t mark_share, int split, int part, const LayerDev *__restrict__ layers,
             int32_t *const *__restrict__ labels, float *const *__restrict__ vecs,
             unsigned long long *__restrict__ counters) {
    __shared__ MarkWarp s_warps[kMarkThreads / 32];
@@ -876,12 +880,16 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
    const int64_t n_warps = (int64_t)gridDim.x * (kMarkThreads / 32);
    unsigned long long n_slow = 0, n_overlap = 0, n_overflow = 0;
    const bool open = *reinterpret_cast<volatile unsigned long long *>(&counters[0]) == 0;
-   const int64_t n = mark_share > 0 ? (int64_t)marks[0].y : brick_end - brick_begin;
-   for (int64_t r = warp; r < n; r += n_warps) {
+   const int64_t n = mark_share > 0 ? (int64_t)marks[0].y : (brick_end - brick_begin) << split;
+   const int parts = (int)kMarkList / part;
+   for (int64_t u = warp; u < n * parts; u += n_warps) {
+      const int64_t r = u % n;
+      const int g = (int)(u / n) * part;
       const unsigned at = mark_share > 0 ? directory[r] : kScanBrick;
-      int64_t brick = brick_begin + r;
+      int64_t place = r;
       if (mark_share > 0)
-         brick = brick_begin + ((at & kScanBrick) ? at & ~kScanBrick : marks[at].x);
+         place = (at & kScanBrick) ? at & ~kScanBrick : marks[at].x;
+      const int64_t brick = brick_begin + (place >> split);
       const unsigned j1 = min(offsets[brick + 1], n_pairs), j0 = min(offsets[brick], j1);
       if (j0 == j1)
          continue;
@@ -895,9 +903,9 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
       C.vec = vecs[C.p.tile];
       C.multi = open && C.p.T->n_bundles > 1;
       if (!(at & kScanBrick)) {
-         const int total = (int)marks[at].y;
+         const int total = min((int)marks[at].y, g + part);
          const unsigned short *voxel = reinterpret_cast<const unsigned short *>(marks + at + 1);
-         for (int m = 0; m < total; m += 32) {
+         for (int m = g; m < total; m += 32) {
             if (m + lane < total)
                W.voxel[lane] = voxel[m + lane];
             __syncwarp();
@@ -905,7 +913,11 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
          }
          continue;
       }
-      for (int row = 0; row < C.p.nx * C.p.ny; row++) {
+      if (g)
+         continue;
+      const int x0 = (int)(place & ((1 << split) - 1)) * (kBrickX >> split);
+      const int x1 = min(x0 + (kBrickX >> split), C.p.nx);
+      for (int row = x0 * C.p.ny; row < x1 * C.p.ny; row++) {
          const int lx = row / C.p.ny, ly = row - lx * C.p.ny;
          const int64_t i =
              ((int64_t)(C.p.ox + lx) * C.p.T->Y + (C.p.oy + ly)) * C.p.T->Z + C.p.oz + lane;
@@ -929,18 +941,15 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
 }
 
 // ------------------------------------------------------------- the brick ---
-// Marked voxels of one brick that get a record; with more of them the labels
-// are as good.
-constexpr unsigned kMarkList = 128;
-
 // Radial orientations a warp has still to compute.
 struct RadialQueue {
    unsigned seg[64];
    unsigned short entry[64]; // voxel of the brick
 };
 
-// One CTA per brick: its warps share the brick's segments in the sweep, then
-// its rows in the decode.  32 warps per SM (64 registers).  Bound by
+// One CTA per brick (or 2^split, each a part of its x range): its warps share
+// the brick's segments in the sweep, then its rows in the decode.  32 warps per
+// SM (64 registers).  Bound by
 // instruction issue (66-75% of the slots) and the shared-memory atomics: about
 // a third of the time goes to the sweep, less than a third to the setup of
 // bricks and segments, the rest to the decode, near half of it for the unit
@@ -958,9 +967,9 @@ __global__ void __launch_bounds__(kBrickThreads<MULTI>, 1024 / kBrickThreads<MUL
 voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
              int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
              const unsigned *__restrict__ list, unsigned n_pairs, unsigned *__restrict__ directory,
-             uint2 *__restrict__ marks, int64_t mark_share, const LayerDev *__restrict__ layers,
-             int32_t *const *__restrict__ labels, float *const *__restrict__ vecs,
-             unsigned long long *__restrict__ counters) {
+             uint2 *__restrict__ marks, int64_t mark_share, int split,
+             const LayerDev *__restrict__ layers, int32_t *const *__restrict__ labels,
+             float *const *__restrict__ vecs, unsigned long long *__restrict__ counters) {
    constexpr int kThreads = kBrickThreads<MULTI>, kWarps = kThreads / 32;
    __shared__ __align__(16) unsigned skey[kBrickVoxels];
    __shared__ SweepRec s_rec[kRecs<MULTI>];
@@ -980,9 +989,15 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    unsigned long long n_slow = 0, n_overlap = 0;
 
-   for (int64_t brick = brick_begin + blockIdx.x; brick < brick_end; brick += gridDim.x) {
+   for (int64_t place = blockIdx.x; place < (brick_end - brick_begin) << split;
+        place += gridDim.x) {
+      const int64_t brick = brick_begin + (place >> split);
       const BrickPlace p = brick_place(tiles, n_tiles, brick);
-      const int ox = p.ox, oy = p.oy, oz = p.oz, nx = p.nx, ny = p.ny, nz = p.nz;
+      const int x0 = (int)(place & ((1 << split) - 1)) * (kBrickX >> split);
+      const int nx = min(p.nx - x0, kBrickX >> split);
+      if (nx <= 0)
+         continue;
+      const int ox = p.ox + x0, oy = p.oy, oz = p.oz, ny = p.ny, nz = p.nz;
       const int Y = p.T->Y, Z = p.T->Z, layer_base = p.T->layer_base;
       const int max_layer = p.T->max_layer, n_bundles = p.T->n_bundles;
       int32_t *label = labels[p.tile];
@@ -1189,7 +1204,7 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
             if (lab == kMarkedLabel) {
                const unsigned at = atomicAdd(&s_marked, 1u);
                if (at < kMarkList)
-                  s_list[at] = (unsigned short)(lx * kPlane + ly * kBrickZ + lane);
+                  s_list[at] = (unsigned short)((x0 + lx) * kPlane + ly * kBrickZ + lane);
             }
             const unsigned m = __ballot_sync(0xFFFFFFFFu, defer);
             if (defer) {
@@ -1211,7 +1226,7 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          radial(lane);
       __syncthreads();
       if (warp == 0 && s_marked && mark_share > 0) { // the brick's record
-         const unsigned n = s_marked, place = (unsigned)(brick - brick_begin);
+         const unsigned n = s_marked;
          unsigned long long got = 0; // {entries taken, records}
          if (lane == 0) // (a record that does not fit takes no entries)
             got = atomicAdd(reinterpret_cast<unsigned long long *>(marks),
@@ -1220,9 +1235,9 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          const uint64_t at = 1u + (unsigned)got;
          const bool fits = n <= kMarkList && at + 1 + (n + 3) / 4 <= (uint64_t)mark_share;
          if (lane == 0) {
-            directory[got >> 32] = fits ? (unsigned)at : kScanBrick | place;
+            directory[got >> 32] = fits ? (unsigned)at : kScanBrick | (unsigned)place;
             if (fits)
-               marks[at] = make_uint2(place, n);
+               marks[at] = make_uint2((unsigned)place, n);
          }
          if (fits)
             for (unsigned e = lane; e < n; e += 32)
@@ -1235,6 +1250,17 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
    if (n_slow)
       atomicAdd(&counters[9], n_slow);
 }
+
+// Small volumes are as long as their longest brick and its marks.  Up to two
+// CTAs per SM a brick is swept by 2, 4 or 8 CTAs, each a part of its x range
+// with the same list; up to 1,216 units (two waves of voxel_marks' CTAs if each
+// held one) eight marked voxels go to a warp instead of a whole record.  Whole
+// calls, two bundles, without either -> with both: 24 x 24 x 24 (9 bricks) 163 ->
+// 118 us, 48 x 40 x 24 (30) 180 -> 156, 64 x 64 x 64 (128) 209 -> 177, with the
+// marks alone 96 x 96 x 60 (288) 295 -> 252, 128 x 128 x 60 (512) 332 -> 284, 160 x
+// 160 x 60 (800) 341 -> 313; 1,725 bricks 296 -> 301, and bricks split above 304
+// units change nothing (288: 253, 512: 285) or cost (288 by four: 269).
+constexpr int64_t kSplitBricks = 304, kSplitMarks = 1216;
 
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
@@ -1288,6 +1314,15 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
          FPGB_CUDA_TRY(cudaGetLastError());
       }
    }
+   // (up to eight times as many records: their directory at the end of their
+   // space)
+   int split = 0;
+   int64_t dir_entries = 0;
+   while (n_launch == 1 && split < 3 && n_bricks << (split + 1) <= kSplitBricks &&
+          mark_share > n_bricks << (split + 2)) {
+      split++;
+      dir_entries = ((n_bricks << split) + 1) / 2;
+   }
    cudaStream_t alt = chunks && chunks->n > 1 ? chunks->alt : nullptr;
    cudaEvent_t joined[2] = {};
    auto launch_all = [&]() -> int {
@@ -1301,21 +1336,27 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
          const int64_t b1 = chunks ? chunks->bound[c + 1] : n_bricks;
          cudaStream_t s = (alt && (c & 1)) ? alt : st;
          if (b1 > b0) {
-            const unsigned grid = (unsigned)std::min<int64_t>(b1 - b0, 0x7FFFFFFF);
-            // a warp per brick, up to about two waves
+            const int64_t n = (b1 - b0) << split;
+            const unsigned grid = (unsigned)std::min<int64_t>(n, 0x7FFFFFFF);
+            // a warp per record, or per part of it, up to about two waves
+            const int part = n <= kSplitMarks ? 8 : (int)kMarkList;
             const unsigned mark_grid = (unsigned)std::min<int64_t>(
-                (b1 - b0 + kMarkThreads / 32 - 1) / (kMarkThreads / 32), 152 * 8);
+                (n * ((int)kMarkList / part) + kMarkThreads / 32 - 1) / (kMarkThreads / 32),
+                152 * 8);
             uint2 *share = marks + c * mark_share;
+            const int64_t room = mark_share - dir_entries;
+            unsigned *directory =
+                split ? reinterpret_cast<unsigned *>(share + room) : counts + b0;
             auto kernel = multi_bundle ? voxel_bricks<true> : voxel_bricks<false>;
             const int threads = multi_bundle ? kBrickThreads<true> : kBrickThreads<false>;
             kernel<<<grid, threads, 0, s>>>(segs, tiles, n_tiles, b0, b1, offsets, list,
-                                                  (unsigned)n_pairs, counts + b0, share,
-                                                  mark_share, layers, labels, vecs, counters);
+                                            (unsigned)n_pairs, directory, share, room, split,
+                                            layers, labels, vecs, counters);
             FPGB_CUDA_TRY(cudaGetLastError());
-            // (the fill's cursors have become the directory of the records)
+            // (unsplit, the fill's cursors have become the directory of the records)
             voxel_marks<<<mark_grid, kMarkThreads, 0, s>>>(
-                segs, tiles, n_tiles, b0, b1, offsets, list, (unsigned)n_pairs, counts + b0,
-                share, mark_share, layers, labels, vecs, counters);
+                segs, tiles, n_tiles, b0, b1, offsets, list, (unsigned)n_pairs, directory, share,
+                room, split, part, layers, labels, vecs, counters);
             FPGB_CUDA_TRY(cudaGetLastError());
          }
          if (chunks && chunks->after)
