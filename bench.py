@@ -61,7 +61,7 @@ N_TILES = 256
 CPU_SAMPLE_STRIDE = 8      # GPU arm's CPU baseline / parity: every 8th tile (32 tiles)
 ONE_THREAD_TILES = (0, 128)  # the CPU baseline's 1-thread figure
 REF_TILES_PER_STEP = 8     # reference arm: 8 consecutive tiles per step, rotating
-VOXELIZER_LAUNCHES = 4     # brick_bin (count), brick_scan, brick_bin (fill), voxel_bricks
+VOXELIZER_LAUNCHES = 5     # brick_bin (count), brick_scan, brick_bin (fill), voxel_bricks, voxel_marks
 MARCH_LAUNCHES = 2         # batch_march untilted, tilted
 E2E_GROUPS = 16            # host-buffer e2e: tile groups pipelined by run_tiles_host (16: 228 ms, 8: 232, 4: 244, 2: 271)
 # units of the committed ncu captures (profiles/*_tiles16.md): the first 16 tiles
@@ -701,8 +701,8 @@ def measure_crossing(dev, steps=10, warmup=3):
 
 def measure_rofl(w, label, images, stream, reps=3, cpu_pixels=48, side=None):
     """ROFL (Simpli.apply_rofl's fit) of the crossing volume's 5-tilt image
-    series, every tissue pixel, on the device (MINPACK, one thread per
-    pixel), and the oracle (scipy's MINPACK, as the reference) on a sample
+    series, every tissue pixel, on the device (MINPACK, a lane or
+    a few per pixel), and the oracle (scipy's MINPACK, as the reference) on a sample
     of the same pixels on one host core (cpu_pixels = 0: no CPU leg).
     ``side``: only the first side x side pixels (a small case for ncu)."""
     import torch

@@ -14,8 +14,8 @@ Flags that matter for parity:
   * ``raymarch.cu``, ``batch.cu``: ``-fmad=false`` with the wanted fused
     multiply-adds written out — every march kernel (plain or batched,
     per-thread or cooperative) then gives the same bits for the same tile.
-  * ``optic.cu``: ``-fmad=false`` — the Gaussian filter sums in scipy's
-    order with separate roundings.
+  * ``optic.cu``: ``-fmad=false`` — the epa sums round as numpy's; the fused
+    multiply-adds of the optic map's weighted sums are written out.
   * ``rofl.cu``: ``-fmad=false`` — MINPACK's and numpy's sums and products
     round separately; the fused forms numpy's matrix product uses are
     written out.

@@ -546,7 +546,8 @@ size_t tissue_workspace_bytes(const TissuePlan &p) {
    return b;
 }
 
-// Bricks of a slabbed launch, at least: a wave of 4 per SM.
+// Bricks of a slabbed launch, at least: 4 per SM (a wave of the 256-thread
+// CTAs, half of one of the 128-thread ones).
 constexpr int64_t kSlabBricks = 608;
 
 int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,

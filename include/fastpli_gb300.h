@@ -102,8 +102,9 @@ int fpgb_generate_tissue(const fpgb_volume *vol, const fpgb_fibers *fibers,
 /* Device-resident variant.  d_label / d_vector are device buffers of the
  * full volume; d_workspace (>= fpgb_generate_workspace_size bytes, 256-byte
  * aligned) holds the segment and layer tables and the segment lists of the
- * voxel bricks (the per-voxel winner keys stay in shared memory), or NULL to
- * use the library's own cached device pool.  props/n_props/warnings are host memory;
+ * voxel bricks (the per-voxel winner keys stay in shared memory) with the
+ * records of the voxels that are decided exactly, or NULL to use the library's
+ * own cached device pool.  props/n_props/warnings are host memory;
  * warnings != NULL synchronises the stream. */
 size_t fpgb_generate_workspace_size(const fpgb_volume *vol,
                                     const fpgb_fibers *fibers);
@@ -238,7 +239,7 @@ int fpgb_epa_device(const double *d_image, int64_t n_pix, int64_t n_rho, double 
  * _ROFL_with_jacobi.py, as Simpli.apply_rofl applies it per pixel,
  * __simpli.py:623-705) of a 5-tilt series d_data [5, n_pix, n_rot] (tilts
  * (0,0), (tau,0), (tau,90), (tau,180), (tau,270) degrees; 4 <= n_rot <= 32),
- * FP64, one thread per pixel.  d_out [n_pix, 8] receives direction,
+ * FP64, 16, 4 or 1 lanes per pixel by n_pix.  d_out [n_pix, 8] receives direction,
  * inclination, t_rel, their standard deviations, chi^2 and MINPACK's
  * evaluation count (the reference's niter).  The fit is MINPACK's
  * Levenberg-Marquardt as scipy.optimize.leastsq runs it for the reference
