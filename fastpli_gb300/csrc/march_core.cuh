@@ -59,8 +59,8 @@ __device__ __forceinline__ float sinc_sq(float y) {
    return fmaf(p, y, 1.f);
 }
 
-// __fdividef(1, x) for x around 1: without its scaling of large divisors, which
-// changes nothing there (the same bits for every float in [0.5, 2]).
+// 1 / x for x around 1 by the approximate reciprocal instruction alone (the bits
+// of __fdividef(1, x) for every float in [0.5, 2], compared one by one).
 __device__ __forceinline__ float rcp_near_one(float x) {
    float r;
    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
