@@ -174,7 +174,9 @@ FPGB_HD void fill_segment(const double *P, const double *Q, double r0, double r1
    fill_fast_fields(S, dim);
    const double rm = r0 < r1 ? r1 : r0;
    S.thr_f = (float)((double)f_ly_squ * rm * rm * (1.0 + 1e-5)) * (1.f + 0x1p-22f);
-   S.mg = seg_margin(S, S.thr_f);
+   // (beyond, differences to base leave 32 bits; from 1e19 on the estimate's
+   // squares overflow, and an infinite one is not a distance)
+   S.mg = S.pscale < 0x1p30f ? seg_margin(S, S.thr_f) : INFINITY;
    const double rn = r0 < r1 ? r0 : r1;
    const double a = (double)f_ly_squ * rn * rn * (1.0 - 1e-5);
    float af = (float)a;

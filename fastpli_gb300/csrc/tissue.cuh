@@ -35,7 +35,8 @@ struct __align__(16) SegDev {
    int32_t lo[3];   // clipped box start (generator.cpp:304)
    int32_t ext[3];  // clipped box extent
    int32_t bundle;
-   float mg;         // bound on |sweep estimate - dist^2| over the box (seg_margin)
+   float mg;         // bound on |sweep estimate - dist^2| over the box (seg_margin);
+                     // infinite: the estimate says nothing
    float dec_rsq;    // float(r^2) at every t of the segment when that is one
                      // certain value (constant radius); NaN otherwise
    float rsq0, rsq1; // float(r^2) at t = 0 and t = 1 (exact)

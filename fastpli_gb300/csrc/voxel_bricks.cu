@@ -38,6 +38,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 
 #include "ff.cuh"
 #include "fpgb_common.cuh"
@@ -310,7 +312,7 @@ constexpr int kPlane = kBrickY * kBrickZ; // distance of x neighbours in the sha
 // Place of (y, z) in a plane of the shared arrays.  A row y is rotated by 9 y:
 // the lanes of a chunk cover several rows of a sub-box some 8 to 13 voxels
 // high, which would else share that many of the 32 banks.
-__device__ __forceinline__ int plane_place(int y, int z) {
+FPGB_HD int plane_place(int y, int z) {
    return y * kBrickZ + ((z + 9 * y) & (kBrickZ - 1));
 }
 
@@ -325,12 +327,45 @@ struct SegSweep {
    float mg;
 };
 
+// a / b within 2 ulps, of the device's approximate division
+FPGB_HD float quotient_est(float a, float b) {
+#ifdef __CUDA_ARCH__
+   return __fdividef(a, b);
+#else
+   return a / b;
+#endif
+}
+
+FPGB_HD int int_min(int a, int b) { return a < b ? a : b; }
+FPGB_HD int int_max(int a, int b) { return a > b ? a : b; }
+
+FPGB_HD int leading_zeros(unsigned v) { // v > 0
+#ifdef __CUDA_ARCH__
+   return __clz((int)v);
+#else
+   return __builtin_clz(v);
+#endif
+}
+
+FPGB_HD int float_bits(float f) {
+#ifdef __CUDA_ARCH__
+   return __float_as_int(f);
+#else
+   int i;
+   std::memcpy(&i, &f, sizeof i);
+   return i;
+#endif
+}
+
 __device__ __forceinline__ SegSweep load_sweep(const SegDev &S) {
    const float4 *f = reinterpret_cast<const float4 *>(&S.pf[0]);
    const int4 *i = reinterpret_cast<const int4 *>(&S.pf[0]);
    return SegSweep{__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(i + 3), __ldg(i + 4),
                    __ldg(&S.mg)};
 }
+
+// Whether the FP32 estimate of the segment bounds anything (SegDev::mg).
+FPGB_HD bool bounded(const SegSweep &w) { return w.mg < INFINITY; }
 
 // The part of segment S's clipped box inside the brick (origin o, extent n),
 // swept as columns along x: its ey x ez (y, z) cells are numbered z fastest,
@@ -342,22 +377,22 @@ struct SubBox {
    float inv_ez; // 1/ez for the division-free cell split
 };
 
-__device__ __forceinline__ bool sub_box(const SegSweep &w, int ox, int oy, int oz, int nx,
-                                        int ny, int nz, SubBox &b) {
-   b.x0 = max(w.d.y, ox);
-   b.y0 = max(w.d.z, oy);
-   b.z0 = max(w.d.w, oz);
-   b.ex = min(w.d.y + w.e.x, ox + nx) - b.x0;
-   b.ey = min(w.d.z + w.e.y, oy + ny) - b.y0;
-   b.ez = min(w.d.w + w.e.z, oz + nz) - b.z0;
+FPGB_HD bool sub_box(const SegSweep &w, int ox, int oy, int oz, int nx, int ny, int nz,
+                     SubBox &b) {
+   b.x0 = int_max(w.d.y, ox);
+   b.y0 = int_max(w.d.z, oy);
+   b.z0 = int_max(w.d.w, oz);
+   b.ex = int_min(w.d.y + w.e.x, ox + nx) - b.x0;
+   b.ey = int_min(w.d.z + w.e.y, oy + ny) - b.y0;
+   b.ez = int_min(w.d.w + w.e.z, oz + nz) - b.z0;
    if (b.ex <= 0 || b.ey <= 0 || b.ez <= 0)
       return false;
    b.ncell = b.ey * b.ez;
-   b.inv_ez = __fdividef(1.f, (float)b.ez);
+   b.inv_ez = quotient_est(1.f, (float)b.ez);
    return true;
 }
 
-__device__ __forceinline__ int brick_index(int x, int y, int z, int ox, int oy, int oz) {
+FPGB_HD int brick_index(int x, int y, int z, int ox, int oy, int oz) {
    return ((x - ox) * kBrickY + (y - oy)) * kBrickZ + (z - oz);
 }
 
@@ -375,19 +410,17 @@ struct BrickScale {
 
 constexpr unsigned kNoKey = 0xFFFFFFFFu;
 
-__device__ __forceinline__ bool key_marked(unsigned key) { return (key & 1u) && key != kNoKey; }
-
-__device__ BrickScale brick_scale(unsigned n_seg, float max_thr2, float max_mg) {
+FPGB_HD BrickScale brick_scale(unsigned n_seg, float max_thr2, float max_mg) {
    BrickScale k;
-   const int bits = n_seg <= 128u ? 8 : min(31, 33 - __clz((int)(n_seg - 1u)));
-   const int qbits = min(23, 32 - bits);
+   const int bits = n_seg <= 128u ? 8 : int_min(31, 33 - leading_zeros(n_seg - 1u));
+   const int qbits = int_min(23, 32 - bits);
    k.bits = bits;
    k.mul = 1u << bits;
    const float top = qbits > 3 ? (float)((1u << qbits) - 4u) : 0.f;
-   k.scale = 0.999999f * __fdividef(top, max_thr2);
+   k.scale = 0.999999f * quotient_est(top, max_thr2);
    if (!(k.scale > 0.f && k.scale < 1e30f))
       k.scale = 0.f;
-   k.quantum = k.scale > 0.f ? __fdividef(1.000001f, k.scale) : INFINITY;
+   k.quantum = k.scale > 0.f ? quotient_est(1.000001f, k.scale) : INFINITY;
    k.mg2 = 2.f * max_mg;
    const float w = fmaf(k.mg2, k.scale, 4.f) * (float)k.mul;
    if (w < 1e9f) {
@@ -401,7 +434,7 @@ __device__ BrickScale brick_scale(unsigned n_seg, float max_thr2, float max_mg) 
 }
 
 // Upper bound of the hi that a voxel's key stands for.
-__device__ __forceinline__ float key_bound(const BrickScale &k, unsigned key) {
+FPGB_HD float key_bound(const BrickScale &k, unsigned key) {
    return ((float)(key >> k.bits) + 1.f) * k.quantum;
 }
 
@@ -415,11 +448,10 @@ struct __align__(16) SweepRec {
    unsigned box;               // ncell, ez << 9, ex << 15, first voxel's place << 19
 };
 
-__device__ __forceinline__ SweepRec sweep_rec(const SegSweep &w, const SubBox &b, bool any,
-                                              int ox, int oy, int oz) {
+FPGB_HD SweepRec sweep_rec(const SegSweep &w, const SubBox &b, bool any, int ox, int oy, int oz) {
    SweepRec r;
-   r.wx0 = ((float)(b.x0 - __float_as_int(w.c.z)) + 0.5f) - w.a.x;
-   r.wy0 = ((float)(b.y0 - __float_as_int(w.c.w)) + 0.5f) - w.a.y;
+   r.wx0 = ((float)(b.x0 - float_bits(w.c.z)) + 0.5f) - w.a.x;
+   r.wy0 = ((float)(b.y0 - float_bits(w.c.w)) + 0.5f) - w.a.y;
    r.wz0 = ((float)(b.z0 - w.d.x) + 0.5f) - w.a.z;
    r.mg = w.mg;
    r.vn2x = -2.f * w.a.w;
@@ -427,8 +459,12 @@ __device__ __forceinline__ SweepRec sweep_rec(const SegSweep &w, const SubBox &b
    r.vn2z = -2.f * w.b.y;
    r.c2f = w.b.z;
    r.rch = -0.5f * w.b.w;
-   // (finite: an infinite hi is outside)
+   // (finite: a radius whose square is not)
    r.thr = fminf(fmaf(2.00001f, w.mg, w.c.x), 3e38f);
+   if (!bounded(w)) { // every voxel of the box counts as inside; W marks it
+      r.wx0 = r.wy0 = r.wz0 = r.mg = 0.f;
+      r.vn2x = r.vn2y = r.vn2z = r.c2f = r.rch = 0.f;
+   }
    r.inv_ez = b.inv_ez;
    r.box = any ? (unsigned)b.ncell | (unsigned)b.ez << 9 | (unsigned)b.ex << 15 |
                      (unsigned)brick_index(b.x0, b.y0, b.z0, ox, oy, oz) << 19
@@ -446,7 +482,7 @@ struct Cell {
    float a2, b; // the y / z parts of the estimate
 };
 
-__device__ __forceinline__ Cell cell_of(const SweepRec &g, float ezf, float c) {
+FPGB_HD Cell cell_of(const SweepRec &g, float ezf, float c) {
    const float iy = truncf((c + 0.5f) * g.inv_ez);
    const float iz = fmaf(-iy, ezf, c);
    const float wy = g.wy0 + iy, wz = g.wz0 + iz;
@@ -627,8 +663,7 @@ constexpr int kLayerCache = 4;
 // (generator.cpp:345-349).  2^-20 covers the rounding of the quotient and of
 // the products here.  -1 when the interval straddles a boundary, the
 // outermost one included.
-__device__ __forceinline__ int certain_layer(const float *sq, int n, float lo, float hi,
-                                             float r_sqr) {
+FPGB_HD int certain_layer(const float *sq, int n, float lo, float hi, float r_sqr) {
    int w = 0;
    bool sure = true;
    for (int l = 0; l < n; l++) {
@@ -823,9 +858,13 @@ __device__ __forceinline__ void resolve_marks(const MarkCtx &C, MarkWarp &W, int
                                           ((float)(y - __float_as_int(w.c.w)) + 0.5f) - w.a.y,
                                           ((float)(z - w.d.x) + 0.5f) - w.a.z, w.a.w, w.b.x,
                                           w.b.y, w.b.z, w.b.w, mg);
+            float hi = __fadd_ru(d2, mg);
             lo = __fsub_rd(d2, mg);
-            const float hi = __fadd_ru(d2, mg);
-            certain = hi <= w.c.y;
+            if (!bounded(w)) {
+               lo = 0.f;
+               hi = INFINITY;
+            }
+            certain = hi <= w.c.y && hi < INFINITY;
             in = !(lo > w.c.x);
             if (certain) {
                atomicMin(&W.bound[m], __float_as_uint(hi));
@@ -1053,7 +1092,8 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          s_rec[j % kRecs<MULTI>] = sweep_rec(w, b, any, ox, oy, oz);
          if (MULTI)
             s_acc[j % kRecs<MULTI>] =
-                make_uint2(__float_as_uint(fminf(w.c.y, 3e38f)), (unsigned)w.e.w);
+                make_uint2(__float_as_uint(bounded(w) ? fminf(w.c.y, 3e38f) : -1.f),
+                           (unsigned)w.e.w);
       };
       { // the first records, and the largest bounds of the list's segments
         // (floats >= 0: bits order like values)

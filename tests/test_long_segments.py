@@ -1,0 +1,76 @@
+"""Segments longer than the volume, up to lengths whose squares overflow in
+FP32 and FP64.  On the CPU a replay of the bricks' sweep (host build of the
+kernel's functions): every voxel that it does not mark has the winner and layer
+of the FP64 evaluation of all candidates.  On the GPU labels, vectors and
+warnings against the oracle bit for bit, with short fibers in the same bricks."""
+
+import os
+import shutil
+import subprocess
+import warnings
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SRC = os.path.join(ROOT, "tests", "native", "voxel_brick_check.cu")
+LENGTHS = ["1e3", "1e6", "1e9", "2e9", "1e12", "1e16", "1e19", "1.6e19", "1e20", "1e160"]
+LY1 = [(1.0, 0.004, 1.0, "r")]
+LY3 = [(0.333, -0.004, 10.0, "p"), (0.666, 0.0, 5.0, "b"), (1.0, 0.004, 1.0, "r")]
+
+
+@pytest.fixture(scope="module")
+def checker(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    exe = str(tmp_path_factory.mktemp("bcheck") / "bcheck")
+    subprocess.run([nvcc, "-O2", "-std=c++17", "-fmad=false", "-Xcompiler",
+                    "-ffp-contract=off,-fopenmp", "-I", os.path.join(ROOT, "include"), SRC,
+                    "-o", exe], check=True, capture_output=True)
+    return exe
+
+
+def replay(checker, *args):
+    r = subprocess.run([checker, *map(str, args)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return dict(zip(r.stdout.split()[::2], r.stdout.split()[1::2]))
+
+
+@pytest.mark.parametrize("length", LENGTHS)
+def test_unmarked_voxels_are_certain(checker, length):
+    replay(checker, 9, 96, 80, 64, 3, 12, 2, 0, length)
+
+
+@pytest.mark.parametrize("radius,points,taper", [(1e20, 3, 0), (4, 9, 0), (4, 9, 0.5)])
+def test_unmarked_voxels_are_certain_at_other_radii(checker, radius, points, taper):
+    replay(checker, 5, 61, 43, 50, radius, 14, points, taper, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", LENGTHS)
+def test_long_segments_match_oracle(cuda, oracle_port, length):
+    from fastpli_gb300.simulation import _Generator
+    rng = np.random.default_rng(11)
+    dim = (48, 57, 40)
+    long, short = [], []
+    for _ in range(8):
+        d = rng.normal(size=3)
+        d = d / np.linalg.norm(d) * float(length)
+        m, e = rng.uniform(0.2, 0.8, 3) * dim, rng.uniform(0.2, 0.8)
+        long.append(np.array([[*(m - e * d), 3.0], [*(m + (1 - e) * d), 3.0]]))
+        q = rng.uniform(0.1, 0.9, 3) * dim + np.linspace(-4, 4, 5)[:, None] * rng.normal(size=3)
+        short.append(np.column_stack([q, np.full(5, 2.0)]))
+    fibers, layers = [long, short], [LY3, LY1]
+    with np.errstate(all="ignore"):
+        olab, ovec, _, owarn = oracle_port.generate(dim, [0.0] * 3, 1.0, fibers, layers)
+    assert (olab > 0).any()
+    g = _Generator()
+    g.set_volume(dim, [0.0] * 3, 1.0)
+    g.set_fiber_bundles(fibers, layers)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        label, vector, _, w = g.run_generation_device()
+    assert np.array_equal(label.cpu().numpy(), olab)
+    assert np.array_equal(vector.cpu().numpy().view(np.uint32), ovec.view(np.uint32))
+    assert w["overlap"] == owarn["overlap"]
