@@ -72,7 +72,7 @@ struct fpgb_batch_impl {
    std::vector<size_t> table_off; // per pair: lut then ztab, relative to ws_tables
    int64_t total_vox = 0, steps = 0;
    int64_t n_bricks = 0, brick_pairs = 0;
-   bool any_multi_bundle = false;
+   bool any_multi_bundle = false, any_long = false;
    int want_epa = 0;
    // bound buffers
    char *arena = nullptr, *ws = nullptr;
@@ -390,6 +390,7 @@ int plan_batch(int64_t n_tiles, const fpgb_volume *vols, const fpgb_fibers *fibe
       if (P.n_bundles == 0)
          B->layers.push_back(LayerDev{});
       B->any_multi_bundle |= P.n_bundles > 1;
+      B->any_long |= P.long_segs;
       vox += T.n_vox;
    }
    if (seg_base[n_tiles] > 0xFFFFFFF0ull) {
@@ -595,7 +596,7 @@ int run_batch(fpgb_batch_impl *B, int march_ctas_per_sm, int chunk, int coop, cu
       FPGB_CUDA_TRY(cudaMemsetAsync(counters, 0,
                                     sizeof(unsigned long long) * (kCounterWords + 2), st));
       FPGB_TRY(launch_voxel_bricks(segs, seg_tile, B->n_segs, tiles, (int64_t)nt,
-                                   B->n_bricks, B->brick_pairs, layers, B->any_multi_bundle,
+                                   B->n_bricks, B->brick_pairs, layers, B->any_multi_bundle, B->any_long,
                                    lptr, vptr, W + B->ws_bricks, counters, st));
    } else {
       // the march's queue counters only: the voxelizer's warnings stay

@@ -45,32 +45,14 @@ FPGB_HD void split2(double d, float &hi, float &lo) {
    lo = (float)(d - (double)hi);
 }
 
-// Bound on |estimate - reference float| of the sweep's FP32 dist^2
-// (sweep_dist2) over the voxels of the segment's box that lie within or next
-// to the segment's thickest end: |w| <= |v| + r' for the voxel's offset w
-// from p.  With u = 2^-24, the rounding of the inputs (w: u (|w0| + |w| + 1)
-// for the offset w0 of the sub-box's first cell, v, c2: u each), of the six
-// operations and of the sum of the margin itself stays below u (15 |w|^2 +
-// 2 |w| |w0| + 12 c2 + 4) (the error of t enters squared: the value is the
-// squared distance to some point of the segment); the reference's own double
-// arithmetic adds 2^-50 pscale |w| and its final rounding u |w|^2.  18 u and
-// 12 u are 1.08e-6 and 7.2e-7.  For a voxel farther away, d >= |w| - |v|, so
-// that error is below 3.3e-6 d^2 + 4e-6 c2 and the estimate stays past the
-// thickest end as the distance does: r' has more than that on top.
-// Evaluated in float, whose own rounding (below 1e-5) the factor 1.001 covers.
+// The segment's own bound (sweep_margin) over its whole box.
 FPGB_HD float seg_margin(const SegDev &S, float thr) {
-   float w2 = 0.f;
+   float first[3], steps[3];
    for (int i = 0; i < 3; i++) {
-      const float a = (float)((double)S.lo[i] + 0.5 - S.p[i]);
-      const float b = a + (float)(S.ext[i] > 0 ? S.ext[i] - 1 : 0);
-      w2 += fmaxf(a * a, b * b);
+      first[i] = (float)((double)S.lo[i] + 0.5 - S.p[i]);
+      steps[i] = (float)(S.ext[i] > 0 ? S.ext[i] - 1 : 0);
    }
-   const float box = sqrtf(w2), v = sqrtf(S.c2f), ps = 1e-14f * S.pscale;
-   const float near = v + sqrtf(thr * 1.0001f + 0.01f + 1e-4f * S.c2f +
-                                10.f * ps * (v + sqrtf(thr) + 1.f));
-   const float w = fminf(box, near);
-   return 1.001f * (1.08e-6f * w * w + 1.5e-7f * w * box + 7.2e-7f * S.c2f + 2e-6f +
-                    ps * (w + 1.f));
+   return sweep_margin(first, steps, S.c2f, S.pscale, thr);
 }
 
 // Host-side constants of the two-float path, all derived in double exactly
@@ -174,15 +156,19 @@ FPGB_HD void fill_segment(const double *P, const double *Q, double r0, double r1
    fill_fast_fields(S, dim);
    const double rm = r0 < r1 ? r1 : r0;
    S.thr_f = (float)((double)f_ly_squ * rm * rm * (1.0 + 1e-5)) * (1.f + 0x1p-22f);
-   // (beyond, differences to base leave 32 bits; from 1e19 on the estimate's
-   // squares overflow, and an infinite one is not a distance)
-   S.mg = S.pscale < 0x1p30f ? seg_margin(S, S.thr_f) : INFINITY;
+   S.mg = seg_margin(S, S.thr_f);
    const double rn = r0 < r1 ? r0 : r1;
    const double a = (double)f_ly_squ * rn * rn * (1.0 - 1e-5);
    float af = (float)a;
    if ((double)af > a)
       af = nextafterf(af, 0.f);
-   S.acc_f = af > 0.f ? af : -1.f;
+   S.acc_f = af > 0.f ? fminf(af, 3e38f) : -1.f; // (finite, as hi)
+   // From 2^30 voxels on differences to base leave 32 bits, from 1e19 on the
+   // estimate's squares overflow, and an infinite one is not a distance.
+   if (!(S.pscale < 0x1p30f)) {
+      S.mg = S.c2f = INFINITY;
+      S.acc_f = -1.f;
+   }
    S.bundle = bundle;
 }
 
@@ -263,6 +249,17 @@ Box fiber_box(const double *xyz, const double *r, int64_t n) {
 // 29.6 and 22.7 ms).
 constexpr size_t kTogetherBytes = size_t(256) << 10;
 
+bool long_segment(const double *p, const double *q) {
+   double c2 = 0.0;
+   bool far = false;
+   for (int i = 0; i < 3; i++) {
+      const double v = q[i] - p[i];
+      c2 = c2 + v * v;
+      far = far || std::fabs(p[i]) > 0x1p29 || std::fabs(q[i]) > 0x1p29;
+   }
+   return (float)c2 > kLongSquared || far;
+}
+
 int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan, bool fill) {
    if (!vol || !fb) {
       set_error("generate_tissue: null volume or fibers");
@@ -294,6 +291,7 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
    plan->Y = vol->dim[1];
    plan->Z = vol->dim[2];
    plan->n_bundles = nb;
+   plan->long_segs = false;
    plan->segs.clear();
    plan->source.clear();
    plan->layers.assign(nb > 0 ? nb : 1, LayerDev{});
@@ -440,7 +438,8 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
       return bundle_on[b] && p1 - p0 > 1 && overlap(volbox, fbox[fi]) && plan->layers[b].n > 0;
    };
    int64_t cand = 0, pairs = 0;
-#pragma omp parallel for schedule(dynamic, 32) reduction(+ : cand, pairs) if (np > kSerialPoints)
+   bool longer = false;
+#pragma omp parallel for schedule(dynamic, 32) reduction(+ : cand, pairs) reduction(|| : longer) if (np > kSerialPoints)
    for (int64_t fi = 0; fi < nf; fi++) {
       const int64_t b = fiber_bundle[fi];
       const int64_t p0 = fb->fiber_point_off[fi], p1 = fb->fiber_point_off[fi + 1];
@@ -460,6 +459,7 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
          n++;
          cand += count;
          pairs += segment_brick_pairs(S);
+         longer = longer || long_segment(&xyz[3 * s], &xyz[3 * (s + 1)]);
       }
       fiber_segs[fi + 1] = n;
    }
@@ -470,6 +470,7 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
    plan->n_segs = fiber_segs[nf];
    plan->candidates = cand;
    plan->brick_pairs = pairs;
+   plan->long_segs = longer;
    if (plan->n_segs > 0xFFFFFFF0ll) {
       set_error("too many fiber segments: %lld", (long long)plan->n_segs);
       return FPGB_EINVAL;
@@ -674,7 +675,7 @@ int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
       chunks = BrickChunks{n, bound, &Slabs::thunk, &slabs, alt};
    }
    FPGB_TRY(launch_voxel_bricks(segs, nullptr, p.n_segs, tile, 1, n_bricks,
-                                p.brick_pairs, layers, p.n_bundles > 1, lp, vp, w, counters, st,
+                                p.brick_pairs, layers, p.n_bundles > 1, p.long_segs, lp, vp, w, counters, st,
                                 n > 1 ? &chunks : nullptr));
    if (n == 1 && after_slab)
       FPGB_TRY(after_slab(ctx, 0, p.X, st));

@@ -36,7 +36,7 @@ struct __align__(16) SegDev {
    int32_t ext[3];  // clipped box extent
    int32_t bundle;
    float mg;         // bound on |sweep estimate - dist^2| over the box (seg_margin);
-                     // infinite: the estimate says nothing
+                     // infinite, and c2f with it: the estimate says nothing
    float dec_rsq;    // float(r^2) at every t of the segment when that is one
                      // certain value (constant radius); NaN otherwise
    float rsq0, rsq1; // float(r^2) at t = 0 and t = 1 (exact)
@@ -111,6 +111,7 @@ struct TissuePlan {
    int64_t candidates = 0;   // sum of clipped box volumes
    int64_t brick_pairs = 0;  // (segment, brick) pairs of the brick voxelizer
    int64_t n_segs = 0;
+   bool long_segs = false; // some segment is long_segment
    // the segment table; or, unfilled, what the device fills it from: n_points x
    // (x, y, z) in voxels, n_points radii, n_segs SegSrc
    RawArray<SegDev> segs;
@@ -120,6 +121,11 @@ struct TissuePlan {
    std::vector<LayerDev> layers;
    std::vector<double> props; // (dn, mu) rows
 };
+
+// Longer than 64 voxels, or 2^29 voxels away: what the sweep takes part by part
+// or without a bound.
+constexpr float kLongSquared = 64.f * 64.f;
+bool long_segment(const double *p, const double *q);
 
 // fill = false leaves a large segment table to the device (run_tissue).
 int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,

@@ -92,6 +92,36 @@ FPGB_HD float sweep_dist2(float wx, float a2, float b, float vn2, float c2f, flo
    return fmaf(t, fmaf(t, c2f, c1n), fmaf(wx, wx, b));
 }
 
+// Bound on |estimate - reference float| of the sweep's FP32 dist^2
+// (sweep_dist2) over a box of voxels, from the offsets `first` of its first
+// voxel from the segment's start and its last one `steps` further, over the
+// voxels that lie within or next to the segment's thickest end (thr): |w| <=
+// |v| + r' for the voxel's offset w from the start.  With u = 2^-24, the
+// rounding of the inputs (w: u (|w0| + |w| + 1) for the offset w0 of the
+// sub-box's first cell, v, c2: u each), of the six operations and of the sum of
+// the margin itself stays below u (15 |w|^2 + 2 |w| |w0| + 12 c2 + 4) (the
+// error of t enters squared: the value is the squared distance to some point
+// of the segment); the reference's own double arithmetic adds 2^-50 pscale |w|
+// and its final rounding u |w|^2.  18 u and 12 u are 1.08e-6 and 7.2e-7.  For a
+// voxel farther away, d >= |w| - |v|, so that error is below 3.3e-6 d^2 + 4e-6
+// c2 and the estimate stays past the thickest end as the distance does: r' has
+// more than that on top.  Evaluated in float, whose own rounding (below 1e-5)
+// the factor 1.001 covers.
+FPGB_HD float sweep_margin(const float first[3], const float steps[3], float c2f, float pscale,
+                           float thr) {
+   float w2 = 0.f;
+   for (int i = 0; i < 3; i++) {
+      const float a = first[i], b = a + steps[i];
+      w2 += fmaxf(a * a, b * b);
+   }
+   const float box = sqrtf(w2), v = sqrtf(c2f), ps = 1e-14f * pscale;
+   const float near = v + sqrtf(thr * 1.0001f + 0.01f + 1e-4f * c2f +
+                                10.f * ps * (v + sqrtf(thr) + 1.f));
+   const float w = fminf(box, near);
+   return 1.001f * (1.08e-6f * w * w + 1.5e-7f * w * box + 7.2e-7f * c2f + 2e-6f +
+                    ps * (w + 1.f));
+}
+
 // float(|cl - pt|^2) and float(r(t)^2) exactly as generator.cpp:327-328.
 FPGB_HD void exact_dist(const SegDev &S, const double pt[3],
                                            double cl[3], float &dist_squ,

@@ -364,9 +364,6 @@ __device__ __forceinline__ SegSweep load_sweep(const SegDev &S) {
                    __ldg(&S.mg)};
 }
 
-// Whether the FP32 estimate of the segment bounds anything (SegDev::mg).
-FPGB_HD bool bounded(const SegSweep &w) { return w.mg < INFINITY; }
-
 // The part of segment S's clipped box inside the brick (origin o, extent n),
 // swept as columns along x: its ey x ez (y, z) cells are numbered z fastest,
 // lane l of chunk c owns cell 32 c + l and visits the ex voxels of that
@@ -448,23 +445,80 @@ struct __align__(16) SweepRec {
    unsigned box;               // ncell, ez << 9, ex << 15, first voxel's place << 19
 };
 
-FPGB_HD SweepRec sweep_rec(const SegSweep &w, const SubBox &b, bool any, int ox, int oy, int oz) {
-   SweepRec r;
-   r.wx0 = ((float)(b.x0 - float_bits(w.c.z)) + 0.5f) - w.a.x;
-   r.wy0 = ((float)(b.y0 - float_bits(w.c.w)) + 0.5f) - w.a.y;
-   r.wz0 = ((float)(b.z0 - w.d.x) + 0.5f) - w.a.z;
-   r.mg = w.mg;
-   r.vn2x = -2.f * w.a.w;
-   r.vn2y = -2.f * w.b.x;
-   r.vn2z = -2.f * w.b.y;
-   r.c2f = w.b.z;
-   r.rch = -0.5f * w.b.w;
-   // (finite: a radius whose square is not)
-   r.thr = fminf(fmaf(2.00001f, w.mg, w.c.x), 3e38f);
-   if (!bounded(w)) { // every voxel of the box counts as inside; W marks it
-      r.wx0 = r.wy0 = r.wz0 = r.mg = 0.f;
-      r.vn2x = r.vn2y = r.vn2z = r.c2f = r.rch = 0.f;
+// A segment as the sweep of one sub-box sees it: the first voxel's offset from
+// its start, its direction, their FP32 invariants and the bound of the estimate.
+struct SegPart {
+   float w0[3], v[3], c2f, c2_rcp, mg;
+};
+
+// The estimate's error grows with the square of a segment's length, and the
+// largest of a brick's margins decides which of its voxels are close calls.  So
+// of a long segment the sweep takes the part that holds the closest point of
+// every voxel of the sub-box: the distances are the same (the rounding of the
+// part's start in double, below 2^-50 pscale, is a ninth of what sweep_margin
+// has for that), the error that of a segment as long as the sub-box.
+__host__ __device__ __noinline__ inline SegPart long_part(const SegDev &S, const SubBox &b) {
+   SegPart r{};
+   r.mg = INFINITY;
+   if (!(S.mg < INFINITY)) // every voxel of the sub-box counts as inside, W marks it
+      return r;
+   const int first[3] = {b.x0, b.y0, b.z0}, ext[3] = {b.ex, b.ey, b.ez};
+   // closest-point parameters of the sub-box: its centre's, give or take half its
+   // extent along v and 1/16 voxel
+   double mid = 0.0, reach = 0.0625 * sqrtf(S.c2f);
+   for (int i = 0; i < 3; i++) {
+      const double half = 0.5 * (ext[i] - 1);
+      mid = mid + ((first[i] + 0.5 + half) - S.p[i]) * S.v[i];
+      reach = reach + half * fabs(S.v[i]);
    }
+   const double rc2 = 1.0 / S.c2;
+   const double t0 = fmin(fmax((mid - reach) * rc2, 0.0), 1.0);
+   const double part = fmin(fmax((mid + reach) * rc2, 0.0), 1.0) - t0;
+   float steps[3];
+   for (int i = 0; i < 3; i++) {
+      r.w0[i] = (float)((first[i] + 0.5) - (S.p[i] + S.v[i] * t0));
+      r.v[i] = (float)(S.v[i] * part);
+      steps[i] = (float)(ext[i] - 1);
+   }
+   r.c2f = (float)(part * part * S.c2);
+   r.c2_rcp = r.c2f > 0.f ? 1.f / r.c2f : 0.f;
+   r.mg = sweep_margin(r.w0, steps, r.c2f, S.pscale, S.thr_f);
+   return r;
+}
+
+template <bool LONG>
+FPGB_HD SegPart seg_part(const SegDev &S, const SegSweep &w, const SubBox &b) {
+   if (LONG && w.b.z > kLongSquared)
+      return long_part(S, b);
+   const int first[3] = {b.x0, b.y0, b.z0}, base[3] = {float_bits(w.c.z), float_bits(w.c.w), w.d.x};
+   const float pf[3] = {w.a.x, w.a.y, w.a.z};
+   SegPart r;
+   for (int i = 0; i < 3; i++)
+      r.w0[i] = ((float)(first[i] - base[i]) + 0.5f) - pf[i];
+   r.v[0] = w.a.w;
+   r.v[1] = w.b.x;
+   r.v[2] = w.b.y;
+   r.c2f = w.b.z;
+   r.c2_rcp = w.b.w;
+   r.mg = w.mg;
+   return r;
+}
+
+template <bool LONG>
+FPGB_HD SweepRec sweep_rec(const SegPart &g, float thr, const SubBox &b, bool any, int ox, int oy,
+                           int oz) {
+   SweepRec r;
+   r.wx0 = g.w0[0];
+   r.wy0 = g.w0[1];
+   r.wz0 = g.w0[2];
+   r.mg = !LONG || g.mg < INFINITY ? g.mg : 0.f;
+   r.vn2x = -2.f * g.v[0];
+   r.vn2y = -2.f * g.v[1];
+   r.vn2z = -2.f * g.v[2];
+   r.c2f = g.c2f;
+   r.rch = -0.5f * g.c2_rcp;
+   // (finite: a radius whose square is not)
+   r.thr = fminf(fmaf(2.00001f, g.mg, thr), 3e38f);
    r.inv_ez = b.inv_ez;
    r.box = any ? (unsigned)b.ncell | (unsigned)b.ez << 9 | (unsigned)b.ex << 15 |
                      (unsigned)brick_index(b.x0, b.y0, b.z0, ox, oy, oz) << 19
@@ -858,13 +912,9 @@ __device__ __forceinline__ void resolve_marks(const MarkCtx &C, MarkWarp &W, int
                                           ((float)(y - __float_as_int(w.c.w)) + 0.5f) - w.a.y,
                                           ((float)(z - w.d.x) + 0.5f) - w.a.z, w.a.w, w.b.x,
                                           w.b.y, w.b.z, w.b.w, mg);
-            float hi = __fadd_ru(d2, mg);
-            lo = __fsub_rd(d2, mg);
-            if (!bounded(w)) {
-               lo = 0.f;
-               hi = INFINITY;
-            }
-            certain = hi <= w.c.y && hi < INFINITY;
+            lo = w.mg < INFINITY ? __fsub_rd(d2, mg) : 0.f;
+            const float hi = __fadd_ru(d2, mg);
+            certain = hi <= w.c.y;
             in = !(lo > w.c.x);
             if (certain) {
                atomicMin(&W.bound[m], __float_as_uint(hi));
@@ -1001,7 +1051,10 @@ struct RadialQueue {
 // sweeps with an exact evaluation of 0.9 candidates per voxel in this one:
 // 523 -> 219 + 45 us and 2,216 -> 929 + 153 us; the marked voxels resolved here
 // instead (a list, a queue and two barriers per brick): 330 and 1,290 us.
-template <bool MULTI>
+// LONG: the list may hold long segments (a kernel of its own: with long_part's
+// call in it the kernel of the others took 888 us on the crossing volume
+// instead of 866).
+template <bool MULTI, bool LONG>
 __global__ void __launch_bounds__(kBrickThreads<MULTI>, 1024 / kBrickThreads<MULTI>)
 voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
              int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
@@ -1085,15 +1138,18 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          s_multi = MULTI && n_bundles > 1 &&
                    *reinterpret_cast<volatile unsigned long long *>(&counters[0]) == 0;
       }
-      auto prepare = [&](unsigned j, unsigned s) {
+      // the record of the list's segment j; the bound of its estimate
+      auto prepare = [&](unsigned j, unsigned s) -> float {
          const SegSweep w = load_sweep(segs[s]);
          SubBox b;
-         const bool any = sub_box(w, ox, oy, oz, nx, ny, nz, b);
-         s_rec[j % kRecs<MULTI>] = sweep_rec(w, b, any, ox, oy, oz);
+         const bool any = sub_box(w, ox, oy, oz, nx, ny, nz, b); // (a brick's part may not)
+         if (LONG && !any)
+            b = SubBox{};
+         const SegPart g = seg_part<LONG>(segs[s], w, b);
+         s_rec[j % kRecs<MULTI>] = sweep_rec<LONG>(g, w.c.x, b, any, ox, oy, oz);
          if (MULTI)
-            s_acc[j % kRecs<MULTI>] =
-                make_uint2(__float_as_uint(bounded(w) ? fminf(w.c.y, 3e38f) : -1.f),
-                           (unsigned)w.e.w);
+            s_acc[j % kRecs<MULTI>] = make_uint2(__float_as_uint(w.c.y), (unsigned)w.e.w);
+         return LONG && !any ? 0.f : g.mg;
       };
       { // the first records, and the largest bounds of the list's segments
         // (floats >= 0: bits order like values)
@@ -1101,15 +1157,20 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
          for (unsigned j = threadIdx.x; j < n_seg; j += kThreads) {
             const unsigned s = list[j0 + j];
             const SegDev &S = segs[s];
-            const float m = __ldg(&S.mg);
+            float m = __ldg(&S.mg);
             if (j < kSegCache) {
                s_seg[j] = s;
                s_rsq[j] = __ldg(&S.dec_rsq);
                if (MULTI)
                   s_bundle[j] = __ldg(&S.bundle);
             }
-            if (j < kRecs<MULTI>)
-               prepare(j, s);
+            if (j < kRecs<MULTI>) {
+               const float part = prepare(j, s);
+               m = LONG ? part : m;
+            } else if (LONG && __ldg(&S.c2f) > kLongSquared) {
+               SubBox b;
+               m = sub_box(load_sweep(S), ox, oy, oz, nx, ny, nz, b) ? long_part(S, b).mg : 0.f;
+            }
             th = max(th, __float_as_uint(fmaf(2.0001f, m, __ldg(&S.thr_f))));
             mg = max(mg, __float_as_uint(m));
          }
@@ -1304,8 +1365,8 @@ constexpr int64_t kSplitBricks = 304, kSplitMarks = 1216;
 
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
-                        const LayerDev *layers, bool multi_bundle, int32_t *const *labels,
-                        float *const *vecs, void *ws, unsigned long long *counters,
+                        const LayerDev *layers, bool multi_bundle, bool long_segs,
+                        int32_t *const *labels, float *const *vecs, void *ws, unsigned long long *counters,
                         cudaStream_t st, const BrickChunks *chunks) {
    if (n_tiles <= 0 || n_bricks <= 0)
       return FPGB_OK;
@@ -1387,7 +1448,10 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
             const int64_t room = mark_share - dir_entries;
             unsigned *directory =
                 split ? reinterpret_cast<unsigned *>(share + room) : counts + b0;
-            auto kernel = multi_bundle ? voxel_bricks<true> : voxel_bricks<false>;
+            auto kernel = multi_bundle ? long_segs ? voxel_bricks<true, true>
+                                                   : voxel_bricks<true, false>
+                          : long_segs  ? voxel_bricks<false, true>
+                                       : voxel_bricks<false, false>;
             const int threads = multi_bundle ? kBrickThreads<true> : kBrickThreads<false>;
             kernel<<<grid, threads, 0, s>>>(segs, tiles, n_tiles, b0, b1, offsets, list,
                                             (unsigned)n_pairs, directory, share, room, split,

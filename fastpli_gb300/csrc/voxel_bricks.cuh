@@ -65,11 +65,12 @@ struct BrickChunks {
 // are the tile's output arrays (vecs[t] may be null: labels only).
 // seg_tile may be null when there is one tile.  `ws` holds
 // brick_workspace_bytes(n_bricks, n_pairs, n_segs) bytes, 256-byte aligned.
+// long_segs: some segment is a long_segment.
 // `chunks` may be null: one launch over every brick.
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
-                        const LayerDev *layers, bool multi_bundle, int32_t *const *labels,
-                        float *const *vecs, void *ws, unsigned long long *counters,
+                        const LayerDev *layers, bool multi_bundle, bool long_segs,
+                        int32_t *const *labels, float *const *vecs, void *ws, unsigned long long *counters,
                         cudaStream_t st, const BrickChunks *chunks = nullptr);
 
 } // namespace fpgb

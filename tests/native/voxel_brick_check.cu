@@ -115,10 +115,12 @@ int main(int argc, char **argv) {
          const SegDev &S = plan.segs[s];
          SegSweep w = host_sweep(S);
          SubBox b;
-         const bool any = sub_box(w, ox, oy, oz, nx, ny, nz, b);
-         rec.push_back(sweep_rec(w, b, any, ox, oy, oz));
-         th = std::max(th, fmaf(2.0001f, w.mg, S.thr_f));
-         mg = std::max(mg, w.mg);
+         if (!sub_box(w, ox, oy, oz, nx, ny, nz, b))
+            std::abort(); // the list has it for this brick
+         const SegPart g = seg_part<true>(S, w, b);
+         rec.push_back(sweep_rec<true>(g, S.thr_f, b, true, ox, oy, oz));
+         th = std::max(th, fmaf(2.0001f, g.mg, S.thr_f));
+         mg = std::max(mg, g.mg);
       }
       const BrickScale k = brick_scale((unsigned)list.size(), th, mg);
       std::vector<unsigned> keys(kBrickVoxels, kNoKey);

@@ -34,7 +34,8 @@ def checker(tmp_path_factory):
 def replay(checker, *args):
     r = subprocess.run([checker, *map(str, args)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
-    return dict(zip(r.stdout.split()[::2], r.stdout.split()[1::2]))
+    words = [w for w in r.stdout.split() if not w.startswith("(")]
+    return dict(zip(words[::2], words[1::2]))
 
 
 @pytest.mark.parametrize("length", LENGTHS)
@@ -45,6 +46,47 @@ def test_unmarked_voxels_are_certain(checker, length):
 @pytest.mark.parametrize("radius,points,taper", [(1e20, 3, 0), (4, 9, 0), (4, 9, 0.5)])
 def test_unmarked_voxels_are_certain_at_other_radii(checker, radius, points, taper):
     replay(checker, 5, 61, 43, 50, radius, 14, points, taper, 0)
+
+
+@pytest.mark.parametrize("args", [
+    (1, 256, 128, 64, 5, 100, 2, 0, 0), (1, 512, 128, 64, 5, 100, 2, 0, 0),
+    (1, 1024, 64, 64, 5, 50, 2, 0, 0), (1, 1024, 64, 64, 1.5, 500, 2, 0, 0),
+    (1, 96, 80, 64, 3, 60, 2, 0, 66), (1, 96, 80, 64, 3, 60, 2, 0, 1e5)])
+def test_few_close_calls_whatever_the_length(checker, args):
+    """A margin of at most 1.1e-6 (2 * 40)^2 = 0.007 either side of the layers
+    at r^2 and 0.56 r^2: 4 * 0.007 / r^2 of a fiber's voxels, and as many where
+    two fibers meet."""
+    bound = 0.015 if args[4] > 2 else 0.03
+    out = replay(checker, *args)
+    assert float(out["marked"]) <= bound * float(out["inside"]) and out["over"] == "0", out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bundles,fibers", [(1, 20), (1, 300), (2, 260)])
+def test_lists_of_two_point_fibers_match_oracle(cuda, oracle_port, bundles, fibers):
+    """More long segments in a brick than it sweeps at a time, and few."""
+    from fastpli_gb300.simulation import _Generator
+    rng = np.random.default_rng(fibers)
+    dim = (43, 37, 70)
+    sets = []
+    for _ in range(bundles):
+        m = rng.uniform(0, 1, (fibers, 3)) * dim
+        d = rng.normal(size=(fibers, 3))
+        d *= 300 / np.linalg.norm(d, axis=1, keepdims=True)
+        r = rng.uniform(1.0, 5.0, fibers)
+        sets.append([np.column_stack([np.stack([a - v, a + v]), [q, q]])
+                     for a, v, q in zip(m, d, r)])
+    layers = [LY3, LY1][:bundles]
+    olab, ovec, _, owarn = oracle_port.generate(dim, [0.0] * 3, 1.0, sets, layers)
+    g = _Generator()
+    g.set_volume(dim, [0.0] * 3, 1.0)
+    g.set_fiber_bundles(sets, layers)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        label, vector, _, w = g.run_generation_device()
+    assert np.array_equal(label.cpu().numpy(), olab)
+    assert np.array_equal(vector.cpu().numpy().view(np.uint32), ovec.view(np.uint32))
+    assert w["overlap"] == owarn["overlap"]
 
 
 @pytest.mark.gpu
