@@ -68,7 +68,7 @@ struct fpgb_batch_impl {
    size_t arena_bytes = 0;
    // workspace layout (bytes)
    size_t ws_bricks = 0, ws_segs = 0, ws_segtile = 0, ws_layers = 0, ws_tiles = 0, ws_prm = 0,
-          ws_items = 0, ws_tables = 0, ws_counters = 0, ws_bytes = 0;
+          ws_items = 0, ws_tables = 0, ws_counters = 0, ws_bytes = 0, ws_bricks_bytes = 0;
    std::vector<size_t> table_off; // per pair: lut then ztab, relative to ws_tables
    int64_t total_vox = 0, steps = 0;
    int64_t n_bricks = 0, brick_pairs = 0;
@@ -458,7 +458,9 @@ int plan_batch(int64_t n_tiles, const fpgb_volume *vols, const fpgb_fibers *fibe
 
    // workspace
    size_t w = 0;
-   B->ws_bricks = take(w, brick_workspace_bytes(B->n_bricks, B->brick_pairs, B->n_segs));
+   B->ws_bricks_bytes = brick_workspace_bytes(B->n_bricks, B->brick_pairs, B->n_segs) +
+                        brick_workspace_more(B->n_bricks);
+   B->ws_bricks = take(w, B->ws_bricks_bytes);
    B->ws_segs = take(w, sizeof(SegDev) * B->n_segs);
    B->ws_segtile = take(w, sizeof(int32_t) * B->seg_tile.size());
    B->ws_layers = take(w, sizeof(LayerDev) * B->layers.size());
@@ -596,8 +598,9 @@ int run_batch(fpgb_batch_impl *B, int march_ctas_per_sm, int chunk, int coop, cu
       FPGB_CUDA_TRY(cudaMemsetAsync(counters, 0,
                                     sizeof(unsigned long long) * (kCounterWords + 2), st));
       FPGB_TRY(launch_voxel_bricks(segs, seg_tile, B->n_segs, tiles, (int64_t)nt,
-                                   B->n_bricks, B->brick_pairs, layers, B->any_multi_bundle, B->any_long,
-                                   lptr, vptr, W + B->ws_bricks, counters, st));
+                                   B->n_bricks, B->brick_pairs, layers, B->any_multi_bundle,
+                                   B->any_long, lptr, vptr, W + B->ws_bricks, B->ws_bricks_bytes,
+                                   counters, st));
    } else {
       // the march's queue counters only: the voxelizer's warnings stay
       FPGB_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned long long) * 2, st));

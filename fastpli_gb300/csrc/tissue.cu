@@ -538,7 +538,7 @@ static int64_t plan_bricks(const TissuePlan &p, int32_t nb[3]) {
    return n;
 }
 
-size_t tissue_workspace_bytes(const TissuePlan &p) {
+size_t tissue_workspace_bytes(const TissuePlan &p, bool most) {
    int32_t nb[3];
    const int64_t n_bricks = plan_bricks(p, nb);
    size_t b = align_up(sizeof(TileDev) + 2 * sizeof(void *), 256);
@@ -546,7 +546,7 @@ size_t tissue_workspace_bytes(const TissuePlan &p) {
    b += align_up(sizeof(LayerDev) * p.layers.size(), 256);
    b += align_up(sizeof(unsigned long long) * kCounterWords, 256);
    b += brick_workspace_bytes(n_bricks, p.brick_pairs, p.n_segs);
-   return b;
+   return b + (most ? brick_workspace_more(n_bricks) : 0);
 }
 
 // Bricks of a slabbed launch, at least: 4 per SM (a wave of the 256-thread
@@ -675,7 +675,8 @@ int run_tissue(const TissuePlan &p, int only_label, int32_t *d_label,
       chunks = BrickChunks{n, bound, &Slabs::thunk, &slabs, alt};
    }
    FPGB_TRY(launch_voxel_bricks(segs, nullptr, p.n_segs, tile, 1, n_bricks,
-                                p.brick_pairs, layers, p.n_bundles > 1, p.long_segs, lp, vp, w, counters, st,
+                                p.brick_pairs, layers, p.n_bundles > 1, p.long_segs, lp, vp, w,
+                                ws_bytes - (size_t)(w - static_cast<char *>(d_ws)), counters, st,
                                 n > 1 ? &chunks : nullptr));
    if (n == 1 && after_slab)
       FPGB_TRY(after_slab(ctx, 0, p.X, st));
@@ -781,8 +782,8 @@ int fpgb_generate_tissue_device(const fpgb_volume *vol, const fpgb_fibers *fiber
       set_error("generate_tissue_device: null output buffer");
       return FPGB_EINVAL;
    }
-   const size_t need = tissue_workspace_bytes(p);
    if (!d_workspace) {
+      const size_t need = tissue_workspace_bytes(p, true);
       FPGB_TRY(pool_get(kSlotKeys, need, &d_workspace, as_stream(stream)));
       workspace_bytes = need;
    }
@@ -808,7 +809,7 @@ int fpgb_generate_tissue(const fpgb_volume *vol, const fpgb_fibers *fibers, int 
    FPGB_TRY(pool_get(kSlotLabel, sizeof(int32_t) * nvox, &d_label));
    if (!only_label)
       FPGB_TRY(pool_get(kSlotVector, sizeof(float) * 3 * nvox, &d_vec));
-   const size_t need = tissue_workspace_bytes(p);
+   const size_t need = tissue_workspace_bytes(p, true);
    FPGB_TRY(pool_get(kSlotKeys, need, &d_ws));
    cudaStream_t st = nullptr;
    unsigned long long *d_counters = nullptr;

@@ -130,7 +130,8 @@ bool long_segment(const double *p, const double *q);
 // fill = false leaves a large segment table to the device (run_tissue).
 int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
                 bool fill = true);
-size_t tissue_workspace_bytes(const TissuePlan &p);
+// Least scratch of run_tissue, or what it can use.
+size_t tissue_workspace_bytes(const TissuePlan &p, bool most = false);
 // Voxelizes the planned volume into d_label / d_vector on stream st.  With
 // n_slabs > 1 the bricks are voxelized in that many x-slabs, one launch each
 // (alternating between st and `alt` when alt is given), and

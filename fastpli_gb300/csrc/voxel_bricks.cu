@@ -75,24 +75,30 @@ int64_t segment_brick_pairs(const SegDev &S) {
           brick_range(S.lo[2], S.ext[2], kBrickZ, b0);
 }
 
-// The marked voxels' records, a share of the space per launch: entry 0 counts
-// {entries taken, records}; a record is {brick, number} and the brick's marked
-// voxels, four 16-bit places to an entry.  The launch's part of the bricks'
-// count array becomes the records' directory.  32 bytes per segment hold
-// several times the marks of the synthetic volumes; a brick whose record does
-// not fit is found again by the labels of its voxels.
-static int64_t mark_entries(int64_t n_segs) {
-   return std::max<int64_t>(0, 4 * n_segs - 32);
-}
+// The marked voxels' records, a share of the space per launch: entries 0 and 1
+// count {entries taken, records} and {full bricks}; a record is {brick, number}
+// and the brick's marked voxels, four 16-bit places to an entry.  The launch's
+// part of the bricks' count array becomes the directory: the records from its
+// start, from its end the bricks with more marked voxels than a record takes.
+// The space is what the workspace has left: the least has 32 bytes per segment,
+// several times the marks of fibers of short segments; with 128 bytes per brick
+// on top few long segments have room as well.
+constexpr int kMarkHead = 2;
 
-size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs, int64_t n_segs) {
+static size_t brick_list_bytes(int64_t n_bricks, int64_t n_pairs) {
    size_t w = 0;
    w += align_up(sizeof(unsigned) * (n_bricks + 1), 256); // offsets
    w += align_up(sizeof(unsigned) * std::max<int64_t>(n_bricks, 1), 256); // counts, then cursors
    w += align_up(sizeof(unsigned) * std::max<int64_t>(n_pairs, 1), 256);  // segment lists
-   w += align_up(sizeof(uint2) * mark_entries(n_segs), 256);              // marked voxels
    return w;
 }
+
+size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs, int64_t n_segs) {
+   return brick_list_bytes(n_bricks, n_pairs) +
+          align_up((size_t)std::max<int64_t>(0, 32 * n_segs - 256), 256);
+}
+
+size_t brick_workspace_more(int64_t n_bricks) { return (size_t(32) << 10) + 128 * n_bricks; }
 
 // ---------------------------------------------------------------- binning ---
 // Pair p of segment S in tile T (x slowest): its brick.
@@ -157,7 +163,7 @@ brick_bin_small(const SegDev *__restrict__ segs, const int32_t *__restrict__ seg
    __shared__ unsigned count[kSmallBricks], wsum[32];
    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
    if (mark_share > 0 && t < n_shares) // the marked voxels' lists start empty
-      marks[t * mark_share] = make_uint2(0u, 0u);
+      marks[t * mark_share] = marks[t * mark_share + 1] = make_uint2(0u, 0u);
    for (int b = t; b < n_bricks; b += 1024)
       count[b] = 0;
    __syncthreads();
@@ -235,7 +241,7 @@ brick_scan(const unsigned *__restrict__ counts, int64_t n, unsigned *__restrict_
            uint2 *__restrict__ marks, int64_t mark_share, int n_shares,
            unsigned long long *__restrict__ counters) {
    if (mark_share > 0 && (int)threadIdx.x < n_shares) // the marked voxels' lists start empty
-      marks[threadIdx.x * mark_share] = make_uint2(0u, 0u);
+      marks[threadIdx.x * mark_share] = marks[threadIdx.x * mark_share + 1] = make_uint2(0u, 0u);
    __shared__ unsigned long long wsum[32];
    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
    // the callers' workspaces are 256-byte aligned; checked anyway before any
@@ -770,11 +776,10 @@ __device__ __forceinline__ BrickPlace brick_place(const TileDev *__restrict__ ti
 }
 
 // --------------------------------------------------------- marked voxels ---
-// Marked voxels of one brick that get a record; with more of them the labels
-// are as good.
+// Marked voxels of one brick that get a record; a brick with more is full.
 constexpr unsigned kMarkList = 128;
 constexpr int kMarkThreads = 128, kMarkQueue = 192;
-constexpr unsigned kScanBrick = 0x80000000u; // directory entry without a record: a brick
+constexpr unsigned kNoRecord = 0x80000000u; // directory entry of a brick whose record had no room
 
 // What one warp of voxel_marks works on: up to 32 marked voxels of its brick,
 // and the candidates found for them.
@@ -947,13 +952,179 @@ __device__ __forceinline__ void resolve_marks(const MarkCtx &C, MarkWarp &W, int
    __syncwarp();
 }
 
-// Resolves the marked voxels of the bricks [brick_begin, brick_end), a brick
-// per warp (bound by latency: 16 warps per SM, each a chain of list, segment
-// and evaluation; a voxel per lane walking the list by itself took 260 us on
-// the crossing volume instead of 153, 6 CTAs per SM at 80 registers 166): from
-// its record, or from the labels of a brick without one (every brick when the
-// launch has no space for records).  Units: 2^split parts of a brick, `part`
-// marked voxels of one of them.
+// Full bricks: where fibers share their course, or a radius changes along a
+// segment (then the shell between a segment's own and its thickest radius is
+// undecided), a sixth to all of the voxels are marked.  A CTA takes half a
+// brick: its warps sweep the segments over the marked voxels (a byte of marks
+// per column lets the others pass) and queue the candidates whose lower bound is
+// not past the smallest certain upper one, for 32 lanes at a time.  Bound by
+// issue (46% of the slots at 14 warps per SM), most of it the exact
+// evaluations.  A warp per brick that walked the list row by row before: 256 x
+// 256 x 64, 58% of the voxels in two copies of a fiber 2,674 -> 444 us, two
+// bundles of them 2,646 -> 459, tapered fibers 515 -> 205.
+constexpr int kHalfX = kBrickX / 2, kFullRecs = 64;
+
+struct FullSeg {
+   float acc, mg2; // surely inside up to acc; hi - mg2 is a lower bound
+   unsigned bundle, seg;
+};
+
+struct FullScratch {
+   unsigned long long key[kHalfX * kPlane]; // winner's; until then {smallest certain hi, ~0}
+   unsigned minb[kHalfX * kPlane];          // smallest bundle the voxel is inside of
+   SweepRec rec[kFullRecs];
+   FullSeg seg[kFullRecs];
+   unsigned q_seg[kMarkThreads / 32][64];
+   unsigned short q_voxel[kMarkThreads / 32][64];
+   unsigned char mark[kPlane]; // a bit per x
+   unsigned next;
+};
+
+// z of a place in the plane's row y (plane_place)
+__device__ __forceinline__ int place_z(int place, int y) {
+   return (place - 9 * y) & (kBrickZ - 1);
+}
+
+// Evaluates n <= 32 queued candidates, a lane each.
+__device__ __forceinline__ void drain_full(const MarkCtx &C, FullScratch &F, int at, int n, int x0,
+                                           int lane, int warp, unsigned long long &n_slow) {
+   __syncwarp();
+   if (lane < n) {
+      const unsigned s = F.q_seg[warp][at + lane];
+      const int li = F.q_voxel[warp][at + lane], y = li >> 5 & 7;
+      const SegDev &S = C.segs[s];
+      float dist_squ, r_sqr;
+      if (cand_dist(S, C.p.ox + x0 + (li >> 8), C.p.oy + y, C.p.oz + place_z(li, y), dist_squ,
+                    r_sqr))
+         n_slow++;
+      if (!(dist_squ > C.layers[S.bundle].f_ly_squ * r_sqr)) { // generator.cpp:329-331
+         atomicMin(&F.key[li], ((unsigned long long)__float_as_uint(dist_squ) << 32) |
+                                   (unsigned long long)(0xFFFFFFFFu - s));
+         if (C.multi)
+            atomicMin(&F.minb[li], (unsigned)S.bundle);
+      }
+   }
+   __syncwarp();
+}
+
+// The marked voxels x0 <= x < x0 + nx <= x0 + kHalfX of a brick, by the CTA.
+__device__ __forceinline__ void resolve_full(const MarkCtx &C, FullScratch &F, int x0, int nx,
+                                             unsigned long long &n_slow,
+                                             unsigned long long &n_overlap,
+                                             unsigned long long &n_overflow) {
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   const int64_t plane = (int64_t)C.p.T->Y * C.p.T->Z;
+   const int64_t corner =
+       (C.p.ox + x0) * plane + (int64_t)C.p.oy * C.p.T->Z + C.p.oz; // of the half brick
+   bool any = false;
+   for (int yz = threadIdx.x; yz < kPlane; yz += kMarkThreads) {
+      const int y = yz >> 5, z = yz & 31, at = plane_place(y, z);
+      unsigned m = 0;
+      for (int x = 0; x < kHalfX; x++) {
+         if (x < nx && y < C.p.ny && z < C.p.nz &&
+             C.label[corner + x * plane + (int64_t)y * C.p.T->Z + z] == kMarkedLabel)
+            m |= 1u << x;
+         F.key[x * kPlane + at] = ~0ull;
+         F.minb[x * kPlane + at] = ~0u;
+      }
+      F.mark[at] = (unsigned char)m;
+      any = any || m;
+   }
+   if (!__syncthreads_or(any))
+      return;
+   int qn = 0;
+   for (unsigned base = 0; base < C.n_seg; base += kFullRecs) {
+      const unsigned n = min(C.n_seg - base, (unsigned)kFullRecs);
+      for (unsigned e = threadIdx.x; e < n; e += kMarkThreads) {
+         const unsigned s = C.list[base + e];
+         const SegSweep w = load_sweep(C.segs[s]);
+         SubBox b;
+         F.rec[e].box = 0u;
+         if (sub_box(w, C.p.ox + x0, C.p.oy, C.p.oz, nx, C.p.ny, C.p.nz, b)) {
+            const SegPart g = seg_part<true>(C.segs[s], w, b);
+            F.rec[e] = sweep_rec<true>(g, w.c.x, b, true, C.p.ox + x0, C.p.oy, C.p.oz);
+            F.seg[e] = FullSeg{w.c.y, 2.00001f * g.mg, (unsigned)w.e.w, s};
+         }
+      }
+      if (threadIdx.x == 0)
+         F.next = kMarkThreads / 32;
+      __syncthreads();
+      for (unsigned j = warp, next; j < n; j = __shfl_sync(0xFFFFFFFFu, next, 0)) {
+         if (lane == 0)
+            next = atomicAdd(&F.next, 1u);
+         const SweepRec g = F.rec[j];
+         const FullSeg f = F.seg[j];
+         const float ezf = (float)(g.box >> 9 & 63u);
+         const int ncell = (int)(g.box & 511u), ex = (int)(g.box >> 15 & 15u);
+         const int first = (int)(g.box >> 27);
+         for (int c0 = 0; c0 < ncell; c0 += 32) {
+            const Cell c = cell_of(g, ezf, (float)min(c0 + lane, ncell - 1));
+            const unsigned m =
+                c0 + lane < ncell ? F.mark[c.yz] >> first & ((1u << ex) - 1u) : 0u;
+            if (!__any_sync(0xFFFFFFFFu, m))
+               continue;
+            unsigned need = 0; // a bit per x
+#pragma unroll
+            for (int i = 0; i < kHalfX; i++) {
+               const float hi = sweep_dist2(g.wx0 + (float)i, c.a2, c.b, g.vn2x, g.c2f, g.rch);
+               if (!(m >> i & 1u) || hi > g.thr)
+                  continue;
+               // (keys only decrease: any value read bounds the last one; ~0 reads
+               // as NaN, past which nothing is)
+               const int li = (first + i) * kPlane + c.yz;
+               volatile const unsigned *cur = reinterpret_cast<unsigned *>(&F.key[li]) + 1;
+               const float best = __uint_as_float(*cur);
+               bool mine = !(hi - f.mg2 > best);
+               if (hi <= f.acc) {
+                  if (!(hi >= best))
+                     atomicMin(&F.key[li], ((unsigned long long)__float_as_uint(hi) << 32) |
+                                               0xFFFFFFFFull);
+                  if (C.multi)
+                     atomicMin(&F.minb[li], f.bundle);
+               } else if (C.multi) {
+                  mine = mine || f.bundle < *reinterpret_cast<volatile unsigned *>(&F.minb[li]);
+               }
+               need |= mine ? 1u << i : 0u;
+            }
+            if (!__any_sync(0xFFFFFFFFu, need))
+               continue;
+            for (int i = 0; i < ex; i++) {
+               const unsigned b = __ballot_sync(0xFFFFFFFFu, need >> i & 1u);
+               if (need >> i & 1u) {
+                  const int at = qn + __popc(b & ((1u << lane) - 1u));
+                  F.q_seg[warp][at] = f.seg;
+                  F.q_voxel[warp][at] = (unsigned short)((first + i) * kPlane + c.yz);
+               }
+               qn += __popc(b);
+               if (qn >= 32) {
+                  qn -= 32;
+                  drain_full(C, F, qn, 32, x0, lane, warp, n_slow);
+               }
+            }
+         }
+      }
+      __syncthreads(); // the records are rewritten
+   }
+   drain_full(C, F, 0, qn, x0, lane, warp, n_slow);
+   __syncthreads();
+   for (int yz = threadIdx.x; yz < C.p.ny * kBrickZ; yz += kMarkThreads) {
+      const int y = yz >> 5, z = yz & 31, at = plane_place(y, z);
+      const unsigned m = F.mark[at];
+      for (int x = 0; x < nx; x++)
+         if (m >> x & 1u)
+            finish_voxel(C, F.key[x * kPlane + at], C.p.ox + x0 + x, C.p.oy + y, C.p.oz + z,
+                         F.minb[x * kPlane + at], n_slow, n_overlap, n_overflow);
+   }
+   __syncthreads(); // the scratch is rewritten for the next
+}
+
+// Resolves the marked voxels of the bricks [brick_begin, brick_end): those of
+// a record by a warp (bound by latency: 16 warps per SM, each a chain of list,
+// segment and evaluation; a voxel per lane walking the list by itself took 260 us
+// on the crossing volume instead of 153, 6 CTAs per SM at 80 registers 166),
+// full bricks by halves, a CTA each, and so every brick when the launch has no
+// space for records.  Units: 2^split parts of a brick, `part` marked voxels of
+// one of them.
 __global__ void __launch_bounds__(kMarkThreads)
 voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, int64_t n_tiles,
             int64_t brick_begin, int64_t brick_end, const unsigned *__restrict__ offsets,
@@ -962,27 +1133,25 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
             int64_t mark_share, int split, int part, const LayerDev *__restrict__ layers,
             int32_t *const *__restrict__ labels, float *const *__restrict__ vecs,
             unsigned long long *__restrict__ counters) {
-   __shared__ MarkWarp s_warps[kMarkThreads / 32];
-   MarkWarp &W = s_warps[threadIdx.x >> 5];
+   __shared__ union Scratch {
+      MarkWarp warps[kMarkThreads / 32];
+      FullScratch full;
+      __device__ Scratch() {}
+   } scratch;
+   MarkWarp &W = scratch.warps[threadIdx.x >> 5];
    const int lane = threadIdx.x & 31;
    const int64_t warp = (blockIdx.x * (int64_t)kMarkThreads + threadIdx.x) >> 5;
    const int64_t n_warps = (int64_t)gridDim.x * (kMarkThreads / 32);
    unsigned long long n_slow = 0, n_overlap = 0, n_overflow = 0;
    const bool open = *reinterpret_cast<volatile unsigned long long *>(&counters[0]) == 0;
-   const int64_t n = mark_share > 0 ? (int64_t)marks[0].y : (brick_end - brick_begin) << split;
-   const int parts = (int)kMarkList / part;
-   for (int64_t u = warp; u < n * parts; u += n_warps) {
-      const int64_t r = u % n;
-      const int g = (int)(u / n) * part;
-      const unsigned at = mark_share > 0 ? directory[r] : kScanBrick;
-      int64_t place = r;
-      if (mark_share > 0)
-         place = (at & kScanBrick) ? at & ~kScanBrick : marks[at].x;
+   const int64_t n_places = (brick_end - brick_begin) << split;
+   const int64_t n = mark_share > 0 ? (int64_t)marks[0].y : 0;
+   // the list of a place's brick; false when it is empty
+   auto brick_of = [&](int64_t place, MarkCtx &C) -> bool {
       const int64_t brick = brick_begin + (place >> split);
       const unsigned j1 = min(offsets[brick + 1], n_pairs), j0 = min(offsets[brick], j1);
       if (j0 == j1)
-         continue;
-      MarkCtx C;
+         return false;
       C.p = brick_place(tiles, n_tiles, brick);
       C.n_seg = j1 - j0;
       C.list = list + j0;
@@ -991,35 +1160,49 @@ voxel_marks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles, 
       C.label = labels[C.p.tile];
       C.vec = vecs[C.p.tile];
       C.multi = open && C.p.T->n_bundles > 1;
-      if (!(at & kScanBrick)) {
-         const int total = min((int)marks[at].y, g + part);
-         const unsigned short *voxel = reinterpret_cast<const unsigned short *>(marks + at + 1);
-         for (int m = g; m < total; m += 32) {
-            if (m + lane < total)
-               W.voxel[lane] = voxel[m + lane];
-            __syncwarp();
-            resolve_marks(C, W, min(32, total - m), lane, n_slow, n_overlap, n_overflow);
-         }
+      return true;
+   };
+   const int parts = (int)kMarkList / part;
+   for (int64_t u = warp; u < n * parts; u += n_warps) {
+      const unsigned at = directory[u % n];
+      const int g = (int)(u / n) * part;
+      MarkCtx C;
+      if ((at & kNoRecord) || !brick_of(marks[at].x, C))
          continue;
-      }
-      if (g)
-         continue;
-      const int x0 = (int)(place & ((1 << split) - 1)) * (kBrickX >> split);
-      const int x1 = min(x0 + (kBrickX >> split), C.p.nx);
-      for (int row = x0 * C.p.ny; row < x1 * C.p.ny; row++) {
-         const int lx = row / C.p.ny, ly = row - lx * C.p.ny;
-         const int64_t i =
-             ((int64_t)(C.p.ox + lx) * C.p.T->Y + (C.p.oy + ly)) * C.p.T->Z + C.p.oz + lane;
-         const bool on = lane < C.p.nz && C.label[i] == kMarkedLabel;
-         const unsigned b = __ballot_sync(0xFFFFFFFFu, on);
-         if (!b)
-            continue;
-         if (on)
-            W.voxel[__popc(b & ((1u << lane) - 1u))] =
-                (unsigned short)(lx * kPlane + ly * kBrickZ + lane);
+      const int total = min((int)marks[at].y, g + part);
+      const unsigned short *voxel = reinterpret_cast<const unsigned short *>(marks + at + 1);
+      for (int m = g; m < total; m += 32) {
+         if (m + lane < total)
+            W.voxel[lane] = voxel[m + lane];
          __syncwarp();
-         resolve_marks(C, W, __popc(b), lane, n_slow, n_overlap, n_overflow);
+         resolve_marks(C, W, min(32, total - m), lane, n_slow, n_overlap, n_overflow);
       }
+   }
+   // full bricks, and where the records ran out of space those without one
+   const int64_t n_full = mark_share > 0 ? (int64_t)marks[1].x : n_places;
+   const int64_t n_more = mark_share > 0 && kMarkHead + (int64_t)marks[0].x > mark_share ? n : 0;
+   const int halves = split ? 1 : 2;
+   if (n_full + n_more > 0)
+      __syncthreads();
+   for (int64_t u = blockIdx.x; u < (n_full + n_more) * halves; u += gridDim.x) {
+      const int64_t r = u / halves;
+      int64_t place = r;
+      if (r >= n_full) {
+         const unsigned at = directory[r - n_full];
+         if (!(at & kNoRecord))
+            continue;
+         place = at & ~kNoRecord;
+      } else if (mark_share > 0) {
+         place = directory[n_places - 1 - r];
+      }
+      MarkCtx C;
+      if (!brick_of(place, C))
+         continue;
+      const int x0 = split ? (int)(place & ((1 << split) - 1)) * (kBrickX >> split)
+                           : (int)(u - r * halves) * kHalfX;
+      const int nx = min(C.p.nx - x0, split ? kBrickX >> split : kHalfX);
+      if (nx > 0)
+         resolve_full(C, scratch.full, x0, nx, n_slow, n_overlap, n_overflow);
    }
    if (n_overlap)
       atomicAdd(&counters[0], n_overlap);
@@ -1328,15 +1511,22 @@ voxel_bricks(const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
       __syncthreads();
       if (warp == 0 && s_marked && mark_share > 0) { // the brick's record
          const unsigned n = s_marked;
+         const bool full = n > kMarkList;
          unsigned long long got = 0; // {entries taken, records}
-         if (lane == 0) // (a record that does not fit takes no entries)
-            got = atomicAdd(reinterpret_cast<unsigned long long *>(marks),
-                            (1ull << 32) | (n <= kMarkList ? 1u + (n + 3u) / 4u : 0u));
-         got = __shfl_sync(0xFFFFFFFFu, got, 0);
-         const uint64_t at = 1u + (unsigned)got;
-         const bool fits = n <= kMarkList && at + 1 + (n + 3) / 4 <= (uint64_t)mark_share;
          if (lane == 0) {
-            directory[got >> 32] = fits ? (unsigned)at : kScanBrick | (unsigned)place;
+            if (full) {
+               const int64_t last = ((brick_end - brick_begin) << split) - 1;
+               directory[last - atomicAdd(&marks[1].x, 1u)] = (unsigned)place;
+            } else {
+               got = atomicAdd(reinterpret_cast<unsigned long long *>(marks),
+                               (1ull << 32) | (1u + (n + 3u) / 4u));
+            }
+         }
+         got = __shfl_sync(0xFFFFFFFFu, got, 0);
+         const uint64_t at = (uint64_t)kMarkHead + (unsigned)got;
+         const bool fits = !full && at + 1 + (n + 3) / 4 <= (uint64_t)mark_share;
+         if (lane == 0 && !full) {
+            directory[got >> 32] = fits ? (unsigned)at : kNoRecord | (unsigned)place;
             if (fits)
                marks[at] = make_uint2((unsigned)place, n);
          }
@@ -1366,7 +1556,8 @@ constexpr int64_t kSplitBricks = 304, kSplitMarks = 1216;
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
                         const LayerDev *layers, bool multi_bundle, bool long_segs,
-                        int32_t *const *labels, float *const *vecs, void *ws, unsigned long long *counters,
+                        int32_t *const *labels, float *const *vecs, void *ws, size_t ws_bytes,
+                        unsigned long long *counters,
                         cudaStream_t st, const BrickChunks *chunks) {
    if (n_tiles <= 0 || n_bricks <= 0)
       return FPGB_OK;
@@ -1379,17 +1570,26 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
                 (long long)n_pairs);
       return FPGB_EINVAL;
    }
+   const size_t lists = brick_list_bytes(n_bricks, n_pairs);
+   if (ws_bytes < lists) {
+      set_error("voxelizer: %zu bytes of scratch, %zu needed", ws_bytes, lists);
+      return FPGB_ENOMEM;
+   }
    char *w = static_cast<char *>(ws);
    auto *offsets = reinterpret_cast<unsigned *>(w);
    w += align_up(sizeof(unsigned) * (n_bricks + 1), 256);
    auto *counts = reinterpret_cast<unsigned *>(w);
    w += align_up(sizeof(unsigned) * std::max<int64_t>(n_bricks, 1), 256);
    auto *list = reinterpret_cast<unsigned *>(w);
-   w += align_up(sizeof(unsigned) * std::max<int64_t>(n_pairs, 1), 256);
-   auto *marks = reinterpret_cast<uint2 *>(w);
+   auto *marks = reinterpret_cast<uint2 *>(static_cast<char *>(ws) + lists);
    const int n_launch = chunks ? chunks->n : 1;
-   // entries of one launch (entry 0 counts)
-   const int64_t mark_share = n_launch <= 1024 ? mark_entries(n_segs) / n_launch : 0;
+   // entries of one launch (kNoRecord is past every place among them)
+   int64_t mark_share =
+       n_launch <= 1024
+           ? std::min<int64_t>((int64_t)((ws_bytes - lists) / sizeof(uint2)), 1 << 30) / n_launch
+           : 0;
+   if (mark_share < kMarkHead)
+      mark_share = 0;
 
    if (n_bricks <= kSmallBricks && n_pairs <= kSmallPairs && n_segs <= kSmallPairs) {
       brick_bin_small<<<1, 1024, 0, st>>>(segs, seg_tile, (int)n_segs, tiles, (int)n_bricks,
@@ -1415,8 +1615,8 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
          FPGB_CUDA_TRY(cudaGetLastError());
       }
    }
-   // (up to eight times as many records: their directory at the end of their
-   // space)
+   // (up to eight times as many places: their directory at the end of the
+   // records' space)
    int split = 0;
    int64_t dir_entries = 0;
    while (n_launch == 1 && split < 3 && n_bricks << (split + 1) <= kSplitBricks &&
@@ -1439,11 +1639,11 @@ int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_s
          if (b1 > b0) {
             const int64_t n = (b1 - b0) << split;
             const unsigned grid = (unsigned)std::min<int64_t>(n, 0x7FFFFFFF);
-            // a warp per record, or per part of it, up to about two waves
+            // a warp per record, or per part of it, a CTA per full brick, up to
+            // about two waves
             const int part = n <= kSplitMarks ? 8 : (int)kMarkList;
             const unsigned mark_grid = (unsigned)std::min<int64_t>(
-                (n * ((int)kMarkList / part) + kMarkThreads / 32 - 1) / (kMarkThreads / 32),
-                152 * 8);
+                n * std::max(1, (int)kMarkList / part / (kMarkThreads / 32)), 152 * 8);
             uint2 *share = marks + c * mark_share;
             const int64_t room = mark_share - dir_entries;
             unsigned *directory =

@@ -41,9 +41,10 @@ void tile_bricks(int64_t X, int64_t Y, int64_t Z, int32_t nb[3], int64_t *n_bric
 // Number of (segment, brick) pairs of one segment (its clipped box).
 int64_t segment_brick_pairs(const SegDev &S);
 
-// Device scratch of the voxelizer for n_bricks bricks, n_pairs pairs and
-// n_segs segments.
+// Least device scratch of the voxelizer for n_bricks bricks, n_pairs pairs and
+// n_segs segments, and what more it can use (records of marked voxels).
 size_t brick_workspace_bytes(int64_t n_bricks, int64_t n_pairs, int64_t n_segs);
+size_t brick_workspace_more(int64_t n_bricks);
 
 // Brick ranges to voxelize as separate launches, in order: launch c covers
 // bricks [bound[c], bound[c + 1]), and after(ctx, c, s) runs on the host once
@@ -64,13 +65,14 @@ struct BrickChunks {
 // Bins the segments to bricks and voxelizes every tile.  labels[t] / vecs[t]
 // are the tile's output arrays (vecs[t] may be null: labels only).
 // seg_tile may be null when there is one tile.  `ws` holds
-// brick_workspace_bytes(n_bricks, n_pairs, n_segs) bytes, 256-byte aligned.
+// ws_bytes >= brick_workspace_bytes(n_bricks, n_pairs, n_segs), 256-byte aligned.
 // long_segs: some segment is a long_segment.
 // `chunks` may be null: one launch over every brick.
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
                         const LayerDev *layers, bool multi_bundle, bool long_segs,
-                        int32_t *const *labels, float *const *vecs, void *ws, unsigned long long *counters,
+                        int32_t *const *labels, float *const *vecs, void *ws, size_t ws_bytes,
+                        unsigned long long *counters,
                         cudaStream_t st, const BrickChunks *chunks = nullptr);
 
 } // namespace fpgb
