@@ -26,6 +26,8 @@
 // share the measurements, the tilts and the Jacobian's columns of a pixel: the
 // chain is a quarter as long, and the sums of the three columns, each in the
 // order MINPACK (sequential) or numpy (pairwise) takes it, run side by side.
+// Small maps, which wait for the longest chain, take 16 lanes, large ones 1
+// (one_lane_pixels).
 // Compiled with -fmad=false: products and sums round separately, as in the
 // reference, except where a fused multiply-add is written out.
 #include <cuda_runtime.h>
@@ -368,7 +370,7 @@ __device__ __forceinline__ double cube_rn(double x) {
 // scipy.optimize.leastsq runs it for the reference (_ROFL_with_jacobi.py:
 // 472-486): ftol = xtol = 1.49012e-8, gtol = 0, maxfev = 150, factor 100,
 // automatic scaling, epsfcn = machine epsilon.  The m x 3 Jacobian and the
-// residual vectors are the thread's own; the loops over the measurements
+// residual vectors are the pixel's lanes'; the loops over the measurements
 // run in MINPACK's order, so the iterates differ from the reference's only
 // where CUDA's FP64 trigonometry rounds differently from the reference's
 // numpy (a last-bit difference in some evaluations, which MINPACK's
@@ -835,10 +837,14 @@ __device__ int mp_fit(const RoflParams &P, PixelArrays<MAXM> &A, int M, double x
 // memory, 33 KB per warp with G = 4 and 10 rotations, 26 KB with 16 and 32; with
 // a lane per pixel in its local memory, interleaved across the warp and cached
 // in L1 (held to 80 registers: 24 warps per SM).
+// With a mask the pixels are those of rofl_select's list, whose length n the
+// kernel finds in status[2]; it is one of those launched for several ranges of
+// n, and the others return at once.
 template <int MAXR, int G>
 __global__ void __launch_bounds__(32, G == 1 ? 24 : 0)
-rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__restrict__ mask,
-         const RoflParams P, double *__restrict__ out, unsigned long long *__restrict__ status) {
+rofl_fit(const double *__restrict__ data, int64_t n_pix, const int64_t *__restrict__ list,
+         int64_t n_least, int64_t n_end, const RoflParams P, double *__restrict__ out,
+         unsigned long long *__restrict__ status) {
    constexpr int MAXM = 5 * MAXR, kPixels = 32 / G;
    extern __shared__ __align__(16) unsigned char s_arrays[];
    PixelArrays<G == 1 ? MAXM : 1> own; // (local memory)
@@ -847,18 +853,19 @@ rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__
        G == 1 ? reinterpret_cast<PixelArrays<MAXM> &>(own)
               : reinterpret_cast<PixelArrays<MAXM> *>(s_arrays)[lane / G];
    const Lanes<G> L;
+   const int64_t n = list ? (int64_t)status[2] : n_pix;
+   if (n < n_least || n >= n_end)
+      return;
    for (;;) {
       unsigned long long first = 0;
       if (lane == 0)
          first = atomicAdd(&status[1], (unsigned long long)kPixels);
       first = __shfl_sync(0xFFFFFFFFu, first, 0);
-      if (first >= (unsigned long long)n_pix)
+      if (first >= (unsigned long long)n)
          break;
-      const int64_t p = (int64_t)first + lane / G;
-      if (p < n_pix && mask && !mask[p]) {
-         for (int e = L.g; e < 8; e += G)
-            out[8 * p + e] = nan("");
-      } else if (p < n_pix) {
+      const int64_t q = (int64_t)first + lane / G;
+      if (q < n) {
+         const int64_t p = list ? list[q] : q;
          // tilt t, rotation k of pixel p: data[(t * n_pix + p) * R + k]
          for (int t = L.g; t < 5; t += G) {
             const double *d = data + (t * n_pix + p) * R;
@@ -959,24 +966,64 @@ rofl_fit(const double *__restrict__ data, int64_t n_pix, const unsigned char *__
    }
 }
 
+// The unmasked pixels, in any order, and their number; NaN for the others.
+__global__ void __launch_bounds__(256)
+rofl_select(const unsigned char *__restrict__ mask, int64_t n_pix, int64_t *__restrict__ list,
+            double *__restrict__ out, unsigned long long *__restrict__ status) {
+   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+   const bool on = p < n_pix && mask[p];
+   const unsigned m = __ballot_sync(0xFFFFFFFFu, on);
+   const int lane = threadIdx.x & 31;
+   unsigned long long at = 0;
+   if (lane == 0 && m)
+      at = atomicAdd(&status[2], (unsigned long long)__popc(m));
+   at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(m & ((1u << lane) - 1u));
+   if (on)
+      list[at] = p;
+   else if (p < n_pix)
+      for (int e = 0; e < 8; e++)
+         out[8 * p + e] = nan("");
+}
+
 // Lanes per pixel.  Up to kRoflFewPixels 16: four warps per SM of two pixels
 // each, which an SM's FP64 unit runs nearly as fast as one, so only the length
-// of a pixel's chain counts.  From kRoflManyPixels on 1: the map keeps every SM
+// of a pixel's chain counts.  From one_lane_pixels on 1: the map keeps every SM
 // busy for many times the longest chain, so only the number of instructions
-// counts.  Between them 4 (GB300, forward differences, 9 rotations):
+// counts.  Between them 4, up to 10 rotations (GB300, forward differences, 9
+// rotations):
 //   30 x 20     16: 1.70 ms   4:   2.72 ms   1:  6.3 ms
 //   77 x 77     16: 4.94      4:   4.68      1:  9.8
 //   160 x 150   16: 18.2      4:  13.8       1: 18.0
 //   320 x 320                 4:  44.0       1: 35.7
 //   512 x 512                 4: 109         1: 84.0
+// With more rotations four lanes per pixel leave an SM two warps (105 KB of
+// arrays each) and lose to 16 from 6,000 pixels on; and one lane wins sooner,
+// the instructions that 16 lanes repeat being in proportion to the pixels, the
+// longest chain to the rotations (ms, two maps of faster and slower fits; the
+// thread per pixel before all of these 16.1 / 20.4, 23.6 / 26.0, 56.5 / 61.1 for
+// 18 rotations and 6,000 / 12,100, 24,000, 79,000 pixels):
+//   11 rotations   12,000: 16  9.7 / 10.9   1  7.3 / 14.1   24,000: 18.9 / 21.0    9.0 / 16.3
+//   18             12,000:    10.8 / 11.8     11.5 / 15.4   24,000: 20.8 / 22.8   14.7 / 19.8
+//   18             79,000:    67.4 / 72.8     33.7 / 43.8
+//   32             24,000:    26.3 / 28.7     28.9 / 32.1   36,000: 38.8 / 41.8   33.8 / 38.2
+// In grad_mode the chain is ten times as long: 16 and 1 lanes level at 79,000
+// pixels of 11 rotations (219 and 222 ms), 16 ahead of 1 with more.
+// Masked pixels do not count: a warp of one-lane pixels idles on those it meets
+// (90% of 24,000 pixels masked, 18 rotations: 12.4 ms so, 4.2 with 16 lanes).
 constexpr int64_t kRoflFewPixels = 1216, kRoflManyPixels = 80000;
 
+static int64_t one_lane_pixels(const RoflParams &P) {
+   return P.n_rot <= kRoflSmallRot || P.grad_mode ? kRoflManyPixels : 1000 * P.n_rot;
+}
+
 // As many warps as are resident (the pixels are taken from the counter), fewer
-// for small maps.
+// for small maps; for n_least <= pixels < n_end.
 template <int MAXR, int G>
-static int launch_rofl(const double *d_data, int64_t n_pix, const unsigned char *d_mask,
-                       const RoflParams &P, double *d_out, unsigned long long *status,
-                       cudaStream_t st) {
+static int launch_rofl(const double *d_data, int64_t n_pix, const int64_t *d_list, int64_t n_least,
+                       int64_t n_end, const RoflParams &P, double *d_out,
+                       unsigned long long *status, cudaStream_t st) {
+   if (n_least >= n_end || n_pix < n_least || (!d_list && n_pix >= n_end))
+      return FPGB_OK;
    constexpr int kPixels = 32 / G;
    constexpr int kBytes = G == 1 ? 0 : kPixels * (int)sizeof(PixelArrays<5 * MAXR>);
    int dev = 0, sms = 0, per_sm = 0;
@@ -986,10 +1033,11 @@ static int launch_rofl(const double *d_data, int64_t n_pix, const unsigned char 
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
    FPGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rofl_fit<MAXR, G>, 32,
                                                                kBytes));
+   const int64_t most = std::min(n_pix, n_end - 1);
    const int64_t blocks = std::max<int64_t>(
-       1, std::min<int64_t>((n_pix + kPixels - 1) / kPixels, (int64_t)sms * std::max(per_sm, 1)));
-   rofl_fit<MAXR, G><<<(unsigned)blocks, 32, kBytes, st>>>(d_data, n_pix, d_mask, P, d_out,
-                                                           status);
+       1, std::min<int64_t>((most + kPixels - 1) / kPixels, (int64_t)sms * std::max(per_sm, 1)));
+   rofl_fit<MAXR, G><<<(unsigned)blocks, 32, kBytes, st>>>(d_data, n_pix, d_list, n_least, n_end,
+                                                           P, d_out, status);
    FPGB_CUDA_TRY(cudaGetLastError());
    return FPGB_OK;
 }
@@ -1050,16 +1098,33 @@ int fpgb_rofl_device(const double *d_data, int64_t n_pix, int64_t n_rot, double 
    void *w = nullptr;
    FPGB_TRY(pool_get(kSlotCounters, sizeof(unsigned long long) * kCounterWords, &w, st));
    auto *status = static_cast<unsigned long long *>(w);
-   // status[0]: pixels at the evaluation limit, status[1]: next pixel
-   FPGB_CUDA_TRY(cudaMemsetAsync(status, 0, 2 * sizeof(unsigned long long), st));
+   // status[0]: pixels at the evaluation limit, [1]: next pixel, [2]: unmasked ones
+   FPGB_CUDA_TRY(cudaMemsetAsync(status, 0, 3 * sizeof(unsigned long long), st));
    if (n_pix > 0) {
-      const bool small = P.n_rot <= kRoflSmallRot;
-      auto launch = n_pix >= kRoflManyPixels
-                        ? (small ? launch_rofl<kRoflSmallRot, 1> : launch_rofl<kRoflMaxRot, 1>)
-                    : small && n_pix > kRoflFewPixels ? launch_rofl<kRoflSmallRot, 4>
-                    : small                           ? launch_rofl<kRoflSmallRot, 16>
-                                                      : launch_rofl<kRoflMaxRot, 16>;
-      FPGB_TRY(launch(d_data, n_pix, d_mask, P, d_out, status, st));
+      int64_t *list = nullptr;
+      if (d_mask) {
+         void *l = nullptr;
+         FPGB_TRY(pool_get(kSlotStaging, sizeof(int64_t) * (size_t)n_pix, &l, st));
+         list = static_cast<int64_t *>(l);
+         rofl_select<<<(unsigned)((n_pix + 255) / 256), 256, 0, st>>>(d_mask, n_pix, list, d_out,
+                                                                     status);
+         FPGB_CUDA_TRY(cudaGetLastError());
+      }
+      const int64_t one = one_lane_pixels(P), none = INT64_MAX;
+      if (P.n_rot <= kRoflSmallRot) {
+         const int64_t few = kRoflFewPixels + 1;
+         FPGB_TRY((launch_rofl<kRoflSmallRot, 16>(d_data, n_pix, list, 0, few, P, d_out, status,
+                                                  st)));
+         FPGB_TRY((launch_rofl<kRoflSmallRot, 4>(d_data, n_pix, list, few, one, P, d_out, status,
+                                                 st)));
+         FPGB_TRY((launch_rofl<kRoflSmallRot, 1>(d_data, n_pix, list, one, none, P, d_out, status,
+                                                 st)));
+      } else {
+         FPGB_TRY((launch_rofl<kRoflMaxRot, 16>(d_data, n_pix, list, 0, one, P, d_out, status,
+                                                st)));
+         FPGB_TRY((launch_rofl<kRoflMaxRot, 1>(d_data, n_pix, list, one, none, P, d_out, status,
+                                               st)));
+      }
    }
    if (n_unconverged) {
       unsigned long long h = 0;
