@@ -78,13 +78,14 @@ __device__ __forceinline__ int64_t block_begin(int64_t u, int64_t n, double scal
 }
 
 // One axis of the map: output u sums input rows first[u] .. + count[u] with
-// weights w[u * pitch ...]; block[u] input pixels go to it.
+// weights w[(u - u0) * pitch ...], kept for the outputs u0 .. + nu at a time;
+// block[u] input pixels go to it.
 struct AxisMap {
    int64_t n, size; // input and output length
-   int pitch;
+   int64_t u0, nu;
+   int64_t pitch;
    double *w;
-   int64_t *first;
-   int *count, *block;
+   int64_t *first, *count, *block;
 };
 
 // The weights of both axes, a CTA per output pixel: the weight of row i is the
@@ -92,35 +93,37 @@ struct AxisMap {
 // every mirror image of it (mode 'reflect': d c b a | a b c d | d c b a,
 // repeated for lines shorter than the kernel).
 __global__ void axis_weights(AxisMap ax, AxisMap ay, double scale, const GaussTaps g) {
-   const bool second = (int64_t)blockIdx.x >= ax.size;
-   const AxisMap A = second ? ay : ax;
-   const int64_t u = (int64_t)blockIdx.x - (second ? ax.size : 0);
-   const int64_t b0 = block_begin(u, A.n, scale), b1 = block_begin(u + 1, A.n, scale);
-   const int64_t r = g.radius;
-   const int64_t lo = b0 - r > 0 ? b0 - r : 0, hi = b1 + r < A.n ? b1 + r : A.n;
-   const int count = b1 > b0 ? (int)(hi - lo) : 0;
-   if (threadIdx.x == 0) {
-      A.first[u] = lo;
-      A.count[u] = count;
-      A.block[u] = (int)(b1 - b0);
-   }
-   const int64_t period = 2 * A.n;
-   for (int t = threadIdx.x; t < count; t += blockDim.x) {
-      double sum = 0.0;
-      for (int side = 0; side < 2; side++) {
-         int64_t p = side ? -1 - (lo + t) : lo + t; // images: p + period * m
-         p += (b0 - r - p) / period * period;       // near the window's lower end
-         while (p < b0 - r)
-            p += period;
-         while (p - period >= b0 - r)
-            p -= period;
-         for (; p < b1 + r; p += period) {
-            const int64_t i0 = p - r > b0 ? p - r : b0, i1 = p + r + 1 < b1 ? p + r + 1 : b1;
-            for (int64_t i = i0; i < i1; i++)
-               sum = sum + g.w[i > p ? i - p : p - i];
-         }
+   for (int64_t q = blockIdx.x; q < ax.nu + ay.nu; q += gridDim.x) {
+      const bool second = q >= ax.nu;
+      const AxisMap A = second ? ay : ax;
+      const int64_t local = q - (second ? ax.nu : 0), u = A.u0 + local;
+      const int64_t b0 = block_begin(u, A.n, scale), b1 = block_begin(u + 1, A.n, scale);
+      const int64_t r = g.radius;
+      const int64_t lo = b0 - r > 0 ? b0 - r : 0, hi = b1 + r < A.n ? b1 + r : A.n;
+      const int64_t count = b1 > b0 ? hi - lo : 0;
+      if (threadIdx.x == 0) {
+         A.first[u] = lo;
+         A.count[u] = count;
+         A.block[u] = b1 - b0;
       }
-      A.w[u * A.pitch + t] = sum;
+      const int64_t period = 2 * A.n;
+      for (int64_t t = threadIdx.x; t < count; t += blockDim.x) {
+         double sum = 0.0;
+         for (int side = 0; side < 2; side++) {
+            int64_t p = side ? -1 - (lo + t) : lo + t; // images: p + period * m
+            p += (b0 - r - p) / period * period;       // near the window's lower end
+            while (p < b0 - r)
+               p += period;
+            while (p - period >= b0 - r)
+               p -= period;
+            for (; p < b1 + r; p += period) {
+               const int64_t i0 = p - r > b0 ? p - r : b0, i1 = p + r + 1 < b1 ? p + r + 1 : b1;
+               for (int64_t i = i0; i < i1; i++)
+                  sum = sum + g.w[i > p ? i - p : p - i];
+            }
+         }
+         A.w[local * A.pitch + t] = sum;
+      }
    }
 }
 
@@ -131,6 +134,8 @@ __global__ void axis_weights(AxisMap ax, AxisMap ay, double scale, const GaussTa
 // 52 us, with the weights 9 and axis 1 15 us; filtering every pixel along both
 // axes (142 M products, reflected index per tap) and then summing the blocks
 // took 273 + 273 + 18 us.
+// Images of fewer than 128 columns share a CTA among groups of outputs
+// (100,000 x 1 x 9 with 481 taps: 0.53 ms, 2.61 with the other lanes idle).
 constexpr int kRows = 4;
 
 __global__ void __launch_bounds__(128)
@@ -138,30 +143,43 @@ map_axis0(const double *__restrict__ in, double *__restrict__ out, int64_t C, co
    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
    if (c >= C)
       return;
-   for (int64_t u0 = blockIdx.y * (int64_t)kRows; u0 < A.size; u0 += gridDim.y * (int64_t)kRows) {
+   const int64_t end = A.u0 + A.nu;
+   for (int64_t u0 = A.u0 + (blockIdx.y * (int64_t)blockDim.y + threadIdx.y) * kRows; u0 < end;
+        u0 += gridDim.y * (int64_t)blockDim.y * kRows) {
       double acc[kRows] = {};
-      int lo = INT32_MAX, hi = 0, first[kRows], count[kRows];
+      int64_t lo = INT64_MAX, hi = 0, first[kRows], count[kRows];
 #pragma unroll
       for (int k = 0; k < kRows; k++) {
-         const int64_t u = u0 + k < A.size ? u0 + k : A.size - 1;
-         first[k] = (int)A.first[u]; // (rows: at most 2^31)
-         count[k] = u0 + k < A.size ? A.count[u] : 0;
+         const int64_t u = u0 + k < end ? u0 + k : end - 1;
+         first[k] = A.first[u];
+         count[k] = u0 + k < end ? A.count[u] : 0;
          if (count[k]) {
             lo = first[k] < lo ? first[k] : lo;
             hi = first[k] + count[k] > hi ? first[k] + count[k] : hi;
          }
       }
-      const double *w = A.w + u0 * A.pitch;
-      for (int i = lo; i < hi; i++) {
-         const double v = in[i * C + c];
+      // (in 32 bits from a base: 64-bit indices cost 10% at 100 taps)
+      for (int64_t base = lo; base < hi; base += 1 << 30) {
+         const int rows = (int)(hi - base < 1 << 30 ? hi - base : 1 << 30);
+         int from[kRows], to[kRows];
 #pragma unroll
-         for (int k = 0; k < kRows; k++) // (the same for every thread of the warp)
-            if (i >= first[k] && i < first[k] + count[k])
-               acc[k] = fma(w[k * A.pitch + (i - first[k])], v, acc[k]);
+         for (int k = 0; k < kRows; k++) {
+            const int64_t a = first[k] - base, b = a + count[k];
+            from[k] = (int)(a < 0 ? 0 : a < rows ? a : rows);
+            to[k] = (int)(b < 0 ? 0 : b < rows ? b : rows);
+         }
+         const double *w = A.w + (u0 - A.u0) * A.pitch + base, *v = in + base * C + c;
+         for (int i = 0; i < rows; i++) {
+            const double x = v[i * C];
+#pragma unroll
+            for (int k = 0; k < kRows; k++) // (the same for every thread of a group)
+               if (i >= from[k] && i < to[k])
+                  acc[k] = fma(w[k * A.pitch - first[k] + i], x, acc[k]);
+         }
       }
 #pragma unroll
       for (int k = 0; k < kRows; k++)
-         if (u0 + k < A.size)
+         if (u0 + k < end)
             out[(u0 + k) * C + c] = acc[k];
    }
 }
@@ -170,16 +188,17 @@ map_axis0(const double *__restrict__ in, double *__restrict__ out, int64_t C, co
 // (an empty block: 0 / 0 = NaN, as numpy's divide).
 __global__ void __launch_bounds__(128)
 map_axis1(const double *__restrict__ in, double *__restrict__ out, int64_t U, int64_t R,
-          const AxisMap A, const int *__restrict__ block0) {
-   const int64_t total = U * A.size * R;
+          const AxisMap A, const int64_t *__restrict__ block0) {
+   const int64_t total = U * A.nu * R;
    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
         e += (int64_t)gridDim.x * blockDim.x) {
       const int64_t r = e % R, uv = e / R;
-      const int64_t u = uv / A.size, v = uv - u * A.size;
+      const int64_t u = uv / A.nu, local = uv - u * A.nu, v = A.u0 + local;
       const double *row = in + (u * A.n + A.first[v]) * R + r;
-      const double *w = A.w + v * A.pitch;
-      const int n = A.count[v];
+      const double *w = A.w + local * A.pitch;
       double even = 0.0, odd = 0.0;
+      const int64_t all = A.count[v];
+      const int n = (int)(all < 1 << 30 ? all : 1 << 30); // (32-bit steps; the rest below)
       int t = 0;
       for (; t + 1 < n; t += 2) {
          even = fma(w[t], row[t * R], even);
@@ -187,7 +206,10 @@ map_axis1(const double *__restrict__ in, double *__restrict__ out, int64_t U, in
       }
       if (t < n)
          even = fma(w[t], row[t * R], even);
-      out[e] = (even + odd) / (double)((int64_t)block0[u] * A.block[v]);
+#pragma unroll 1
+      for (int64_t i = n; i < all; i++)
+         even = fma(w[i], row[i * R], even);
+      out[(u * A.size + v) * R + r] = (even + odd) / (double)(block0[u] * A.block[v]);
    }
 }
 
@@ -372,6 +394,9 @@ static unsigned grid_for(int64_t n, int threads) {
    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, 152 * 64));
 }
 
+// Weights of one axis held at a time.
+constexpr int64_t kWeightBytes = int64_t(256) << 20;
+
 } // namespace fpgb
 
 using namespace fpgb;
@@ -418,9 +443,11 @@ int fpgb_optic_filter_resample_device(const double *d_image, int64_t X, int64_t 
    ay.size = SY;
    size_t bytes = align_up(sizeof(double) * (SX * Y * n_rho), 256);
    for (AxisMap *A : {&ax, &ay}) {
-      A->pitch = (int)std::min<double>((double)A->n, widest);
-      bytes += align_up(sizeof(double) * A->size * A->pitch, 256) +
-               align_up(sizeof(int64_t) * A->size, 256) + 2 * align_up(sizeof(int) * A->size, 256);
+      A->pitch = (int64_t)std::min<double>((double)A->n, widest);
+      A->nu = std::max<int64_t>(
+          1, std::min<int64_t>(A->size, kWeightBytes / ((int64_t)sizeof(double) * A->pitch)));
+      bytes += align_up(sizeof(double) * A->nu * A->pitch, 256) +
+               3 * align_up(sizeof(int64_t) * A->size, 256);
    }
    void *ws = nullptr;
    FPGB_TRY(pool_get(kSlotOptic, bytes, &ws, st));
@@ -432,20 +459,46 @@ int fpgb_optic_filter_resample_device(const double *d_image, int64_t X, int64_t 
    };
    double *tmp = reinterpret_cast<double *>(take(sizeof(double) * (SX * Y * n_rho)));
    for (AxisMap *A : {&ax, &ay}) {
-      A->w = reinterpret_cast<double *>(take(sizeof(double) * A->size * A->pitch));
+      A->w = reinterpret_cast<double *>(take(sizeof(double) * A->nu * A->pitch));
       A->first = reinterpret_cast<int64_t *>(take(sizeof(int64_t) * A->size));
-      A->count = reinterpret_cast<int *>(take(sizeof(int) * A->size));
-      A->block = reinterpret_cast<int *>(take(sizeof(int) * A->size));
+      A->count = reinterpret_cast<int64_t *>(take(sizeof(int64_t) * A->size));
+      A->block = reinterpret_cast<int64_t *>(take(sizeof(int64_t) * A->size));
    }
-   axis_weights<<<(unsigned)(SX + SY), 64, 0, st>>>(ax, ay, scale, g);
-   FPGB_CUDA_TRY(cudaGetLastError());
+   auto weights = [&](const AxisMap &a, const AxisMap &b) -> int {
+      axis_weights<<<(unsigned)std::min<int64_t>(a.nu + b.nu, 0x7FFFFFFF), 64, 0, st>>>(a, b,
+                                                                                    scale, g);
+      FPGB_CUDA_TRY(cudaGetLastError());
+      return FPGB_OK;
+   };
+   // the outputs of an axis part by part: one but for very long axes
+   const AxisMap none{};
+   auto next = [](AxisMap &A) {
+      A.u0 += A.nu;
+      A.nu = std::min(A.nu, A.size - A.u0);
+      return A.nu > 0;
+   };
+   FPGB_TRY(weights(ax, ay));
    const int64_t C = Y * n_rho;
-   const dim3 grid((unsigned)((C + 127) / 128),
-                   (unsigned)std::min<int64_t>((SX + kRows - 1) / kRows, 65535));
-   map_axis0<<<grid, 128, 0, st>>>(d_image, tmp, C, ax);
-   FPGB_CUDA_TRY(cudaGetLastError());
-   map_axis1<<<grid_for(SX * SY * n_rho, 128), 128, 0, st>>>(tmp, d_out, SX, n_rho, ay, ax.block);
-   FPGB_CUDA_TRY(cudaGetLastError());
+   const int wide = (int)std::min<int64_t>(C, 128);
+   for (;;) {
+      const dim3 block(wide, 128 / wide);
+      const int64_t groups = (ax.nu + kRows * block.y - 1) / (kRows * block.y);
+      const dim3 grid((unsigned)((C + wide - 1) / wide),
+                      (unsigned)std::min<int64_t>(groups, 65535));
+      map_axis0<<<grid, block, 0, st>>>(d_image, tmp, C, ax);
+      FPGB_CUDA_TRY(cudaGetLastError());
+      if (!next(ax))
+         break;
+      FPGB_TRY(weights(ax, none));
+   }
+   for (;;) {
+      map_axis1<<<grid_for(SX * ay.nu * n_rho, 128), 128, 0, st>>>(tmp, d_out, SX, n_rho, ay,
+                                                                   ax.block);
+      FPGB_CUDA_TRY(cudaGetLastError());
+      if (!next(ay))
+         break;
+      FPGB_TRY(weights(none, ay));
+   }
    return FPGB_OK;
 }
 
