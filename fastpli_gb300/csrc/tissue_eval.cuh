@@ -152,9 +152,26 @@ FPGB_HD void exact_dist(const SegDev &S, const double pt[3],
 //
 // The pairs are kept unnormalised where the next operation does not need
 // them normalised: products contribute their rounding error (one fused
-// multiply-add) to a single low word, whose own rounding is a few units of
-// 2^-48 of the terms' magnitudes — the form every bound here is stated in
-// (2^-41 and 2^-42 of them, at least 2^3 units of slack).
+// multiply-add) to a single low word.  The bounds count roundings at their
+// worst, in units of u^2 = 2^-48 of the terms' magnitudes; wm and vm are the
+// 1-norms of point - p and of v, b the parameter, d the offset, m = wm + vm b + 1.
+//   ff_dot3    the low word holds three product and two sum errors and the cross
+//              terms, five u |a| |b| in all (|a| |b| the sum of the products'
+//              sizes): 32 for its ten roundings, 11 for the terms left out and
+//              for a sum that cancels (none in |d|^2)
+//   w . v      45 |w| |v| with the rounding of the inputs, and 5 vm from the low
+//              part of p - base, which is not relative to |w|: branch_bound
+//              has 64 and 8
+//   b          that over v.v, and 25 b of the quotient
+//   d          14 |v| b + 4 |w| + 4 across the segment (the products, three sums
+//              and the inputs' low parts); along it |v| times b's error; 49 m
+//              with both
+//   |d|^2      an error of d along the segment counts squared only: 2 * 14 m |d| +
+//              32 |d|^2 <= 60 m |d|
+//   unit       49 m / |d| of d, and 37: half of |d|^2's 32, 16 of the Newton step
+//              and its product, 5 of the components' products
+// and the reference's double arithmetic, 2^-50.5 pscale in d, 2^-48.5 pscale |d|
+// in |d|^2.
 struct FastCand {
    float dist_squ, r_sqr;
    ff d[3];  // closest - point
@@ -173,6 +190,17 @@ FPGB_HD float rsqrt_est(float x) {
 #endif
 }
 
+FPGB_HD float branch_bound(float wm, float vm) {
+   return 0x1p-42f * ((wm + 0.125f) * vm + 1.f); // 64, 8
+}
+FPGB_HD float dist_bound(const FastCand &c, float pscale) {
+   return 0x1.ep-43f * c.m * (c.dn + 0x1p-20f * c.m) + // 60
+          0x1.8p-50f * pscale * (2.f * c.dn + 1.f);
+}
+FPGB_HD float unit_bound(const FastCand &c, float pscale) {
+   return (0x1.ap-43f * c.m + 0x1.2p-50f * pscale) * (1.001f * c.y0) + 0x1.4p-43f; // 52, 40
+}
+
 // closest - point of the candidate (generator.cpp:475-494) with its squared
 // length, and r^2 where it needs no rounding decision (rsq0, rsq1, rsq_const;
 // NaN: interior of a segment whose radius changes, b holds the parameter).
@@ -189,7 +217,7 @@ FPGB_HD bool fast_offset(const SegDev &S, const float pt[3], FastCand &c, ff &b)
       vm += fabsf(S.vf[i]);
    }
    const ff c1 = ff_dot3(w, v);
-   const float ec = 0x1p-42f * (wm * vm + 1.f);
+   const float ec = branch_bound(wm, vm);
    const float dq = (c1.hi - S.c2f) + (c1.lo - S.c2_lo);
    b = ff{0.f, 0.f};
    if (c1.hi < -ec) { // c1 < 0: closest = s0, t = 0 (generator.cpp:483-484)
@@ -228,15 +256,14 @@ FPGB_HD bool fast_candidate(const SegDev &S, const float pt[3], FastCand &c) {
    if (!(c.r_sqr == c.r_sqr)) { // r = r0 (1 - t) + r1 t  (fiber.cpp:115-120)
       const ff R = ff_add(ff{S.r0_hi, S.r0_lo}, ff_mul(ff{S.dr_hi, S.dr_lo}, b));
       const ff R2 = ff_sqr(R);
-      // b's error is that of c1: 2^-42 (|w| |v| + 1) / c2
+      // b's error, at most 25 u^2 b + (45 |w| |v| + 5 vm) u^2 / c2, is below a
+      // quarter of 2^-40 eb
       const float eb = c.m * c.m * S.c2_rcp + b.hi + 1.f;
       const float er = 0x1p-40f * (R2.hi + fabsf(R.hi) * fabsf(S.dr_hi) * eb);
       if (!ff_round_unique(R2, er, c.r_sqr))
          return false;
    }
-   const float ed = 0x1p-43f * c.m * (c.dn + 0x1p-20f * c.m) +
-                    0x1p-49f * S.pscale * (2.f * c.dn + 1.f);
-   return ff_round_unique(c.D, ed, c.dist_squ);
+   return ff_round_unique(c.D, dist_bound(c, S.pscale), c.dist_squ);
 }
 
 // float(unit(point - closest)) of the 'r' layer (generator.cpp:370-371)
@@ -247,7 +274,7 @@ FPGB_HD bool fast_radial(const SegDev &S, const FastCand &c, float out[3]) {
    const ff t = two_prod(c.y0, c.y0);
    const float e = fmaf(-c.D.lo, t.hi, fmaf(-c.D.hi, t.lo, fmaf(-c.D.hi, t.hi, 1.f)));
    const ff inv = quick_two_sum(c.y0, c.y0 * fmaf(0.375f * e, e, 0.5f * e));
-   const float ex = (0x1p-43f * c.m + 0x1p-49f * S.pscale) * (1.001f * c.y0) + 0x1p-44f;
+   const float ex = unit_bound(c, S.pscale);
 #pragma unroll
    for (int i = 0; i < 3; i++) { // nv = -d
       const ff p = two_prod(-c.d[i].hi, inv.hi);
