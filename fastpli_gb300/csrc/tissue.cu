@@ -249,17 +249,6 @@ Box fiber_box(const double *xyz, const double *r, int64_t n) {
 // 29.6 and 22.7 ms).
 constexpr size_t kTogetherBytes = size_t(256) << 10;
 
-bool long_segment(const double *p, const double *q) {
-   double c2 = 0.0;
-   bool far = false;
-   for (int i = 0; i < 3; i++) {
-      const double v = q[i] - p[i];
-      c2 = c2 + v * v;
-      far = far || std::fabs(p[i]) > 0x1p29 || std::fabs(q[i]) > 0x1p29;
-   }
-   return (float)c2 > kLongSquared || far;
-}
-
 int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan, bool fill) {
    if (!vol || !fb) {
       set_error("generate_tissue: null volume or fibers");
@@ -449,18 +438,25 @@ int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,
          continue;
       int64_t n = 0;
       SegDev S;
+      double longest = 0.0; // squared
       for (int64_t s = p0; s + 1 < p1; s++) {
-         const int64_t count =
-             segment_box(&xyz[3 * s], &xyz[3 * (s + 1)], rad[s], rad[s + 1],
-                         plan->layers[b].sqrt_last, vol->dim, S.lo, S.ext);
+         const double *P = &xyz[3 * s], *Q = P + 3;
+         const int64_t count = segment_box(P, Q, rad[s], rad[s + 1], plan->layers[b].sqrt_last,
+                                           vol->dim, S.lo, S.ext);
          kept[s] = count > 0;
          if (count == 0)
             continue;
          n++;
          cand += count;
          pairs += segment_brick_pairs(S);
-         longer = longer || long_segment(&xyz[3 * s], &xyz[3 * (s + 1)]);
+         const double c2 = (Q[0] - P[0]) * (Q[0] - P[0]) + (Q[1] - P[1]) * (Q[1] - P[1]) +
+                           (Q[2] - P[2]) * (Q[2] - P[2]);
+         longest = c2 > longest ? c2 : longest;
       }
+      // (the fiber's box has its points: no coordinate is past it)
+      for (int i = 0; i < 3; i++)
+         longer = longer || !(fbox[fi].mn[i] > -0x1p29 && fbox[fi].mx[i] < 0x1p29);
+      longer = longer || (float)longest > kLongSquared;
       fiber_segs[fi + 1] = n;
    }
    for (int64_t fi = 0; fi < nf; fi++) {

@@ -111,7 +111,7 @@ struct TissuePlan {
    int64_t candidates = 0;   // sum of clipped box volumes
    int64_t brick_pairs = 0;  // (segment, brick) pairs of the brick voxelizer
    int64_t n_segs = 0;
-   bool long_segs = false; // some segment is long_segment
+   bool long_segs = false; // some segment is longer than 64 voxels or far away
    // the segment table; or, unfilled, what the device fills it from: n_points x
    // (x, y, z) in voxels, n_points radii, n_segs SegSrc
    RawArray<SegDev> segs;
@@ -122,10 +122,9 @@ struct TissuePlan {
    std::vector<double> props; // (dn, mu) rows
 };
 
-// Longer than 64 voxels, or 2^29 voxels away: what the sweep takes part by part
-// or without a bound.
+// Segments longer than 64 voxels (and those 2^30 voxels away, which have no
+// bound) are swept by voxel_bricks<., true>.
 constexpr float kLongSquared = 64.f * 64.f;
-bool long_segment(const double *p, const double *q);
 
 // fill = false leaves a large segment table to the device (run_tissue).
 int plan_tissue(const fpgb_volume *vol, const fpgb_fibers *fb, TissuePlan *plan,

@@ -66,7 +66,7 @@ struct BrickChunks {
 // are the tile's output arrays (vecs[t] may be null: labels only).
 // seg_tile may be null when there is one tile.  `ws` holds
 // ws_bytes >= brick_workspace_bytes(n_bricks, n_pairs, n_segs), 256-byte aligned.
-// long_segs: some segment is a long_segment.
+// long_segs: TissuePlan's.
 // `chunks` may be null: one launch over every brick.
 int launch_voxel_bricks(const SegDev *segs, const int32_t *seg_tile, int64_t n_segs,
                         const TileDev *tiles, int64_t n_tiles, int64_t n_bricks, int64_t n_pairs,
