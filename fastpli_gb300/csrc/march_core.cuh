@@ -89,9 +89,9 @@ __device__ __forceinline__ float acos_sq(float x) {
 // accurate as th -> 0.  Larger angles use acosf and the hardware sine.  The
 // reference's flip of u (when v.u < 0) is carried as the sign of u's weight.
 //
-// Out of line, as are the rare wide angles within, and the zero cases are
-// weights, not branches of their own: seven copies of this body in a marching
-// kernel, which the warps run through out of step, do not fit the instruction
+// The rare wide angles are out of line, and the zero cases weights, not branches
+// of their own: a marching kernel has seven copies of this body, which the warps
+// run through out of step, and the whole of them does not fit the instruction
 // cache.
 static __device__ __noinline__ float2 slerp_weights_wide(float c, float t) {
    // th in [0.6, pi/2]: the hardware sine is accurate to ~5e-7 here
@@ -694,7 +694,7 @@ __device__ __forceinline__ void march_one_ray_column(const MarchParams &P, int64
 // every step.  Here each warp takes its 32 rays through kCoopSteps steps at a
 // time in three phases:
 //   1. every lane loads its steps' labels (all in flight together), adds up
-//      their attenuation and lists its birefringent steps, packed by ballot;
+//      their attenuation and lists its birefringent steps;
 //   2. the warp's jobs are shared out to all 32 lanes, each job producing that
 //      step's rotation (cos 2phi, sin 2phi, cos/sin ret) from the interpolated
 //      axis, which depends only on the step's position, not on the state;
@@ -705,11 +705,15 @@ __device__ __forceinline__ void march_one_ray_column(const MarchParams &P, int64
 // is added up again without it.
 // Bound by instruction issue (56% of the slots) and the latency of the 8-corner
 // gathers: about 250 issue slots per ray and step on the crossing volume, 670
-// per job.  Against windows of 4 steps with the corners worked out in phase 1
-// (a warp pays for it when one lane has a job), a shuffle scan and every step
-// applied in turn: crossing, one tilt 478 -> 430 us, Lerp tile 146 -> 106 us;
-// with windows of 4 steps 5% slower, of 16 (half the L1 gone to scratch) 30%.
-// The loops below stay rolled: unrolled, the kernel outgrows the instruction
+// per job.  The list has a ray's jobs together (a shuffle scan): its steps are
+// neighbours along z, so the lanes of phase 2 read a few columns' lines instead
+// of 32 (listed step by step, by ballots: 256 x 256 x 60 all birefringent, Lerp
+// 248 against 141 us, L1 hits 84 and 92%; crossing, five tilts 1,610 and 1,594).
+// Against windows of 4 steps with the corners worked out in phase 1 (a warp pays
+// for it when one lane has a job) and every step applied in turn: crossing, one
+// tilt 478 -> 430 us, Lerp tile 146 -> 106 us; with windows of 4 steps 5%
+// slower, of 16 (half the L1 gone to scratch) 30%.
+// The loops over jobs stay rolled: unrolled, the kernel outgrows the instruction
 // cache (119 KB: 660 us).
 // ----------------------------------------------------------------------------
 constexpr int kCoopSteps = 8;
@@ -717,13 +721,14 @@ constexpr int kCoopSlots = kCoopSteps * 32; // per warp
 constexpr float kNoRotation = 2.f;          // in the place of cos 2phi
 
 struct CoopScratch {
-   float f[4][kCoopSlots]; // cos 2phi, sin 2phi, cos ret, sin ret; slot = step * 32 + lane
+   // of a job, at step * 32 + ray: cos 2phi (until it is done the label), sin 2phi,
+   // cos ret, sin ret
+   float f[4][kCoopSlots];
    int64_t px[32], py[32]; // the rays' positions at the window's first step
-   int lab[kCoopSlots];    // of a job
    unsigned flags[32];     // per ray: bit j: the axis of step j is zero; bit 31: not normalised
-   unsigned char list[kCoopSlots]; // slots of the jobs
+   unsigned char list[kCoopSlots]; // the jobs' places, a ray's together
 };
-static_assert(kCoopSlots <= 256 && kCoopSteps < 31, "slots are bytes, steps flag bits");
+static_assert(kCoopSlots <= 256 && kCoopSteps < 31, "places are bytes, steps flag bits");
 
 // Label optics in shared memory (labels below kLutCache).
 constexpr int kLutCache = 64;
@@ -763,7 +768,8 @@ __device__ __forceinline__ void coop_job(const MarchParams &P, const CoopLut &lu
                                          const int32_t *__restrict__ label,
                                          const float *__restrict__ vec, CoopScratch &S, int k0,
                                          int t) {
-   const int slot = S.list[t], lab = S.lab[t], ray = slot & 31, j = slot >> 5;
+   const int at = S.list[t], ray = at & 31, j = at >> 5;
+   const int lab = __float_as_int(S.f[0][at]);
    int64_t px = S.px[ray], py = S.py[ray];
    if (TILT) {
       px += j * P.dx_fx;
@@ -786,10 +792,10 @@ __device__ __forceinline__ void coop_job(const MarchParams &P, const CoopLut &lu
       if (!retard_params(v, n2, kret, c, s, cr, sr))
          c = kNoRotation;
    }
-   S.f[0][slot] = c;
-   S.f[1][slot] = s;
-   S.f[2][slot] = cr;
-   S.f[3][slot] = sr;
+   S.f[0][at] = c;
+   S.f[1][at] = s;
+   S.f[2][at] = cr;
+   S.f[3][at] = sr;
 }
 
 template <int MODE, bool TILT, bool WIDE>
@@ -826,7 +832,6 @@ __device__ __forceinline__ void march_ray_coop(const MarchParams &P, int64_t ray
          }
       }
       unsigned jobs = 0;
-      int total = 0;
 #pragma unroll
       for (int j = 0; j < kCoopSteps; j++) {
          if ((unsigned)lab[j] >= (unsigned)P.n_props) {
@@ -835,16 +840,21 @@ __device__ __forceinline__ void march_ray_coop(const MarchParams &P, int64_t ray
          }
          const float2 o = step_optics(P, lut, lab[j]);
          L += k0 + j < P.n_z ? o.x : 0.f; // (0 for labels without effect)
-         const bool job = active && __float_as_int(o.y) == 2;
-         const unsigned m = __ballot_sync(0xffffffffu, job);
-         if (job) {
-            const int at = total + __popc(m & ((1u << lane) - 1u));
-            S.list[at] = (unsigned char)(j * 32 + lane);
-            S.lab[at] = lab[j];
+         if (active && __float_as_int(o.y) == 2) {
+            S.f[0][j * 32 + lane] = __int_as_float(lab[j]);
             jobs |= 1u << j;
          }
-         total += __popc(m);
       }
+      int end = __popc(jobs); // of this lane's jobs in the list
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+         const int before = __shfl_up_sync(0xffffffffu, end, o);
+         end += lane >= o ? before : 0;
+      }
+      const int total = __shfl_sync(0xffffffffu, end, 31);
+#pragma unroll 1
+      for (unsigned m = jobs, t = end - __popc(jobs); m; m &= m - 1)
+         S.list[t++] = (unsigned char)((__ffs((int)m) - 1) * 32 + lane);
       __syncwarp();
       // phase 2: the jobs
 #pragma unroll 1
@@ -854,10 +864,10 @@ __device__ __forceinline__ void march_ray_coop(const MarchParams &P, int64_t ray
       // phase 3: this lane's rotations, in order
 #pragma unroll 1
       for (unsigned m = jobs; m; m &= m - 1) {
-         const int slot = (__ffs((int)m) - 1) * 32 + lane;
-         const float c = S.f[0][slot];
+         const int at = (__ffs((int)m) - 1) * 32 + lane;
+         const float c = S.f[0][at];
          if (c != kNoRotation)
-            apply_retard(u1, u2, u3, c, S.f[1][slot], S.f[2][slot], S.f[3][slot]);
+            apply_retard(u1, u2, u3, c, S.f[1][at], S.f[2][at], S.f[3][at]);
       }
       const unsigned flags = jobs ? S.flags[lane] : 0u;
       if (flags) {
@@ -867,17 +877,20 @@ __device__ __forceinline__ void march_ray_coop(const MarchParams &P, int64_t ray
             w_zero = true;
             L = L0;
             int64_t qx = S.px[lane], qy = S.py[lane];
-#pragma unroll 1
-            for (int j = 0; j < kCoopSteps && k0 + j < P.n_z; j++) {
-               int l = step_label<WIDE>(P, label, qx, qy, k0 + j);
-               if ((unsigned)l >= (unsigned)P.n_props)
-                  l = 0;
-               if (!(zero >> j & 1u))
-                  L += step_optics(P, lut, l).x;
+            int again[kCoopSteps]; // (their loads in flight together)
+#pragma unroll
+            for (int j = 0; j < kCoopSteps; j++) {
+               again[j] = k0 + j < P.n_z ? step_label<WIDE>(P, label, qx, qy, k0 + j) : 0;
                if (TILT) {
                   qx += P.dx_fx;
                   qy += P.dy_fx;
                }
+            }
+#pragma unroll
+            for (int j = 0; j < kCoopSteps; j++) {
+               const int l = (unsigned)again[j] < (unsigned)P.n_props ? again[j] : 0;
+               if (k0 + j < P.n_z && !(zero >> j & 1u))
+                  L += step_optics(P, lut, l).x;
             }
          }
          S.flags[lane] = 0;
