@@ -271,9 +271,6 @@ int plan_march(const fpgb_setup *s, const int64_t *dim, const double *props, int
    // with step 1 (simulator.cpp:259-261 then gives z = k + 1/2); at those
    // exact voxel centres Lerp and Slerp reduce to the voxel's own axis
    // (simulator.cpp:518-519)
-   // Lerp / Slerp: the warp-cooperative march (the faster variant on every
-   // volume measured; the batched path's autotuner may pick either)
-   P.coop = P.mode != 0 ? 1 : 0;
    P.column = 0;
    if (theta == 0 && P.n_z == P.Z && step[0] == 0 && step[1] == 0) {
       bool seq = true;
@@ -317,13 +314,16 @@ int plan_march(const fpgb_setup *s, const int64_t *dim, const double *props, int
 // ======================================================================
 // device
 // ======================================================================
+// Lerp and Slerp run the cooperative march (the faster variant on every volume
+// measured; the batched path's autotuner may pick either), NN and vertical
+// columns in any mode the kernels of MODE 0.
 // 7 resident blocks per SM for the per-thread and column kernels (72
 // registers: 3% faster than the 80-register default on config 2; 8 blocks
 // spill too much); the cooperative kernels 5 for Slerp (96 registers, and less
 // of L1 gone to scratch: five tilts of the crossing volume 1,657 us against
 // 1,726 with 6) and 6 for Lerp (a tile 181 us against 233 with 5).
-template <int MODE, bool TILT, bool COOP, bool WIDE>
-__global__ void __launch_bounds__(128, COOP ? (MODE == 2 ? 5 : 6) : 7)
+template <int MODE, bool TILT, bool WIDE>
+__global__ void __launch_bounds__(128, MODE == 2 ? 5 : MODE == 1 ? 6 : 7)
 march_rays(const MarchParams P, int64_t unit0, const int32_t *__restrict__ label,
            const float *__restrict__ vec, double *__restrict__ image,
            double *__restrict__ epa_t, double *__restrict__ epa_d, double *__restrict__ epa_r,
@@ -331,15 +331,15 @@ march_rays(const MarchParams P, int64_t unit0, const int32_t *__restrict__ label
    // launches may cover a range of units, in either order
    const int64_t unit = P.reverse ? unit0 + (int64_t)gridDim.x - 1 - blockIdx.x
                                   : unit0 + (int64_t)blockIdx.x;
-   if (!TILT && P.column) { // 128 consecutive vertical rays per block
+   if (MODE == 0 && !TILT && P.column) { // 128 consecutive vertical rays per block
       const int64_t ray = unit * (int64_t)blockDim.x + threadIdx.x;
       if (ray < P.X * P.Y)
          march_one_ray_column(P, ray, label, vec, image, epa_t, epa_d, epa_r, counters);
       return;
    }
    int64_t ray; // one 4 x 32 tile of rays per block (tile_ray)
-   const bool valid = tile_ray<MODE != 0 && COOP>(P, unit, threadIdx.x, ray);
-   if (MODE == 0 || !COOP) {
+   const bool valid = tile_ray<MODE != 0>(P, unit, threadIdx.x, ray);
+   if constexpr (MODE == 0) {
       if (valid)
          march_one_ray<MODE, TILT, WIDE>(P, ray, label, vec, image, epa_t, epa_d, epa_r,
                                          counters);
@@ -447,28 +447,23 @@ static int launch_march_units(const MarchParams &P, const int32_t *d_label, cons
    // separate kernels per march variant: the cooperative one holds shared
    // scratch and more registers, which must not cap the occupancy of the
    // per-thread one
-#define FPGB_LAUNCH(M, T, C)                                                               \
+#define FPGB_LAUNCH(M, T)                                                                   \
    if (narrow)                                                                              \
-      march_rays<M, T, C, false><<<grid, 128, 0, st>>>(P, u0, d_label, d_vec, d_image, d_t, \
-                                                       d_d, d_r, d_counters);                \
+      march_rays<M, T, false><<<grid, 128, 0, st>>>(P, u0, d_label, d_vec, d_image, d_t,    \
+                                                    d_d, d_r, d_counters);                  \
    else                                                                                     \
-      march_rays<M, T, C, true><<<grid, 128, 0, st>>>(P, u0, d_label, d_vec, d_image, d_t,  \
-                                                      d_d, d_r, d_counters)
-   const bool coop = P.coop != 0;
+      march_rays<M, T, true><<<grid, 128, 0, st>>>(P, u0, d_label, d_vec, d_image, d_t,     \
+                                                   d_d, d_r, d_counters)
    const bool narrow = march_narrow(P);
    // (vertical columns need no interpolation: the kernel with the fewest
    // registers and no scratch; 1024 x 1024 x 240 1,120 -> 940 us)
-   switch (!tilt && P.column ? 0 : P.mode * 4 + (tilt ? 2 : 0) + (coop ? 1 : 0)) {
-   case 0: case 1: FPGB_LAUNCH(0, false, false); break;
-   case 2: case 3: FPGB_LAUNCH(0, true, false); break;
-   case 4: FPGB_LAUNCH(1, false, false); break;
-   case 5: FPGB_LAUNCH(1, false, true); break;
-   case 6: FPGB_LAUNCH(1, true, false); break;
-   case 7: FPGB_LAUNCH(1, true, true); break;
-   case 8: FPGB_LAUNCH(2, false, false); break;
-   case 9: FPGB_LAUNCH(2, false, true); break;
-   case 10: FPGB_LAUNCH(2, true, false); break;
-   default: FPGB_LAUNCH(2, true, true); break;
+   switch (!tilt && P.column ? 0 : P.mode * 2 + (tilt ? 1 : 0)) {
+   case 0: FPGB_LAUNCH(0, false); break;
+   case 1: FPGB_LAUNCH(0, true); break;
+   case 2: FPGB_LAUNCH(1, false); break;
+   case 3: FPGB_LAUNCH(1, true); break;
+   case 4: FPGB_LAUNCH(2, false); break;
+   default: FPGB_LAUNCH(2, true); break;
    }
 #undef FPGB_LAUNCH
    FPGB_CUDA_TRY(cudaGetLastError());

@@ -55,10 +55,7 @@ struct MarchParams {
    int32_t tilted; // x/y advance or the axis rotates
    int32_t column; // vertical ray reading z = 0..Z-1 (or mirrored) in order:
                    // the column path applies (16-byte loads when Z % 4 == 0)
-   // Lerp/Slerp rays that are not vertical columns: 1 = warp-cooperative
-   // march (steps needing interpolation compacted across the warp), 0 = one
-   // thread per ray.  Both give the same bits; the choice is speed only.
-   int32_t coop;
+   int32_t pad_;
    // kinds of labels 0..15, two bits each (kind_packed = 1 when every label
    // fits): the march reads a step's kind without a table load
    uint32_t kind_mask;
