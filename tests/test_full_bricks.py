@@ -62,12 +62,17 @@ def test_full_bricks_match_oracle(cuda, oracle_port, name, dim):
         label, vector, _, w = g.run_generation_device()
         only, _, _, _ = g.run_generation_device(only_label=True)
         hlab, hvec, _ = g.run_generation()
+        # the least workspace: records' space by segments only, or none
+        least = cuda.empty(g.workspace_size(), dtype=cuda.uint8, device="cuda")
+        llab, lvec, _, lw = g.run_generation_device(workspace=least)
     assert np.array_equal(label.cpu().numpy(), olab)
     assert np.array_equal(vector.cpu().numpy().view(np.uint32), ovec.view(np.uint32))
     assert np.array_equal(only.cpu().numpy(), olab)
     assert np.array_equal(hlab, olab) and np.array_equal(hvec.view(np.uint32),
                                                          ovec.view(np.uint32))
-    assert w["overlap"] == owarn["overlap"]
+    assert np.array_equal(llab.cpu().numpy(), olab)
+    assert np.array_equal(lvec.cpu().numpy().view(np.uint32), ovec.view(np.uint32))
+    assert w["overlap"] == lw["overlap"] == owarn["overlap"]
 
 
 @pytest.mark.gpu
