@@ -48,10 +48,9 @@ FPGB_HD void closest_point(const SegDev &S, const double pt[3],
 // v.v, 0, 1) — the closest-point parameter, so no branch: for t = 0 it is
 // |w|^2, for t = 1 |w - v|^2, in between |w|^2 - (w.v)^2 / v.v.  An error in
 // t only raises the value by v.v (dt)^2 (the expression is the squared
-// distance to a point of the segment, minimal at the exact t).  The y and z
-// parts of w.w and w.v are passed in (a = wy vy + wz vz, b = wy^2 + wz^2):
-// the voxelizer's sweep computes them once per (y, z) cell and visits the x
-// of the cell's column, so the per-candidate work is six fused operations.
+// distance to a point of the segment, minimal at the exact t).  This form,
+// with a bound of the candidate's own, is what voxel_marks filters by; the sweep
+// takes the same estimate with the segment's bound (sweep_dist2).
 // The bound covers the rounding of the float inputs, of every FP32 operation
 // (fused multiply-adds: one rounding each, the same on the host and the
 // device) and of the reference's own final rounding; a host build checks it
@@ -98,8 +97,8 @@ FPGB_HD float sweep_dist2(float wx, float a2, float b, float vn2, float c2f, flo
 // voxels that lie within or next to the segment's thickest end (thr): |w| <=
 // |v| + r' for the voxel's offset w from the start.  With u = 2^-24, the
 // rounding of the inputs (w: u (|w0| + |w| + 1) for the offset w0 of the
-// sub-box's first cell, v, c2: u each), of the six operations and of the sum of
-// the margin itself stays below u (15 |w|^2 + 2 |w| |w0| + 12 c2 + 4) (the
+// sub-box's first cell, v, c2: u each), of the operations and of the sum of the
+// margin itself stays below u (15 |w|^2 + 2 |w| |w0| + 12 c2 + 4) (the
 // error of t enters squared: the value is the squared distance to some point
 // of the segment); the reference's own double arithmetic adds 2^-50 pscale |w|
 // and its final rounding u |w|^2.  18 u and 12 u are 1.08e-6 and 7.2e-7.  For a

@@ -7,7 +7,7 @@
 // owns one brick: it keeps the voxels' winner keys and, for multi-bundle
 // volumes, the per-voxel bundle minimum in shared memory, sweeps the brick's
 // segments over them, and finally decodes every voxel's winner into label
-// and orientation, written once to HBM.
+// and orientation, but for the close calls, which voxel_marks resolves.
 #pragma once
 
 #include <cuda_runtime.h>
