@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "fpgb_common.cuh"
@@ -138,6 +139,12 @@ __global__ void axis_weights(AxisMap ax, AxisMap ay, double scale, const GaussTa
 // (100,000 x 1 x 9 with 481 taps: 0.53 ms, 2.61 with the other lanes idle).
 constexpr int kRows = 4;
 
+// The rows of an axis of 2^30 and more (LONG) are counted in 64 bits, which costs
+// 10% at 100 taps.
+template <bool LONG> using RowIndex = std::conditional_t<LONG, int64_t, int>;
+constexpr int64_t kLongAxis = 1 << 30;
+
+template <bool LONG>
 __global__ void __launch_bounds__(128)
 map_axis0(const double *__restrict__ in, double *__restrict__ out, int64_t C, const AxisMap A) {
    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -158,24 +165,21 @@ map_axis0(const double *__restrict__ in, double *__restrict__ out, int64_t C, co
             hi = first[k] + count[k] > hi ? first[k] + count[k] : hi;
          }
       }
-      // (in 32 bits from a base: 64-bit indices cost 10% at 100 taps)
-      for (int64_t base = lo; base < hi; base += 1 << 30) {
-         const int rows = (int)(hi - base < 1 << 30 ? hi - base : 1 << 30);
-         int from[kRows], to[kRows];
+      using I = RowIndex<LONG>;
+      const I rows = hi > lo ? (I)(hi - lo) : I(0);
+      I from[kRows], to[kRows];
 #pragma unroll
-         for (int k = 0; k < kRows; k++) {
-            const int64_t a = first[k] - base, b = a + count[k];
-            from[k] = (int)(a < 0 ? 0 : a < rows ? a : rows);
-            to[k] = (int)(b < 0 ? 0 : b < rows ? b : rows);
-         }
-         const double *w = A.w + (u0 - A.u0) * A.pitch + base, *v = in + base * C + c;
-         for (int i = 0; i < rows; i++) {
-            const double x = v[i * C];
+      for (int k = 0; k < kRows; k++) {
+         from[k] = count[k] ? (I)(first[k] - lo) : I(0);
+         to[k] = from[k] + (I)count[k];
+      }
+      const double *w = A.w + (u0 - A.u0) * A.pitch, *v = in + lo * C + c;
+      for (I i = 0; i < rows; i++) {
+         const double x = v[i * C];
 #pragma unroll
-            for (int k = 0; k < kRows; k++) // (the same for every thread of a group)
-               if (i >= from[k] && i < to[k])
-                  acc[k] = fma(w[k * A.pitch - first[k] + i], x, acc[k]);
-         }
+         for (int k = 0; k < kRows; k++) // (the same for every thread of a group)
+            if (i >= from[k] && i < to[k])
+               acc[k] = fma(w[k * A.pitch + (i - from[k])], x, acc[k]);
       }
 #pragma unroll
       for (int k = 0; k < kRows; k++)
@@ -186,6 +190,7 @@ map_axis0(const double *__restrict__ in, double *__restrict__ out, int64_t C, co
 
 // Axis 1 of [U, n, R] -> [U, size, R], divided by the blocks' pixel counts
 // (an empty block: 0 / 0 = NaN, as numpy's divide).
+template <bool LONG>
 __global__ void __launch_bounds__(128)
 map_axis1(const double *__restrict__ in, double *__restrict__ out, int64_t U, int64_t R,
           const AxisMap A, const int64_t *__restrict__ block0) {
@@ -197,18 +202,14 @@ map_axis1(const double *__restrict__ in, double *__restrict__ out, int64_t U, in
       const double *row = in + (u * A.n + A.first[v]) * R + r;
       const double *w = A.w + local * A.pitch;
       double even = 0.0, odd = 0.0;
-      const int64_t all = A.count[v];
-      const int n = (int)(all < 1 << 30 ? all : 1 << 30); // (32-bit steps; the rest below)
-      int t = 0;
+      const RowIndex<LONG> n = (RowIndex<LONG>)A.count[v];
+      RowIndex<LONG> t = 0;
       for (; t + 1 < n; t += 2) {
          even = fma(w[t], row[t * R], even);
          odd = fma(w[t + 1], row[(t + 1) * R], odd);
       }
       if (t < n)
          even = fma(w[t], row[t * R], even);
-#pragma unroll 1
-      for (int64_t i = n; i < all; i++)
-         even = fma(w[i], row[i * R], even);
       out[(u * A.size + v) * R + r] = (even + odd) / (double)(block0[u] * A.block[v]);
    }
 }
@@ -485,15 +486,17 @@ int fpgb_optic_filter_resample_device(const double *d_image, int64_t X, int64_t 
       const int64_t groups = (ax.nu + kRows * block.y - 1) / (kRows * block.y);
       const dim3 grid((unsigned)((C + wide - 1) / wide),
                       (unsigned)std::min<int64_t>(groups, 65535));
-      map_axis0<<<grid, block, 0, st>>>(d_image, tmp, C, ax);
+      auto kernel = X < kLongAxis ? map_axis0<false> : map_axis0<true>;
+      kernel<<<grid, block, 0, st>>>(d_image, tmp, C, ax);
       FPGB_CUDA_TRY(cudaGetLastError());
       if (!next(ax))
          break;
       FPGB_TRY(weights(ax, none));
    }
    for (;;) {
-      map_axis1<<<grid_for(SX * ay.nu * n_rho, 128), 128, 0, st>>>(tmp, d_out, SX, n_rho, ay,
-                                                                   ax.block);
+      auto kernel = Y < kLongAxis ? map_axis1<false> : map_axis1<true>;
+      kernel<<<grid_for(SX * ay.nu * n_rho, 128), 128, 0, st>>>(tmp, d_out, SX, n_rho, ay,
+                                                                ax.block);
       FPGB_CUDA_TRY(cudaGetLastError());
       if (!next(ay))
          break;
