@@ -130,9 +130,9 @@ __global__ void axis_weights(AxisMap ax, AxisMap ay, double scale, const GaussTa
 
 // Axis 0 of [n, C] -> [size, C]: a thread takes one column and kRows outputs,
 // whose windows overlap: each input row is loaded once for all of them.  Bound
-// by FP64 fused multiply-adds (pipe 83% busy): 512 x 512 x 9 at sigma 0.71,
+// by FP64 fused multiply-adds (pipe 86% busy): 512 x 512 x 9 at sigma 0.71,
 // scale 0.2 / 1.33 takes 16 M of them (39 + 6.6 taps, 77 of 512 rows) and
-// 52 us, with the weights 9 and axis 1 15 us; filtering every pixel along both
+// 49 us, with the weights 10 and axis 1 15 us; filtering every pixel along both
 // axes (142 M products, reflected index per tap) and then summing the blocks
 // took 273 + 273 + 18 us.
 // Images of fewer than 128 columns share a CTA among groups of outputs

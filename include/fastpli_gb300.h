@@ -239,9 +239,9 @@ int fpgb_epa_device(const double *d_image, int64_t n_pix, int64_t n_rho, double 
  * _ROFL_with_jacobi.py, as Simpli.apply_rofl applies it per pixel,
  * __simpli.py:623-705) of a 5-tilt series d_data [5, n_pix, n_rot] (tilts
  * (0,0), (tau,0), (tau,90), (tau,180), (tau,270) degrees; 4 <= n_rot <= 32),
- * FP64, 16, 4 or 1 lanes per pixel by the number of
- * (unmasked) pixels and n_rot; d_mask != NULL takes 8 n_pix bytes of scratch.  d_out [n_pix, 8] receives direction,
- * inclination, t_rel, their standard deviations, chi^2 and MINPACK's
+ * FP64, 16, 4 or 1 lanes per pixel by the number of unmasked pixels and n_rot;
+ * d_mask != NULL takes 8 n_pix bytes of scratch.  d_out [n_pix, 8] receives
+ * direction, inclination, t_rel, their standard deviations, chi^2 and MINPACK's
  * evaluation count (the reference's niter).  The fit is MINPACK's
  * Levenberg-Marquardt as scipy.optimize.leastsq runs it for the reference
  * (_ROFL_with_jacobi.py:472-486): forward differences, or with grad_mode
