@@ -20,7 +20,7 @@ LY3 = [(0.333, -0.004, 10.0, "p"), (0.666, 0.0, 5.0, "b"), (1.0, 0.004, 1.0, "r"
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def program(tmp_path_factory):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not available")
@@ -31,33 +31,33 @@ def checker(tmp_path_factory):
     return exe
 
 
-def replay(checker, *args):
-    r = subprocess.run([checker, *map(str, args)], capture_output=True, text=True)
+def replay(program, *args):
+    r = subprocess.run([program, *map(str, args)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     words = [w for w in r.stdout.split() if not w.startswith("(")]
     return dict(zip(words[::2], words[1::2]))
 
 
 @pytest.mark.parametrize("length", LENGTHS)
-def test_unmarked_voxels_are_certain(checker, length):
-    replay(checker, 9, 96, 80, 64, 3, 12, 2, 0, length)
+def test_unmarked_voxels_are_certain(program, length):
+    replay(program, 9, 96, 80, 64, 3, 12, 2, 0, length)
 
 
 @pytest.mark.parametrize("radius,points,taper", [(1e20, 3, 0), (4, 9, 0), (4, 9, 0.5)])
-def test_unmarked_voxels_are_certain_at_other_radii(checker, radius, points, taper):
-    replay(checker, 5, 61, 43, 50, radius, 14, points, taper, 0)
+def test_unmarked_voxels_are_certain_at_other_radii(program, radius, points, taper):
+    replay(program, 5, 61, 43, 50, radius, 14, points, taper, 0)
 
 
 @pytest.mark.parametrize("args", [
     (1, 256, 128, 64, 5, 100, 2, 0, 0), (1, 512, 128, 64, 5, 100, 2, 0, 0),
     (1, 1024, 64, 64, 5, 50, 2, 0, 0), (1, 1024, 64, 64, 1.5, 500, 2, 0, 0),
     (1, 96, 80, 64, 3, 60, 2, 0, 66), (1, 96, 80, 64, 3, 60, 2, 0, 1e5)])
-def test_few_close_calls_whatever_the_length(checker, args):
+def test_few_close_calls_whatever_the_length(program, args):
     """A margin of at most 1.1e-6 (2 * 40)^2 = 0.007 either side of the layers
     at r^2 and 0.56 r^2: 4 * 0.007 / r^2 of a fiber's voxels, and as many where
     two fibers meet."""
     bound = 0.015 if args[4] > 2 else 0.03
-    out = replay(checker, *args)
+    out = replay(program, *args)
     assert float(out["marked"]) <= bound * float(out["inside"]) and out["over"] == "0", out
 
 

@@ -13,7 +13,7 @@ SRC = os.path.join(ROOT, "tests", "native", "voxel_bound_check.cu")
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def program(tmp_path_factory):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not available")
@@ -25,6 +25,6 @@ def checker(tmp_path_factory):
 
 
 @pytest.mark.parametrize("length", ["1e-3", "1", "10", "1e3", "1e5"])
-def test_errors_stay_well_inside_the_bounds(checker, length):
-    r = subprocess.run([checker, "3", length, "400000", "0.25"], capture_output=True, text=True)
+def test_errors_stay_well_inside_the_bounds(program, length):
+    r = subprocess.run([program, "3", length, "400000", "0.25"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
